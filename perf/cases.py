@@ -311,9 +311,9 @@ def work(case):
         pre = 2 * _fft_flops(H, W) + 16 * n
         if kind == "dense_precondition":
             return dict(bytes=16 * n * S, flops=pre * S)
-        # about 100 Arnoldi steps of restart 24: the preconditioned vector and the
+        # about 72 Arnoldi steps of restart 24: the preconditioned vector and the
         # operator in and out, the basis (12 vectors on average) read twice
-        steps = 100
+        steps = 72
         return dict(bytes=steps * n * S * 8 * (4 + 24), flops=steps * S * (pre + n * (120 + 16 * 24)))
     n = case["nz"] * case["nx"]
     if kind == "learned_setup":
@@ -325,7 +325,7 @@ def work(case):
         it = 120 * case["angles"]
         return dict(bytes=it * n * 88, flops=it * (4 * _fft_flops(case["nz"], case["nx"]) + n * 150))
     if kind == "record":
-        it = (85 if case["learned"] else 270) * case["bins"] * case["angles"]
+        it = (50 if case["learned"] else 160) * case["bins"] * case["angles"]
         return dict(bytes=it * n * 88, flops=it * (4 * _fft_flops(case["nz"], case["nx"]) + n * 150))
     S = case["systems"]
     if kind == "apply":
