@@ -158,6 +158,93 @@ __device__ __forceinline__ typename CxT<T>::type stencil(const Geo& g, const Sys
   return y;
 }
 
+// The same stencil from separable PML factors: every stretch ratio
+// sz(i) / sx(j +- 1/2) or sx(j) / sz(i +- 1/2) is a product of a factor of the
+// row and one of the column, so a thread that walks down a column divides once
+// per column and row and not four times per node.  Off the PML every factor is
+// one and the fluxes are real.
+// The factors are formed in double and rounded once to T.
+template <typename T>
+struct ColFactors {
+  typename CxT<T>::type s, inv_e, inv_w;   // sx(j), 1/sx(j + 1/2), 1/sx(j - 1/2)
+  bool plain;                              // all three equal one
+};
+template <typename T>
+struct RowFactors {
+  typename CxT<T>::type s, inv_s, inv_n;   // sz(i), 1/sz(i + 1/2), 1/sz(i - 1/2)
+  bool plain;
+};
+__device__ __forceinline__ double2 inv_stretch(double y) {   // 1 / (1 + i y)
+  const double d = 1.0 / (1.0 + y * y);
+  return make_double2(d, -y * d);
+}
+template <typename T>
+__device__ __forceinline__ ColFactors<T> col_factors(const Geo& g, const SysScalars& s, int j) {
+  typedef typename CxT<T>::type C;
+  ColFactors<T> c;
+  c.plain = j > g.n_pml && j < g.nx - 1 - g.n_pml;
+  c.s = c.inv_e = c.inv_w = cx<C>(T(1), T(0));
+  if (!c.plain) {
+    c.s.y = (T)(s.sig * pml_profile<double>((double)j, g.nx, g.n_pml));
+    const double2 e = inv_stretch(s.sig * pml_profile<double>(j + 0.5, g.nx, g.n_pml));
+    const double2 w = inv_stretch(s.sig * pml_profile<double>(j - 0.5, g.nx, g.n_pml));
+    c.inv_e = cx<C>((T)e.x, (T)e.y);
+    c.inv_w = cx<C>((T)w.x, (T)w.y);
+  }
+  return c;
+}
+template <typename T>
+__device__ __forceinline__ RowFactors<T> row_factors(const Geo& g, const SysScalars& s, int i) {
+  typedef typename CxT<T>::type C;
+  RowFactors<T> r;
+  r.plain = i > g.n_pml && i < g.nz - 1 - g.n_pml;
+  r.s = r.inv_s = r.inv_n = cx<C>(T(1), T(0));
+  if (!r.plain) {
+    r.s.y = (T)(s.sig * pml_profile<double>((double)i, g.nz, g.n_pml));
+    const double2 so = inv_stretch(s.sig * pml_profile<double>(i + 0.5, g.nz, g.n_pml));
+    const double2 no = inv_stretch(s.sig * pml_profile<double>(i - 0.5, g.nz, g.n_pml));
+    r.inv_s = cx<C>((T)so.x, (T)so.y);
+    r.inv_n = cx<C>((T)no.x, (T)no.y);
+  }
+  return r;
+}
+template <typename T, bool ADJ>
+__device__ __forceinline__ typename CxT<T>::type stencil_sep(T kh2, T fpow, const RowFactors<T>& rf,
+                                                             const ColFactors<T>& cf, T a_c, T a_e, T a_w, T a_s,
+                                                             T a_n, T b_c, T t_c, typename CxT<T>::type pc,
+                                                             typename CxT<T>::type pe, typename CxT<T>::type pw,
+                                                             typename CxT<T>::type ps, typename CxT<T>::type pn) {
+  typedef typename CxT<T>::type C;
+  const T e = t_c * fpow, mb = kh2 * b_c;
+  C mass = cx<C>(mb * (T(1) - e * e), (ADJ ? T(-2) : T(2)) * mb * e);
+  const T he = T(0.5) * (a_c + a_e), hw = T(0.5) * (a_c + a_w), hs = T(0.5) * (a_c + a_s), hn = T(0.5) * (a_c + a_n);
+  C y;
+  if (rf.plain && cf.plain) {
+    y = mass * pc;
+    y = y + he * (pe - pc);
+    y = y + hw * (pw - pc);
+    y = y + hs * (ps - pc);
+    y = y + hn * (pn - pc);
+    return y;
+  }
+  C fe = he * (rf.s * cf.inv_e), fw = hw * (rf.s * cf.inv_w);
+  C fs = hs * (cf.s * rf.inv_s), fn = hn * (cf.s * rf.inv_n);
+  const C sxz = cf.s * rf.s;
+  mass = mass * (ADJ ? conjc(sxz) : sxz);
+  if (ADJ) { fe = conjc(fe); fw = conjc(fw); fs = conjc(fs); fn = conjc(fn); }
+  y = mass * pc;
+  y = y + fe * (pe - pc);
+  y = y + fw * (pw - pc);
+  y = y + fs * (ps - pc);
+  y = y + fn * (pn - pc);
+  return y;
+}
+
+// Coefficients of the dense path's 8th-order staggered derivative.
+__host__ __device__ constexpr double nsr_dense_stencil(int k) {
+  return k == 0 ? 1225.0 / 1024.0 : k == 1 ? -245.0 / 3072.0 : k == 2 ? 49.0 / 5120.0 : -5.0 / 7168.0;
+}
+
 // Plane-wave source line value at column j (SI line amplitude, no 1/h^2):
 // taper(x) exp(-i k0 x sin(theta)), nsrno/wave_operator.py:114-115.
 __device__ __forceinline__ double2 source_line(const Geo& g, double k0, double sin_theta, int j) {

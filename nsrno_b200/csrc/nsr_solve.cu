@@ -31,7 +31,8 @@
 #include <type_traits>
 #include <string.h>
 
-enum { MODE_EMPTY = 0, MODE_INIT = 1, MODE_ITER_A = 2, MODE_ITER_B = 3, MODE_RES = 4, MODE_EMIT = 5 };
+// MODE_FINISH lives only between finalize and finish_block, inside one CTA.
+enum { MODE_EMPTY = 0, MODE_INIT = 1, MODE_ITER_A = 2, MODE_ITER_B = 3, MODE_RES = 4, MODE_EMIT = 5, MODE_FINISH = 6 };
 
 #define NSR_LAUNCHES_PER_IT 9
 #define NSR_MAX_GROUPS 4        // slot groups on parallel graph branches
@@ -82,7 +83,6 @@ struct SolveArgs {
   int n_systems;
   int rows;      // rows per fwd CTA
   int tc;        // columns per cols CTA
-  int tz;        // band rows per inv CTA
   int nb_inv;    // inv CTAs per slot
   double tol2;
   double shift;
@@ -384,27 +384,41 @@ __device__ void pop_next(const SolveArgs& A, SlotState& S) {
   }
 }
 
+// Marks a system as finished with its outputs.  The receiver values are
+// gathered afterwards by the whole block (finish_block), so a finish costs one
+// round of loads and not one per receiver in a single thread.
 __device__ void finish_system(const SolveArgs& A, SlotState& S, int reason, double rel) {
-  const long long n = (long long)A.g.nz * A.g.nx;
-  const int slot = (int)(&S - A.B.slots);
-  const double2* x = A.B.x + (2LL * slot + S.xpar) * n;
-  for (int k = 0; k < A.n_rx; ++k) {
-    const int idx = A.rx[k];
-    const bool ok = idx >= 0 && (long long)idx < n;   // out-of-range receivers read as NaN
-    A.iq[(long long)S.sys * A.n_rx + k] = !ok ? make_double2(NAN, NAN)
-                                         : (S.zero_rhs ? make_double2(0.0, 0.0) : __ldcg(&x[idx]));
-  }
   A.residual[S.sys] = rel;
   A.iterations[S.sys] = S.iters;
   A.status[S.sys] = reason;
-  if (A.fields) {
-    // counted as done once the emit pass has written its field
-    S.mode = MODE_EMIT;
-    return;
+  S.mode = MODE_FINISH;
+}
+
+// Second part of a finish, run by `nt` threads of the slot's last CTA (thread
+// index t) after finalize: receiver values, then thread 0 hands the slot on.
+// `sync` is a barrier over those threads.
+template <typename SYNC>
+__device__ __forceinline__ void finish_block(const SolveArgs& A, SlotState& S, int t, int nt, SYNC sync) {
+  const long long n = (long long)A.g.nz * A.g.nx;
+  const int slot = (int)(&S - A.B.slots);
+  const double2* x = A.B.x + (2LL * slot + S.xpar) * n;
+  const bool zero = S.zero_rhs != 0;
+  double2* iq = A.iq + (long long)S.sys * A.n_rx;
+  for (int k = t; k < A.n_rx; k += nt) {
+    const int idx = A.rx[k];
+    const bool ok = idx >= 0 && (long long)idx < n;   // out-of-range receivers read as NaN
+    iq[k] = !ok ? make_double2(NAN, NAN) : (zero ? make_double2(0.0, 0.0) : __ldcg(&x[idx]));
   }
-  __threadfence();
-  atomicAdd(A.B.done, 1);
-  pop_next(A, S);
+  sync();
+  if (t == 0) {
+    if (A.fields) {
+      S.mode = MODE_EMIT;   // counted as done once the emit pass has written its field
+    } else {
+      __threadfence();
+      atomicAdd(A.B.done, 1);
+      pop_next(A, S);
+    }
+  }
 }
 
 // Scalar recurrence of one slot, run by thread 0 of the slot's last CTA.
@@ -574,11 +588,40 @@ __device__ void finalize(const SolveArgs& A, SlotState& S, int mode, const doubl
 // ---------------------------------------------------------------------------
 // Per-CTA partials, arrival, and the last CTA's finalize (no waiting).
 // ---------------------------------------------------------------------------
+// Deterministic sum of `count` rows of NSR_NPART partials into tot, by `nt`
+// threads (a multiple of 32): thread (c, q) adds a contiguous run of rows of
+// column q into run[c][q] (nt doubles of shared memory), then column q's runs
+// are added in order.  One thread per column
+// over every row (the earlier form) was a chain of `count` dependent
+// L2 reads: about 50 us at 768 rows.
+template <typename SYNC>
+__device__ __forceinline__ void sum_partials(const double* part, int count, int t, int nt, double* run, double* tot,
+                                             SYNC sync) {
+  const int nc = nt / NSR_NPART;
+  const int q = t % NSR_NPART, c = t / NSR_NPART;
+  if (c < nc) {
+    const int per = (count + nc - 1) / nc;
+    const int b1 = min(count, (c + 1) * per);
+    double s = 0.0;
+#pragma unroll 4
+    for (int b = c * per; b < b1; ++b) s += __ldcg(&part[(long long)b * NSR_NPART + q]);
+    run[t] = s;
+  }
+  sync();
+  if (t < NSR_NPART) {
+    double s = 0.0;
+    for (int k = 0; k < nc; ++k) s += run[k * NSR_NPART + t];
+    tot[t] = s;
+  }
+  sync();
+}
+
 __device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotState& S, int slot, int mode,
                                                     double* acc) {
   __shared__ double red[NSR_NPART];
   __shared__ double tot[NSR_NPART];
-  __shared__ int am_last;
+  __shared__ double run[256];   // the blocks have 256 threads
+  __shared__ int am_last, finished;
   block_sum<NSR_NPART>(acc, red);
   double* part = A.B.partials + (long long)slot * A.nb_inv * NSR_NPART;
   if (threadIdx.x == 0) {
@@ -590,18 +633,15 @@ __device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotStat
   __syncthreads();
   if (!am_last) return;
   __threadfence();
-  // Deterministic sum over CTAs: thread q sums column q in CTA order.
-  if (threadIdx.x < NSR_NPART) {
-    double sacc = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) sacc += __ldcg(&part[b * NSR_NPART + threadIdx.x]);
-    tot[threadIdx.x] = sacc;
-  }
-  __syncthreads();
+  sum_partials(part, (int)gridDim.x, threadIdx.x, blockDim.x, run, tot, [] { __syncthreads(); });
   if (threadIdx.x == 0) {
     A.B.arrive[slot] = 0;
     finalize(A, S, mode, tot);
+    finished = S.mode == MODE_FINISH;
     __threadfence();
   }
+  __syncthreads();
+  if (finished) finish_block(A, S, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 }
 
 // ---------------------------------------------------------------------------
@@ -796,7 +836,8 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
   volatile int& abort_flag = abort_word;
   __shared__ double wsum[NC / 32][NSR_NPART];
   __shared__ double tot[NSR_NPART];
-  // Each consumer's FP64 accumulators live in shared memory (column tid): in
+  // Each consumer's FP64 accumulators live in shared memory (column tid; reused
+  // as scratch of the slot's last sum): in
   // registers they pushed the 96-register budget of four CTAs per SM into
   // spills inside the row loop.
   __shared__ double accs[NP][NC];
@@ -1057,15 +1098,10 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     named_sync(1, NC);
     if (am_last) {
       __threadfence();
-      if (tid < NSR_NPART) {
-        double sacc = 0.0;
-        for (int b = 0; b < it.per_slot; ++b) sacc += __ldcg(&part[b * NSR_NPART + tid]);
-        tot[tid] = sacc;
-      }
-      named_sync(1, NC);
+      sum_partials(part, it.per_slot, tid, NC, &accs[0][0], tot, [] { named_sync(1, NC); });
       if (tid == 0) {
         A.B.arrive[slot] = 0;
-        finalize(A, S, want, tot);
+        finalize(A, S, want, tot);   // ITER modes never finish a system: no finish_block here
         __threadfence();
       }
     }
@@ -1151,40 +1187,56 @@ __global__ void __launch_bounds__(256, 4) k_inv1(SolveArgs A, int half) {
 // ---------------------------------------------------------------------------
 // res: FP64 true residual r = b - A x of a replacement (x += M^-1 y) or of a
 // new system (x = x0); emit passes only arrive and hand the slot on.
+// One thread per column of a NSR_RES_TZ x NSR_RES_TX tile walks down its rows
+// with the north/centre/south values of x and a in registers; the east and west
+// neighbours come from the adjacent lanes, the PML factors from the separable
+// form of stencil_sep (no division per node).  Bound by its FP64 arithmetic
+// and 64 B per node; 44 systems of 768 x 1024 spent 15.9 ms in this launch with
+// one thread per node, four complex divisions each, and receivers gathered
+// by one thread, 7.6 ms in this form.
 // ---------------------------------------------------------------------------
+#define NSR_RES_TZ 8      // rows of one residual tile: 384 tiles of one 768 x 1024 system
+#define NSR_RES_TX 256
+#define NSR_RES_CTAS 1184 // CTAs of one launch over all its slots (8 per SM): most launches find no slot to
+                          // serve, and 4,224 idle CTAs cost 8 us more than 1,184
+__host__ __device__ inline int res_tiles(int nz, int nx) {
+  return ((nz + NSR_RES_TZ - 1) / NSR_RES_TZ) * ((nx + NSR_RES_TX - 1) / NSR_RES_TX);
+}
 template <bool ADJ>
-__global__ void __launch_bounds__(256) k_res(SolveArgs A) {
+__global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
   const int slot = A.slot0 + blockIdx.y;
   SlotState& S = A.B.slots[slot];
   const int mode = S.mode;
   if (!(mode == MODE_RES || mode == MODE_INIT || mode == MODE_EMIT)) return;
   const Geo& g = A.g;
   const long long n = (long long)g.nz * g.nx;
-  const int tz = A.tz;
-  const int z0 = blockIdx.x * tz;
-  const int nb = min(tz, g.nz - z0);
   const int nx = g.nx;
-  const SysScalars sc = sys_scalars(g, S.freq);
-  const double* ca = A.mat.a64;
-  const double* cb = A.mat.b64;
-  const double* ct = A.mat.t64;
-  auto Aa64 = [&](int i2, int j2) -> double {
-    if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= nx) return 1.0;
-    return __ldg(&ca[(long long)i2 * nx + j2]);
-  };
+  const int nbx = (nx + NSR_RES_TX - 1) / NSR_RES_TX;
+  const int n_tiles = res_tiles(g.nz, nx);
+  const int lane = threadIdx.x & 31;
   double acc[NSR_NPART];
 #pragma unroll
   for (int q = 0; q < NSR_NPART; ++q) acc[q] = 0.0;
   const long long soff = slot * n;
-  if (mode == MODE_RES || mode == MODE_INIT) {
+  const bool init = mode == MODE_INIT;
+  const SysScalars sc = sys_scalars(g, S.freq);
+  __shared__ RowFactors<double> rowf[NSR_RES_TZ];
+  for (int tile = mode == MODE_EMIT ? n_tiles : blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int rb = tile / nbx, cb = tile - rb * nbx;
+    const int z0 = rb * NSR_RES_TZ, z1 = min(z0 + NSR_RES_TZ, g.nz);
+    const int j = cb * NSR_RES_TX + threadIdx.x;
+    const bool own = j < nx;
+    __syncthreads();   // rowf of the tile before has been read
+    if (threadIdx.x < z1 - z0) rowf[threadIdx.x] = row_factors<double>(g, sc, z0 + threadIdx.x);
+    __syncthreads();
+    const ColFactors<double> cf = col_factors<double>(g, sc, j);
     const float2* zw = A.B.w + soff;   // z = M^-1 y after the rinv pass
     const double2* xo = A.B.x + (2LL * slot + S.xpar) * n;
     double2* xn = A.B.x + (2LL * slot + (S.xpar ^ 1)) * n;
     const float2* x0 = (A.x0 && S.sys >= 0 && !S.x0_off) ? A.x0 + (long long)S.sys * n : nullptr;
-    auto P = [&](int i2, int j2) -> double2 {
-      if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= nx) return make_double2(0.0, 0.0);
-      const long long id = (long long)i2 * nx + j2;
-      if (mode == MODE_INIT) return x0 ? to_d(x0[id]) : make_double2(0.0, 0.0);
+    const double2 zero = make_double2(0.0, 0.0);
+    auto P = [&](long long id) -> double2 {
+      if (init) return x0 ? to_d(x0[id]) : zero;
       return xo[id] + to_d(zw[id]);
     };
     const double h2 = g.h * g.h;
@@ -1192,31 +1244,53 @@ __global__ void __launch_bounds__(256) k_res(SolveArgs A) {
     const double st = sin(S.angle);
     float2* r = A.B.r + soff;
     float2* rh = A.B.rh + soff;
-    for (int k = threadIdx.x; k < nb * nx; k += blockDim.x) {
-      const int i = z0 + k / nx, j = k % nx;
-      const long long idx = (long long)i * nx + j;
-      double2 b;
-      if (rhs) {
-        b = h2 * to_d(rhs[idx]);
-      } else if (i == g.face) {
-        double2 l = source_line(g, sc.k0, st, j);
-        b = make_double2(-l.x, -l.y);
-      } else {
-        b = make_double2(0.0, 0.0);
+    const bool edge_w = lane == 0, edge_e = lane == 31 || j + 1 >= nx;
+    long long idx = (long long)z0 * nx + (own ? j : 0);
+    double2 pn = own && z0 > 0 ? P(idx - nx) : zero;
+    double2 pc = own ? P(idx) : zero;
+    double an = own && z0 > 0 ? __ldg(&A.mat.a64[idx - nx]) : 1.0;
+    double ac = own ? __ldg(&A.mat.a64[idx]) : 1.0;
+    for (int i = z0; i < z1; ++i, idx += nx) {
+      const bool has_s = own && i + 1 < g.nz;
+      const double2 ps = has_s ? P(idx + nx) : zero;
+      const double as = has_s ? __ldg(&A.mat.a64[idx + nx]) : 1.0;
+      double2 pw = make_double2(__shfl_up_sync(0xffffffffu, pc.x, 1), __shfl_up_sync(0xffffffffu, pc.y, 1));
+      double2 pe = make_double2(__shfl_down_sync(0xffffffffu, pc.x, 1), __shfl_down_sync(0xffffffffu, pc.y, 1));
+      double aw = __shfl_up_sync(0xffffffffu, ac, 1), ae = __shfl_down_sync(0xffffffffu, ac, 1);
+      if (own && edge_w) {
+        pw = j > 0 ? P(idx - 1) : zero;
+        aw = j > 0 ? __ldg(&A.mat.a64[idx - 1]) : 1.0;
       }
-      const double2 ax = stencil<double, ADJ>(g, sc, i, j, __ldg(&cb[idx]), __ldg(&ct[idx]), P, Aa64);
-      const double2 res = b - ax;
-      xn[idx] = P(i, j);
-      const float2 rf = to_f(res);
-      r[idx] = rf;
-      if (mode == MODE_INIT) {
-        rh[idx] = rf;
-        acc[0] += b.x * b.x + b.y * b.y;
-        acc[1] += (double)rf.x * rf.x + (double)rf.y * rf.y;
-      } else {
-        acc[0] += (double)rf.x * rf.x + (double)rf.y * rf.y;
-        dot_acc(acc[1], acc[2], rh[idx], rf);
+      if (own && edge_e) {
+        pe = j + 1 < nx ? P(idx + 1) : zero;
+        ae = j + 1 < nx ? __ldg(&A.mat.a64[idx + 1]) : 1.0;
       }
+      if (own) {
+        double2 b = zero;
+        if (rhs) {
+          b = h2 * to_d(rhs[idx]);
+        } else if (i == g.face) {
+          const double2 l = source_line(g, sc.k0, st, j);
+          b = make_double2(-l.x, -l.y);
+        }
+        const double2 ax = stencil_sep<double, ADJ>(sc.kh2, sc.fpow, rowf[i - z0], cf, ac, ae, aw, as, an, __ldg(&A.mat.b64[idx]),
+                                            __ldg(&A.mat.t64[idx]), pc, pe, pw, ps, pn);
+        xn[idx] = pc;
+        const float2 rf = to_f(b - ax);
+        r[idx] = rf;
+        if (init) {
+          rh[idx] = rf;
+          acc[0] += b.x * b.x + b.y * b.y;
+          acc[1] += (double)rf.x * rf.x + (double)rf.y * rf.y;
+        } else {
+          acc[0] += (double)rf.x * rf.x + (double)rf.y * rf.y;
+          dot_acc(acc[1], acc[2], rh[idx], rf);
+        }
+      }
+      pn = pc;
+      pc = ps;
+      an = ac;
+      ac = as;
     }
   }
   reduce_and_finalize(A, S, slot, mode, acc);
@@ -1319,7 +1393,7 @@ struct TileChoice {
 };
 
 static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileChoice* c) {
-  c->sw = 256; c->sd = 4; c->sr = 64; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
+  c->sw = 256; c->sd = 4; c->sr = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
   c->tc = nsr_cols_tc(g);
   c->rows = nsr_rows_per_cta(g);
   c->groups = n_slots >= 8 ? 2 : 1;
@@ -1336,21 +1410,29 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     c->rows_staged = t->rows_staged != 0;
   }
   if (!stn_kernel(c->sw, c->sd, c->scpt, false, 1)) return NSR_ERR_ARGUMENT;
-  if (c->sr < NSR_STN_MIN_ROWS || c->sr > 64 || c->sctas < 0 || c->sctas > 8) return NSR_ERR_ARGUMENT;
+  if (c->sr != 0 && (c->sr < NSR_STN_MIN_ROWS || c->sr > 64)) return NSR_ERR_ARGUMENT;
+  if (c->sctas < 0 || c->sctas > 8) return NSR_ERR_ARGUMENT;
   if (!(c->tc == 8 || c->tc == 16) || (size_t)g->nz * c->tc * sizeof(float2) > 200 * 1024) return NSR_ERR_ARGUMENT;
   if (c->rows < 1 || c->rows > 8 || sizeof(float2) * (size_t)c->rows * nsr_row_stride(g->nx) > 200 * 1024)
     return NSR_ERR_ARGUMENT;
   if (c->groups < 1 || c->groups > NSR_MAX_GROUPS) return NSR_ERR_ARGUMENT;
   if (c->groups > n_slots) c->groups = n_slots;
+  if (c->sr == 0) {
+    // Band height of the stencil: the tallest whose items give every SM about
+    // three CTAs.  Tall bands re-read the fewest halo rows, but a band is walked
+    // row by row, about 0.8 us each: three 256 x 256 systems in 64-row bands
+    // were 12 CTAs and 52 us a launch, in 4-row bands 192 CTAs.
+    const int strips = (g->nx + c->sw - 1) / c->sw, ns = (n_slots + c->groups - 1) / c->groups;
+    c->sr = 64;
+    while (c->sr > NSR_STN_MIN_ROWS && (long long)ns * ((g->nz + c->sr - 1) / c->sr) * strips < 3 * 148) c->sr /= 2;
+  }
   return 0;
 }
 
-static int band_rows(const NsrGrid* g) {
-  int budget = g->nx <= 1024 ? 8192 : 16384;
-  int tz = budget / g->nx - 2;
-  if (tz < 1) tz = 1;
-  if (tz > g->nz) tz = g->nz;
-  return tz;
+// Residual CTAs per slot of a launch over ns slots.
+static int res_ctas(const NsrGrid* g, int ns) {
+  const int tiles = res_tiles(g->nz, g->nx), share = NSR_RES_CTAS / ns > 1 ? NSR_RES_CTAS / ns : 1;
+  return tiles < share ? tiles : share;
 }
 
 struct Layout {
@@ -1361,8 +1443,7 @@ struct Layout {
 static Layout layout(const NsrGrid* g, int n_slots) {
   Layout L;
   const size_t n = (size_t)g->nz * g->nx;
-  const int tz = band_rows(g);
-  const int nb_res = (g->nz + tz - 1) / tz;
+  const int nb_res = res_ctas(g, 1);
   int nb_st = stencil_ctas(g);
   if (stn_ok(g) && stn_items_max(g) > nb_st) nb_st = stn_items_max(g);
   L.nb_inv = nb_res > nb_st ? nb_res : nb_st;
@@ -1481,7 +1562,6 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     A.n_systems = n_systems;
     A.rows = T.rows;
     A.tc = T.tc;
-    A.tz = band_rows(grid);
     A.nb_inv = L.nb_inv;
     A.tol2 = params->tolerance * params->tolerance;
     A.restart2 = params->restart_factor * params->restart_factor;
@@ -1505,7 +1585,6 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
 
     const size_t fwd_smem = sizeof(float2) * A.rows * nsr_row_stride(grid->nx);
     const size_t col_smem = nsr_cols_smem(grid);
-    const int nb_res = (grid->nz + A.tz - 1) / A.tz;
     const int nb_st = stencil_ctas(grid);
     const bool pairs = grid->nx % 2 == 0;
     const bool use_stn = stn_ok(grid);
@@ -1579,7 +1658,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
       const dim3 g_fwd(ns, (grid->nz + A.rows - 1) / A.rows);
       const dim3 g_col(ns, (grid->nx + A.tc - 1) / A.tc);
       const dim3 g_inv(nb_st, ns);
-      const dim3 g_res(nb_res, ns);
+      const dim3 g_res(res_ctas(grid, ns), ns);
       if (which == 0) {
         int hv = half;
         void* args[] = {&Ag, &hv};
@@ -1589,8 +1668,8 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
         void* args[] = {&Ag, &hv};
         cudaLaunchKernel((const void*)cols_fn, g_col, dim3(512), args, col_smem, sq);
       } else if (which == 2) {
-        if (A.adjoint) k_res<true><<<g_res, 256, 0, sq>>>(Ag);
-        else k_res<false><<<g_res, 256, 0, sq>>>(Ag);
+        if (A.adjoint) k_res<true><<<g_res, NSR_RES_TX, 0, sq>>>(Ag);
+        else k_res<false><<<g_res, NSR_RES_TX, 0, sq>>>(Ag);
       } else if (which == 3 && use_stn) {
         StnItems si;
         si.tz = T.sr;
