@@ -385,63 +385,195 @@ extern "C" int nsr_plane_wave_rhs(const NsrGrid* grid, const double* freq_hz, co
 // each edge e=(i,j): d(lam^H A u)/d log rho_i = a_i w_e conj(lam_j - lam_i)(u_j - u_i),
 // w_e = stretch_e / (2 h^2).
 // ---------------------------------------------------------------------------
-template <typename CT>
-__global__ void k_grad(Geo g, const void* __restrict__ mat, const double* __restrict__ freq, int ns,
-                       const CT* __restrict__ u, const CT* __restrict__ lam,
-                       double* __restrict__ gc, double* __restrict__ gr) {
-  const long long n = (long long)g.nz * g.nx;
-  const double inv_h2 = 1.0 / (g.h * g.h);
-  const MatPlanes mp = nsr_planes(mat, n);
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k / g.nx), j = (int)(k - (long long)i * g.nx);
-    const double a_c = mp.a64[k], b_c = mp.b64[k], t_c = mp.t64[k];
-    double acc_c = 0.0, acc_r = 0.0;
-    for (int sidx = 0; sidx < ns; ++sidx) {
-      const SysScalars s = sys_scalars(g, freq[sidx]);
-      const CT* us = u + sidx * n;
-      const CT* ls = lam + sidx * n;
-      auto U = [&](int i2, int j2) -> double2 {
-        if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= g.nx) return make_double2(0.0, 0.0);
-        const CT q = us[(long long)i2 * g.nx + j2];
-        return make_double2((double)q.x, (double)q.y);
-      };
-      auto L = [&](int i2, int j2) -> double2 {
-        if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= g.nx) return make_double2(0.0, 0.0);
-        const CT q = ls[(long long)i2 * g.nx + j2];
-        return make_double2((double)q.x, (double)q.y);
-      };
-      const double2 uc = U(i, j), lc = L(i, j);
-      const double2 lu = conjc(lc) * uc;
-      const double sig = s.sig;
-      const double2 sx = make_double2(1.0, sig * pml_profile<double>((double)j, g.nx, g.n_pml));
-      const double2 sz = make_double2(1.0, sig * pml_profile<double>((double)i, g.nz, g.n_pml));
-      const double e = t_c * s.fpow;
-      const double2 onepie = make_double2(1.0, e);
-      const double2 cell = (s.kh2 * b_c) * (sx * sz);          // h^2 k0^2 sx sz b
-      const double2 dm_c = (-2.0) * (cell * onepie);
-      const double2 dm_r = (-1.0) * (cell * (onepie * onepie));
-      double2 edge = make_double2(0.0, 0.0);
-      const int di[4] = {0, 0, 1, -1}, dj[4] = {1, -1, 0, 0};
+//
+// A thread owns one column of a TZ-row tile and keeps its nodes' sums in
+// registers while the systems go by; the tile of u and lam of the next system is
+// copied into shared memory (cp.async) while the present one is summed.  The edge term is the same product at both
+// ends of an edge, so each south edge is formed once and carried to the next
+// row.  With c = (k0 h)^2 sx sz and onepie = 1 + i e the sums are kept without
+// b and a:  acc_c = 2 sum Re(conj(lam) u c onepie),  acc_r = sum Re(conj(lam) u
+// c onepie^2),  acc_e = sum Re(edges); everything is FP64 as before.  Bound by
+// FP64 issue and conversions (about 30 FP64 operations and 8 conversions per
+// node and system).  22 systems of 1024 x 1536: 1,152 us with one thread per
+// node, a pow and six PML profiles per node and system; 270 us in this form.
+#define NSR_GRAD_TX 128      // threads of a block, one column each
+#define NSR_GRAD_CHUNK 64    // systems whose scalars are staged in shared memory at a time
+
+__device__ __forceinline__ void cp_async_zfill(float2* dst, const float2* src, bool live) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_zfill(double2* dst, const double2* src, bool live) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+// Columns c0 - 1 .. c0 + NSR_GRAD_TX of the rows z0 - 1 .. z0 + TZ of a field
+// (zero outside the grid).
+template <typename CT, int TZ>
+struct GradTile {
+  CT u[TZ + 2][NSR_GRAD_TX + 2], l[TZ + 2][NSR_GRAD_TX + 2];
+};
+template <typename CT, int TZ>
+__device__ __forceinline__ void grad_fetch(GradTile<CT, TZ>& t, const Geo& g, const CT* us, const CT* ls, int z0,
+                                           int c0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        double2 st;
-        if (q < 2) {
-          double2 sh = make_double2(1.0, sig * pml_profile<double>(j + 0.5 * dj[q], g.nx, g.n_pml));
-          st = divc(sz, sh);
-        } else {
-          double2 sh = make_double2(1.0, sig * pml_profile<double>(i + 0.5 * di[q], g.nz, g.n_pml));
-          st = divc(sx, sh);
-        }
-        const double2 du = U(i + di[q], j + dj[q]) - uc;
-        const double2 dl = conjc(L(i + di[q], j + dj[q]) - lc);
-        edge = edge + (0.5 * st) * (dl * du);
-      }
-      acc_c += -(lu * dm_c).x;
-      acc_r += -(lu * dm_r).x - a_c * edge.x;
-    }
-    gc[k] += acc_c * inv_h2;
-    gr[k] += acc_r * inv_h2;
+  for (int r = 0; r < TZ + 2; ++r) {
+    const int i = z0 - 1 + r;
+    const bool row = i >= 0 && i < g.nz;
+    const int j = c0 + threadIdx.x;
+    const bool live = row && j < g.nx;
+    const long long id = live ? (long long)i * g.nx + j : 0;
+    cp_async_zfill(&t.u[r][threadIdx.x + 1], us + id, live);
+    cp_async_zfill(&t.l[r][threadIdx.x + 1], ls + id, live);
   }
+  // the two halo columns
+  for (int q = threadIdx.x; q < 2 * (TZ + 2); q += NSR_GRAD_TX) {
+    const int r = q >> 1, i = z0 - 1 + r, j = (q & 1) ? c0 + NSR_GRAD_TX : c0 - 1;
+    const bool live = i >= 0 && i < g.nz && j >= 0 && j < g.nx;
+    const long long id = live ? (long long)i * g.nx + j : 0;
+    const int c = (q & 1) ? NSR_GRAD_TX + 1 : 0;
+    cp_async_zfill(&t.u[r][c], us + id, live);
+    cp_async_zfill(&t.l[r][c], ls + id, live);
+  }
+  cp_async_commit();
+}
+
+template <typename CT, int TZ>
+__global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, const void* __restrict__ mat,
+                                                         const double* __restrict__ freq, int ns,
+                                                         const CT* __restrict__ u, const CT* __restrict__ lam,
+                                                         double* __restrict__ gc, double* __restrict__ gr) {
+  __shared__ SysScalars scs[NSR_GRAD_CHUNK];
+  extern __shared__ __align__(16) unsigned char grad_smem[];
+  GradTile<CT, TZ>* tiles = reinterpret_cast<GradTile<CT, TZ>*>(grad_smem);   // two: one in use, one in flight
+  const long long n = (long long)g.nz * g.nx;
+  const int nx = g.nx, nz = g.nz;
+  const int nbx = (nx + NSR_GRAD_TX - 1) / NSR_GRAD_TX;
+  const int c0 = (blockIdx.x % nbx) * NSR_GRAD_TX;
+  const int j = c0 + threadIdx.x, tx = threadIdx.x + 1;
+  const int z0 = (blockIdx.x / nbx) * TZ;
+  const bool own = j < nx;
+  const int jc = own ? j : nx - 1;
+  const MatPlanes mp = nsr_planes(mat, n);
+  grad_fetch(tiles[0], g, u, lam, z0, c0);
+  const bool col_plain = j > g.n_pml && j < nx - 1 - g.n_pml;
+  // PML profiles of the column at j, j + 1/2, j - 1/2 (zero off the PML)
+  const double px = col_plain ? 0.0 : pml_profile<double>((double)jc, nx, g.n_pml);
+  const double pxe = col_plain ? 0.0 : pml_profile<double>(jc + 0.5, nx, g.n_pml);
+  const double pxw = col_plain ? 0.0 : pml_profile<double>(jc - 0.5, nx, g.n_pml);
+  const bool warp_plain = __all_sync(0xffffffffu, col_plain || !own);
+  double acc_c[TZ], acc_r[TZ], acc_e[TZ];
+  double t64[TZ];
+#pragma unroll
+  for (int q = 0; q < TZ; ++q) {
+    acc_c[q] = acc_r[q] = acc_e[q] = 0.0;
+    t64[q] = z0 + q < nz ? __ldg(&mp.t64[(long long)(z0 + q) * nx + jc]) : 0.0;
+  }
+  auto D = [](CT v) { return make_double2((double)v.x, (double)v.y); };
+  // conj(dl) du
+  auto prod = [](double2 dl, double2 du) {
+    return make_double2(dl.x * du.x + dl.y * du.y, dl.x * du.y - dl.y * du.x);
+  };
+  for (int s0 = 0; s0 < ns; s0 += NSR_GRAD_CHUNK) {
+    const int cnt = min(NSR_GRAD_CHUNK, ns - s0);
+    __syncthreads();
+    for (int q = threadIdx.x; q < cnt; q += NSR_GRAD_TX) scs[q] = sys_scalars(g, freq[s0 + q]);
+    for (int q = 0; q < cnt; ++q) {
+      const int sys = s0 + q;
+      __syncthreads();   // the tile about to be refilled has been read
+      if (sys + 1 < ns) {
+        grad_fetch(tiles[(sys + 1) & 1], g, u + (long long)(sys + 1) * n, lam + (long long)(sys + 1) * n, z0, c0);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+      const GradTile<CT, TZ>& t = tiles[sys & 1];
+      const SysScalars s = scs[q];
+      // 1 / (1 + i sig p) of the column's east and west half nodes
+      double2 ie = make_double2(1.0, 0.0), iw = ie;
+      if (!warp_plain) { ie = inv_stretch(s.sig * pxe); iw = inv_stretch(s.sig * pxw); }
+      const double2 sx = make_double2(1.0, s.sig * px);
+      double2 uc = D(t.u[1][tx]), lc = D(t.l[1][tx]);
+      double north;   // Re(w conj(dl) du) of the edge to the row above
+      {
+        const double2 p = prod(D(t.l[0][tx]) - lc, D(t.u[0][tx]) - uc);
+        north = p.x;
+        if (!(warp_plain && z0 > g.n_pml && z0 <= nz - 1 - g.n_pml)) {
+          const double2 w = sx * inv_stretch(s.sig * pml_profile<double>(z0 - 0.5, nz, g.n_pml));
+          north = w.x * p.x - w.y * p.y;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < TZ; ++r) {
+        const int i = z0 + r;
+        const double2 un = D(t.u[r + 2][tx]), ln = D(t.l[r + 2][tx]);
+        const double2 due = D(t.u[r + 1][tx + 1]) - uc, dle = D(t.l[r + 1][tx + 1]) - lc;
+        const double2 duw = D(t.u[r + 1][tx - 1]) - uc, dlw = D(t.l[r + 1][tx - 1]) - lc;
+        const double2 dus = un - uc, dls = ln - lc;
+        const double2 lu = prod(lc, uc);
+        const double e = t64[r] * s.fpow;
+        const bool row_plain = i > g.n_pml && i < nz - 1 - g.n_pml;
+        if (row_plain && warp_plain) {
+          const double south = dls.x * dus.x + dls.y * dus.y;
+          const double ew = dle.x * due.x + dle.y * due.y + (dlw.x * duw.x + dlw.y * duw.y);
+          acc_e[r] += 0.5 * (ew + south + north);
+          north = south;
+          const double ei = e * lu.y;
+          acc_c[r] += s.kh2 * (lu.x - ei);
+          acc_r[r] += s.kh2 * (lu.x * (1.0 - e * e) - 2.0 * ei);
+        } else {
+          const double2 pe = prod(dle, due), pw = prod(dlw, duw), ps = prod(dls, dus);
+          const double2 sz = make_double2(1.0, s.sig * pml_profile<double>((double)i, nz, g.n_pml));
+          const double2 we = sz * ie, ww = sz * iw;
+          const double2 ws = sx * inv_stretch(s.sig * pml_profile<double>(i + 0.5, nz, g.n_pml));
+          const double south = ws.x * ps.x - ws.y * ps.y;
+          acc_e[r] += 0.5 * ((we.x * pe.x - we.y * pe.y) + (ww.x * pw.x - ww.y * pw.y) + south + north);
+          north = south;
+          const double2 cell = sx * sz;
+          const double2 c1 = cell * make_double2(1.0, e), c2 = cell * make_double2(1.0 - e * e, 2.0 * e);
+          acc_c[r] += s.kh2 * (lu.x * c1.x - lu.y * c1.y);
+          acc_r[r] += s.kh2 * (lu.x * c2.x - lu.y * c2.y);
+        }
+        uc = un;
+        lc = ln;
+      }
+    }
+  }
+  if (!own) return;
+  const double inv_h2 = 1.0 / (g.h * g.h);
+#pragma unroll
+  for (int r = 0; r < TZ; ++r) {
+    if (z0 + r >= nz) break;
+    const long long k = (long long)(z0 + r) * nx + j;
+    const double b = mp.b64[k], a = mp.a64[k];
+    gc[k] += 2.0 * b * acc_c[r] * inv_h2;
+    gr[k] += (b * acc_r[r] - a * acc_e[r]) * inv_h2;
+  }
+}
+
+template <typename CT>
+static cudaError_t launch_grad(const Geo& g, const void* coef, const double* freq, int ns, const void* u,
+                               const void* lam, double* gc, double* gr, cudaStream_t st) {
+  // 4-row tiles read 6 rows for 4, from L2; a grid whose 4-row tiles would
+  // leave SMs without four blocks takes 2-row tiles.
+  const int bx = (g.nx + NSR_GRAD_TX - 1) / NSR_GRAD_TX;
+  const CT *pu = (const CT*)u, *pl = (const CT*)lam;
+  cudaError_t ce;
+  if ((long long)bx * ((g.nz + 3) / 4) >= 4 * 148) {
+    const int smem = 2 * (int)sizeof(GradTile<CT, 4>);
+    ce = cudaFuncSetAttribute(k_grad<CT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (ce != cudaSuccess) return ce;
+    k_grad<CT, 4><<<bx * ((g.nz + 3) / 4), NSR_GRAD_TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
+  } else {
+    const int smem = 2 * (int)sizeof(GradTile<CT, 2>);
+    k_grad<CT, 2><<<bx * ((g.nz + 1) / 2), NSR_GRAD_TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
+  }
+  return cudaGetLastError();
 }
 
 extern "C" int nsr_grad_accum(const NsrGrid* grid, const void* coef, const double* freq_hz,
@@ -452,17 +584,11 @@ extern "C" int nsr_grad_accum(const NsrGrid* grid, const void* coef, const doubl
   if (!coef || !freq_hz || !u || !lam || !g_logc || !g_logrho || n_systems < 0) return NSR_ERR_ARGUMENT;
   if (precision != 0 && precision != 1) return NSR_ERR_ARGUMENT;
   if (n_systems == 0) return 0;
-  long long n = (long long)grid->nz * grid->nx;
-  int bx = (int)((n + 255) / 256);
-  if (bx > 148 * 16) bx = 148 * 16;
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == 0)
-    k_grad<float2><<<bx, 256, 0, st>>>(make_geo(*grid), coef, freq_hz, n_systems, (const float2*)u,
-                                        (const float2*)lam, g_logc, g_logrho);
-  else
-    k_grad<double2><<<bx, 256, 0, st>>>(make_geo(*grid), coef, freq_hz, n_systems, (const double2*)u,
-                                         (const double2*)lam, g_logc, g_logrho);
-  return last_error();
+  const Geo g = make_geo(*grid);
+  const cudaError_t ce = precision == 0 ? launch_grad<float2>(g, coef, freq_hz, n_systems, u, lam, g_logc, g_logrho, st)
+                                        : launch_grad<double2>(g, coef, freq_hz, n_systems, u, lam, g_logc, g_logrho, st);
+  return ce == cudaSuccess ? 0 : (int)ce;
 }
 
 // ---------------------------------------------------------------------------
