@@ -10,7 +10,8 @@
 //   (D p)[n]     = (1/dx) sum_k a_k (p[n+1+k] - p[n-k])
 //   (-D^H f)[n]  = (1/dx) sum_k a_k (f[n+k]   - f[n-1-k])
 // with a = (1225/1024, -245/3072, 49/5120, -5/7168).
-// Pass 1 writes the staggered fluxes, pass 2 takes their divergence.
+// One kernel forms the staggered fluxes of a tile in shared memory and takes
+// their divergence.
 #include "nsr_internal.cuh"
 
 #include <string.h>
@@ -56,119 +57,214 @@ __device__ __forceinline__ bool dense_inside(const DenseGeo& g, int i, int j) {
   return i >= g.pz && i < g.pz + g.h && j >= g.px && j < g.px + g.w;
 }
 
-// Pass 1.  Forward: X = ax svx D_x(mask p), gX = gvx X, and the same along z.
-// Adjoint: w = conj(scal) mask p, flux_x = conj(ax svx) (-D_x(conj(lx) w) - conj(gvx) D_x(conj(rx) w)).
-template <typename T, bool ADJ>
-__global__ void k_dense_flux(DenseGeo g, const double* __restrict__ coef, const typename DC<T>::C* __restrict__ p,
-                             typename DC<T>::C* __restrict__ tmp, int nf) {
+// One pass over a TZ x DA_TX tile.  The x part of a node needs p along its row
+// only and the z part along its column only, 7 nodes each way: the tile of
+// mask p with those halos is staged in shared memory, the staggered fluxes of
+// the tile (3 or 4 nodes beyond it) are formed there, and their divergence is
+// taken from there, so that HBM carries p, y and the coefficients once.  (Two
+// passes with four flux planes through memory moved 80 B per node and field.)
+//   Forward: X = ax svx D_x(mask p), likewise Z;
+//            y = mask (scal (lx div X + rx div(gvx X) + lz div Z + rz div(gvz Z)) + mass p) + (1 - mask) p.
+//   Adjoint: w = conj(scal) mask p;
+//            X = conj(ax svx) (-D_x(conj(lx) w) - conj(gvx) D_x(conj(rx) w)), likewise Z;
+//            y = mask (-div X - div Z + conj(mass) p) + (1 - mask) p.
+// Off the PML gv = sv = 1, the left factor is zero and the right one is one
+// constant: a tile all of whose profiles say so takes a shorter form.
+// Eleven complex64 fields on 1056 x 1216: 695 us in two passes, 316 us here,
+// bound by its shared-memory reads (about 33 a node).
+#define DA_TX 64
+#define DA_THREADS 256
+#define DA_R 7    // reach of the two staggered stencils
+
+template <typename T, int TZ>
+struct DenseTile {
   typedef typename DC<T>::C C;
+  C p[TZ + 2 * DA_R][DA_TX + 2 * DA_R];   // mask p; rows and columns start at (z0 - 7, c0 - 7)
+  C x[TZ][DA_TX + 7];                     // X at columns c0 - 4 .. c0 + DA_TX + 2
+  C z[TZ + 7][DA_TX];                     // Z at rows z0 - 4 .. z0 + TZ + 2
+  C prx[4][DA_TX + 2 * DA_R];             // sv, gv, l, r of the columns
+  C prz[4][TZ + 2 * DA_R];                // and of the rows
+};
+
+template <typename C>
+__device__ __forceinline__ bool is_real(C v, double re) { return v.x == (decltype(v.x))re && v.y == 0; }
+
+template <typename T, bool ADJ, int TZ>
+__global__ void __launch_bounds__(DA_THREADS) k_dense_apply(DenseGeo g, const double* __restrict__ coef,
+                                                            const typename DC<T>::C* __restrict__ p,
+                                                            typename DC<T>::C* __restrict__ y, int nf) {
+  typedef typename DC<T>::C C;
+  extern __shared__ __align__(16) unsigned char da_smem[];
+  DenseTile<T, TZ>& t = *reinterpret_cast<DenseTile<T, TZ>*>(da_smem);
   const DenseCoef dc = dense_unpack(coef, g.H, g.W);
   const long long n = (long long)g.H * g.W;
-  const int f = blockIdx.y;
-  const C* pf = p + f * n;
-  C* t = tmp + f * 4 * n;
+  // The fields run fastest, so the coefficients of a tile come from L2 after
+  // the first field.
+  const int f = blockIdx.x % nf, tile = blockIdx.x / nf;
+  const int nbx = (g.W + DA_TX - 1) / DA_TX;
+  const int z0 = (tile / nbx) * TZ, c0 = (tile % nbx) * DA_TX;
+  const C* pf = p + (long long)f * n;
+  C* yf = y + (long long)f * n;
   const C zero = cx<C>(T(0), T(0));
+  const int tid = threadIdx.x;
+  // A tile with no node of the native region copies.
+  const bool touched = z0 < g.pz + g.h && z0 + TZ > g.pz && c0 < g.px + g.w && c0 + DA_TX > g.px;
+  if (!touched) {
+    for (int k = tid; k < TZ * DA_TX; k += DA_THREADS) {
+      const int i = z0 + k / DA_TX, j = c0 + k % DA_TX;
+      if (i < g.H && j < g.W) yf[(long long)i * g.W + j] = pf[(long long)i * g.W + j];
+    }
+    return;
+  }
+  constexpr int PW = DA_TX + 2 * DA_R, PH = TZ + 2 * DA_R;
+  // The corners of the halo are never read.
+  for (int k = tid; k < PW * PH; k += DA_THREADS) {
+    const int r = k / PW, c = k - r * PW;
+    const int i = z0 - DA_R + r, j = c0 - DA_R + c;
+    const bool cross = (r >= DA_R && r < DA_R + TZ) || (c >= DA_R && c < DA_R + DA_TX);
+    if (cross) t.p[r][c] = i >= 0 && i < g.H && j >= 0 && j < g.W && dense_inside(g, i, j)
+                               ? pf[(long long)i * g.W + j] : zero;
+  }
+  bool plain_x = true, plain_z = true;
+  C r0x = zero, r0z = zero;   // the right factors of the first column and row
+  {
+    const int jm = min(max(c0, 0), g.W - 1), im = min(max(z0, 0), g.H - 1);
+    r0x = DC<T>::from(dc.rx[jm]);
+    r0z = DC<T>::from(dc.rz[im]);
+  }
+  for (int c = tid; c < PW; c += DA_THREADS) {
+    const int j = c0 - DA_R + c;
+    const bool in = j >= 0 && j < g.W;
+    const C sv = in ? DC<T>::from(dc.svx[j]) : zero, gv = in ? DC<T>::from(dc.gvx[j]) : zero;
+    const C l = in ? DC<T>::from(dc.lx[j]) : zero, r = in ? DC<T>::from(dc.rx[j]) : zero;
+    t.prx[0][c] = sv; t.prx[1][c] = gv; t.prx[2][c] = l; t.prx[3][c] = r;
+    plain_x = plain_x && is_real(sv, 1.0) && is_real(gv, 1.0) && is_real(l, 0.0) && r.x == r0x.x && r.y == r0x.y;
+  }
+  for (int c = tid; c < PH; c += DA_THREADS) {
+    const int i = z0 - DA_R + c;
+    const bool in = i >= 0 && i < g.H;
+    const C sv = in ? DC<T>::from(dc.svz[i]) : zero, gv = in ? DC<T>::from(dc.gvz[i]) : zero;
+    const C l = in ? DC<T>::from(dc.lz[i]) : zero, r = in ? DC<T>::from(dc.rz[i]) : zero;
+    t.prz[0][c] = sv; t.prz[1][c] = gv; t.prz[2][c] = l; t.prz[3][c] = r;
+    plain_z = plain_z && is_real(sv, 1.0) && is_real(gv, 1.0) && is_real(l, 0.0) && r.x == r0z.x && r.y == r0z.y;
+  }
+  plain_x = __syncthreads_and(plain_x) != 0;
+  plain_z = __syncthreads_and(plain_z) != 0;
+  const T a4[4] = {(T)nsr_dense_stencil(0), (T)nsr_dense_stencil(1), (T)nsr_dense_stencil(2), (T)nsr_dense_stencil(3)};
   const T inv_dx = (T)(1.0 / g.dx);
-  const C wscal = DC<T>::from(conjc(g.scal));
-  auto PM = [&](int i2, int j2) -> C {
-    if (i2 < 0 || i2 >= g.H || j2 < 0 || j2 >= g.W || !dense_inside(g, i2, j2)) return zero;
-    return pf[(long long)i2 * g.W + j2];
+  const C scal = DC<T>::from(g.scal);
+  // D along a line of stride s: sum a_q (p[+1+q] - p[-q])
+  auto grad = [&](const C* q, int s) -> C {
+    C v = a4[0] * (q[s] - q[0]);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) v = v + a4[k] * (q[(1 + k) * s] - q[-k * s]);
+    return v;
   };
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k / g.W), j = (int)(k - (long long)i * g.W);
+  // divergence: sum a_q (f[+q] - f[-1-q])
+  auto div = [&](const C* q, int s) -> C {
+    C v = a4[0] * (q[0] - q[-s]);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) v = v + a4[k] * (q[k * s] - q[-(1 + k) * s]);
+    return v;
+  };
+  // D of (conj(factor) p) with a factor per node of the line
+  auto grad_of = [&](const C* q, int s, const C* fac) -> C {
+    C v = zero;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v = v + a4[k] * (conjc(fac[1 + k]) * q[(1 + k) * s] - conjc(fac[-k]) * q[-k * s]);
+    return v;
+  };
+  auto div_of = [&](const C* q, int s, const C* fac) -> C {
+    C v = zero;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v = v + a4[k] * (fac[k] * q[k * s] - fac[-1 - k] * q[-(1 + k) * s]);
+    return v;
+  };
+  // fluxes along x: node (z0 + r, c0 - 4 + c)
+  for (int k = tid; k < TZ * (DA_TX + 7); k += DA_THREADS) {
+    const int r = k / (DA_TX + 7), c = k - r * (DA_TX + 7);
+    const int i = z0 + r, j = c0 - 4 + c;
+    C v = zero;
+    if (i < g.H && j >= 0 && j < g.W) {
+      const C* q = &t.p[r + DA_R][c + 3];
+      const T ax = (T)dc.ax[(long long)i * g.W + j];
+      if (!ADJ) {
+        const C gx = grad(q, 1);
+        v = plain_x ? (inv_dx * ax) * gx : (inv_dx * ax) * (t.prx[0][c + 3] * gx);
+      } else if (plain_x) {
+        v = (T(-1) * inv_dx * ax) * (conjc(scal * r0x) * grad(q, 1));
+      } else {
+        const C fl = grad_of(q, 1, &t.prx[2][c + 3]), fr = grad_of(q, 1, &t.prx[3][c + 3]);
+        v = (T(-1) * inv_dx * ax) * (conjc(t.prx[0][c + 3] * scal) * (fl + conjc(t.prx[1][c + 3]) * fr));
+      }
+    }
+    t.x[r][c] = v;
+  }
+  // fluxes along z: node (z0 - 4 + r, c0 + c)
+  for (int k = tid; k < (TZ + 7) * DA_TX; k += DA_THREADS) {
+    const int r = k / DA_TX, c = k - r * DA_TX;
+    const int i = z0 - 4 + r, j = c0 + c;
+    C v = zero;
+    if (i >= 0 && i < g.H && j < g.W) {
+      const C* q = &t.p[r + 3][c + DA_R];
+      const T az = (T)dc.az[(long long)i * g.W + j];
+      if (!ADJ) {
+        const C gz = grad(q, PW);
+        v = plain_z ? (inv_dx * az) * gz : (inv_dx * az) * (t.prz[0][r + 3] * gz);
+      } else if (plain_z) {
+        v = (T(-1) * inv_dx * az) * (conjc(scal * r0z) * grad(q, PW));
+      } else {
+        const C fl = grad_of(q, PW, &t.prz[2][r + 3]), fr = grad_of(q, PW, &t.prz[3][r + 3]);
+        v = (T(-1) * inv_dx * az) * (conjc(t.prz[0][r + 3] * scal) * (fl + conjc(t.prz[1][r + 3]) * fr));
+      }
+    }
+    t.z[r][c] = v;
+  }
+  __syncthreads();
+  for (int k = tid; k < TZ * DA_TX; k += DA_THREADS) {
+    const int r = k / DA_TX, c = k - r * DA_TX;
+    const int i = z0 + r, j = c0 + c;
+    if (i >= g.H || j >= g.W) continue;
+    const long long id = (long long)i * g.W + j;
+    if (!dense_inside(g, i, j)) { yf[id] = pf[id]; continue; }
+    const C* qx = &t.x[r][c + 4];
+    const C* qz = &t.z[r + 4][c];
+    const C pk = t.p[r + DA_R][c + DA_R];
+    const C mass = DC<T>::from(dc.mass[id]);
     if (!ADJ) {
-      C gx = zero, gz = zero;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T a = (T)c_dense_a[q];
-        gx = gx + a * (PM(i, j + 1 + q) - PM(i, j - q));
-        gz = gz + a * (PM(i + 1 + q, j) - PM(i - q, j));
-      }
-      const C X = (inv_dx * (T)dc.ax[k]) * (DC<T>::from(dc.svx[j]) * gx);
-      const C Z = (inv_dx * (T)dc.az[k]) * (DC<T>::from(dc.svz[i]) * gz);
-      t[k] = X;
-      t[n + k] = DC<T>::from(dc.gvx[j]) * X;
-      t[2 * n + k] = Z;
-      t[3 * n + k] = DC<T>::from(dc.gvz[i]) * Z;
+      C part;
+      const C dX = div(qx, 1), dZ = div(qz, DA_TX);
+      part = plain_x ? r0x * dX
+                     : t.prx[2][c + DA_R] * dX + t.prx[3][c + DA_R] * div_of(qx, 1, &t.prx[1][c + DA_R]);
+      part = part + (plain_z ? r0z * dZ
+                             : t.prz[2][r + DA_R] * dZ + t.prz[3][r + DA_R] * div_of(qz, DA_TX, &t.prz[1][r + DA_R]));
+      yf[id] = scal * (inv_dx * part) + mass * pk;
     } else {
-      // along x the left/right factors depend on the column of each node
-      C fl = zero, fr = zero, zl = zero, zr = zero;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T a = (T)c_dense_a[q];
-        const int je = j + 1 + q, jw = j - q;
-        const C we = PM(i, je), ww = PM(i, jw);
-        const C le = je < g.W ? conjc(DC<T>::from(dc.lx[je])) * we : zero;
-        const C lw = jw >= 0 ? conjc(DC<T>::from(dc.lx[jw])) * ww : zero;
-        const C re = je < g.W ? conjc(DC<T>::from(dc.rx[je])) * we : zero;
-        const C rw = jw >= 0 ? conjc(DC<T>::from(dc.rx[jw])) * ww : zero;
-        fl = fl + a * (le - lw);
-        fr = fr + a * (re - rw);
-        const int is = i + 1 + q, in = i - q;
-        const C ws = PM(is, j), wn = PM(in, j);
-        const C ls = is < g.H ? conjc(DC<T>::from(dc.lz[is])) * ws : zero;
-        const C ln = in >= 0 ? conjc(DC<T>::from(dc.lz[in])) * wn : zero;
-        const C rs = is < g.H ? conjc(DC<T>::from(dc.rz[is])) * ws : zero;
-        const C rn = in >= 0 ? conjc(DC<T>::from(dc.rz[in])) * wn : zero;
-        zl = zl + a * (ls - ln);
-        zr = zr + a * (rs - rn);
-      }
-      // w = conj(scal) mask p was left out of the sums: apply it once here
-      const C fx = (T(-1) * inv_dx) * (wscal * (fl + conjc(DC<T>::from(dc.gvx[j])) * fr));
-      const C fz = (T(-1) * inv_dx) * (wscal * (zl + conjc(DC<T>::from(dc.gvz[i])) * zr));
-      t[k] = conjc(DC<T>::from(dc.svx[j]) * cx<C>((T)dc.ax[k], T(0))) * fx;
-      t[2 * n + k] = conjc(DC<T>::from(dc.svz[i]) * cx<C>((T)dc.az[k], T(0))) * fz;
+      yf[id] = (T(-1) * inv_dx) * (div(qx, 1) + div(qz, DA_TX)) + conjc(mass) * pk;
     }
   }
 }
 
-// Pass 2.  Forward: y = mask (scal (lx divX + rx div gX + lz divZ + rz div gZ) + mass p) + (1 - mask) p.
-// Adjoint: y = mask (D^H flux_x + D^H flux_z + conj(mass) p) + (1 - mask) p.
-template <typename T, bool ADJ>
-__global__ void k_dense_div(DenseGeo g, const double* __restrict__ coef, const typename DC<T>::C* __restrict__ p,
-                            const typename DC<T>::C* __restrict__ tmp, typename DC<T>::C* __restrict__ y, int nf) {
+template <typename T, bool ADJ, int TZ>
+static cudaError_t launch_dense_apply(const DenseGeo& g, const double* coef, int nf, const void* x, void* y,
+                                      cudaStream_t st) {
   typedef typename DC<T>::C C;
-  const DenseCoef dc = dense_unpack(coef, g.H, g.W);
-  const long long n = (long long)g.H * g.W;
-  const int f = blockIdx.y;
-  const C* pf = p + f * n;
-  const C* t = tmp + f * 4 * n;
-  C* yf = y + f * n;
-  const C zero = cx<C>(T(0), T(0));
-  const T inv_dx = (T)(1.0 / g.dx);
-  auto F = [&](int plane, int i2, int j2) -> C {
-    if (i2 < 0 || i2 >= g.H || j2 < 0 || j2 >= g.W) return zero;
-    return t[plane * n + (long long)i2 * g.W + j2];
-  };
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k / g.W), j = (int)(k - (long long)i * g.W);
-    const C pk = pf[k];
-    if (!dense_inside(g, i, j)) { yf[k] = pk; continue; }
-    if (!ADJ) {
-      C dX = zero, dgX = zero, dZ = zero, dgZ = zero;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T a = (T)c_dense_a[q];
-        dX = dX + a * (F(0, i, j + q) - F(0, i, j - 1 - q));
-        dgX = dgX + a * (F(1, i, j + q) - F(1, i, j - 1 - q));
-        dZ = dZ + a * (F(2, i + q, j) - F(2, i - 1 - q, j));
-        dgZ = dgZ + a * (F(3, i + q, j) - F(3, i - 1 - q, j));
-      }
-      const C part = DC<T>::from(dc.lx[j]) * dX + DC<T>::from(dc.rx[j]) * dgX +
-                     DC<T>::from(dc.lz[i]) * dZ + DC<T>::from(dc.rz[i]) * dgZ;
-      yf[k] = DC<T>::from(g.scal) * (inv_dx * part) + DC<T>::from(dc.mass[k]) * pk;
-    } else {
-      C dX = zero, dZ = zero;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T a = (T)c_dense_a[q];
-        dX = dX + a * (F(0, i, j + q) - F(0, i, j - 1 - q));
-        dZ = dZ + a * (F(2, i + q, j) - F(2, i - 1 - q, j));
-      }
-      // D^H f = -(-D^H f)
-      yf[k] = (T(-1) * inv_dx) * (dX + dZ) + conjc(DC<T>::from(dc.mass[k])) * pk;
-    }
-  }
+  const int smem = (int)sizeof(DenseTile<T, TZ>);
+  const cudaError_t ce = cudaFuncSetAttribute(k_dense_apply<T, ADJ, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (ce != cudaSuccess) return ce;
+  const long long tiles = (long long)((g.W + DA_TX - 1) / DA_TX) * ((g.H + TZ - 1) / TZ);
+  k_dense_apply<T, ADJ, TZ><<<(unsigned)(tiles * nf), DA_THREADS, smem, st>>>(g, coef, (const C*)x, (C*)y, nf);
+  return cudaGetLastError();
+}
+
+// Tile height: tall tiles form the fewest fluxes twice (23 rows for 16); grids
+// whose 16-row tiles are fewer than three per SM take 8-row ones.
+template <typename T, bool ADJ>
+static cudaError_t dense_apply_t(const DenseGeo& g, const double* coef, int nf, const void* x, void* y,
+                                 cudaStream_t st) {
+  const long long tiles = (long long)((g.W + DA_TX - 1) / DA_TX) * ((g.H + 15) / 16) * nf;
+  return tiles >= 3 * 148 ? launch_dense_apply<T, ADJ, 16>(g, coef, nf, x, y, st)
+                          : launch_dense_apply<T, ADJ, 8>(g, coef, nf, x, y, st);
 }
 
 extern "C" size_t nsr_dense_coef_bytes(const NsrDenseGrid* g) {
@@ -178,7 +274,7 @@ extern "C" size_t nsr_dense_coef_bytes(const NsrDenseGrid* g) {
 
 extern "C" size_t nsr_dense_workspace_size(const NsrDenseGrid* g, int32_t n_fields, int32_t precision) {
   if (!g || g->H <= 0 || g->W <= 0 || n_fields < 0 || (precision != 0 && precision != 1)) return 0;
-  return (size_t)4 * g->H * g->W * n_fields * (precision ? 16 : 8);
+  return n_fields > 0 ? 256 : 0;   // the fluxes live in shared memory
 }
 
 extern "C" int nsr_dense_apply(const NsrDenseGrid* grid, const double* coef, double scal_re, double scal_im,
@@ -194,31 +290,12 @@ extern "C" int nsr_dense_apply(const NsrDenseGrid* grid, const double* coef, dou
   DenseGeo g;
   g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
   g.scal = make_double2(scal_re, scal_im);
-  const long long n = (long long)g.H * g.W;
-  int bx = (int)((n + 255) / 256);
-  if (bx > 4096) bx = 4096;
-  const dim3 gr(bx, n_fields);
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == 0) {
-    float2* t = (float2*)workspace;
-    if (adjoint) {
-      k_dense_flux<float, true><<<gr, 256, 0, st>>>(g, coef, (const float2*)x, t, n_fields);
-      k_dense_div<float, true><<<gr, 256, 0, st>>>(g, coef, (const float2*)x, t, (float2*)y, n_fields);
-    } else {
-      k_dense_flux<float, false><<<gr, 256, 0, st>>>(g, coef, (const float2*)x, t, n_fields);
-      k_dense_div<float, false><<<gr, 256, 0, st>>>(g, coef, (const float2*)x, t, (float2*)y, n_fields);
-    }
-  } else {
-    double2* t = (double2*)workspace;
-    if (adjoint) {
-      k_dense_flux<double, true><<<gr, 256, 0, st>>>(g, coef, (const double2*)x, t, n_fields);
-      k_dense_div<double, true><<<gr, 256, 0, st>>>(g, coef, (const double2*)x, t, (double2*)y, n_fields);
-    } else {
-      k_dense_flux<double, false><<<gr, 256, 0, st>>>(g, coef, (const double2*)x, t, n_fields);
-      k_dense_div<double, false><<<gr, 256, 0, st>>>(g, coef, (const double2*)x, t, (double2*)y, n_fields);
-    }
-  }
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      precision == 0 ? (adjoint ? dense_apply_t<float, true>(g, coef, n_fields, x, y, st)
+                                : dense_apply_t<float, false>(g, coef, n_fields, x, y, st))
+                     : (adjoint ? dense_apply_t<double, true>(g, coef, n_fields, x, y, st)
+                                : dense_apply_t<double, false>(g, coef, n_fields, x, y, st));
   return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -261,7 +338,7 @@ __global__ void k_dense_grad(DenseGeo g, const double* __restrict__ coef, const 
       double2 gx = zero, gz = zero, qxl = zero, qxr = zero, qzl = zero, qzr = zero;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const double a = c_dense_a[q];
+        const double a = nsr_dense_stencil(q);
         gx = gx + a * (U(i, j + 1 + q) - U(i, j - q));
         gz = gz + a * (U(i + 1 + q, j) - U(i - q, j));
         const int jw = j - q, je = j + 1 + q, in_ = i - q, is = i + 1 + q;
