@@ -11,7 +11,7 @@
 
 #define NSR_MAX_RADIX_STAGES 12
 #define NSR_MAX_LINE 2048
-// Largest prime radix of the transforms (direct DFT stages, see fft_stage_prime).
+// Largest prime radix of the transforms (direct DFT stages, see small_dft and gen_stage_prime).
 #define NSR_MAX_PRIME_RADIX 61
 #define NSR_PI 3.14159265358979323846
 
@@ -276,9 +276,58 @@ struct FftPlan {
   const float2* tws;
 };
 
+// cos and sin of 2 pi k / R for the odd prime radices, from the Taylor series
+// of the angle reduced to [-pi, pi] (30 terms in double, rounded once).
+template <int R>
+struct PrimeTable {
+  float c[R], s[R];
+};
+template <int R>
+__host__ __device__ constexpr PrimeTable<R> make_prime_table() {
+  PrimeTable<R> t{};
+  for (int k = 0; k < R; ++k) {
+    const double x = 2.0 * NSR_PI * (2 * k > R ? k - R : k) / R;
+    double c = 1.0, s = x, tc = 1.0, ts = x;
+    for (int q = 1; q < 15; ++q) {
+      tc *= -x * x / ((2 * q - 1) * (2 * q));
+      ts *= -x * x / ((2 * q) * (2 * q + 1));
+      c += tc;
+      s += ts;
+    }
+    t.c[k] = (float)c;
+    t.s[k] = (float)s;
+  }
+  return t;
+}
+
 template <int R, bool INV>
 __device__ __forceinline__ void small_dft(float2* x) {
-  if (R == 2) {
+  if constexpr (R == 5 || R == 7 || R == 11 || R == 13 || R == 17 || R == 19) {
+    // Direct DFT of an odd prime length on the sums and differences of x[q] and
+    // x[R - q]: (R - 1)^2 real multiply-adds instead of 4 (R - 1)^2.
+    constexpr PrimeTable<R> T = make_prime_table<R>();
+    constexpr int M = (R - 1) / 2;
+    float2 a[M], b[M], x0 = x[0], sum = x[0];
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+      a[q] = x[q + 1] + x[R - 1 - q];
+      b[q] = x[q + 1] - x[R - 1 - q];
+      sum = sum + a[q];
+    }
+    x[0] = sum;
+#pragma unroll
+    for (int k = 1; k <= M; ++k) {
+      float2 c = x0, d = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int q = 1; q <= M; ++q) {
+        c = c + T.c[(q * k) % R] * a[q - 1];
+        d = d + T.s[(q * k) % R] * b[q - 1];
+      }
+      const float2 t = INV ? make_float2(-d.y, d.x) : make_float2(d.y, -d.x);   // -+ i d
+      x[k] = c + t;
+      x[R - k] = c - t;
+    }
+  } else if (R == 2) {
     float2 a = x[0], b = x[1];
     x[0] = a + b; x[1] = a - b;
   } else if (R == 3) {
@@ -339,111 +388,282 @@ __device__ __forceinline__ void small_dft(float2* x) {
   }
 }
 
-// One DIF stage (forward) or its inverse over `nl` lines.
-// Element k of line l lives at s[l*lstride + k*estride].  When `line_fast`
-// the thread index runs over lines first (columns held side by side in
-// shared memory), otherwise over butterflies of one line first (rows).
+// Row layout in shared memory: one pad element after every 16 (element k of a
+// row at k + k/16), which keeps the stages with power-of-two strides free of
+// bank conflicts.
+__host__ __device__ inline int nsr_row_stride(int n) { return n + (n >> 4); }
+__device__ __forceinline__ int row_pos(int k) { return k + (k >> 4); }
+
+// Stages of any length the plan takes, with the length, the radix order and
+// the strides known at run time.  TC = 0: `nl` rows in the padded row layout;
+// TC > 0: TC columns side by side (element k of column l at l + k TC).
+// Twiddles come from the stage tables of FftPlan::tws.
 template <int R, bool INV>
-__device__ __forceinline__ void fft_stage(float2* s, int nl, int lstride, int estride, bool line_fast,
-                                          const FftPlan& P, int L) {
-  const int m = L / R;
-  const int per_line = P.n / R;
-  const int nb = nl * per_line;
-  const int tstep = P.n / L;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    int l, bb;
-    if (line_fast) { l = b % nl; bb = b / nl; } else { l = b / per_line; bb = b % per_line; }
-    const int o = bb / m, j = bb - o * m;
-    float2* base = s + l * lstride + (o * L + j) * estride;
-    float2 v[R];
+__device__ __forceinline__ void gen_twiddle(float2* v, const float2* __restrict__ tst, int j, int m) {
+  if (m == 1) return;   // unit twiddles
 #pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = base[q * m * estride];
-    if (!INV) {
-      small_dft<R, false>(v);
-#pragma unroll
-      for (int k = 1; k < R; ++k) v[k] = v[k] * __ldg(&P.tw[j * k * tstep]);
-    } else {
-#pragma unroll
-      for (int k = 1; k < R; ++k) v[k] = v[k] * conjc(__ldg(&P.tw[j * k * tstep]));
-      small_dft<R, true>(v);
-    }
-#pragma unroll
-    for (int q = 0; q < R; ++q) base[q * m * estride] = v[q];
+  for (int k = 1; k < R; ++k) {
+    const float2 w = __ldg(tst + (k - 1) * m + j);
+    v[k] = v[k] * (INV ? conjc(w) : w);
   }
 }
 
-// One DIF stage (forward) or its inverse for a prime radix R > 3, as a direct
-// R-point DFT: y_k = sum_q v_q W_R^(q k), W_R^e = tw[e n / R].  The cost is
-// R complex multiply-adds per point, which the sizes that need these stages
-// (paddings such as 1056 = 2^5 3 11 and 1216 = 2^6 19) can afford.
-template <bool INV>
-__device__ __noinline__ void fft_stage_prime(float2* s, int nl, int lstride, int estride, bool line_fast,
-                                             const FftPlan& P, int L, int R) {
-  const int m = L / R;
-  const int per_line = P.n / R;
-  const int nb = nl * per_line;
-  const int tstep = P.n / L;
-  const int rstep = P.n / R;
+template <int R, bool INV, int TC>
+__device__ __forceinline__ void gen_stage(float2* s, int nl, int N, int L, const float2* __restrict__ tst) {
+  const int m = L / R, per = N / R, nb = (TC ? TC : nl) * per;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    int l, bb;
+    if constexpr (TC > 0) { l = b % TC; bb = b / TC; } else { l = b / per; bb = b - l * per; }
+    const int o = bb / m, j = bb - o * m, e = o * L + j;
+    float2* base = TC ? s + l : s + l * nsr_row_stride(N);
+    float2 v[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = base[TC ? (e + q * m) * TC : row_pos(e + q * m)];
+    if (INV) gen_twiddle<R, true>(v, tst, j, m);
+    small_dft<R, INV>(v);
+    if (!INV) gen_twiddle<R, false>(v, tst, j, m);
+#pragma unroll
+    for (int q = 0; q < R; ++q) base[TC ? (e + q * m) * TC : row_pos(e + q * m)] = v[q];
+  }
+}
+
+// The stage of a prime radix above 19: a direct R-point DFT,
+// y_k = sum_q v_q W_R^(q k) with W_R^e = tw[e n / R].
+template <bool INV, int TC>
+__device__ __noinline__ void gen_stage_prime(float2* s, int nl, const FftPlan& P, int R, int L,
+                                             const float2* __restrict__ tst) {
+  const int N = P.n, m = L / R, per = N / R, nb = (TC ? TC : nl) * per;
   float2 v[NSR_MAX_PRIME_RADIX], y[NSR_MAX_PRIME_RADIX];
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     int l, bb;
-    if (line_fast) { l = b % nl; bb = b / nl; } else { l = b / per_line; bb = b % per_line; }
-    const int o = bb / m, j = bb - o * m;
-    float2* base = s + l * lstride + (o * L + j) * estride;
-    for (int q = 0; q < R; ++q) v[q] = base[q * m * estride];
-    if (INV)
-      for (int k = 1; k < R; ++k) v[k] = v[k] * conjc(__ldg(&P.tw[j * k * tstep]));
+    if constexpr (TC > 0) { l = b % TC; bb = b / TC; } else { l = b / per; bb = b - l * per; }
+    const int o = bb / m, j = bb - o * m, e = o * L + j;
+    float2* base = TC ? s + l : s + l * nsr_row_stride(N);
+    for (int q = 0; q < R; ++q) v[q] = base[TC ? (e + q * m) * TC : row_pos(e + q * m)];
+    if (INV && m > 1)
+      for (int k = 1; k < R; ++k) v[k] = v[k] * conjc(__ldg(tst + (k - 1) * m + j));
     for (int k = 0; k < R; ++k) {
       float2 acc = v[0];
-      int e = 0;
+      int f = 0;
       for (int q = 1; q < R; ++q) {
-        e += k;
-        if (e >= R) e -= R;
-        const float2 w = __ldg(&P.tw[e * rstep]);
+        f += k;
+        if (f >= R) f -= R;
+        const float2 w = __ldg(&P.tw[f * per]);
         acc = acc + v[q] * (INV ? conjc(w) : w);
       }
       y[k] = acc;
     }
-    if (!INV)
-      for (int k = 1; k < R; ++k) y[k] = y[k] * __ldg(&P.tw[j * k * tstep]);
-    for (int q = 0; q < R; ++q) base[q * m * estride] = y[q];
+    if (!INV && m > 1)
+      for (int k = 1; k < R; ++k) y[k] = y[k] * __ldg(tst + (k - 1) * m + j);
+    for (int q = 0; q < R; ++q) base[TC ? (e + q * m) * TC : row_pos(e + q * m)] = y[q];
   }
 }
 
-template <bool INV>
-__device__ void fft_lines(float2* s, int nl, int lstride, int estride, bool line_fast, const FftPlan& P) {
-  if (!INV) {
-    int L = P.n;
-    for (int st = 0; st < P.nst; ++st) {
-      const int R = P.radix[st];
-      switch (R) {
-        case 2: fft_stage<2, false>(s, nl, lstride, estride, line_fast, P, L); break;
-        case 3: fft_stage<3, false>(s, nl, lstride, estride, line_fast, P, L); break;
-        case 4: fft_stage<4, false>(s, nl, lstride, estride, line_fast, P, L); break;
-        case 8: fft_stage<8, false>(s, nl, lstride, estride, line_fast, P, L); break;
-        case 16: fft_stage<16, false>(s, nl, lstride, estride, line_fast, P, L); break;
-        default: fft_stage_prime<false>(s, nl, lstride, estride, line_fast, P, L, R); break;
-      }
-      __syncthreads();
-      L /= R;
-    }
+// Calls f(RadixTag<R>{}) for the radices with a register butterfly, g() for the others.
+template <int R>
+struct RadixTag { static constexpr int value = R; };
+template <typename F, typename G>
+__device__ __forceinline__ void gen_radix(int R, F f, G g) {
+  switch (R) {
+    case 2: f(RadixTag<2>{}); break;
+    case 3: f(RadixTag<3>{}); break;
+    case 4: f(RadixTag<4>{}); break;
+    case 5: f(RadixTag<5>{}); break;
+    case 7: f(RadixTag<7>{}); break;
+    case 8: f(RadixTag<8>{}); break;
+    case 11: f(RadixTag<11>{}); break;
+    case 13: f(RadixTag<13>{}); break;
+    case 16: f(RadixTag<16>{}); break;
+    case 17: f(RadixTag<17>{}); break;
+    case 19: f(RadixTag<19>{}); break;
+    default: g(); break;
+  }
+}
+
+// Length and twiddle table of stage `st`.
+struct StageAt {
+  int L;
+  const float2* tst;
+};
+__device__ __forceinline__ StageAt gen_stage_at(const FftPlan& P, int st) {
+  int L = P.n, off = 0;
+  for (int k = 0; k < st; ++k) {
+    const int m = L / P.radix[k];
+    if (m > 1) off += m * (P.radix[k] - 1);
+    L = m;
+  }
+  return StageAt{L, P.tws + off};
+}
+
+// Stages [first, last) in shared memory, forwards or (INV) backwards.
+template <bool INV, int TC>
+__device__ __forceinline__ void gen_stages(float2* s, int nl, const FftPlan& P, int first, int last) {
+  for (int k = first; k < last; ++k) {
+    const int st = INV ? last - 1 - (k - first) : k;
+    const StageAt a = gen_stage_at(P, st);
+    gen_radix(P.radix[st], [&](auto tag) { gen_stage<decltype(tag)::value, INV, TC>(s, nl, P.n, a.L, a.tst); },
+              [&] { gen_stage_prime<INV, TC>(s, nl, P, P.radix[st], a.L, a.tst); });
+    __syncthreads();
+  }
+}
+
+// Row transforms of any length between global memory (nl contiguous rows of N
+// points, flat index l N + c) and the padded rows, with the elementwise work at
+// the natural-order end fused into the first (forward) or last (inverse)
+// stage, as in ct_rows_forward_direct and ct_rows_inverse_direct.
+template <typename IN>
+__device__ __forceinline__ void gen_rows_forward(float2* s, int nl, const FftPlan& P, float2* __restrict__ g, IN in) {
+  const int N = P.n, rs = nsr_row_stride(N);
+  gen_radix(P.radix[0],
+            [&](auto tag) {
+              constexpr int R = decltype(tag)::value;
+              const int m = N / R;
+              for (int b = threadIdx.x; b < nl * m; b += blockDim.x) {
+                const int l = b / m, j = b - l * m;
+                float2 v[R];
+                in(RadixTag<R>{}, l * N + j, m, v);
+                small_dft<R, false>(v);
+                gen_twiddle<R, false>(v, P.tws, j, m);
+#pragma unroll
+                for (int q = 0; q < R; ++q) s[l * rs + row_pos(j + q * m)] = v[q];
+              }
+            },
+            [&] {
+              for (int l = 0; l < nl; ++l)
+                for (int c = threadIdx.x; c < N; c += blockDim.x) {
+                  float2 v[1];
+                  in(RadixTag<1>{}, l * N + c, 0, v);
+                  s[l * rs + row_pos(c)] = v[0];
+                }
+              __syncthreads();
+              gen_stage_prime<false, 0>(s, nl, P, P.radix[0], N, P.tws);
+            });
+  __syncthreads();
+  gen_stages<false, 0>(s, nl, P, 1, P.nst);
+  for (int l = 0; l < nl; ++l)
+    for (int c = threadIdx.x; c < N; c += blockDim.x) g[(long long)l * N + c] = s[l * rs + row_pos(c)];
+}
+
+template <typename OUT>
+__device__ __forceinline__ void gen_rows_inverse(float2* s, int nl, const FftPlan& P, const float2* g, OUT out) {
+  const int N = P.n, rs = nsr_row_stride(N);
+  for (int l = 0; l < nl; ++l)
+    for (int c = threadIdx.x; c < N; c += blockDim.x) s[l * rs + row_pos(c)] = g[(long long)l * N + c];
+  __syncthreads();
+  gen_stages<true, 0>(s, nl, P, 1, P.nst);
+  gen_radix(P.radix[0],
+            [&](auto tag) {
+              constexpr int R = decltype(tag)::value;
+              const int m = N / R;
+              for (int b = threadIdx.x; b < nl * m; b += blockDim.x) {
+                const int l = b / m, j = b - l * m;
+                float2 v[R];
+#pragma unroll
+                for (int q = 0; q < R; ++q) v[q] = s[l * rs + row_pos(j + q * m)];
+                gen_twiddle<R, true>(v, P.tws, j, m);
+                small_dft<R, true>(v);
+#pragma unroll
+                for (int q = 0; q < R; ++q) out(l * N + j + q * m, v[q]);
+              }
+            },
+            [&] {
+              gen_stage_prime<true, 0>(s, nl, P, P.radix[0], N, P.tws);
+              __syncthreads();
+              for (int l = 0; l < nl; ++l)
+                for (int c = threadIdx.x; c < N; c += blockDim.x) out(l * N + c, s[l * rs + row_pos(c)]);
+            });
+}
+
+// The column pass of any length, as ct_cols_direct: first forward and last
+// inverse stage between registers and global memory, the multiplier applied
+// between the last forward and the first inverse stage.
+template <int TC, typename MUL>
+__device__ __forceinline__ void gen_cols(float2* s, const FftPlan& P, float2* __restrict__ g, int nx, int ncol, MUL mul) {
+  const int N = P.n, last = P.nst - 1;
+  const float2 zero = make_float2(0.f, 0.f);
+  if (last > 0) {
+    gen_radix(P.radix[0],
+              [&](auto tag) {
+                constexpr int R = decltype(tag)::value;
+                const int m = N / R;
+                for (int b = threadIdx.x; b < TC * m; b += blockDim.x) {
+                  const int l = b % TC, j = b / TC;
+                  float2 v[R];
+#pragma unroll
+                  for (int q = 0; q < R; ++q) v[q] = l < ncol ? g[(long long)(j + q * m) * nx + l] : zero;
+                  small_dft<R, false>(v);
+                  gen_twiddle<R, false>(v, P.tws, j, m);
+#pragma unroll
+                  for (int q = 0; q < R; ++q) s[l + (j + q * m) * TC] = v[q];
+                }
+              },
+              [&] {
+                for (int k = threadIdx.x; k < N * TC; k += blockDim.x)
+                  s[k] = k % TC < ncol ? g[(long long)(k / TC) * nx + k % TC] : zero;
+                __syncthreads();
+                gen_stage_prime<false, TC>(s, TC, P, P.radix[0], N, P.tws);
+              });
+    __syncthreads();
+    gen_stages<false, TC>(s, TC, P, 1, last);
   } else {
-    // Lengths of the forward stages, replayed backwards.
-    int Ls[NSR_MAX_RADIX_STAGES];
-    int L = P.n;
-    for (int st = 0; st < P.nst; ++st) { Ls[st] = L; L /= P.radix[st]; }
-    for (int st = P.nst - 1; st >= 0; --st) {
-      const int R = P.radix[st];
-      switch (R) {
-        case 2: fft_stage<2, true>(s, nl, lstride, estride, line_fast, P, Ls[st]); break;
-        case 3: fft_stage<3, true>(s, nl, lstride, estride, line_fast, P, Ls[st]); break;
-        case 4: fft_stage<4, true>(s, nl, lstride, estride, line_fast, P, Ls[st]); break;
-        case 8: fft_stage<8, true>(s, nl, lstride, estride, line_fast, P, Ls[st]); break;
-        case 16: fft_stage<16, true>(s, nl, lstride, estride, line_fast, P, Ls[st]); break;
-        default: fft_stage_prime<true>(s, nl, lstride, estride, line_fast, P, Ls[st], R); break;
-      }
-      __syncthreads();
-    }
+    for (int k = threadIdx.x; k < N * TC; k += blockDim.x)
+      s[k] = k % TC < ncol ? g[(long long)(k / TC) * nx + k % TC] : zero;
+    __syncthreads();
+  }
+  gen_radix(P.radix[last],
+            [&](auto tag) {
+              constexpr int R = decltype(tag)::value;
+              for (int b = threadIdx.x; b < TC * (N / R); b += blockDim.x) {
+                const int l = b % TC, o = b / TC;
+                float2* base = s + l + o * R * TC;
+                float2 v[R];
+#pragma unroll
+                for (int q = 0; q < R; ++q) v[q] = base[q * TC];
+                small_dft<R, false>(v);
+#pragma unroll
+                for (int q = 0; q < R; ++q) v[q] = v[q] * mul(l, o * R + q);
+                small_dft<R, true>(v);
+#pragma unroll
+                for (int q = 0; q < R; ++q) base[q * TC] = v[q];
+              }
+            },
+            [&] {
+              const StageAt a = gen_stage_at(P, last);
+              gen_stage_prime<false, TC>(s, TC, P, P.radix[last], a.L, a.tst);
+              __syncthreads();
+              for (int k = threadIdx.x; k < N * TC; k += blockDim.x) s[k] = s[k] * mul(k % TC, k / TC);
+              __syncthreads();
+              gen_stage_prime<true, TC>(s, TC, P, P.radix[last], a.L, a.tst);
+            });
+  __syncthreads();
+  if (last > 0) {
+    gen_stages<true, TC>(s, TC, P, 1, last);
+    gen_radix(P.radix[0],
+              [&](auto tag) {
+                constexpr int R = decltype(tag)::value;
+                const int m = N / R;
+                for (int b = threadIdx.x; b < TC * m; b += blockDim.x) {
+                  const int l = b % TC, j = b / TC;
+                  float2 v[R];
+#pragma unroll
+                  for (int q = 0; q < R; ++q) v[q] = s[l + (j + q * m) * TC];
+                  gen_twiddle<R, true>(v, P.tws, j, m);
+                  small_dft<R, true>(v);
+                  if (l < ncol) {
+#pragma unroll
+                    for (int q = 0; q < R; ++q) g[(long long)(j + q * m) * nx + l] = v[q];
+                  }
+                }
+              },
+              [&] {
+                gen_stage_prime<true, TC>(s, TC, P, P.radix[0], N, P.tws);
+                __syncthreads();
+                for (int k = threadIdx.x; k < N * TC; k += blockDim.x)
+                  if (k % TC < ncol) g[(long long)(k / TC) * nx + k % TC] = s[k];
+              });
+  } else {
+    for (int k = threadIdx.x; k < N * TC; k += blockDim.x)
+      if (k % TC < ncol) g[(long long)(k / TC) * nx + k % TC] = s[k];
   }
 }
 
@@ -612,19 +832,16 @@ __device__ __forceinline__ void ct_fft(float2* s, int nl, const float2* __restri
   else ct_inverse<N, RL.nst - 1, LF, LS, ES, PAD>(s, nl, tws);
 }
 
-// Row layout in shared memory: the specialised sizes insert one pad element
-// after every 16 (element k of a row at k + k/16), which keeps every row FFT
-// stage free of shared-memory bank conflicts.
-__host__ __device__ inline bool nsr_row_padded(int n) {
+// Line lengths with compile-time specialised transforms; the others run the
+// run-time stages.
+__host__ __device__ inline bool nsr_specialised(int n) {
   switch (n) {
     case 256: case 384: case 512: case 768: case 1024: case 1536: case 2048: return true;
     default: return false;
   }
 }
-__host__ __device__ inline int nsr_row_stride(int n) { return nsr_row_padded(n) ? n + (n >> 4) : n; }
 
-// Rows: nl lines of length n, row stride nsr_row_stride(n) (padded for the
-// specialised sizes, plain otherwise).
+// Rows: nl lines of length n in the padded row layout.
 template <bool INV>
 __device__ void fft_rows(float2* s, int nl, const FftPlan& P) {
   switch (P.n) {
@@ -635,7 +852,7 @@ __device__ void fft_rows(float2* s, int nl, const FftPlan& P) {
     case 1024: ct_fft<1024, INV, false, 1024 + 64, 1, true>(s, nl, P.tws); return;
     case 1536: ct_fft<1536, INV, false, 1536 + 96, 1, true>(s, nl, P.tws); return;
     case 2048: ct_fft<2048, INV, false, 2048 + 128, 1, true>(s, nl, P.tws); return;
-    default: fft_lines<INV>(s, nl, P.n, 1, false, P); return;
+    default: gen_stages<INV, 0>(s, nl, P, 0, P.nst); return;
   }
 }
 
@@ -650,7 +867,7 @@ __device__ void fft_cols(float2* s, const FftPlan& P) {
     case 1024: ct_fft<1024, INV, true, 1, TC, false>(s, TC, P.tws); return;
     case 1536: ct_fft<1536, INV, true, 1, TC, false>(s, TC, P.tws); return;
     case 2048: ct_fft<2048, INV, true, 1, TC, false>(s, TC, P.tws); return;
-    default: fft_lines<INV>(s, TC, 1, TC, true, P); return;
+    default: gen_stages<INV, TC>(s, TC, P, 0, P.nst); return;
   }
 }
 
@@ -809,9 +1026,6 @@ __device__ __forceinline__ bool fft_cols_direct(float2* s, const FftPlan& P, flo
 //    memory, and `out(k, v)` receives each output of stage 0 (flat index k)
 //    and stores it.
 // Two shared-memory round trips fewer than load, transform, store.
-template <int R>
-struct RadixTag { static constexpr int value = R; };
-
 template <int N, typename IN>
 __device__ __forceinline__ void ct_rows_forward_direct(float2* s, int nl, const float2* __restrict__ tws,
                                                        float2* __restrict__ g, IN in) {
@@ -925,6 +1139,25 @@ __device__ __forceinline__ bool fft_rows_inverse_direct(float2* s, int nl, const
     case 2048: ct_rows_inverse_direct<2048>(s, nl, P.tws, g, out); return true;
     default: return false;
   }
+}
+
+// Row and column passes of any plan: GEN selects the run-time stages (sizes
+// nsr_specialised does not name; their kernels get more registers).
+template <bool GEN, typename IN>
+__device__ __forceinline__ void rows_forward(float2* s, int nl, const FftPlan& P, float2* __restrict__ g, IN in) {
+  if constexpr (GEN) gen_rows_forward(s, nl, P, g, in);
+  else fft_rows_forward_direct(s, nl, P, g, in);
+}
+template <bool GEN, typename OUT>
+__device__ __forceinline__ void rows_inverse(float2* s, int nl, const FftPlan& P, const float2* g, OUT out) {
+  if constexpr (GEN) gen_rows_inverse(s, nl, P, g, out);
+  else fft_rows_inverse_direct(s, nl, P, g, out);
+}
+template <bool GEN, int TC, typename MUL>
+__device__ __forceinline__ void cols_multiply(float2* s, const FftPlan& P, float2* __restrict__ g, int nx, int ncol,
+                                              MUL mul) {
+  if constexpr (GEN) gen_cols<TC>(s, P, g, nx, ncol, mul);
+  else fft_cols_direct<TC>(s, P, g, nx, ncol, mul);
 }
 
 // Column pass with the fused middle stage for the specialised sizes; other

@@ -16,8 +16,6 @@
 
 #include <string.h>
 
-__constant__ double c_dense_a[4] = {1225.0 / 1024.0, -245.0 / 3072.0, 49.0 / 5120.0, -5.0 / 7168.0};
-
 struct DenseCoef {
   // planes [H][W]
   const double* ax;
@@ -398,73 +396,60 @@ extern "C" int nsr_dense_grad(const NsrDenseGrid* grid, const double* coef, doub
 // The transforms are the solver's row and column FFTs (sizes 8..2048 whose
 // prime factors are at most 61, e.g. the 1056 x 1216 padding of the reference).
 // ---------------------------------------------------------------------------
-__global__ void k_dense_symbol(int n, FftPlan plan, float* d2) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int f = nsr_digit_reverse(k, n, plan.radix, plan.nst);
-    const double q = 2.0 * NSR_PI * f / n;
-    double s = 0.0;
-    for (int j = 0; j < 4; ++j) s += c_dense_a[j] * sin((j + 0.5) * q);
-    d2[k] = (float)(4.0 * s * s);   // |D|^2 dx^2
-  }
+// Eleven 1056 x 1216 fields (radices 11 3 2 16 and 19 4 16): 1,365 us with the
+// prime radices as loops over local arrays and unpadded rows, 490 us with
+// register butterflies and the ends of the transforms fused.
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_dense_rows_fwd(int nz, int nx, PrecTables t,
+                                                                     const float2* __restrict__ x,
+                                                                     float2* __restrict__ w, int rows) {
+  extern __shared__ float2 sm[];
+  const int z0 = blockIdx.x * rows;
+  const long long off = blockIdx.y * (long long)nz * nx + (long long)z0 * nx;
+  const float2* __restrict__ xs = x + off;
+  rows_forward<GEN>(sm, min(rows, nz - z0), t.px, w + off, [&](auto tag, int k0, int step, float2* v) {
+#pragma unroll
+    for (int q = 0; q < decltype(tag)::value; ++q) v[q] = xs[k0 + q * step];
+  });
 }
 
-template <int TC>
-__global__ void __launch_bounds__(512) k_dense_cols(int nz, int nx, PrecTables t, const float* __restrict__ d2z,
-                                                    const float* __restrict__ d2x, float2* __restrict__ w,
-                                                    float inv_k0dx2, float shift, int adjoint) {
+template <int TC, bool GEN>
+__global__ void __launch_bounds__(GEN ? 256 : 512, 2) k_dense_cols(int nz, int nx, PrecTables t,
+                                                                   const float* __restrict__ d2z,
+                                                                   const float* __restrict__ d2x,
+                                                                   float2* __restrict__ w, float inv_k0dx2,
+                                                                   float shift, int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)nz * nx;
-  float2* ws = w + blockIdx.y * n;
   const int c0 = blockIdx.x * TC;
   const int ncol = min(TC, nx - c0);
-  for (int k = threadIdx.x; k < nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    sm[k] = c < ncol ? ws[(long long)z * nx + c0 + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_cols<false, TC>(sm, t.pz);
   const float inv_n = 1.0f / (float)n;
-  for (int k = threadIdx.x; k < nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    if (c < ncol) {
-      const float re = 1.0f - (d2z[z] + d2x[c0 + c]) * inv_k0dx2;
-      float2 mul = divc(make_float2(inv_n, 0.f), make_float2(re, -shift));
-      if (adjoint) mul = conjc(mul);
-      sm[k] = sm[k] * mul;
-    }
-  }
-  __syncthreads();
-  fft_cols<true, TC>(sm, t.pz);
-  for (int k = threadIdx.x; k < nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    if (c < ncol) ws[(long long)z * nx + c0 + c] = sm[k];
-  }
+  cols_multiply<GEN, TC>(sm, t.pz, w + blockIdx.y * n + c0, nx, ncol, [&](int c, int z) -> float2 {
+    if (c >= ncol) return make_float2(0.f, 0.f);
+    const float re = 1.0f - (d2z[z] + d2x[c0 + c]) * inv_k0dx2;
+    const float2 mul = divc(make_float2(inv_n, 0.f), make_float2(re, -shift));
+    return adjoint ? conjc(mul) : mul;
+  });
 }
 
-__global__ void k_dense_rows(int nz, int nx, int pz, int px, int h, int w, PrecTables t,
-                             const float2* __restrict__ x, float2* __restrict__ y, int rows, int inverse) {
+// Inverse rows, masked to the native region: a tile of rows outside it is zero
+// without a transform.
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_dense_rows_inv(DenseGeo g, PrecTables t,
+                                                                     const float2* __restrict__ w,
+                                                                     float2* __restrict__ y, int rows) {
   extern __shared__ float2 sm[];
-  const long long n = (long long)nz * nx;
-  const int z0 = blockIdx.x * rows;
-  const int nr = min(rows, nz - z0);
-  const float2* xs = x + blockIdx.y * n + (long long)z0 * nx;
-  const int rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
-  for (int k = threadIdx.x; k < nr * nx; k += blockDim.x) {
-    const int l = k / nx, c = k - l * nx;
-    sm[l * rs + (pad ? c + (c >> 4) : c)] = xs[k];
+  const int nz = g.H, nx = g.W, z0 = blockIdx.x * rows, nr = min(rows, nz - z0);
+  const long long off = blockIdx.y * (long long)nz * nx + (long long)z0 * nx;
+  float2* __restrict__ ys = y + off;
+  if (z0 >= g.pz + g.h || z0 + nr <= g.pz) {
+    for (int k = threadIdx.x; k < nr * nx; k += blockDim.x) ys[k] = make_float2(0.f, 0.f);
+    return;
   }
-  __syncthreads();
-  if (inverse) fft_rows<true>(sm, nr, t.px);
-  else fft_rows<false>(sm, nr, t.px);
-  __syncthreads();
-  float2* ys = y + blockIdx.y * n + (long long)z0 * nx;
-  for (int k = threadIdx.x; k < nr * nx; k += blockDim.x) {
-    const int l = k / nx, c = k - l * nx;
-    const int i = z0 + l;
-    const bool in = !inverse || (i >= pz && i < pz + h && c >= px && c < px + w);
-    ys[k] = in ? sm[l * rs + (pad ? c + (c >> 4) : c)] : make_float2(0.f, 0.f);
-  }
+  rows_inverse<GEN>(sm, nr, t.px, w + off, [&](int k, float2 v) {
+    const int l = k / nx;
+    ys[k] = dense_inside(g, z0 + l, k - l * nx) ? v : make_float2(0.f, 0.f);
+  });
 }
 
 static NsrGrid dense_fft_grid(const NsrDenseGrid* g) {
@@ -501,31 +486,30 @@ extern "C" int nsr_dense_precondition(const NsrDenseGrid* grid, double k0dx2, do
   NsrGrid q = dense_fft_grid(grid);
   char* ws = (char*)workspace;
   PrecTables t;
-  int err = nsr_prec_setup(&q, &t, ws, st);
-  if (err) return err;
   float* d2x = (float*)(ws + nsr_align(nsr_prec_table_bytes(&q)));
   float* d2z = d2x + grid->W;
+  int err = nsr_prec_setup(&q, &t, ws, st, d2x, d2z);
+  if (err) return err;
   float2* w = (float2*)(ws + nsr_align(nsr_prec_table_bytes(&q)) + nsr_align(sizeof(float) * (grid->H + grid->W)));
-  k_dense_symbol<<<(grid->W + 255) / 256, 256, 0, st>>>(grid->W, t.px, d2x);
-  k_dense_symbol<<<(grid->H + 255) / 256, 256, 0, st>>>(grid->H, t.pz, d2z);
   const int rows = nsr_rows_per_cta(&q);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->W);
   const dim3 gr((grid->H + rows - 1) / rows, n_fields);
-  k_dense_rows<<<gr, 256, row_smem, st>>>(grid->H, grid->W, grid->pz, grid->px, grid->h, grid->w, t,
-                                          (const float2*)x, w, rows, 0);
+  const bool gx = !nsr_specialised(grid->W), gz = !nsr_specialised(grid->H);
+  DenseGeo g;
+  g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
+  g.scal = make_double2(0.0, 0.0);
+  const auto fwd = gx ? k_dense_rows_fwd<true> : k_dense_rows_fwd<false>;
+  const auto inv = gx ? k_dense_rows_inv<true> : k_dense_rows_inv<false>;
+  fwd<<<gr, 256, row_smem, st>>>(grid->H, grid->W, t, (const float2*)x, w, rows);
   const int tc = nsr_cols_tc(&q);
   const dim3 gc((grid->W + tc - 1) / tc, n_fields);
   const size_t csm = nsr_cols_smem(&q);
-  const float inv = (float)(1.0 / k0dx2);
-  if (tc == 16) {
-    cudaFuncSetAttribute(k_dense_cols<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_dense_cols<16><<<gc, 512, csm, st>>>(grid->H, grid->W, t, d2z, d2x, w, inv, (float)shift, adjoint);
-  } else {
-    cudaFuncSetAttribute(k_dense_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_dense_cols<8><<<gc, 512, csm, st>>>(grid->H, grid->W, t, d2z, d2x, w, inv, (float)shift, adjoint);
-  }
-  k_dense_rows<<<gr, 256, row_smem, st>>>(grid->H, grid->W, grid->pz, grid->px, grid->h, grid->w, t, w,
-                                          (float2*)y, rows, 1);
+  const auto cols = tc == 16 ? (gz ? k_dense_cols<16, true> : k_dense_cols<16, false>)
+                             : (gz ? k_dense_cols<8, true> : k_dense_cols<8, false>);
+  cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+  cols<<<gc, nsr_cols_threads(gz), csm, st>>>(grid->H, grid->W, t, d2z, d2x, w, (float)(1.0 / k0dx2), (float)shift,
+                                              adjoint);
+  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }

@@ -189,60 +189,41 @@ __device__ __forceinline__ float2 learned_symbol(const LearnedSpec& L, float s2z
   return make_float2(er * dr + ei * di, ei * dr - er * di);
 }
 
-// Column pass with an arbitrary multiplier: `mul(c, z)` is the factor of tile
-// column c at digit-reversed z position, including the 1/n of the transform
-// pair; columns at or beyond the grid edge are never multiplied.
-template <int TC, typename MUL>
+// Column pass of the columns [c0, c0 + TC) of a field with a multiplier:
+// `mul(c, z)` is the factor of tile column c at digit-reversed z position,
+// including the 1/n of the transform pair; columns at or beyond the grid edge
+// are never multiplied.  STAGED (specialised sizes only, a launch shape the
+// autotuner can choose): load, every stage in shared memory, store.
+template <int TC, bool GEN, bool STAGED, typename MUL>
 __device__ __forceinline__ void cols_pass_with(float2* sm, const Geo& g, const PrecTables& tab,
                                                float2* __restrict__ ws, int c0, MUL mul) {
   const int ncol = min(TC, g.nx - c0);
-  for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    sm[k] = c < ncol ? ws[(long long)z * g.nx + c0 + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
   auto m = [&](int c, int z) -> float2 { return c < ncol ? mul(c, z) : make_float2(0.f, 0.f); };
-  if (!fft_cols_fused<TC>(sm, tab.pz, m)) {
-    // Sizes without a specialised transform: separate passes.
-    fft_cols<false, TC>(sm, tab.pz);
+  if constexpr (STAGED) {
     for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
       const int z = k / TC, c = k - z * TC;
-      sm[k] = sm[k] * m(c, z);
+      sm[k] = c < ncol ? ws[(long long)z * g.nx + c0 + c] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    fft_cols<true, TC>(sm, tab.pz);
-  }
-  for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    if (c < ncol) ws[(long long)z * g.nx + c0 + c] = sm[k];
-  }
-}
-
-// The same pass with the first forward and the last inverse stage fused into
-// the global load and store (the specialised sizes of nsr_row_padded only);
-// STAGED selects cols_pass_with instead (every size: load, every stage in
-// shared memory, store).
-template <int TC, bool STAGED, typename MUL>
-__device__ __forceinline__ void cols_pass_direct(float2* sm, const Geo& g, const PrecTables& tab,
-                                                 float2* __restrict__ ws, int c0, MUL mul) {
-  if constexpr (STAGED) {
-    cols_pass_with<TC>(sm, g, tab, ws, c0, mul);
+    fft_cols_fused<TC>(sm, tab.pz, m);
+    for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
+      const int z = k / TC, c = k - z * TC;
+      if (c < ncol) ws[(long long)z * g.nx + c0 + c] = sm[k];
+    }
   } else {
-    const int ncol = min(TC, g.nx - c0);
-    auto m = [&](int c, int z) -> float2 { return c < ncol ? mul(c, z) : make_float2(0.f, 0.f); };
-    fft_cols_direct<TC>(sm, tab.pz, ws + c0, g.nx, ncol, m);
+    cols_multiply<GEN, TC>(sm, tab.pz, ws + c0, g.nx, ncol, m);
   }
 }
 
 // Fixed shifted-Laplace multiplier 1 / (n (-4 (s2z + s2x) + (k0 h)^2 (1 + i shift))).
-template <int TC>
+template <int TC, bool GEN>
 __device__ __forceinline__ void cols_pass_fixed(float2* sm, const Geo& g, const PrecTables& tab,
                                                 float2* __restrict__ ws, double freq, double shift, int adjoint,
                                                 int c0) {
   const SysScalars s = sys_scalars(g, freq);
   const float inv_n = 1.0f / (float)((long long)g.nz * g.nx);
   const float2 shiftc = make_float2((float)s.kh2, (float)(s.kh2 * shift));
-  cols_pass_with<TC>(sm, g, tab, ws, c0, [&](int c, int z) -> float2 {
+  cols_pass_with<TC, GEN, false>(sm, g, tab, ws, c0, [&](int c, int z) -> float2 {
     const float sym = -4.0f * (tab.s2z[z] + tab.s2x[c0 + c]);
     const float2 mul = divc(make_float2(inv_n, 0.f), make_float2(sym + shiftc.x, shiftc.y));
     return adjoint ? conjc(mul) : mul;
@@ -259,49 +240,22 @@ __device__ __forceinline__ float2 learned_plane_value(const LearnedSpec& L, cons
   return inv_n * learned_symbol(L, tab.s2z[z], tab.s2x[x], kh2, h2);
 }
 
-// Column pass of either preconditioner, chosen at run time: the learned
-// multiplier evaluated on the fly from `lp` (non-null), else the fixed one.
-template <int TC>
-__device__ __forceinline__ void cols_pass(float2* sm, const Geo& g, const PrecTables& tab, float2* __restrict__ ws,
-                                          double freq, double shift, int adjoint, int c0,
-                                          const float* __restrict__ lp = nullptr) {
-  if (!lp) {
-    cols_pass_fixed<TC>(sm, g, tab, ws, freq, shift, adjoint, c0);
-    return;
-  }
+// Column pass with the learned multiplier evaluated on the fly.
+template <int TC, bool GEN>
+__device__ __forceinline__ void cols_pass_learned(float2* sm, const Geo& g, const PrecTables& tab,
+                                                  float2* __restrict__ ws, double freq, int adjoint, int c0,
+                                                  const float* __restrict__ lp) {
   // The spectral parameters go through shared memory so that the fused radix
   // stage keeps its registers for the butterfly.
   __shared__ LearnedSpec Ls;
   if (threadIdx.x == 0) Ls = load_learned_spec(lp);
   __syncthreads();
   const float kh2 = (float)sys_scalars(g, freq).kh2;
-  cols_pass_with<TC>(sm, g, tab, ws, c0, [&](int c, int z) -> float2 {
+  cols_pass_with<TC, GEN, false>(sm, g, tab, ws, c0, [&](int c, int z) -> float2 {
     const float2 mul = learned_plane_value(Ls, g, tab, kh2, z, c0 + c);
     return adjoint ? conjc(mul) : mul;
   });
 }
-
-// Rows z0-1 .. z0+nb of w (zero outside the grid) into the padded row layout
-// of shared memory, inverse row FFT.  Row rr of the band is sm[(rr+1)*rs].
-__device__ __forceinline__ void band_inverse_rows(float2* sm, const Geo& g, const PrecTables& tab,
-                                                  const float2* __restrict__ w, int z0, int nb) {
-  const int nx = g.nx;
-  const int rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
-  const int nl = nb + 2;
-  for (int rr = 0; rr < nl; ++rr) {
-    const int z = z0 - 1 + rr;
-    const bool in = z >= 0 && z < g.nz;
-#pragma unroll 4
-    for (int j = threadIdx.x; j < nx; j += blockDim.x)
-      sm[rr * rs + (pad ? j + (j >> 4) : j)] = in ? w[(long long)z * nx + j] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_rows<true>(sm, nl, tab.px);
-}
-
-// Stores `val` for element (l, c) of a row tile in the padded row layout.
-__device__ __forceinline__ int row_slot(int l, int c, int rs, bool pad) { return l * rs + (pad ? c + (c >> 4) : c); }
 
 // Diagonal gains of the learned preconditioner.  Plane 0 of a gain pair is the
 // inner gain (applied before the FFTs), plane 1 the outer one (after them);
@@ -331,24 +285,4 @@ __device__ __forceinline__ float2 gain_mul(const float2* plane, long long idx, b
   float2 gv = __ldg(&plane[idx]);
   if (cj) gv.y = -gv.y;
   return gv * v;
-}
-
-// After band_inverse_rows: multiply band rows z0-1 .. z0+nb (those inside the
-// grid) by the post gain.
-__device__ __forceinline__ void band_post_gain(float2* sm, const Geo& g, const float2* __restrict__ post, bool cj,
-                                               int z0, int nb) {
-  if (!post) return;
-  const int nx = g.nx;
-  const int rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
-  __syncthreads();
-  for (int rr = 0; rr < nb + 2; ++rr) {
-    const int z = z0 - 1 + rr;
-    if (z < 0 || z >= g.nz) continue;
-    for (int j = threadIdx.x; j < nx; j += blockDim.x) {
-      float2& v = sm[rr * rs + (pad ? j + (j >> 4) : j)];
-      v = gain_mul(post, (long long)z * nx + j, cj, v);
-    }
-  }
-  __syncthreads();
 }

@@ -128,7 +128,8 @@ __device__ bool g_reduce(const GArgs& A, int slot, const double* vals, int nv, d
 // ---------------------------------------------------------------------------
 // fwd: v_j from r (j = 0) or w (j > 0), stored in V and transformed by rows.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gk_fwd(GArgs A, int j) {
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -138,40 +139,40 @@ __global__ void __launch_bounds__(256) gk_fwd(GArgs A, int j) {
   const int z0 = blockIdx.x * A.rows;
   const int nr = min(A.rows, g.nz - z0);
   const long long off = (long long)z0 * g.nx;
-  const float2* src = (j == 0 ? A.r : A.w) + slot * n + off;
+  const float2* __restrict__ src = (j == 0 ? A.r : A.w) + slot * n + off;
   const float scale = (float)(1.0 / (j == 0 ? S.beta : S.hlast));   // both real and positive
-  float2* vj = A.V + ((long long)slot * (A.m + 1) + j) * n + off;
-  const int nx = g.nx, rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
+  float2* __restrict__ vj = A.V + ((long long)slot * (A.m + 1) + j) * n + off;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) {
-      const float2 v = scale * src[l * nx + c];
-      vj[l * nx + c] = v;
-      sm[row_slot(l, c, rs, pad)] = G.pre ? gain_mul(G.pre, off + l * nx + c, G.conj, v) : v;
+  rows_forward<GEN>(sm, nr, A.tab.px, A.W + slot * n + off, [&](auto tag, int k0, int step, float2* v) {
+    constexpr int R = decltype(tag)::value;
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = scale * src[k0 + q * step];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      vj[k0 + q * step] = v[q];
+      if (G.pre) v[q] = gain_mul(G.pre, off + k0 + q * step, G.conj, v[q]);
     }
-  __syncthreads();
-  fft_rows<false>(sm, nr, A.tab.px);
-  float2* Wp = A.W + slot * n + off;
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) Wp[l * nx + c] = sm[row_slot(l, c, rs, pad)];
+  });
 }
 
 // cols for slots active at step j (j < 0: slots that run a cycle-end update)
-template <int TC>
-__global__ void __launch_bounds__(512) gk_cols(GArgs A, int j) {
+template <int TC, bool GEN>
+__global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
   const bool on = j >= 0 ? g_active(S, j) : (S.sys >= 0 && !S.done && S.used > 0);
   if (!on) return;
   const long long n = (long long)A.g.nz * A.g.nx;
-  cols_pass<TC>(sm, A.g, A.tab, A.W + slot * n, S.freq, A.shift, A.adjoint, blockIdx.x * TC, A.lp);
+  float2* w = A.W + slot * n;
+  if (A.lp) cols_pass_learned<TC, GEN>(sm, A.g, A.tab, w, S.freq, A.adjoint, blockIdx.x * TC, A.lp);
+  else cols_pass_fixed<TC, GEN>(sm, A.g, A.tab, w, S.freq, A.shift, A.adjoint, blockIdx.x * TC);
 }
 
 // rinv: inverse row FFT of W in place, times the outer gain (W becomes M^-1 v_j,
 // or M^-1 u at the end of a cycle when j < 0).
-__global__ void __launch_bounds__(256, 4) gk_rinv(GArgs A, int j) {
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -182,20 +183,11 @@ __global__ void __launch_bounds__(256, 4) gk_rinv(GArgs A, int j) {
   const int z0 = blockIdx.x * A.rows;
   const int nr = min(A.rows, g.nz - z0);
   const long long off = (long long)z0 * g.nx;
-  float2* __restrict__ Wp = A.W + slot * n + off;
-  const int nx = g.nx, rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) sm[row_slot(l, c, rs, pad)] = Wp[l * nx + c];
-  __syncthreads();
-  fft_rows<true>(sm, nr, A.tab.px);
-  __syncthreads();
+  float2* Wp = A.W + slot * n + off;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) {
-      const float2 v = sm[row_slot(l, c, rs, pad)];
-      Wp[l * nx + c] = G.post ? gain_mul(G.post, off + l * nx + c, G.conj, v) : v;
-    }
+  rows_inverse<GEN>(sm, nr, A.tab.px, Wp, [&](int k, float2 v) {
+    Wp[k] = G.post ? gain_mul(G.post, off + k, G.conj, v) : v;
+  });
 }
 
 // inv: w = A z with z = M^-1 v_j in W.  One thread per column of a
@@ -377,7 +369,8 @@ __global__ void gk_solve(GArgs A) {
 }
 
 // u = V y, forward row FFT into W.
-__global__ void __launch_bounds__(256) gk_comb(GArgs A) {
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_comb(GArgs A) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -391,20 +384,23 @@ __global__ void __launch_bounds__(256) gk_comb(GArgs A) {
   const int z0 = blockIdx.x * A.rows;
   const int nr = min(A.rows, g.nz - z0);
   const long long off = (long long)z0 * g.nx;
-  const int nx = g.nx, rs = nsr_row_stride(nx);
-  const bool pad = nsr_row_padded(nx);
+  const float2* __restrict__ V = A.V + (long long)slot * (m + 1) * n + off;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) {
-      float2 acc = make_float2(0.f, 0.f);
-      for (int i = 0; i < u; ++i) acc = acc + yc[i] * A.V[((long long)slot * (m + 1) + i) * n + off + l * nx + c];
-      sm[row_slot(l, c, rs, pad)] = G.pre ? gain_mul(G.pre, off + l * nx + c, G.conj, acc) : acc;
+  rows_forward<GEN>(sm, nr, A.tab.px, A.W + slot * n + off, [&](auto tag, int k0, int step, float2* v) {
+    constexpr int R = decltype(tag)::value;
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = make_float2(0.f, 0.f);
+    for (int i = 0; i < u; ++i) {
+      const float2 c = yc[i];
+      const float2* __restrict__ Vi = V + i * n;
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = v[q] + c * Vi[k0 + q * step];
     }
-  __syncthreads();
-  fft_rows<false>(sm, nr, A.tab.px);
-  float2* Wp = A.W + slot * n + off;
-  for (int l = 0; l < nr; ++l)
-    for (int c = threadIdx.x; c < nx; c += blockDim.x) Wp[l * nx + c] = sm[row_slot(l, c, rs, pad)];
+    if (G.pre) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = gain_mul(G.pre, off + k0 + q * step, G.conj, v[q]);
+    }
+  });
 }
 
 // FP64 true residual.  init = 1: x = x0 (or 0); init = 0: x += M^-1 V y.
@@ -697,15 +693,19 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
       A.gain_index = params->learned->gain_index;
     }
 
-    const int rs = nsr_row_stride(grid->nx);
-    const size_t fwd_smem = sizeof(float2) * A.rows * rs;
+    const size_t fwd_smem = sizeof(float2) * A.rows * nsr_row_stride(grid->nx);
     const size_t col_smem = nsr_cols_smem(grid);
     const int nb_st = ((grid->nz + NSR_GST_TZ - 1) / NSR_GST_TZ) * ((grid->nx + NSR_GST_TX - 1) / NSR_GST_TX);
-    NSR_TRY(cudaFuncSetAttribute(gk_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
-    NSR_TRY(cudaFuncSetAttribute(gk_comb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
-    NSR_TRY(cudaFuncSetAttribute(gk_cols<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
-    NSR_TRY(cudaFuncSetAttribute(gk_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
-    NSR_TRY(cudaFuncSetAttribute(gk_rinv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
+    const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
+    const auto fwd_fn = gx ? gk_fwd<true> : gk_fwd<false>;
+    const auto rinv_fn = gx ? gk_rinv<true> : gk_rinv<false>;
+    const auto comb_fn = gx ? gk_comb<true> : gk_comb<false>;
+    const auto cols_fn = A.tc == 16 ? (gz ? gk_cols<16, true> : gk_cols<16, false>)
+                                    : (gz ? gk_cols<8, true> : gk_cols<8, false>);
+    NSR_TRY(cudaFuncSetAttribute((const void*)fwd_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
+    NSR_TRY(cudaFuncSetAttribute((const void*)comb_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
+    NSR_TRY(cudaFuncSetAttribute((const void*)cols_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
+    NSR_TRY(cudaFuncSetAttribute((const void*)rinv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
 
     const dim3 g_rows((grid->nz + A.rows - 1) / A.rows, n_slots);
     const dim3 g_col((grid->nx + A.tc - 1) / A.tc, n_slots);
@@ -713,8 +713,7 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     const dim3 g_st(nb_st, n_slots);
     const dim3 g_dot(L.nb_dot, n_slots);
     auto cols = [&](int j) {
-      if (A.tc == 16) gk_cols<16><<<g_col, 512, col_smem, st>>>(A, j);
-      else gk_cols<8><<<g_col, 512, col_smem, st>>>(A, j);
+      cols_fn<<<g_col, nsr_cols_threads(gz), col_smem, st>>>(A, j);
     };
     auto res = [&](int init) {
       if (A.adjoint) gk_res<true><<<g_band, 256, 0, st>>>(A, init);
@@ -724,9 +723,9 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     // One restart cycle.
     NSR_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     for (int j = 0; j < m; ++j) {
-      gk_fwd<<<g_rows, 256, fwd_smem, st>>>(A, j);
+      fwd_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
       cols(j);
-      gk_rinv<<<g_rows, 256, fwd_smem, st>>>(A, j);
+      rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
       if (A.adjoint) gk_inv<true><<<g_st, 256, 0, st>>>(A, j);
       else gk_inv<false><<<g_st, 256, 0, st>>>(A, j);
       gk_dot<<<g_dot, 256, 0, st>>>(A, j);
@@ -735,9 +734,9 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
       gk_axpy<<<g_dot, 256, 0, st>>>(A, j, 2);
     }
     gk_solve<<<(n_slots + 127) / 128, 128, 0, st>>>(A);
-    gk_comb<<<g_rows, 256, fwd_smem, st>>>(A);
+    comb_fn<<<g_rows, 256, fwd_smem, st>>>(A);
     cols(-1);
-    gk_rinv<<<g_rows, 256, fwd_smem, st>>>(A, -1);
+    rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, -1);
     res(0);
     gk_count<<<1, 256, 0, st>>>(A, remaining);
     ce = cudaStreamEndCapture(st, &graph);

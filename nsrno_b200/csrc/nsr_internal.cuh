@@ -13,10 +13,16 @@ struct PrecTables {
 inline size_t nsr_align(size_t b) { return (b + 255) & ~(size_t)255; }
 
 int nsr_check_grid(const NsrGrid* g, bool need_fft);
-int nsr_prec_setup(const NsrGrid* g, PrecTables* t, void* table_mem, cudaStream_t st);
+// Tables of a grid, one launch; d2x, d2z (optional): the dense path's symbols.
+int nsr_prec_setup(const NsrGrid* g, PrecTables* t, void* table_mem, cudaStream_t st, float* d2x = nullptr,
+                   float* d2z = nullptr);
 size_t nsr_prec_table_bytes(const NsrGrid* g);
 int nsr_cols_tc(const NsrGrid* g);
 size_t nsr_cols_smem(const NsrGrid* g);
 int nsr_rows_per_cta(const NsrGrid* g);
+
+// Threads of a column-pass CTA: the run-time transforms take half as many
+// (their butterflies hold up to 19 points in registers).
+inline int nsr_cols_threads(bool gen) { return gen ? 256 : 512; }
 
 int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st);

@@ -271,65 +271,52 @@ int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int lp_gidx(const int* gain_index, int s) { return gain_index ? gain_index[s] : s; }
 
-__global__ void __launch_bounds__(256) k_lp_rows_fwd(Geo g, PrecTables t, const float2* __restrict__ x,
-                                                     float2* __restrict__ w, int rows, const float2* gains,
-                                                     const int* gain_index, int adjoint) {
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_lp_rows_fwd(Geo g, PrecTables t, const float2* __restrict__ x,
+                                                                  float2* __restrict__ w, int rows,
+                                                                  const float2* gains, const int* gain_index,
+                                                                  int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
-  const int nr = min(rows, g.nz - z0);
   const long long off = (long long)z0 * g.nx;
-  const float2* xs = x + blockIdx.y * n + off;
+  const float2* __restrict__ xs = x + blockIdx.y * n + off;
   const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y) : 0, n, adjoint);
-  const int rs = nsr_row_stride(g.nx);
-  const bool pad = nsr_row_padded(g.nx);
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    const float2 v = xs[k];
-    sm[l * rs + (pad ? c + (c >> 4) : c)] = G.pre ? gain_mul(G.pre, off + k, G.conj, v) : v;
-  }
-  __syncthreads();
-  fft_rows<false>(sm, nr, t.px);
-  float2* ws = w + blockIdx.y * n + off;
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    ws[k] = sm[l * rs + (pad ? c + (c >> 4) : c)];
-  }
+  rows_forward<GEN>(sm, min(rows, g.nz - z0), t.px, w + blockIdx.y * n + off,
+                    [&](auto tag, int k0, int step, float2* v) {
+                      constexpr int R = decltype(tag)::value;
+#pragma unroll
+                      for (int q = 0; q < R; ++q) v[q] = xs[k0 + q * step];
+                      if (G.pre) {
+#pragma unroll
+                        for (int q = 0; q < R; ++q) v[q] = gain_mul(G.pre, off + k0 + q * step, G.conj, v[q]);
+                      }
+                    });
 }
 
-template <int TC>
-__global__ void __launch_bounds__(512) k_lp_cols(Geo g, PrecTables t, const double* __restrict__ freq,
-                                                 float2* __restrict__ w, const float* __restrict__ lp, int adjoint) {
+template <int TC, bool GEN>
+__global__ void __launch_bounds__(GEN ? 256 : 512, 2) k_lp_cols(Geo g, PrecTables t, const double* __restrict__ freq,
+                                                                float2* __restrict__ w, const float* __restrict__ lp,
+                                                                int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
-  cols_pass<TC>(sm, g, t, w + blockIdx.y * n, freq[blockIdx.y], 0.0, adjoint, blockIdx.x * TC, lp);
+  cols_pass_learned<TC, GEN>(sm, g, t, w + blockIdx.y * n, freq[blockIdx.y], adjoint, blockIdx.x * TC, lp);
 }
 
-__global__ void __launch_bounds__(256) k_lp_rows_inv(Geo g, PrecTables t, const float2* __restrict__ w,
-                                                     float2* __restrict__ y, int rows, const float2* gains,
-                                                     const int* gain_index, int adjoint) {
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_lp_rows_inv(Geo g, PrecTables t, const float2* __restrict__ w,
+                                                                  float2* __restrict__ y, int rows,
+                                                                  const float2* gains, const int* gain_index,
+                                                                  int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
-  const int nr = min(rows, g.nz - z0);
   const long long off = (long long)z0 * g.nx;
-  const float2* ws = w + blockIdx.y * n + off;
   const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y) : 0, n, adjoint);
-  const int rs = nsr_row_stride(g.nx);
-  const bool pad = nsr_row_padded(g.nx);
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    sm[l * rs + (pad ? c + (c >> 4) : c)] = ws[k];
-  }
-  __syncthreads();
-  fft_rows<true>(sm, nr, t.px);
-  __syncthreads();
-  float2* ys = y + blockIdx.y * n + off;
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    const float2 v = sm[l * rs + (pad ? c + (c >> 4) : c)];
+  float2* __restrict__ ys = y + blockIdx.y * n + off;
+  rows_inverse<GEN>(sm, min(rows, g.nz - z0), t.px, w + blockIdx.y * n + off, [&](int k, float2 v) {
     ys[k] = G.post ? gain_mul(G.post, off + k, G.conj, v) : v;
-  }
+  });
 }
 
 extern "C" int nsr_learned_precondition(const NsrGrid* grid, const NsrLearned* learned, const double* freq_hz,
@@ -353,18 +340,18 @@ extern "C" int nsr_learned_precondition(const NsrGrid* grid, const NsrLearned* l
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
   const float2* gains = (const float2*)learned->gains;
-  k_lp_rows_fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows, gains, learned->gain_index, adjoint);
+  const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
+  const auto fwd = gx ? k_lp_rows_fwd<true> : k_lp_rows_fwd<false>;
+  const auto inv = gx ? k_lp_rows_inv<true> : k_lp_rows_inv<false>;
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows, gains, learned->gain_index, adjoint);
   const int tc = nsr_cols_tc(grid);
   const dim3 gc((grid->nx + tc - 1) / tc, n_systems);
   const size_t csm = nsr_cols_smem(grid);
-  if (tc == 16) {
-    cudaFuncSetAttribute(k_lp_cols<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_lp_cols<16><<<gc, 512, csm, st>>>(g, t, freq_hz, w, learned->params, adjoint);
-  } else {
-    cudaFuncSetAttribute(k_lp_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_lp_cols<8><<<gc, 512, csm, st>>>(g, t, freq_hz, w, learned->params, adjoint);
-  }
-  k_lp_rows_inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, adjoint);
+  const auto cols = tc == 16 ? (gz ? k_lp_cols<16, true> : k_lp_cols<16, false>)
+                             : (gz ? k_lp_cols<8, true> : k_lp_cols<8, false>);
+  cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+  cols<<<gc, nsr_cols_threads(gz), csm, st>>>(g, t, freq_hz, w, learned->params, adjoint);
+  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, adjoint);
   return last_error();
 }
 
@@ -745,8 +732,9 @@ extern "C" int nsr_learned_spectral_backward(const NsrGrid* grid, const float* p
   const int rows = nsr_rows_per_cta(grid);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
-  k_lp_rows_fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, xr, rows, nullptr, nullptr, 0);
-  k_lp_rows_fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)y, yr, rows, nullptr, nullptr, 0);
+  const auto fwd = nsr_specialised(grid->nx) ? k_lp_rows_fwd<false> : k_lp_rows_fwd<true>;
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, xr, rows, nullptr, nullptr, 0);
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)y, yr, rows, nullptr, nullptr, 0);
   const int tc = spec_tc(grid);
   const int nb = (grid->nx + tc - 1) / tc;
   const size_t smem = sizeof(float2) * 2 * (size_t)grid->nz * tc;

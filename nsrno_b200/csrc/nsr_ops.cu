@@ -3,6 +3,7 @@
 // right-hand sides and the adjoint-state material gradient.
 #include "nsr_common.cuh"
 #include "nsr_internal.cuh"
+#include "nsr_device.cuh"
 
 #include <string.h>
 
@@ -198,58 +199,83 @@ extern "C" int nsr_apply(const NsrGrid* grid, const void* coef, const double* fr
 // ---------------------------------------------------------------------------
 // Preconditioner tables and passes (shared with the solver).
 // ---------------------------------------------------------------------------
-__global__ void k_fft_tables(int n, FftPlan plan, float2* tw, float* s2) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    double sn, cs;
-    sincospi(-2.0 * k / n, &sn, &cs);
-    tw[k] = make_float2((float)cs, (float)sn);
-    int f = nsr_digit_reverse(k, n, plan.radix, plan.nst);
-    double sp = sinpi((double)f / n);
-    s2[k] = (float)(sp * sp);
+// Twiddle tw[k] and symbols of output position k of a line of n points:
+// s2 = sin^2(pi f / n) of its frequency f, and (dense path) d2 = |D|^2 dx^2 of
+// the 8th-order staggered derivative.
+__device__ void table_entry(int n, const FftPlan& plan, int k, float2* tw, float* s2, float* d2) {
+  double sn, cs;
+  sincospi(-2.0 * k / n, &sn, &cs);
+  tw[k] = make_float2((float)cs, (float)sn);
+  const int f = nsr_digit_reverse(k, n, plan.radix, plan.nst);
+  const double sp = sinpi((double)f / n);
+  s2[k] = (float)(sp * sp);
+  if (d2) {
+    const double q = 2.0 * NSR_PI * f / n;
+    double s = 0.0;
+    for (int j = 0; j < 4; ++j) s += nsr_dense_stencil(j) * sin((j + 0.5) * q);
+    d2[k] = (float)(4.0 * s * s);
   }
 }
 
-// Per-stage twiddle rows of the specialised transforms (layout: FftPlan::tws),
-// with the same rounding of the same angles as k_fft_tables.
-__global__ void k_fft_stage_twiddles(int n, FftPlan plan, float2* tws, int total) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    int l = n, off = 0;
-    for (int st = 0; st < plan.nst; ++st) {
-      const int r = plan.radix[st], m = l / r;
-      if (m > 1) {
-        if (e < off + m * (r - 1)) {
-          const int k = (e - off) / m + 1, j = (e - off) % m;
-          double sn, cs;
-          sincospi(-2.0 * (j * k * (n / l)) / n, &sn, &cs);
-          tws[e] = make_float2((float)cs, (float)sn);
-          break;
-        }
-        off += m * (r - 1);
+// Entry e of the per-stage twiddle rows (layout: FftPlan::tws), with the same
+// rounding of the same angles as tw.
+__device__ void stage_twiddle_entry(int n, const FftPlan& plan, int e, float2* tws) {
+  int l = n, off = 0;
+  for (int st = 0; st < plan.nst; ++st) {
+    const int r = plan.radix[st], m = l / r;
+    if (m > 1) {
+      if (e < off + m * (r - 1)) {
+        const int k = (e - off) / m + 1, j = (e - off) % m;
+        double sn, cs;
+        sincospi(-2.0 * (j * k * (n / l)) / n, &sn, &cs);
+        tws[e] = make_float2((float)cs, (float)sn);
+        break;
       }
-      l = m;
+      off += m * (r - 1);
     }
+    l = m;
   }
 }
 
-int nsr_prec_setup(const NsrGrid* g, PrecTables* t, void* table_mem, cudaStream_t st) {
+// Every table of a grid in one launch (four to six small launches before, about
+// 2.5 us each in front of every preconditioner call).
+struct TableOut {
+  float2 *twx, *twz, *twsx, *twsz;
+  float *s2x, *s2z, *d2x, *d2z;
+  int nwx, nwz;
+};
+__global__ void __launch_bounds__(128) k_fft_tables(FftPlan px, FftPlan pz, TableOut o) {
+  int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < px.n) { table_entry(px.n, px, k, o.twx, o.s2x, o.d2x); return; }
+  k -= px.n;
+  if (k < pz.n) { table_entry(pz.n, pz, k, o.twz, o.s2z, o.d2z); return; }
+  k -= pz.n;
+  if (k < o.nwx) { stage_twiddle_entry(px.n, px, k, o.twsx); return; }
+  k -= o.nwx;
+  if (k < o.nwz) stage_twiddle_entry(pz.n, pz, k, o.twsz);
+}
+
+int nsr_prec_setup(const NsrGrid* g, PrecTables* t, void* table_mem, cudaStream_t st, float* d2x, float* d2z) {
   char* p = (char*)table_mem;
   t->px.n = g->nx;
   t->pz.n = g->nz;
   if (!nsr_make_radices(g->nx, t->px.radix, &t->px.nst)) return NSR_ERR_UNSUPPORTED_SIZE;
   if (!nsr_make_radices(g->nz, t->pz.radix, &t->pz.nst)) return NSR_ERR_UNSUPPORTED_SIZE;
-  float2* twx = (float2*)p; p += nsr_align(sizeof(float2) * g->nx);
-  float2* twz = (float2*)p; p += nsr_align(sizeof(float2) * g->nz);
-  float* s2x = (float*)p; p += nsr_align(sizeof(float) * g->nx);
-  float* s2z = (float*)p; p += nsr_align(sizeof(float) * g->nz);
-  const int nwx = nsr_twiddle_offset(g->nx, 0), nwz = nsr_twiddle_offset(g->nz, 0);
-  float2* twsx = (float2*)p; p += nsr_align(sizeof(float2) * nwx);
-  float2* twsz = (float2*)p; p += nsr_align(sizeof(float2) * nwz);
-  t->px.tw = twx; t->pz.tw = twz; t->s2x = s2x; t->s2z = s2z;
-  t->px.tws = twsx; t->pz.tws = twsz;
-  k_fft_tables<<<(g->nx + 255) / 256, 256, 0, st>>>(g->nx, t->px, twx, s2x);
-  k_fft_tables<<<(g->nz + 255) / 256, 256, 0, st>>>(g->nz, t->pz, twz, s2z);
-  if (nwx > 0) k_fft_stage_twiddles<<<(nwx + 255) / 256, 256, 0, st>>>(g->nx, t->px, twsx, nwx);
-  if (nwz > 0) k_fft_stage_twiddles<<<(nwz + 255) / 256, 256, 0, st>>>(g->nz, t->pz, twsz, nwz);
+  TableOut o;
+  o.twx = (float2*)p; p += nsr_align(sizeof(float2) * g->nx);
+  o.twz = (float2*)p; p += nsr_align(sizeof(float2) * g->nz);
+  o.s2x = (float*)p; p += nsr_align(sizeof(float) * g->nx);
+  o.s2z = (float*)p; p += nsr_align(sizeof(float) * g->nz);
+  o.nwx = nsr_twiddle_offset(g->nx, 0);
+  o.nwz = nsr_twiddle_offset(g->nz, 0);
+  o.twsx = (float2*)p; p += nsr_align(sizeof(float2) * o.nwx);
+  o.twsz = (float2*)p; p += nsr_align(sizeof(float2) * o.nwz);
+  o.d2x = d2x;
+  o.d2z = d2z;
+  t->px.tw = o.twx; t->pz.tw = o.twz; t->s2x = o.s2x; t->s2z = o.s2z;
+  t->px.tws = o.twsx; t->pz.tws = o.twsz;
+  const int total = g->nx + g->nz + o.nwx + o.nwz;
+  k_fft_tables<<<(total + 127) / 128, 128, 0, st>>>(t->px, t->pz, o);
   return last_error();
 }
 
@@ -260,91 +286,45 @@ size_t nsr_prec_table_bytes(const NsrGrid* g) {
          nsr_align(sizeof(float2) * nsr_twiddle_offset(g->nz, 0));
 }
 
-// Column pass: forward DIF along z, multiply by the shifted-Laplace symbol in
-// the digit-reversed domain, inverse along z.  In place on w.
-template <int TC>
-__global__ void __launch_bounds__(512) k_prec_cols(Geo g, PrecTables t, const double* __restrict__ freq,
-                                                   float2* __restrict__ w, double shift, int adjoint) {
-  extern __shared__ float2 sm[];
-  const int sysi = blockIdx.y;
-  const long long n = (long long)g.nz * g.nx;
-  float2* ws = w + sysi * n;
-  const int c0 = blockIdx.x * TC;
-  const int ncol = min(TC, g.nx - c0);
-  for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    sm[k] = c < ncol ? ws[(long long)z * g.nx + c0 + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_cols<false, TC>(sm, t.pz);
-  const SysScalars s = sys_scalars(g, freq[sysi]);
-  const float kh2 = (float)s.kh2;
-  const float inv_n = 1.0f / (float)n;
-  const float2 shiftc = make_float2(kh2, (float)(s.kh2 * shift));
-  for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    if (c < ncol) {
-      const float sym = -4.0f * (t.s2z[z] + t.s2x[c0 + c]);
-      float2 mul = divc(make_float2(inv_n, 0.f), make_float2(sym + shiftc.x, shiftc.y));
-      if (adjoint) mul = conjc(mul);
-      sm[k] = sm[k] * mul;
-    }
-  }
-  __syncthreads();
-  fft_cols<true, TC>(sm, t.pz);
-  for (int k = threadIdx.x; k < g.nz * TC; k += blockDim.x) {
-    const int z = k / TC, c = k - z * TC;
-    if (c < ncol) ws[(long long)z * g.nx + c0 + c] = sm[k];
-  }
-}
-
 int nsr_cols_tc(const NsrGrid* g) { return g->nz <= 1024 ? 16 : 8; }
-int nsr_cols_threads() { return 512; }
 size_t nsr_cols_smem(const NsrGrid* g) { return sizeof(float2) * (size_t)g->nz * nsr_cols_tc(g); }
 
-// Stand-alone row passes of nsr_precondition.
-__global__ void __launch_bounds__(256) k_prec_rows_fwd(Geo g, PrecTables t, const float2* __restrict__ x,
-                                                       float2* __restrict__ w, int rows) {
+// Stand-alone passes of nsr_precondition.  The ends of the transforms run
+// between registers and global memory (rows_forward, cols_multiply,
+// rows_inverse); each pass reads and writes a field once.  Eleven 768 x 1024
+// fields, rows / columns / rows: 75 / 113 / 58 us staged through shared memory,
+// 46 / 67 / 38 us in this form (21 us each at the copy rate).
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_prec_rows_fwd(Geo g, PrecTables t, const float2* __restrict__ x,
+                                                                    float2* __restrict__ w, int rows) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
-  const int nr = min(rows, g.nz - z0);
-  const float2* xs = x + blockIdx.y * n + (long long)z0 * g.nx;
-  const int rs = nsr_row_stride(g.nx);
-  const bool pad = nsr_row_padded(g.nx);
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    sm[l * rs + (pad ? c + (c >> 4) : c)] = xs[k];
-  }
-  __syncthreads();
-  fft_rows<false>(sm, nr, t.px);
-  float2* ws = w + blockIdx.y * n + (long long)z0 * g.nx;
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    ws[k] = sm[l * rs + (pad ? c + (c >> 4) : c)];
-  }
+  const long long off = blockIdx.y * n + (long long)z0 * g.nx;
+  const float2* __restrict__ xs = x + off;
+  rows_forward<GEN>(sm, min(rows, g.nz - z0), t.px, w + off, [&](auto tag, int k0, int step, float2* v) {
+#pragma unroll
+    for (int q = 0; q < decltype(tag)::value; ++q) v[q] = xs[k0 + q * step];
+  });
 }
 
-__global__ void __launch_bounds__(256) k_prec_rows_inv(Geo g, PrecTables t, const float2* __restrict__ w,
-                                                       float2* __restrict__ y, int rows) {
+template <int TC, bool GEN>
+__global__ void __launch_bounds__(GEN ? 256 : 512, 2) k_prec_cols(Geo g, PrecTables t, const double* __restrict__ freq,
+                                                                  float2* __restrict__ w, double shift, int adjoint) {
+  extern __shared__ float2 sm[];
+  const long long n = (long long)g.nz * g.nx;
+  cols_pass_fixed<TC, GEN>(sm, g, t, w + blockIdx.y * n, freq[blockIdx.y], shift, adjoint, blockIdx.x * TC);
+}
+
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) k_prec_rows_inv(Geo g, PrecTables t, const float2* __restrict__ w,
+                                                                    float2* __restrict__ y, int rows) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
-  const int nr = min(rows, g.nz - z0);
-  const float2* ws = w + blockIdx.y * n + (long long)z0 * g.nx;
-  const int rs = nsr_row_stride(g.nx);
-  const bool pad = nsr_row_padded(g.nx);
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    sm[l * rs + (pad ? c + (c >> 4) : c)] = ws[k];
-  }
-  __syncthreads();
-  fft_rows<true>(sm, nr, t.px);
-  float2* ys = y + blockIdx.y * n + (long long)z0 * g.nx;
-  for (int k = threadIdx.x; k < nr * g.nx; k += blockDim.x) {
-    const int l = k / g.nx, c = k - l * g.nx;
-    ys[k] = sm[l * rs + (pad ? c + (c >> 4) : c)];
-  }
+  const long long off = blockIdx.y * n + (long long)z0 * g.nx;
+  float2* __restrict__ ys = y + off;
+  rows_inverse<GEN>(sm, min(rows, g.nz - z0), t.px, w + off, [&](int k, float2 v) { ys[k] = v; });
 }
 
 extern "C" size_t nsr_precondition_workspace_size(const NsrGrid* grid, int32_t n_systems) {
@@ -369,18 +349,18 @@ extern "C" int nsr_precondition(const NsrGrid* grid, const double* freq_hz, int3
   const int rows = nsr_rows_per_cta(grid);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   dim3 gr((grid->nz + rows - 1) / rows, n_systems);
-  k_prec_rows_fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
+  if (nsr_specialised(grid->nx)) k_prec_rows_fwd<false><<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
+  else k_prec_rows_fwd<true><<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
   const int tc = nsr_cols_tc(grid);
-  dim3 gc((grid->nx + tc - 1) / tc, n_systems);
-  size_t csm = nsr_cols_smem(grid);
-  if (tc == 16) {
-    cudaFuncSetAttribute(k_prec_cols<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_prec_cols<16><<<gc, 512, csm, st>>>(g, t, freq_hz, w, shift, adjoint);
-  } else {
-    cudaFuncSetAttribute(k_prec_cols<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-    k_prec_cols<8><<<gc, 512, csm, st>>>(g, t, freq_hz, w, shift, adjoint);
-  }
-  k_prec_rows_inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
+  const bool gen = !nsr_specialised(grid->nz);
+  const dim3 gc((grid->nx + tc - 1) / tc, n_systems);
+  const size_t csm = nsr_cols_smem(grid);
+  const auto cols = tc == 16 ? (gen ? k_prec_cols<16, true> : k_prec_cols<16, false>)
+                             : (gen ? k_prec_cols<8, true> : k_prec_cols<8, false>);
+  cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
+  cols<<<gc, nsr_cols_threads(gen), csm, st>>>(g, t, freq_hz, w, shift, adjoint);
+  if (nsr_specialised(grid->nx)) k_prec_rows_inv<false><<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
+  else k_prec_rows_inv<true><<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
   return last_error();
 }
 

@@ -126,12 +126,10 @@ __device__ __forceinline__ double abs2(double2 a) { return a.x * a.x + a.y * a.y
 __device__ __forceinline__ void fwd_staged(const SolveArgs& A, const SlotState& S, const GainPair& G, float2* sm,
                                            int mode, int nr, long long off, long long goff, int cnt, float2 sv,
                                            float2 rt, float2 yp, float2 ys, float2 pp, float2 pv) {
-  const Geo& g = A.g;
   float2 *r = A.B.r + off, *p = A.B.p + off, *v = A.B.v + off, *t = A.B.t + off, *y = A.B.y + off;
   // The tile's rows are contiguous in HBM, so one flat index k = l*nx + c runs
   // over them.  The padded row layout puts (l, c) at l*(nx + nx/16) + c + c/16,
-  // which equals k + k/16 because every padded width is a multiple of 16.
-  const bool pad = nsr_row_padded(g.nx);
+  // which equals k + k/16 because every specialised width is a multiple of 16.
   float2* __restrict__ rr_ = r;
   float2* __restrict__ pp_ = p;
   float2* __restrict__ yy_ = y;
@@ -149,19 +147,19 @@ __device__ __forceinline__ void fwd_staged(const SolveArgs& A, const SlotState& 
       const float2 pn = rn + pp * pk + pv * vk;
       rr_[k] = rn; pp_[k] = pn; yy_[k] = yn;
       if (restart) rh[k] = rn;
-      sm[pad ? k + (k >> 4) : k] = G.pre ? gain_mul(G.pre, goff + k, G.conj, pn) : pn;
+      sm[row_pos(k)] = G.pre ? gain_mul(G.pre, goff + k, G.conj, pn) : pn;
     }
   } else if (mode == MODE_ITER_B) {
 #pragma unroll 8
     for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
       const float2 s1 = rr_[k] + sv * vv_[k];
-      sm[pad ? k + (k >> 4) : k] = G.pre ? gain_mul(G.pre, goff + k, G.conj, s1) : s1;
+      sm[row_pos(k)] = G.pre ? gain_mul(G.pre, goff + k, G.conj, s1) : s1;
     }
   } else {  // MODE_RES: apply the pending update to y, transform y, clear it
     for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
       const float2 s1 = rr_[k] + sv * vv_[k];
       const float2 yn = yy_[k] + yp * pp_[k] + ys * s1;
-      sm[pad ? k + (k >> 4) : k] = G.pre ? gain_mul(G.pre, goff + k, G.conj, yn) : yn;
+      sm[row_pos(k)] = G.pre ? gain_mul(G.pre, goff + k, G.conj, yn) : yn;
       yy_[k] = make_float2(0.f, 0.f);
     }
   }
@@ -169,18 +167,21 @@ __device__ __forceinline__ void fwd_staged(const SolveArgs& A, const SlotState& 
   fft_rows<false>(sm, nr, A.tab.px);
   float2* __restrict__ w = A.B.w + off;
 #pragma unroll 8
-  for (int k = threadIdx.x; k < cnt; k += blockDim.x) w[k] = sm[pad ? k + (k >> 4) : k];
+  for (int k = threadIdx.x; k < cnt; k += blockDim.x) w[k] = sm[row_pos(k)];
 }
 
+// How a row or column kernel runs its transform: the specialised sizes with the
+// transform's ends between registers and global memory (PASS_DIRECT) or staged
+// in shared memory (PASS_STAGED, a launch shape the autotuner can choose), every
+// other size by the run-time stages (PASS_GENERIC).
+enum { PASS_STAGED = 0, PASS_DIRECT = 1, PASS_GENERIC = 2 };
+
 // ---------------------------------------------------------------------------
-// fwd: elementwise update + forward row FFT into w.  DIRECT (row widths
-// 256 ... 2048 of the form 2^a 3^b): the update runs inside the transform's
-// first stage and its last stage writes w straight from registers
-// (ct_rows_forward_direct); otherwise the updated tile is staged in shared
-// memory first.
+// fwd: elementwise update + forward row FFT into w.  Unless staged, the update
+// runs inside the transform's first stage (rows_forward).
 // ---------------------------------------------------------------------------
-template <bool DIRECT>
-__global__ void __launch_bounds__(256, 4) k_fwd(SolveArgs A, int half) {
+template <int PASS>
+__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const SlotState& S = A.B.slots[slot];
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(256, 4) k_fwd(SolveArgs A, int half) {
   float2* __restrict__ yy_ = y;
   const float2* __restrict__ vv_ = v;
   const float2* __restrict__ tt_ = t;
-  if constexpr (DIRECT) {
+  if constexpr (PASS != PASS_STAGED) {
     const bool restart = S.restart != 0;
     float2* __restrict__ rh = A.B.rh + off;
     // Values of one stage-0 butterfly: elements k0 + q*step, q < R.  The
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(256, 4) k_fwd(SolveArgs A, int half) {
     // and radix-16 first stages, whose results already hold 16-32 registers).
     auto in = [&](auto tag, int k0, int step, float2* out) {
       constexpr int R = decltype(tag)::value;
-      constexpr int CH = R <= 4 ? R : 2;
+      constexpr int CH = R <= 4 ? R : R % 2 == 0 ? 2 : 1;
       if (mode == MODE_ITER_A) {
 #pragma unroll
         for (int c = 0; c < R; c += CH) {
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(256, 4) k_fwd(SolveArgs A, int half) {
         for (int q = 0; q < R; ++q) out[q] = gain_mul(G.pre, goff + k0 + q * step, G.conj, out[q]);
       }
     };
-    fft_rows_forward_direct(sm, nr, A.tab.px, A.B.w + off, in);
+    rows_forward<PASS == PASS_GENERIC>(sm, nr, A.tab.px, A.B.w + off, in);
   } else {
     fwd_staged(A, S, G, sm, mode, nr, off, goff, cnt, sv, rt, yp, ys, pp, pv);
   }
@@ -293,8 +294,8 @@ __global__ void __launch_bounds__(256, 4) k_fwd(SolveArgs A, int half) {
 // ---------------------------------------------------------------------------
 // cols: column FFT, preconditioner multiply, inverse column FFT (in place).
 // ---------------------------------------------------------------------------
-template <int TC, bool LEARNED, bool STAGED>
-__global__ void __launch_bounds__(512, 2) k_cols(SolveArgs A, int half) {
+template <int TC, bool LEARNED, int PASS>
+__global__ void __launch_bounds__(PASS == PASS_GENERIC ? 256 : 512, 2) k_cols(SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const int mode = A.B.slots[slot].mode;
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(512, 2) k_cols(SolveArgs A, int half) {
   const int adjoint = A.adjoint;
   if (LEARNED) {
     const float2* __restrict__ symp = A.B.sym + slot * n;
-    cols_pass_direct<TC, STAGED>(sm, g, A.tab, A.B.w + slot * n, c0, [&](int c, int z) -> float2 {
+    cols_pass_with<TC, PASS == PASS_GENERIC, PASS == PASS_STAGED>(sm, g, A.tab, A.B.w + slot * n, c0, [&](int c, int z) -> float2 {
       const float2 mul = symp[(long long)z * g.nx + c0 + c];
       return adjoint ? conjc(mul) : mul;
     });
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(512, 2) k_cols(SolveArgs A, int half) {
     const float inv_n = 1.0f / (float)n;
     const float2 shiftc = make_float2((float)s.kh2, (float)(s.kh2 * A.shift));
     const PrecTables& tab = A.tab;
-    cols_pass_direct<TC, STAGED>(sm, g, tab, A.B.w + slot * n, c0, [&](int c, int z) -> float2 {
+    cols_pass_with<TC, PASS == PASS_GENERIC, PASS == PASS_STAGED>(sm, g, tab, A.B.w + slot * n, c0, [&](int c, int z) -> float2 {
       const float sym = -4.0f * (tab.s2z[z] + tab.s2x[c0 + c]);
       const float2 mul = divc(make_float2(inv_n, 0.f), make_float2(sym + shiftc.x, shiftc.y));
       return adjoint ? conjc(mul) : mul;
@@ -324,12 +325,12 @@ __global__ void __launch_bounds__(512, 2) k_cols(SolveArgs A, int half) {
 
 // ---------------------------------------------------------------------------
 // rinv: inverse row FFT in place on w, times the outer gain of the learned
-// preconditioner; afterwards w holds z = M^-1 (input of the half).  DIRECT:
-// the transform's first stage reads w and its last stage writes it, with the
-// gain, straight from registers (ct_rows_inverse_direct).
+// preconditioner; afterwards w holds z = M^-1 (input of the half).  Unless
+// staged, the transform's last stage writes w, with the gain, straight from
+// registers (rows_inverse).
 // ---------------------------------------------------------------------------
-template <bool DIRECT>
-__global__ void __launch_bounds__(256, 4) k_rinv(SolveArgs A, int half) {
+template <int PASS>
+__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_rinv(SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const SlotState& S = A.B.slots[slot];
@@ -341,22 +342,21 @@ __global__ void __launch_bounds__(256, 4) k_rinv(SolveArgs A, int half) {
   const long long goff = (long long)z0 * g.nx;
   float2* w = A.B.w + slot * n + goff;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
-  if constexpr (DIRECT) {
-    fft_rows_inverse_direct(sm, nr, A.tab.px, w, [&](int k, float2 v) {
+  if constexpr (PASS != PASS_STAGED) {
+    rows_inverse<PASS == PASS_GENERIC>(sm, nr, A.tab.px, w, [&](int k, float2 v) {
       w[k] = G.post ? gain_mul(G.post, goff + k, G.conj, v) : v;
     });
     return;
   }
-  const bool pad = nsr_row_padded(g.nx);   // flat index k + k/16, as in k_fwd
   const int cnt = nr * g.nx;
 #pragma unroll 8
-  for (int k = threadIdx.x; k < cnt; k += blockDim.x) sm[pad ? k + (k >> 4) : k] = w[k];
+  for (int k = threadIdx.x; k < cnt; k += blockDim.x) sm[row_pos(k)] = w[k];
   __syncthreads();
   fft_rows<true>(sm, nr, A.tab.px);
   __syncthreads();
 #pragma unroll 8
   for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-    const float2 v = sm[pad ? k + (k >> 4) : k];
+    const float2 v = sm[row_pos(k)];
     w[k] = G.post ? gain_mul(G.post, goff + k, G.conj, v) : v;
   }
 }
@@ -1297,13 +1297,17 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
 }
 
 
-__global__ void k_solve_init(SolveArgs A, int n_slots) {
+__global__ void k_solve_outputs(SolveArgs A) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < A.n_systems; s += gridDim.x * blockDim.x) {
     A.status[s] = NSR_NOT_RUN;
     A.iterations[s] = 0;
     A.residual[s] = NAN;
   }
+}
+
+__global__ void k_solve_init(SolveArgs A, int n_slots) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < n_slots; s += gridDim.x * blockDim.x) {
     SlotState st;
     memset(&st, 0, sizeof(st));
@@ -1610,28 +1614,33 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
         }
       }
     }
-    // row kernels: direct (specialised widths) or staged through shared memory
-    const bool direct_rows = nsr_row_padded(grid->nx) && !T.rows_staged;
+    // row and column kernels: run-time stages, or direct / staged for the specialised sizes
+    const int row_pass = !nsr_specialised(grid->nx) ? PASS_GENERIC : T.rows_staged ? PASS_STAGED : PASS_DIRECT;
+    const int col_pass = !nsr_specialised(grid->nz) ? PASS_GENERIC : T.cols_staged ? PASS_STAGED : PASS_DIRECT;
     typedef void (*RowKernel)(SolveArgs, int);
-    const RowKernel fwd_fn = direct_rows ? k_fwd<true> : k_fwd<false>;
-    const RowKernel rinv_fn = direct_rows ? k_rinv<true> : k_rinv<false>;
+    const RowKernel fwd_fn = row_pass == PASS_GENERIC ? k_fwd<PASS_GENERIC>
+                             : row_pass == PASS_DIRECT ? k_fwd<PASS_DIRECT> : k_fwd<PASS_STAGED>;
+    const RowKernel rinv_fn = row_pass == PASS_GENERIC ? k_rinv<PASS_GENERIC>
+                              : row_pass == PASS_DIRECT ? k_rinv<PASS_DIRECT> : k_rinv<PASS_STAGED>;
     NSR_TRY(cudaFuncSetAttribute((const void*)fwd_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
-    // column kernel: transform tile width, learned or fixed multiplier, direct
-    // (specialised sizes) or staged through shared memory
+    // column kernel: transform tile width, learned or fixed multiplier
     typedef void (*ColsKernel)(SolveArgs, int);
-    const bool generic_cols = !nsr_row_padded(grid->nz) || T.cols_staged;
+    const int col_threads = nsr_cols_threads(col_pass == PASS_GENERIC);
     ColsKernel cols_fn = nullptr;
 #define NSR_COLS_PICK(TC_, L_) \
-    if (A.tc == TC_ && (A.lp != nullptr) == L_) cols_fn = generic_cols ? k_cols<TC_, L_, true> : k_cols<TC_, L_, false>;
+    if (A.tc == TC_ && (A.lp != nullptr) == L_) \
+      cols_fn = col_pass == PASS_GENERIC ? k_cols<TC_, L_, PASS_GENERIC> \
+                : col_pass == PASS_DIRECT ? k_cols<TC_, L_, PASS_DIRECT> : k_cols<TC_, L_, PASS_STAGED>;
     NSR_COLS_PICK(16, false) NSR_COLS_PICK(8, false) NSR_COLS_PICK(16, true) NSR_COLS_PICK(8, true)
 #undef NSR_COLS_PICK
     if (!cols_fn) { err = NSR_ERR_ARGUMENT; goto cleanup; }
     NSR_TRY(cudaFuncSetAttribute((const void*)cols_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
     NSR_TRY(cudaFuncSetAttribute((const void*)rinv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
 
+    k_solve_outputs<<<64, 256, 0, st>>>(A);
     k_solve_init<<<64, 256, 0, st>>>(A, n_slots);
     NSR_TRY(cudaGetLastError());
-    launches = 3;  // two table kernels and the slot initialisation
+    launches = 3;  // the tables, the outputs and the slots
 
     // The slots run as independent groups on branches of the captured graph,
     // so that one group's kernels fill the tail waves of the others'.
@@ -1666,7 +1675,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
       } else if (which == 1) {
         int hv = half;
         void* args[] = {&Ag, &hv};
-        cudaLaunchKernel((const void*)cols_fn, g_col, dim3(512), args, col_smem, sq);
+        cudaLaunchKernel((const void*)cols_fn, g_col, dim3(col_threads), args, col_smem, sq);
       } else if (which == 2) {
         if (A.adjoint) k_res<true><<<g_res, NSR_RES_TX, 0, sq>>>(Ag);
         else k_res<false><<<g_res, NSR_RES_TX, 0, sq>>>(Ag);
