@@ -580,7 +580,7 @@ __device__ __forceinline__ void gen_rows_inverse(float2* s, int nl, const FftPla
 template <int TC, typename MUL>
 __device__ __forceinline__ void gen_cols(float2* s, const FftPlan& P, float2* __restrict__ g, int nx, int ncol, MUL mul) {
   const int N = P.n, last = P.nst - 1;
-  const float2 zero = make_float2(0.f, 0.f);
+  const float2 zero = make_float2(0.f, 0.f);   // columns at or beyond ncol are never stored
   if (last > 0) {
     gen_radix(P.radix[0],
               [&](auto tag) {
@@ -590,7 +590,7 @@ __device__ __forceinline__ void gen_cols(float2* s, const FftPlan& P, float2* __
                   const int l = b % TC, j = b / TC;
                   float2 v[R];
 #pragma unroll
-                  for (int q = 0; q < R; ++q) v[q] = l < ncol ? g[(long long)(j + q * m) * nx + l] : zero;
+                  for (int q = 0; q < R; ++q) v[q] = g[(long long)(j + q * m) * nx + min(l, ncol - 1)];
                   small_dft<R, false>(v);
                   gen_twiddle<R, false>(v, P.tws, j, m);
 #pragma unroll
@@ -918,7 +918,7 @@ __device__ __forceinline__ void ct_inverse_downto(float2* s, int nl, const float
 // nx), with the first forward stage computed straight from the global loads
 // and the last inverse stage written straight to global memory: the tile
 // crosses shared memory two times fewer than load-transform-store.  Columns
-// at or beyond `ncol` read as zero and are not written.  `mul(l, k)` as in
+// at or beyond `ncol` are not written.  `mul(l, k)` as in
 // ct_cols_fused.  Needs at least two stages (every specialised size has).
 template <int N, int TC, typename MUL>
 __device__ __forceinline__ void ct_cols_direct(float2* s, const float2* __restrict__ tws, float2* __restrict__ g,

@@ -286,3 +286,97 @@ __device__ __forceinline__ float2 gain_mul(const float2* plane, long long idx, b
   if (cj) gv.y = -gv.y;
   return gv * v;
 }
+
+// ---------------------------------------------------------------------------
+// FP64 residual tiles shared by the Krylov solvers.
+// ---------------------------------------------------------------------------
+// One thread per column of a NSR_RES_TZ x NSR_RES_TX tile walks down its rows
+// with the north/centre/south values of x and a in registers; the east and west
+// neighbours come from the adjacent lanes, the PML factors from the separable
+// form of stencil_sep (no division per node).
+#define NSR_RES_TZ 8      // rows of one tile: 384 tiles of one 768 x 1024 system
+#define NSR_RES_TX 256    // threads of a block
+#define NSR_RES_CTAS 1184 // CTAs of one launch over all its slots (8 per SM): most launches find no slot to
+                          // serve, and 4,224 idle CTAs cost 8 us more than 1,184
+__host__ __device__ inline int res_tiles(int nz, int nx) {
+  return ((nz + NSR_RES_TZ - 1) / NSR_RES_TZ) * ((nx + NSR_RES_TX - 1) / NSR_RES_TX);
+}
+// CTAs per slot of a launch over ns slots.
+inline int res_ctas(const NsrGrid* g, int ns) {
+  const int tiles = res_tiles(g->nz, g->nx), share = NSR_RES_CTAS / ns > 1 ? NSR_RES_CTAS / ns : 1;
+  return tiles < share ? tiles : share;
+}
+
+// Tiles blockIdx.x, blockIdx.x + gridDim.x, ... : `P(id)` is x at node id,
+// `b_at(idx, i, j)` the h^2-scaled right-hand side, `out(idx, x, b, r)` takes
+// each node's x, b and r = b - A x.
+template <bool ADJ, typename XF, typename BF, typename OUT>
+__device__ __forceinline__ void residual_tiles(const Geo& g, const MatPlanes& mat, const SysScalars& sc, XF P,
+                                               BF b_at, OUT out) {
+  __shared__ RowFactors<double> rowf[NSR_RES_TZ];
+  const int nx = g.nx;
+  const int nbx = (nx + NSR_RES_TX - 1) / NSR_RES_TX;
+  const int n_tiles = res_tiles(g.nz, nx);
+  const int lane = threadIdx.x & 31;
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int rb = tile / nbx, cb = tile - rb * nbx;
+    const int z0 = rb * NSR_RES_TZ, z1 = min(z0 + NSR_RES_TZ, g.nz);
+    const int j = cb * NSR_RES_TX + threadIdx.x;
+    const bool own = j < nx;
+    __syncthreads();   // rowf of the tile before has been read
+    if (threadIdx.x < z1 - z0) rowf[threadIdx.x] = row_factors<double>(g, sc, z0 + threadIdx.x);
+    __syncthreads();
+    const ColFactors<double> cf = col_factors<double>(g, sc, j);
+    const bool edge_w = lane == 0, edge_e = lane == 31 || j + 1 >= nx;
+    // Loads take clamped addresses and are selected afterwards; the south values
+    // are loaded one row ahead of their use.
+    const int jc = min(j, nx - 1);
+    auto row = [&](int i) -> long long { return (long long)min(i, g.nz - 1) * nx + jc; };
+    long long idx = row(z0);
+    double2 pn = P(z0 > 0 ? idx - nx : idx), pc = P(idx), ps_next = P(row(z0 + 1));
+    double an = __ldg(&mat.a64[z0 > 0 ? idx - nx : idx]), ac = __ldg(&mat.a64[idx]);
+    double as_next = __ldg(&mat.a64[row(z0 + 1)]);
+    if (z0 == 0) { pn = zero; an = 1.0; }
+    for (int i = z0; i < z1; ++i, idx += nx) {
+      double2 ps = ps_next;
+      double as = as_next;
+      const long long ahead = row(min(i + 2, z1));
+      ps_next = P(ahead);
+      as_next = __ldg(&mat.a64[ahead]);
+      const double b_c = __ldg(&mat.b64[idx]), t_c = __ldg(&mat.t64[idx]);
+      if (i + 1 >= g.nz) { ps = zero; as = 1.0; }
+      double2 pw = make_double2(__shfl_up_sync(0xffffffffu, pc.x, 1), __shfl_up_sync(0xffffffffu, pc.y, 1));
+      double2 pe = make_double2(__shfl_down_sync(0xffffffffu, pc.x, 1), __shfl_down_sync(0xffffffffu, pc.y, 1));
+      double aw = __shfl_up_sync(0xffffffffu, ac, 1), ae = __shfl_down_sync(0xffffffffu, ac, 1);
+      if (own && edge_w) {
+        pw = j > 0 ? P(idx - 1) : zero;
+        aw = j > 0 ? __ldg(&mat.a64[idx - 1]) : 1.0;
+      }
+      if (own && edge_e) {
+        pe = j + 1 < nx ? P(idx + 1) : zero;
+        ae = j + 1 < nx ? __ldg(&mat.a64[idx + 1]) : 1.0;
+      }
+      if (own) {
+        const double2 b = b_at(idx, i, j);
+        const double2 ax = stencil_sep<double, ADJ>(sc.kh2, sc.fpow, rowf[i - z0], cf, ac, ae, aw, as, an,
+                                                    b_c, t_c, pc, pe, pw, ps, pn);
+        out(idx, pc, b, b - ax);
+      }
+      pn = pc;
+      pc = ps;
+      an = ac;
+      ac = as;
+    }
+  }
+}
+
+// h^2-scaled right-hand side at a node: the given SI field, or the plane-wave
+// source on the array row.
+__device__ __forceinline__ double2 rhs_at(const Geo& g, double k0, double sin_theta, const float2* rhs, long long idx,
+                                          int i, int j) {
+  if (rhs) return (g.h * g.h) * to_d(rhs[idx]);
+  if (i != g.face) return make_double2(0.0, 0.0);
+  const double2 l = source_line(g, k0, sin_theta, j);
+  return make_double2(-l.x, -l.y);
+}

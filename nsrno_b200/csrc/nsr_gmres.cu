@@ -4,29 +4,32 @@
 // (nsrno/dense_wave.py:212-220).
 //
 // The systems of a batch share the Arnoldi index j, so j is a launch argument
-// and one restart cycle is a fixed sequence of launches captured once in a
-// CUDA graph.  Per Arnoldi step (8 launches):
-//   fwd   v_j = (j ? w / h_{j,j-1} : r / beta), forward row FFT of v_j
+// and one restart cycle is a fixed sequence of launches, replayed as a CUDA
+// graph from the second cycle on.  Per Arnoldi step (5 launches):
+//   fwd   v_j = (w - sum_i h'_i v_i) / h_{j,j-1} (the correction of the second
+//         Gram-Schmidt pass; r / beta for j = 0), stored and row-transformed
 //   cols  column FFT, shifted-Laplace multiply, inverse column FFT
 //   rinv  inverse row FFT in place: W = M^-1 v_j
-//   inv   5-point stencil: w = A W
-//   dot   h_i = <v_i, w> (i <= j), FP64 partials, last-CTA sum
-//   axpy  w -= sum_i h_i v_i                (classical Gram-Schmidt, pass 1)
-//   dot   h'_i = <v_i, w>                   (pass 2)
-//   axpy  w -= sum_i h'_i v_i, ||w||^2; the last CTA applies the previous
-//         Givens rotations to column j, forms the new one and the residual
-//         estimate, all in FP64 on the device (no host least squares).
+//   inv   5-point stencil: w = A W, and h_i = <v_i, w> (i <= j) of each tile
+//   gs    w -= sum_i h_i v_i (classical Gram-Schmidt, pass 1), and of the
+//         result h'_i = <v_i, w> (pass 2) and ||w||^2; the last CTA takes
+//         ||w - V h'||^2 = ||w||^2 - sum |h'_i|^2 (V is orthonormal and h' is
+//         of rounding size), applies the previous Givens rotations to column j
+//         and forms the new one, all in FP64 on the device.
+// So the basis is read three times a step (four, with w twice more, when every
+// dot and axpy was its own launch).  Eleven 768 x 1024 systems, 8 steps: 9.1 ms
+// with eight launches a step and one-thread-per-node dots, 4.9 ms in this form.
 // At the end of a cycle: back substitution for y (FP64), u = V y fused with
 // the forward row FFT, the column and inverse row passes, and an FP64 pass
 // that applies x += M^-1 u and recomputes the true residual b - A x.
 #include "nsr_internal.cuh"
 #include "nsr_device.cuh"
+#include "nsr_gs.cuh"
 
 #include <stdlib.h>
 #include <string.h>
 
 #define NSR_GMRES_MAX_M 64
-#define NSR_GDOT_CELLS 8     // nodes per thread in the dot / axpy kernels
 
 struct __align__(16) GSlot {
   int sys;        // system index, -1 when the slot is empty
@@ -42,6 +45,7 @@ struct __align__(16) GSlot {
   double resid;   // true relative residual at the start of the cycle
   double hlast;   // h_{j+1,j} of the last step (the norm that normalises v_{j+1})
   double freq, angle;
+  SysScalars sc;  // scalars of freq (a double pow: formed once, not by every thread)
 };
 
 struct GArgs {
@@ -50,25 +54,26 @@ struct GArgs {
   MatPlanes mat;
   int m;               // restart length
   int n_slots;
-  int nb_band;         // CTAs of the band kernels per slot
-  int nb_dot;          // CTAs of the dot/axpy kernels per slot
-  int tz, rows, tc;
+  int nb_max;          // most CTAs per slot of a reducing kernel
+  int rows, tc;
   double tol;
   double shift;
   int max_it;
   int adjoint;
   GSlot* slots;
   int* arrive;         // [n_slots]
-  double* partials;    // [n_slots][max(nb_dot, nb_band)][2 (m+1)]
+  double* partials;    // [n_slots][2 (m+1) + 1][nb_max]: value-major, the launch's CTAs contiguous
   double2* H;          // [n_slots][(m+1) m] column-major: H[j*(m+1) + i]
   double* cs;          // [n_slots][m]
   double2* sn;         // [n_slots][m]
   double2* gv;         // [n_slots][m+1]
-  double2* hc;         // [n_slots][m+1]  coefficients of the current CGS pass
+  double2* hc;         // [n_slots][m+1]  coefficients of the first CGS pass
+  double2* hc2;        // [n_slots][m+1]  and of the second
   double2* y;          // [n_slots][m]
   float2* V;           // [n_slots][m+1][n]
   float2* w;           // [n_slots][n]
   float2* W;           // [n_slots][n]   FFT work field
+  float2* sym;         // [n_slots][n]   learned multiplier of the slot's system (learned solves only)
   float2* r;           // [n_slots][n]
   double2* x;          // [n_slots][2][n]
   const double* freq;
@@ -88,45 +93,13 @@ __device__ __forceinline__ bool g_active(const GSlot& S, int j) {
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) { return a * b; }
 __device__ __forceinline__ double cabs(double2 a) { return sqrt(a.x * a.x + a.y * a.y); }
 
-// Per-CTA partials of NV doubles, arrival counter, last CTA returns true with
-// the column sums in `tot` (shared, length NV).
-template <int NVMAX>
-__device__ bool g_reduce(const GArgs& A, int slot, const double* vals, int nv, double* tot) {
-  __shared__ double wsum[32][2];
-  __shared__ int am_last;
-  double* part = A.partials + (long long)slot * max(A.nb_dot, A.nb_band) * 2 * (NSR_GMRES_MAX_M + 1);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int q = 0; q < nv; ++q) {
-    double s = warp_sum(vals[q]);
-    if (lane == 0) wsum[wid][q & 1] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int u = 0; u < nw; ++u) t += wsum[u][q & 1];
-      part[blockIdx.x * 2 * (NSR_GMRES_MAX_M + 1) + q] = t;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const int prev = atomicAdd(&A.arrive[slot], 1);
-    am_last = (prev == (int)gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!am_last) return false;
-  __threadfence();
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) s += __ldcg(&part[b * 2 * (NSR_GMRES_MAX_M + 1) + q]);
-    tot[q] = s;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) A.arrive[slot] = 0;
-  return true;
+__device__ __forceinline__ double* g_part(const GArgs& A, int slot) {
+  return A.partials + (long long)slot * (2 * (A.m + 1) + 1) * A.nb_max;
 }
 
 // ---------------------------------------------------------------------------
-// fwd: v_j from r (j = 0) or w (j > 0), stored in V and transformed by rows.
+// fwd: v_j from r (j = 0) or w and the second pass's coefficients (j > 0),
+// stored in V and transformed by rows.
 // ---------------------------------------------------------------------------
 template <bool GEN>
 __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
@@ -141,12 +114,24 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
   const long long off = (long long)z0 * g.nx;
   const float2* __restrict__ src = (j == 0 ? A.r : A.w) + slot * n + off;
   const float scale = (float)(1.0 / (j == 0 ? S.beta : S.hlast));   // both real and positive
+  __shared__ float2 c2[NSR_GMRES_MAX_M];
+  for (int i = threadIdx.x; i < j; i += blockDim.x) c2[i] = to_f(A.hc2[(long long)slot * (A.m + 1) + i]);
+  __syncthreads();
+  const float2* __restrict__ V = A.V + (long long)slot * (A.m + 1) * n + off;
   float2* __restrict__ vj = A.V + ((long long)slot * (A.m + 1) + j) * n + off;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
   rows_forward<GEN>(sm, nr, A.tab.px, A.W + slot * n + off, [&](auto tag, int k0, int step, float2* v) {
     constexpr int R = decltype(tag)::value;
 #pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = scale * src[k0 + q * step];
+    for (int q = 0; q < R; ++q) v[q] = src[k0 + q * step];
+    for (int i = 0; i < j; ++i) {
+      const float2 c = c2[i];
+      const float2* __restrict__ Vi = V + i * n;
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = v[q] - c * Vi[k0 + q * step];
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = scale * v[q];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
       vj[k0 + q * step] = v[q];
@@ -156,7 +141,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
 }
 
 // cols for slots active at step j (j < 0: slots that run a cycle-end update)
-template <int TC, bool GEN>
+template <int TC, bool GEN, bool LEARNED>
 __global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
@@ -165,8 +150,34 @@ __global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(GArgs A, int j) {
   if (!on) return;
   const long long n = (long long)A.g.nz * A.g.nx;
   float2* w = A.W + slot * n;
-  if (A.lp) cols_pass_learned<TC, GEN>(sm, A.g, A.tab, w, S.freq, A.adjoint, blockIdx.x * TC, A.lp);
-  else cols_pass_fixed<TC, GEN>(sm, A.g, A.tab, w, S.freq, A.shift, A.adjoint, blockIdx.x * TC);
+  const int c0 = blockIdx.x * TC;
+  if (LEARNED) {
+    const float2* __restrict__ symp = A.sym + slot * n;
+    const int nx = A.g.nx, adjoint = A.adjoint;
+    cols_pass_with<TC, GEN, false>(sm, A.g, A.tab, w, c0, [&](int c, int z) -> float2 {
+      const float2 mul = symp[(long long)z * nx + c0 + c];
+      return adjoint ? conjc(mul) : mul;
+    });
+  } else {
+    cols_pass_fixed<TC, GEN>(sm, A.g, A.tab, w, S.freq, A.shift, A.adjoint, c0);
+  }
+}
+
+// The learned multiplier depends on the system's frequency only: it is evaluated
+// once per system, in the digit-reversed (z, x) order of the transformed field,
+// and read by every column pass (94 us for eleven 768 x 1024 systems with the
+// two tanh, the exponential and the sincos evaluated in the pass).
+__global__ void __launch_bounds__(256) gk_sym(GArgs A) {
+  const GSlot& S = A.slots[blockIdx.y];
+  if (S.sys < 0) return;
+  const Geo& g = A.g;
+  const long long n = (long long)g.nz * g.nx;
+  const LearnedSpec L = load_learned_spec(A.lp);
+  const float kh2 = (float)S.sc.kh2;
+  float2* __restrict__ sym = A.sym + blockIdx.y * n;
+  for (int z = blockIdx.x; z < g.nz; z += gridDim.x)
+    for (int x = threadIdx.x; x < g.nx; x += blockDim.x)
+      sym[(long long)z * g.nx + x] = learned_plane_value(L, g, A.tab, kh2, z, x);
 }
 
 // rinv: inverse row FFT of W in place, times the outer gain (W becomes M^-1 v_j,
@@ -190,13 +201,15 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(GArgs A, int j) {
   });
 }
 
-// inv: w = A z with z = M^-1 v_j in W.  One thread per column of a
-// NSR_GST_TZ x NSR_GST_TX tile walks down its rows with the north/centre/south
-// values of z and a in registers.
-#define NSR_GST_TZ 32
-#define NSR_GST_TX 256
-template <bool ADJ>
-__global__ void __launch_bounds__(256, 4) gk_inv(GArgs A, int j) {
+// inv: w = A z with z = M^-1 v_j in W, and the tile's inner products with the
+// basis.  One thread per column of a TZ x NSR_GST_TX tile walks down its rows
+// with the north/centre/south values of z and a in registers.
+#define NSR_GST_TX NSR_GS_THREADS
+template <bool ADJ, int TZ>
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_inv(GArgs A, int j) {
+  extern __shared__ __align__(16) double2 wt[];   // TZ x NSR_GST_TX nodes of w
+  __shared__ double tot[2 * (NSR_GMRES_MAX_M + 1)];
+  __shared__ RowFactors<float> rowf[TZ];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
   if (!g_active(S, j)) return;
@@ -205,109 +218,107 @@ __global__ void __launch_bounds__(256, 4) gk_inv(GArgs A, int j) {
   const int nx = g.nx;
   const int nbx = (nx + NSR_GST_TX - 1) / NSR_GST_TX;
   const int rb = blockIdx.x / nbx, cb = blockIdx.x - rb * nbx;
-  const int z0 = rb * NSR_GST_TZ;
-  const int z1 = min(z0 + NSR_GST_TZ, g.nz);
-  const int jj = cb * NSR_GST_TX + threadIdx.x;
-  if (jj >= nx) return;
-  const SysScalars sc = sys_scalars(g, S.freq);
-  const float* __restrict__ ca = A.mat.a32;
-  const float2* __restrict__ z = A.W + slot * n;
-  float2* __restrict__ w = A.w + slot * n;
-  const float2 zero = make_float2(0.f, 0.f);
-  const bool has_e = jj + 1 < nx, has_w = jj > 0;
-  long long idx = (long long)z0 * nx + jj;
-  float2 zu = z0 > 0 ? z[idx - nx] : zero;
-  float2 zc = z[idx];
-  float a_n = z0 > 0 ? __ldg(&ca[idx - nx]) : 1.0f;
-  float a_c = __ldg(&ca[idx]);
-  for (int i = z0; i < z1; ++i, idx += nx) {
-    const bool has_s = i + 1 < g.nz;
-    const float2 zd = has_s ? z[idx + nx] : zero;
-    const float a_s = has_s ? __ldg(&ca[idx + nx]) : 1.0f;
-    const float2 ze = has_e ? z[idx + 1] : zero;
-    const float2 zw = has_w ? z[idx - 1] : zero;
-    const float a_e = has_e ? __ldg(&ca[idx + 1]) : 1.0f;
-    const float a_w = has_w ? __ldg(&ca[idx - 1]) : 1.0f;
-    w[idx] = stencil_pts<ADJ>(g, sc, i, jj, a_c, a_e, a_w, a_s, a_n, __ldg(&A.mat.b32[idx]), __ldg(&A.mat.t32[idx]),
-                              zc, ze, zw, zd, zu);
-    zu = zc;
-    zc = zd;
-    a_n = a_c;
-    a_c = a_s;
-  }
-}
-
-// dot: hc_i = <v_i, w> for i <= j (FP64), into hc (pass 1 overwrites, pass 2 too)
-__global__ void __launch_bounds__(256) gk_dot(GArgs A, int j) {
-  __shared__ double tot[2 * (NSR_GMRES_MAX_M + 1)];
-  const int slot = blockIdx.y;
-  const GSlot& S = A.slots[slot];
-  if (!g_active(S, j)) return;
-  const long long n = (long long)A.g.nz * A.g.nx;
-  const long long base = (long long)blockIdx.x * blockDim.x * NSR_GDOT_CELLS;
-  const float2* w = A.w + slot * n;
-  float2 wl[NSR_GDOT_CELLS];
+  const int z0 = rb * TZ, c0 = cb * NSR_GST_TX;
+  const int jj = c0 + threadIdx.x;
+  {
+    // The loads of RB rows are issued together; the north and centre values are
+    // carried, east and west come from the adjacent lanes (loads at the warp's
+    // ends).
+    constexpr int RB = TZ < 4 ? TZ : 4;
+    const SysScalars& sc = S.sc;
+    const float kh2 = (float)sc.kh2, fpow = (float)sc.fpow;
+    if (threadIdx.x < TZ) rowf[threadIdx.x] = row_factors<float>(g, sc, z0 + threadIdx.x);
+    const ColFactors<float> cf = col_factors<float>(g, sc, jj);
+    __syncthreads();
+    const float* __restrict__ ca = A.mat.a32;
+    const float* __restrict__ cbp = A.mat.b32;
+    const float* __restrict__ ctp = A.mat.t32;
+    const float2* __restrict__ z = A.W + slot * n;
+    float2* __restrict__ w = A.w + slot * n;
+    const float2 zero = make_float2(0.f, 0.f);
+    const bool own = jj < nx;
+    const int lane = threadIdx.x & 31;
+    // lane 0 loads its west, lane 31 its east neighbour
+    const int je = lane == 0 ? jj - 1 : jj + 1;
+    const bool edge = (lane == 0 || lane == 31) && je >= 0 && je < nx;
+    const bool has_e = jj + 1 < nx, has_w = jj > 0;
+    const long long i0 = (long long)z0 * nx;
+    // Loads take clamped addresses and are selected afterwards: a condition
+    // around them would keep them from being issued together.
+    const int jc = min(jj, nx - 1), jx = edge ? je : jc;
+    const long long up = z0 > 0 ? i0 - nx : i0;
+    float2 zu = z[up + jc], zc = z[i0 + jc];
+    float a_n = __ldg(&ca[up + jc]), a_c = __ldg(&ca[i0 + jc]);
+    if (z0 == 0) { zu = zero; a_n = 1.0f; }
+    if (!own) { zc = zero; a_c = 1.0f; }
 #pragma unroll
-  for (int c = 0; c < NSR_GDOT_CELLS; ++c) {
-    const long long k = base + (long long)c * blockDim.x + threadIdx.x;
-    wl[c] = k < n ? w[k] : make_float2(0.f, 0.f);
-  }
-  double vals[2 * (NSR_GMRES_MAX_M + 1)];
-  for (int i = 0; i <= j; ++i) {
-    const float2* v = A.V + ((long long)slot * (A.m + 1) + i) * n;
-    double re = 0.0, im = 0.0;
+    for (int r0 = 0; r0 < TZ; r0 += RB) {
+      float2 zs[RB], zx[RB];
+      float as[RB], ax[RB], bb[RB], tt[RB];
 #pragma unroll
-    for (int c = 0; c < NSR_GDOT_CELLS; ++c) {
-      const long long k = base + (long long)c * blockDim.x + threadIdx.x;
-      if (k < n) dot_acc(re, im, v[k], wl[c]);
+      for (int q = 0; q < RB; ++q) {
+        const int i = z0 + r0 + q;
+        const long long ro = (long long)min(i, g.nz - 1) * nx, so = (long long)min(i + 1, g.nz - 1) * nx;
+        zs[q] = z[so + jc];
+        as[q] = __ldg(&ca[so + jc]);
+        bb[q] = __ldg(&cbp[ro + jc]);
+        tt[q] = __ldg(&ctp[ro + jc]);
+        zx[q] = z[ro + jx];
+        ax[q] = __ldg(&ca[ro + jx]);
+      }
+#pragma unroll
+      for (int q = 0; q < RB; ++q)
+        if (!own || z0 + r0 + q + 1 >= g.nz) { zs[q] = zero; as[q] = 1.0f; }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        const int i = z0 + r0 + q;
+        float2 zw = make_float2(__shfl_up_sync(0xffffffffu, zc.x, 1), __shfl_up_sync(0xffffffffu, zc.y, 1));
+        float2 ze = make_float2(__shfl_down_sync(0xffffffffu, zc.x, 1), __shfl_down_sync(0xffffffffu, zc.y, 1));
+        float a_w = __shfl_up_sync(0xffffffffu, a_c, 1), a_e = __shfl_down_sync(0xffffffffu, a_c, 1);
+        if (lane == 0) { zw = zx[q]; a_w = ax[q]; }
+        if (lane == 31) { ze = zx[q]; a_e = ax[q]; }
+        if (!has_e) { ze = zero; a_e = 1.0f; }
+        if (!has_w) { zw = zero; a_w = 1.0f; }
+        float2 v = zero;
+        if (own && i < g.nz) {
+          v = stencil_sep<float, ADJ>(kh2, fpow, rowf[r0 + q], cf, a_c, a_e, a_w, as[q], a_n, bb[q], tt[q], zc, ze, zw,
+                                      zs[q], zu);
+          w[(long long)i * nx + jj] = v;
+        }
+        wt[(r0 + q) * NSR_GST_TX + threadIdx.x] = to_d(v);
+        zu = zc;
+        zc = zs[q];
+        a_n = a_c;
+        a_c = as[q];
+      }
     }
-    vals[2 * i] = re;
-    vals[2 * i + 1] = im;
   }
-  if (g_reduce<2 * (NSR_GMRES_MAX_M + 1)>(A, slot, vals, 2 * (j + 1), tot)) {
-    for (int i = threadIdx.x; i <= j; i += blockDim.x)
+  __syncthreads();
+  const int nv = j + 1, nb = gridDim.x;
+  double* part = g_part(A, slot);
+  gs_dots<TZ * NSR_GST_TX>(wt, A.V + (long long)slot * (A.m + 1) * n, n, nv, [&](int e) -> long long {
+    return (long long)min(z0 + e / NSR_GST_TX, g.nz - 1) * nx + min(c0 + e % NSR_GST_TX, nx - 1);
+  }, part, nb, blockIdx.x);
+  if (gs_arrive(part, nb, 2 * nv, &A.arrive[slot], tot))
+    for (int i = threadIdx.x; i < nv; i += blockDim.x)
       A.hc[(long long)slot * (A.m + 1) + i] = make_double2(tot[2 * i], tot[2 * i + 1]);
-  }
 }
 
-// axpy: w -= sum_i hc_i v_i.  Pass 1 adds hc into H; pass 2 adds hc into H,
-// takes ||w||, applies the Givens rotations and decides whether the cycle stops.
-__global__ void __launch_bounds__(256) gk_axpy(GArgs A, int j, int pass) {
-  __shared__ double tot[2];
-  __shared__ float2 coef[NSR_GMRES_MAX_M + 1];
-  const int slot = blockIdx.y;
-  GSlot& S = A.slots[slot];
-  if (!g_active(S, j)) return;
-  const long long n = (long long)A.g.nz * A.g.nx;
+// Column j of the Hessenberg matrix, its Givens rotations, and whether the
+// cycle stops (one thread).
+__device__ void g_finish_step(const GArgs& A, GSlot& S, int slot, int j, const double* tot) {
   const int m = A.m;
-  const double2* hc = A.hc + (long long)slot * (m + 1);
-  for (int i = threadIdx.x; i <= j; i += blockDim.x) coef[i] = to_f(hc[i]);
-  __syncthreads();
-  const long long base = (long long)blockIdx.x * blockDim.x * NSR_GDOT_CELLS;
-  float2* w = A.w + slot * n;
-  double nrm = 0.0;
-#pragma unroll
-  for (int c = 0; c < NSR_GDOT_CELLS; ++c) {
-    const long long k = base + (long long)c * blockDim.x + threadIdx.x;
-    if (k >= n) continue;
-    float2 acc = w[k];
-    for (int i = 0; i <= j; ++i) acc = acc - coef[i] * A.V[((long long)slot * (m + 1) + i) * n + k];
-    w[k] = acc;
-    nrm += (double)acc.x * acc.x + (double)acc.y * acc.y;
-  }
-  double vals[1] = {nrm};
-  // Pass 1 needs no reduction: the coefficients go into H by the first CTA.
-  if (pass == 1) {
-    if (blockIdx.x == 0)
-      for (int i = threadIdx.x; i <= j; i += blockDim.x)
-        A.H[(long long)slot * (m + 1) * m + j * (m + 1) + i] = hc[i];
-    return;
-  }
-  if (!g_reduce<2>(A, slot, vals, 1, tot)) return;
-  if (threadIdx.x != 0) return;
   double2* Hc = A.H + (long long)slot * (m + 1) * m + j * (m + 1);   // column j
-  for (int i = 0; i <= j; ++i) Hc[i] = Hc[i] + hc[i];
-  const double hnext = sqrt(tot[0]);
+  const double2* hc = A.hc + (long long)slot * (m + 1);
+  double2* hc2 = A.hc2 + (long long)slot * (m + 1);
+  double nrm = tot[2 * (j + 1)];
+  for (int i = 0; i <= j; ++i) {
+    const double2 h2 = make_double2(tot[2 * i], tot[2 * i + 1]);
+    hc2[i] = h2;
+    Hc[i] = hc[i] + h2;
+    nrm -= h2.x * h2.x + h2.y * h2.y;
+  }
+  const double hnext = nrm > 0.0 ? sqrt(nrm) : (nrm <= 0.0 ? 0.0 : nrm);   // a NaN stays one
   Hc[j + 1] = make_double2(hnext, 0.0);
   S.hlast = hnext;
   double* cs = A.cs + (long long)slot * m;
@@ -349,6 +360,59 @@ __global__ void __launch_bounds__(256) gk_axpy(GArgs A, int j, int pass) {
   // (nsrno/wave_solver.py:31-32), at the restart length or at the budget.
   if (est < 0.5 * A.tol || !(hnext > 1e-12 * S.beta) || j + 1 == m || S.iters >= A.max_it || !isfinite(est))
     S.stop = 1;
+}
+
+// gs: w -= sum_i h_i v_i, then of the new w the second pass's inner products and
+// ||w||^2; the last CTA finishes the step.
+template <int TILE>
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_gs(GArgs A, int j) {
+  extern __shared__ __align__(16) double2 wt[];   // TILE nodes of w
+  __shared__ double tot[2 * (NSR_GMRES_MAX_M + 1) + 1];
+  __shared__ float2 coef[NSR_GMRES_MAX_M + 1];
+  const int slot = blockIdx.y;
+  GSlot& S = A.slots[slot];
+  if (!g_active(S, j)) return;
+  const long long n = (long long)A.g.nz * A.g.nx;
+  const int nv = j + 1, nb = gridDim.x;
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) coef[i] = to_f(A.hc[(long long)slot * (A.m + 1) + i]);
+  __syncthreads();
+  constexpr int C = TILE / NSR_GS_THREADS;
+  const long long base = (long long)blockIdx.x * TILE;
+  float2* __restrict__ w = A.w + slot * n;
+  const float2* __restrict__ V = A.V + (long long)slot * (A.m + 1) * n;
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
+    acc[c] = k < n ? w[k] : zero;
+  }
+  for (int i = 0; i < nv; ++i) {
+    const float2 h = coef[i];
+    const float2* __restrict__ v = V + i * n;
+    float2 x[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
+      x[c] = k < n ? v[k] : zero;
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = acc[c] - h * x[c];
+  }
+  double nrm = 0.0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int e = c * NSR_GS_THREADS + threadIdx.x;
+    const double2 d = to_d(acc[c]);
+    if (base + e < n) w[base + e] = acc[c];
+    wt[e] = d;
+    nrm += d.x * d.x + d.y * d.y;
+  }
+  double* part = g_part(A, slot);
+  nrm = gs_block_sum(nrm);   // its barriers also publish wt
+  if (threadIdx.x == 0) part[(long long)(2 * nv) * nb + blockIdx.x] = nrm;
+  gs_dots<TILE>(wt, V, n, nv, [&](int e) -> long long { return min(base + e, n - 1); }, part, nb, blockIdx.x);
+  if (gs_arrive(part, nb, 2 * nv + 1, &A.arrive[slot], tot) && threadIdx.x == 0) g_finish_step(A, S, slot, j, tot);
 }
 
 // Back substitution R y = g for the slots that ran a cycle.
@@ -405,77 +469,47 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_comb(GArgs A) {
 
 // FP64 true residual.  init = 1: x = x0 (or 0); init = 0: x += M^-1 V y.
 template <bool ADJ>
-__global__ void __launch_bounds__(256) gk_res(GArgs A, int init) {
+__global__ void __launch_bounds__(NSR_RES_TX) gk_res(GArgs A, int init) {
+  __shared__ double tot[2];
   const int slot = blockIdx.y;
   GSlot& S = A.slots[slot];
   if (S.sys < 0 || S.done) return;
   if (!init && S.used == 0) return;
   const Geo& g = A.g;
   const long long n = (long long)g.nz * g.nx;
-  const int z0 = blockIdx.x * A.tz;
-  const int nb = min(A.tz, g.nz - z0);
-  const int nx = g.nx;
   const float2* zW = A.W + slot * n;   // M^-1 u after the rinv pass
-  const SysScalars sc = sys_scalars(g, S.freq);
+  const SysScalars sc = S.sc;
   const double2* xo = A.x + (2LL * slot + S.xpar) * n;
   double2* xn = A.x + (2LL * slot + (S.xpar ^ 1)) * n;
   const float2* x0 = (init && A.x0) ? A.x0 + (long long)S.sys * n : nullptr;
-  auto P = [&](int i2, int j2) -> double2 {
-    if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= nx) return make_double2(0.0, 0.0);
-    const long long id = (long long)i2 * nx + j2;
-    if (init) return x0 ? to_d(x0[id]) : make_double2(0.0, 0.0);
-    return xo[id] + to_d(zW[id]);
-  };
-  auto Aa = [&](int i2, int j2) -> double {
-    if (i2 < 0 || i2 >= g.nz || j2 < 0 || j2 >= nx) return 1.0;
-    return __ldg(&A.mat.a64[(long long)i2 * nx + j2]);
-  };
-  const double h2 = g.h * g.h;
   const float2* rhs = A.rhs ? A.rhs + (long long)S.sys * n : nullptr;
   const double st = sin(S.angle);
   float2* r = A.r + slot * n;
-  double acc[2] = {0.0, 0.0};
-  for (int k = threadIdx.x; k < nb * nx; k += blockDim.x) {
-    const int i = z0 + k / nx, jj = k % nx;
-    const long long idx = (long long)i * nx + jj;
-    double2 b;
-    if (rhs) {
-      b = h2 * to_d(rhs[idx]);
-    } else if (i == g.face) {
-      const double2 l = source_line(g, sc.k0, st, jj);
-      b = make_double2(-l.x, -l.y);
-    } else {
-      b = make_double2(0.0, 0.0);
-    }
-    const double2 ax = stencil<double, ADJ>(g, sc, i, jj, __ldg(&A.mat.b64[idx]), __ldg(&A.mat.t64[idx]), P, Aa);
-    const double2 res = b - ax;
-    xn[idx] = P(i, jj);
-    const float2 rf = to_f(res);
-    r[idx] = rf;
-    acc[0] += res.x * res.x + res.y * res.y;
-    acc[1] += b.x * b.x + b.y * b.y;
-  }
-  __shared__ double red[NSR_NPART];
-  double vals[NSR_NPART] = {acc[0], acc[1], 0, 0, 0, 0, 0, 0};
-  block_sum<NSR_NPART>(vals, red);
-  double* part = A.partials + (long long)slot * max(A.nb_dot, A.nb_band) * 2 * (NSR_GMRES_MAX_M + 1);
-  __shared__ int am_last;
+  double rr = 0.0, bb = 0.0;
+  residual_tiles<ADJ>(
+      g, A.mat, sc,
+      [&](long long id) -> double2 {
+        if (init) return x0 ? to_d(x0[id]) : make_double2(0.0, 0.0);
+        return xo[id] + to_d(zW[id]);
+      },
+      [&](long long idx, int i, int jj) { return rhs_at(g, sc.k0, st, rhs, idx, i, jj); },
+      [&](long long idx, double2 x, double2 b, double2 res) {
+        xn[idx] = x;
+        r[idx] = to_f(res);
+        rr += res.x * res.x + res.y * res.y;
+        bb += b.x * b.x + b.y * b.y;
+      });
+  double* part = g_part(A, slot);
+  const int nb = gridDim.x;
+  rr = gs_block_sum(rr);
+  bb = gs_block_sum(bb);
   if (threadIdx.x == 0) {
-    part[blockIdx.x * 2 * (NSR_GMRES_MAX_M + 1)] = red[0];
-    part[blockIdx.x * 2 * (NSR_GMRES_MAX_M + 1) + 1] = red[1];
-    __threadfence();
-    am_last = atomicAdd(&A.arrive[slot], 1) == (int)gridDim.x - 1;
+    part[blockIdx.x] = rr;
+    part[nb + blockIdx.x] = bb;
   }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  if (threadIdx.x == 0) {
-    double rr = 0.0, bb = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) {
-      rr += __ldcg(&part[b * 2 * (NSR_GMRES_MAX_M + 1)]);
-      bb += __ldcg(&part[b * 2 * (NSR_GMRES_MAX_M + 1) + 1]);
-    }
-    A.arrive[slot] = 0;
+  if (gs_arrive(part, nb, 2, &A.arrive[slot], tot) && threadIdx.x == 0) {
+    rr = tot[0];
+    bb = tot[1];
     S.xpar ^= 1;
     if (init) S.bnorm = sqrt(bb);
     const double rn = sqrt(rr);
@@ -545,6 +579,7 @@ __global__ void gk_load(GArgs A, int first, int count, const double* freq, const
     S.gidx = A.gain_index ? A.gain_index[first + slot] : first + slot;
     S.freq = freq[first + slot];
     S.angle = angle ? angle[first + slot] : 0.0;
+    S.sc = sys_scalars(A.g, S.freq);
   } else {
     S.sys = -1;
     S.done = 1;
@@ -567,40 +602,40 @@ __global__ void gk_count(GArgs A, int* remaining) {
 // Host side.
 // ---------------------------------------------------------------------------
 struct GLayout {
-  size_t tables, slots, arrive, count, partials, H, cs, sn, gv, hc, y, V, w, W, r, x, total;
-  int nb_band, nb_dot, tz;
+  size_t tables, slots, arrive, count, partials, H, cs, sn, gv, hc, hc2, y, V, w, W, sym, r, x, total;
+  int tz, tile, nb_st, nb_gs, nb_max;   // stencil rows and Gram-Schmidt nodes of a CTA, CTAs per slot
 };
-
-static int g_band_rows(const NsrGrid* g) {
-  int budget = g->nx <= 1024 ? 8192 : 16384;
-  int tz = budget / g->nx - 2;
-  if (tz < 1) tz = 1;
-  if (tz > g->nz) tz = g->nz;
-  return tz;
-}
 
 static GLayout g_layout(const NsrGrid* g, int n_slots, int m) {
   GLayout L;
   const size_t n = (size_t)g->nz * g->nx;
-  L.tz = g_band_rows(g);
-  L.nb_band = (g->nz + L.tz - 1) / L.tz;
-  L.nb_dot = (int)((n + 256 * NSR_GDOT_CELLS - 1) / (256 * NSR_GDOT_CELLS));
-  const int nbm = L.nb_band > L.nb_dot ? L.nb_band : L.nb_dot;
+  // Tall tiles (8 rows, 2,048 nodes) amortise the reductions; a batch whose tall
+  // tiles are fewer than three CTAs per SM takes 2-row tiles of 512 nodes.
+  const int bx = (g->nx + NSR_GST_TX - 1) / NSR_GST_TX;
+  const bool tall = (long long)bx * ((g->nz + 7) / 8) * n_slots >= 3 * 148;
+  L.tz = tall ? 8 : 2;
+  L.tile = L.tz * NSR_GST_TX;
+  L.nb_st = bx * ((g->nz + L.tz - 1) / L.tz);
+  L.nb_gs = (int)((n + L.tile - 1) / L.tile);
+  L.nb_max = L.nb_st > L.nb_gs ? L.nb_st : L.nb_gs;
+  if (res_ctas(g, 1) > L.nb_max) L.nb_max = res_ctas(g, 1);
   size_t off = 0;
   L.tables = off; off += nsr_align(nsr_prec_table_bytes(g));
   L.slots = off; off += nsr_align(sizeof(GSlot) * n_slots);
   L.arrive = off; off += nsr_align(sizeof(int) * n_slots);
   L.count = off; off += nsr_align(sizeof(int));
-  L.partials = off; off += nsr_align(sizeof(double) * (size_t)n_slots * nbm * 2 * (NSR_GMRES_MAX_M + 1));
+  L.partials = off; off += nsr_align(sizeof(double) * (size_t)n_slots * L.nb_max * (2 * (m + 1) + 1));
   L.H = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * (m + 1) * m);
   L.cs = off; off += nsr_align(sizeof(double) * (size_t)n_slots * m);
   L.sn = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * m);
   L.gv = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * (m + 1));
   L.hc = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * (m + 1));
+  L.hc2 = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * (m + 1));
   L.y = off; off += nsr_align(sizeof(double2) * (size_t)n_slots * m);
   L.V = off; off += nsr_align(sizeof(float2) * n * (m + 1) * n_slots);
   L.w = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.W = off; off += nsr_align(sizeof(float2) * n * n_slots);
+  L.sym = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.r = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.x = off; off += nsr_align(sizeof(double2) * n * 2 * n_slots);
   L.total = off;
@@ -659,9 +694,7 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     A.mat = nsr_planes(material, (long long)n);
     A.m = m;
     A.n_slots = n_slots;
-    A.nb_band = L.nb_band;
-    A.nb_dot = L.nb_dot;
-    A.tz = L.tz;
+    A.nb_max = L.nb_max;
     A.rows = nsr_rows_per_cta(grid);
     A.tc = nsr_cols_tc(grid);
     A.tol = params->tolerance;
@@ -677,10 +710,12 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     A.sn = (double2*)(ws + L.sn);
     A.gv = (double2*)(ws + L.gv);
     A.hc = (double2*)(ws + L.hc);
+    A.hc2 = (double2*)(ws + L.hc2);
     A.y = (double2*)(ws + L.y);
     A.V = (float2*)(ws + L.V);
     A.w = (float2*)(ws + L.w);
     A.W = (float2*)(ws + L.W);
+    A.sym = (float2*)(ws + L.sym);
     A.r = (float2*)(ws + L.r);
     A.x = (double2*)(ws + L.x);
     A.freq = freq_hz;
@@ -695,13 +730,15 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
 
     const size_t fwd_smem = sizeof(float2) * A.rows * nsr_row_stride(grid->nx);
     const size_t col_smem = nsr_cols_smem(grid);
-    const int nb_st = ((grid->nz + NSR_GST_TZ - 1) / NSR_GST_TZ) * ((grid->nx + NSR_GST_TX - 1) / NSR_GST_TX);
     const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
     const auto fwd_fn = gx ? gk_fwd<true> : gk_fwd<false>;
     const auto rinv_fn = gx ? gk_rinv<true> : gk_rinv<false>;
     const auto comb_fn = gx ? gk_comb<true> : gk_comb<false>;
-    const auto cols_fn = A.tc == 16 ? (gz ? gk_cols<16, true> : gk_cols<16, false>)
-                                    : (gz ? gk_cols<8, true> : gk_cols<8, false>);
+    const auto cols_fn =
+        A.lp ? (A.tc == 16 ? (gz ? gk_cols<16, true, true> : gk_cols<16, false, true>)
+                           : (gz ? gk_cols<8, true, true> : gk_cols<8, false, true>))
+             : (A.tc == 16 ? (gz ? gk_cols<16, true, false> : gk_cols<16, false, false>)
+                           : (gz ? gk_cols<8, true, false> : gk_cols<8, false, false>));
     NSR_TRY(cudaFuncSetAttribute((const void*)fwd_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
     NSR_TRY(cudaFuncSetAttribute((const void*)comb_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
     NSR_TRY(cudaFuncSetAttribute((const void*)cols_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
@@ -709,49 +746,66 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
 
     const dim3 g_rows((grid->nz + A.rows - 1) / A.rows, n_slots);
     const dim3 g_col((grid->nx + A.tc - 1) / A.tc, n_slots);
-    const dim3 g_band(L.nb_band, n_slots);
-    const dim3 g_st(nb_st, n_slots);
-    const dim3 g_dot(L.nb_dot, n_slots);
+    const dim3 g_res(res_ctas(grid, n_slots), n_slots);
+    const dim3 g_st(L.nb_st, n_slots);
+    const dim3 g_gs(L.nb_gs, n_slots);
+    const bool tall = L.tz == 8;
+    const auto inv_fn = A.adjoint ? (tall ? gk_inv<true, 8> : gk_inv<true, 2>) : (tall ? gk_inv<false, 8> : gk_inv<false, 2>);
+    const auto gs_fn = tall ? gk_gs<8 * NSR_GST_TX> : gk_gs<2 * NSR_GST_TX>;
+    const size_t gs_smem = sizeof(double2) * L.tile;
     auto cols = [&](int j) {
       cols_fn<<<g_col, nsr_cols_threads(gz), col_smem, st>>>(A, j);
     };
     auto res = [&](int init) {
-      if (A.adjoint) gk_res<true><<<g_band, 256, 0, st>>>(A, init);
-      else gk_res<false><<<g_band, 256, 0, st>>>(A, init);
+      if (A.adjoint) gk_res<true><<<g_res, NSR_RES_TX, 0, st>>>(A, init);
+      else gk_res<false><<<g_res, NSR_RES_TX, 0, st>>>(A, init);
     };
 
     // One restart cycle.
-    NSR_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    for (int j = 0; j < m; ++j) {
-      fwd_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
-      cols(j);
-      rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
-      if (A.adjoint) gk_inv<true><<<g_st, 256, 0, st>>>(A, j);
-      else gk_inv<false><<<g_st, 256, 0, st>>>(A, j);
-      gk_dot<<<g_dot, 256, 0, st>>>(A, j);
-      gk_axpy<<<g_dot, 256, 0, st>>>(A, j, 1);
-      gk_dot<<<g_dot, 256, 0, st>>>(A, j);
-      gk_axpy<<<g_dot, 256, 0, st>>>(A, j, 2);
-    }
-    gk_solve<<<(n_slots + 127) / 128, 128, 0, st>>>(A);
-    comb_fn<<<g_rows, 256, fwd_smem, st>>>(A);
-    cols(-1);
-    rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, -1);
-    res(0);
-    gk_count<<<1, 256, 0, st>>>(A, remaining);
-    ce = cudaStreamEndCapture(st, &graph);
-    if (ce != cudaSuccess) { err = (int)ce; goto cleanup; }
-    NSR_TRY(cudaGraphInstantiate(&exec, graph, 0));
+    auto cycle = [&]() -> cudaError_t {
+      for (int j = 0; j < m; ++j) {
+        fwd_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
+        cols(j);
+        rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, j);
+        inv_fn<<<g_st, NSR_GS_THREADS, gs_smem, st>>>(A, j);
+        gs_fn<<<g_gs, NSR_GS_THREADS, gs_smem, st>>>(A, j);
+      }
+      gk_solve<<<(n_slots + 127) / 128, 128, 0, st>>>(A);
+      comb_fn<<<g_rows, 256, fwd_smem, st>>>(A);
+      cols(-1);
+      rinv_fn<<<g_rows, 256, fwd_smem, st>>>(A, -1);
+      res(0);
+      gk_count<<<1, 256, 0, st>>>(A, remaining);
+      return cudaGetLastError();
+    };
 
+    // The first cycle of the call is launched directly, so that a solve of one
+    // cycle (a warm start) never waits for a graph to be built; later ones
+    // replay it.
     const int max_cycles = (params->max_iterations + m - 1) / m + 1;
+    bool first_cycle = true;
     for (int first = 0; first < n_systems; first += n_slots) {
       const int count = (n_systems - first) < n_slots ? (n_systems - first) : n_slots;
       gk_load<<<(n_slots + 127) / 128, 128, 0, st>>>(A, first, count, freq_hz, A.angle);
+      if (A.lp) gk_sym<<<dim3(grid->nz < 256 ? grid->nz : 256, n_slots), 256, 0, st>>>(A);
       NSR_TRY(cudaGetLastError());
       res(1);
       NSR_TRY(cudaGetLastError());
       for (int cyc = 0; cyc < max_cycles; ++cyc) {
-        NSR_TRY(cudaGraphLaunch(exec, st));
+        if (first_cycle) {
+          NSR_TRY(cycle());
+          first_cycle = false;
+        } else {
+          if (!exec) {
+            NSR_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            ce = cycle();
+            const cudaError_t ce2 = cudaStreamEndCapture(st, &graph);
+            if (ce == cudaSuccess) ce = ce2;
+            if (ce != cudaSuccess) { err = (int)ce; goto cleanup; }
+            NSR_TRY(cudaGraphInstantiate(&exec, graph, 0));
+          }
+          NSR_TRY(cudaGraphLaunch(exec, st));
+        }
         NSR_TRY(cudaMemcpyAsync(&remaining_host, remaining, sizeof(int), cudaMemcpyDeviceToHost, st));
         NSR_TRY(cudaStreamSynchronize(st));
         if (remaining_host == 0) break;

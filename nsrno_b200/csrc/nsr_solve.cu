@@ -50,6 +50,7 @@ struct __align__(16) SlotState {
   unsigned long long t_start;   // global timer (ns) when the system started
   double bnorm2, rnorm2, resid, r0norm2;
   double freq, angle;
+  SysScalars sc;                    // scalars of freq (set when the slot starts)
   float kh2f, sigf, fpowf, pad_f;   // per-system stencil scalars in float (set when the slot starts)
   double2 rho, alpha, omega, beta;
   // s = r + c_sv v ; r_new = s + c_rt t ; y += c_yp p + c_ys s ; p_new = r_new + c_pp p + c_pv v
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(Solve
       // evaluate it once per system, in the digit-reversed (z, x) order of the
       // transformed field, for k_cols to read.
       const LearnedSpec L = load_learned_spec(A.lp);
-      const float kh2 = (float)sys_scalars(g, S.freq).kh2;
+      const float kh2 = S.kh2f;
       float2* __restrict__ sym = A.B.sym + off;
       for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
         const int l = k / g.nx;
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(PASS == PASS_GENERIC ? 256 : 512, 2) k_cols(So
       return adjoint ? conjc(mul) : mul;
     });
   } else {
-    const SysScalars s = sys_scalars(g, A.B.slots[slot].freq);
+    const SysScalars s = A.B.slots[slot].sc;
     const float inv_n = 1.0f / (float)n;
     const float2 shiftc = make_float2((float)s.kh2, (float)(s.kh2 * A.shift));
     const PrecTables& tab = A.tab;
@@ -362,10 +363,10 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_rinv(Solv
 }
 
 __device__ __forceinline__ void set_float_scalars(const Geo& g, SlotState& S) {
-  const SysScalars sc = sys_scalars(g, S.freq);
-  S.kh2f = (float)sc.kh2;
-  S.sigf = (float)sc.sig;
-  S.fpowf = (float)sc.fpow;
+  S.sc = sys_scalars(g, S.freq);
+  S.kh2f = (float)S.sc.kh2;
+  S.sigf = (float)S.sc.sig;
+  S.fpowf = (float)S.sc.fpow;
 }
 
 __device__ void pop_next(const SolveArgs& A, SlotState& S) {
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(256, 4) k_inv(SolveArgs A, int half) {
   // Every thread of a warp takes part in the shuffles; threads past the last
   // column carry zeros and store nothing.
   {
-    const SysScalars sc = sys_scalars(g, S.freq);
+    const SysScalars sc = S.sc;
     const float* __restrict__ ca = A.mat.a32;
     const float* __restrict__ cb_ = A.mat.b32;
     const float* __restrict__ ct = A.mat.t32;
@@ -1136,7 +1137,7 @@ __global__ void __launch_bounds__(256, 4) k_inv1(SolveArgs A, int half) {
 #pragma unroll
   for (int q = 0; q < NSR_NPART; ++q) acc[q] = 0.0;
   if (j < nx) {
-    const SysScalars sc = sys_scalars(g, S.freq);
+    const SysScalars sc = S.sc;
     const float* __restrict__ ca = A.mat.a32;
     const float* __restrict__ cb_ = A.mat.b32;
     const float* __restrict__ ct = A.mat.t32;
@@ -1187,21 +1188,10 @@ __global__ void __launch_bounds__(256, 4) k_inv1(SolveArgs A, int half) {
 // ---------------------------------------------------------------------------
 // res: FP64 true residual r = b - A x of a replacement (x += M^-1 y) or of a
 // new system (x = x0); emit passes only arrive and hand the slot on.
-// One thread per column of a NSR_RES_TZ x NSR_RES_TX tile walks down its rows
-// with the north/centre/south values of x and a in registers; the east and west
-// neighbours come from the adjacent lanes, the PML factors from the separable
-// form of stencil_sep (no division per node).  Bound by its FP64 arithmetic
-// and 64 B per node; 44 systems of 768 x 1024 spent 15.9 ms in this launch with
-// one thread per node, four complex divisions each, and receivers gathered
-// by one thread, 7.6 ms in this form.
+// Bound by its FP64 arithmetic and 64 B per node; 44 systems of 768 x 1024
+// spent 15.9 ms in this launch with one thread per node, four complex divisions
+// each, and receivers gathered by one thread, 9 ms on residual_tiles.
 // ---------------------------------------------------------------------------
-#define NSR_RES_TZ 8      // rows of one residual tile: 384 tiles of one 768 x 1024 system
-#define NSR_RES_TX 256
-#define NSR_RES_CTAS 1184 // CTAs of one launch over all its slots (8 per SM): most launches find no slot to
-                          // serve, and 4,224 idle CTAs cost 8 us more than 1,184
-__host__ __device__ inline int res_tiles(int nz, int nx) {
-  return ((nz + NSR_RES_TZ - 1) / NSR_RES_TZ) * ((nx + NSR_RES_TX - 1) / NSR_RES_TX);
-}
 template <bool ADJ>
 __global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
   const int slot = A.slot0 + blockIdx.y;
@@ -1210,88 +1200,40 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
   if (!(mode == MODE_RES || mode == MODE_INIT || mode == MODE_EMIT)) return;
   const Geo& g = A.g;
   const long long n = (long long)g.nz * g.nx;
-  const int nx = g.nx;
-  const int nbx = (nx + NSR_RES_TX - 1) / NSR_RES_TX;
-  const int n_tiles = res_tiles(g.nz, nx);
-  const int lane = threadIdx.x & 31;
   double acc[NSR_NPART];
 #pragma unroll
   for (int q = 0; q < NSR_NPART; ++q) acc[q] = 0.0;
-  const long long soff = slot * n;
-  const bool init = mode == MODE_INIT;
-  const SysScalars sc = sys_scalars(g, S.freq);
-  __shared__ RowFactors<double> rowf[NSR_RES_TZ];
-  for (int tile = mode == MODE_EMIT ? n_tiles : blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int rb = tile / nbx, cb = tile - rb * nbx;
-    const int z0 = rb * NSR_RES_TZ, z1 = min(z0 + NSR_RES_TZ, g.nz);
-    const int j = cb * NSR_RES_TX + threadIdx.x;
-    const bool own = j < nx;
-    __syncthreads();   // rowf of the tile before has been read
-    if (threadIdx.x < z1 - z0) rowf[threadIdx.x] = row_factors<double>(g, sc, z0 + threadIdx.x);
-    __syncthreads();
-    const ColFactors<double> cf = col_factors<double>(g, sc, j);
-    const float2* zw = A.B.w + soff;   // z = M^-1 y after the rinv pass
+  if (mode != MODE_EMIT) {
+    const bool init = mode == MODE_INIT;
+    const SysScalars sc = S.sc;
+    const float2* zw = A.B.w + slot * n;   // z = M^-1 y after the rinv pass
     const double2* xo = A.B.x + (2LL * slot + S.xpar) * n;
     double2* xn = A.B.x + (2LL * slot + (S.xpar ^ 1)) * n;
     const float2* x0 = (A.x0 && S.sys >= 0 && !S.x0_off) ? A.x0 + (long long)S.sys * n : nullptr;
-    const double2 zero = make_double2(0.0, 0.0);
-    auto P = [&](long long id) -> double2 {
-      if (init) return x0 ? to_d(x0[id]) : zero;
-      return xo[id] + to_d(zw[id]);
-    };
-    const double h2 = g.h * g.h;
     const float2* rhs = A.rhs ? A.rhs + (long long)S.sys * n : nullptr;
     const double st = sin(S.angle);
-    float2* r = A.B.r + soff;
-    float2* rh = A.B.rh + soff;
-    const bool edge_w = lane == 0, edge_e = lane == 31 || j + 1 >= nx;
-    long long idx = (long long)z0 * nx + (own ? j : 0);
-    double2 pn = own && z0 > 0 ? P(idx - nx) : zero;
-    double2 pc = own ? P(idx) : zero;
-    double an = own && z0 > 0 ? __ldg(&A.mat.a64[idx - nx]) : 1.0;
-    double ac = own ? __ldg(&A.mat.a64[idx]) : 1.0;
-    for (int i = z0; i < z1; ++i, idx += nx) {
-      const bool has_s = own && i + 1 < g.nz;
-      const double2 ps = has_s ? P(idx + nx) : zero;
-      const double as = has_s ? __ldg(&A.mat.a64[idx + nx]) : 1.0;
-      double2 pw = make_double2(__shfl_up_sync(0xffffffffu, pc.x, 1), __shfl_up_sync(0xffffffffu, pc.y, 1));
-      double2 pe = make_double2(__shfl_down_sync(0xffffffffu, pc.x, 1), __shfl_down_sync(0xffffffffu, pc.y, 1));
-      double aw = __shfl_up_sync(0xffffffffu, ac, 1), ae = __shfl_down_sync(0xffffffffu, ac, 1);
-      if (own && edge_w) {
-        pw = j > 0 ? P(idx - 1) : zero;
-        aw = j > 0 ? __ldg(&A.mat.a64[idx - 1]) : 1.0;
-      }
-      if (own && edge_e) {
-        pe = j + 1 < nx ? P(idx + 1) : zero;
-        ae = j + 1 < nx ? __ldg(&A.mat.a64[idx + 1]) : 1.0;
-      }
-      if (own) {
-        double2 b = zero;
-        if (rhs) {
-          b = h2 * to_d(rhs[idx]);
-        } else if (i == g.face) {
-          const double2 l = source_line(g, sc.k0, st, j);
-          b = make_double2(-l.x, -l.y);
-        }
-        const double2 ax = stencil_sep<double, ADJ>(sc.kh2, sc.fpow, rowf[i - z0], cf, ac, ae, aw, as, an, __ldg(&A.mat.b64[idx]),
-                                            __ldg(&A.mat.t64[idx]), pc, pe, pw, ps, pn);
-        xn[idx] = pc;
-        const float2 rf = to_f(b - ax);
-        r[idx] = rf;
-        if (init) {
-          rh[idx] = rf;
-          acc[0] += b.x * b.x + b.y * b.y;
-          acc[1] += (double)rf.x * rf.x + (double)rf.y * rf.y;
-        } else {
-          acc[0] += (double)rf.x * rf.x + (double)rf.y * rf.y;
-          dot_acc(acc[1], acc[2], rh[idx], rf);
-        }
-      }
-      pn = pc;
-      pc = ps;
-      an = ac;
-      ac = as;
-    }
+    float2* r = A.B.r + slot * n;
+    float2* rh = A.B.rh + slot * n;
+    residual_tiles<ADJ>(
+        g, A.mat, sc,
+        [&](long long id) -> double2 {
+          if (init) return x0 ? to_d(x0[id]) : make_double2(0.0, 0.0);
+          return xo[id] + to_d(zw[id]);
+        },
+        [&](long long idx, int i, int j) { return rhs_at(g, sc.k0, st, rhs, idx, i, j); },
+        [&](long long idx, double2 x, double2 b, double2 res) {
+          xn[idx] = x;
+          const float2 rf = to_f(res);
+          r[idx] = rf;
+          if (init) {
+            rh[idx] = rf;
+            acc[0] += b.x * b.x + b.y * b.y;
+            acc[1] += (double)rf.x * rf.x + (double)rf.y * rf.y;
+          } else {
+            acc[0] += (double)rf.x * rf.x + (double)rf.y * rf.y;
+            dot_acc(acc[1], acc[2], rh[idx], rf);
+          }
+        });
   }
   reduce_and_finalize(A, S, slot, mode, acc);
 }
@@ -1431,12 +1373,6 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     while (c->sr > NSR_STN_MIN_ROWS && (long long)ns * ((g->nz + c->sr - 1) / c->sr) * strips < 3 * 148) c->sr /= 2;
   }
   return 0;
-}
-
-// Residual CTAs per slot of a launch over ns slots.
-static int res_ctas(const NsrGrid* g, int ns) {
-  const int tiles = res_tiles(g->nz, g->nx), share = NSR_RES_CTAS / ns > 1 ? NSR_RES_CTAS / ns : 1;
-  return tiles < share ? tiles : share;
 }
 
 struct Layout {
