@@ -817,10 +817,59 @@ __host__ __device__ constexpr int stn_depth0(int D) {
 
 template <int W, int D, int CPT, int H>
 __host__ __device__ constexpr int stn_min_blocks() {
-  // ring, barriers and block sums (2 KB), FP64 accumulators of the consumers
-  constexpr int by_smem = (227 * 1024) / (D * StnLayout<W, H>::SLOT + 2048 + 8 * stn_parts(H) * (W / CPT));
+  // ring, barriers and block sums (2 KB), PML factors, FP64 accumulators of the consumers
+  constexpr int by_smem =
+      (227 * 1024) / (D * StnLayout<W, H>::SLOT + 2048 + 12 * (W + 66) + 8 * stn_parts(H) * (W / CPT));
   constexpr int cap = (W / CPT + 32) > 256 ? 2 : 4;
   return by_smem < 1 ? 1 : (by_smem > cap ? cap : by_smem);
+}
+
+// PML factors of one work item in shared memory: of its rows and columns
+// y = sig * profile (stretch 1 + i y), and 1 / (1 + i y) at the half nodes.
+// Half node k lies before row (column) k of the item.
+#define NSR_STN_MAX_ROWS 64
+template <int W>
+struct StnPml {
+  float yx[W], yz[NSR_STN_MAX_ROWS];
+  float2 hx[W + 1], hz[NSR_STN_MAX_ROWS + 1];
+};
+__device__ __forceinline__ float2 inv_stretch_f(float y) {   // 1 / (1 + i y)
+  const float d = 1.0f / (1.0f + y * y);
+  return make_float2(d, -y * d);
+}
+
+// The stencil at a node of the PML from those factors (r, c: its row and column
+// within the item).
+template <bool ADJ, int W>
+__device__ __forceinline__ float2 stencil_pml(const StnPml<W>& t, int r, int c, float kh2, float fpow, float a_c,
+                                              float a_e, float a_w, float a_s, float a_n, float b_c, float t_c,
+                                              float2 pc, float2 pe, float2 pw, float2 ps, float2 pn) {
+  const float2 sx = make_float2(1.0f, t.yx[c]), sz = make_float2(1.0f, t.yz[r]);
+  const float e = t_c * fpow, mb = kh2 * b_c;
+  const float2 sxz = sx * sz;
+  float2 mass = make_float2(mb * (1.0f - e * e), (ADJ ? -2.0f : 2.0f) * mb * e) * (ADJ ? conjc(sxz) : sxz);
+  float2 fe = (0.5f * (a_c + a_e)) * (sz * t.hx[c + 1]), fw = (0.5f * (a_c + a_w)) * (sz * t.hx[c]);
+  float2 fs = (0.5f * (a_c + a_s)) * (sx * t.hz[r + 1]), fn = (0.5f * (a_c + a_n)) * (sx * t.hz[r]);
+  if (ADJ) { fe = conjc(fe); fw = conjc(fw); fs = conjc(fs); fn = conjc(fn); }
+  float2 y = mass * pc;
+  y = y + fe * (pe - pc);
+  y = y + fw * (pw - pc);
+  y = y + fs * (ps - pc);
+  y = y + fn * (pn - pc);
+  return y;
+}
+// Off the PML: real fluxes.
+template <bool ADJ>
+__device__ __forceinline__ float2 stencil_plain(float kh2, float fpow, float a_c, float a_e, float a_w, float a_s,
+                                                float a_n, float b_c, float t_c, float2 pc, float2 pe, float2 pw,
+                                                float2 ps, float2 pn) {
+  const float e = t_c * fpow, mb = kh2 * b_c;
+  float2 y = make_float2(mb * (1.0f - e * e), (ADJ ? -2.0f : 2.0f) * mb * e) * pc;
+  y = y + (0.5f * (a_c + a_e)) * (pe - pc);
+  y = y + (0.5f * (a_c + a_w)) * (pw - pc);
+  y = y + (0.5f * (a_c + a_s)) * (ps - pc);
+  y = y + (0.5f * (a_c + a_n)) * (pn - pc);
+  return y;
 }
 
 template <int W, int D, int CPT, bool ADJ, int H>
@@ -842,6 +891,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
   // registers they pushed the 96-register budget of four CTAs per SM into
   // spills inside the row loop.
   __shared__ double accs[NP][NC];
+  __shared__ StnPml<W> pml;
   __shared__ int am_last;
   const Geo& g = A.g;
   const int nz = g.nz, nx = g.nx;
@@ -930,14 +980,25 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     const bool has_w = j > 0, has_e = j + CPT < nx;
     const long long soff = slot * n;
     float2* __restrict__ out = (half == 0 ? A.B.v : A.B.t) + soff;
-    SysScalarsF sf;
-    sf.kh2 = S.kh2f;
-    sf.sig = S.sigf;
-    sf.fpow = S.fpowf;
-    sf.inv_npml = g.n_pml > 0 ? 1.0f / (float)g.n_pml : 0.0f;
-    sf.lo = g.n_pml;
-    sf.hi_z = nz - 1 - g.n_pml;
-    sf.hi_x = nx - 1 - g.n_pml;
+    const float kh2 = S.kh2f, fpow = S.fpowf;
+    // interior: lo < i < hi_z, lo < j < hi_x
+    const int lo = g.n_pml, hi_z = nz - 1 - g.n_pml, hi_x = nx - 1 - g.n_pml;
+    if (z0 <= lo || z1 - 1 >= hi_z || c0 <= lo || min(c0 + W, nx) - 1 >= hi_x) {
+      // The item touches the PML: its factors, once per row and column (four
+      // complex divisions and six profiles per PML node before).
+      const float sig = S.sigf, inv_npml = g.n_pml > 0 ? 1.0f / (float)g.n_pml : 0.0f;
+      for (int k = tid; k <= W; k += NC) {
+        const float x = (float)(c0 + k);
+        if (k < W) pml.yx[k] = sig * pml_profile_f(x, nx, g.n_pml, inv_npml);
+        pml.hx[k] = inv_stretch_f(sig * pml_profile_f(x - 0.5f, nx, g.n_pml, inv_npml));
+      }
+      for (int k = tid; k <= nrows; k += NC) {
+        const float z = (float)(z0 + k);
+        if (k < nrows) pml.yz[k] = sig * pml_profile_f(z, nz, g.n_pml, inv_npml);
+        pml.hz[k] = inv_stretch_f(sig * pml_profile_f(z - 0.5f, nz, g.n_pml, inv_npml));
+      }
+      named_sync(1, NC);
+    }
     const float2 sv = f2(S.c_sv);
     // Inner products: float partial sums over NSR_STN_FLUSH rows (2 NSR_STN_FLUSH
     // products per thread), accumulated in FP64.
@@ -977,10 +1038,10 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     };
     AT bNext = bt(bpl, z0), tNext = bt(tpl, z0);
     // Interior test (no PML stretch) per column, once per item; per row below.
-    const bool col_in0 = j > sf.lo && j < sf.hi_x, col_in1 = j + CPT - 1 > sf.lo && j + CPT - 1 < sf.hi_x;
+    const bool cols_in = j > lo && j + CPT - 1 < hi_x;
     for (int k = 0; k < nrows; ++k) {
       const int i = z0 + k;
-      const bool row_in = i > sf.lo && i < sf.hi_z;
+      const bool inside = i > lo && i < hi_z && cols_in;
       const AT bRow = bNext, tRow = tNext;
       if (k + 1 < nrows) { bNext = bt(bpl, i + 1); tNext = bt(tpl, i + 1); }
       const uint32_t sS = q0 + k + 2;
@@ -1004,10 +1065,17 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
           const float2 bb = bRow, tt = tRow;
           const float4 rk = *reinterpret_cast<const float4*>(bC + Ly::ORH + 16 * tid);
           const float2 c0v = lo2(zc), c1v = hi2(zc);
-          const float2 av0 = stencil_pts_f<ADJ>(g, sf, row_in && col_in0, i, j, ac.x, ac.y, aw, as.x, an.x, bb.x,
-                                                tt.x, c0v, c1v, zw, lo2(zs), lo2(zn));
-          const float2 av1 = stencil_pts_f<ADJ>(g, sf, row_in && col_in1, i, j + 1, ac.y, ae, ac.x, as.y, an.y, bb.y,
-                                                tt.y, c1v, ze, c0v, hi2(zs), hi2(zn));
+          float2 av0, av1;
+          if (inside) {
+            av0 = stencil_plain<ADJ>(kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs), lo2(zn));
+            av1 = stencil_plain<ADJ>(kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v, hi2(zs), hi2(zn));
+          } else {
+            const int c = CPT * tid;
+            av0 = stencil_pml<ADJ>(pml, k, c, kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs),
+                                   lo2(zn));
+            av1 = stencil_pml<ADJ>(pml, k, c + 1, kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v,
+                                   hi2(zs), hi2(zn));
+          }
           *reinterpret_cast<float4*>(out + (long long)i * nx + j) = pack2(av0, av1);
           if (half == 0) {
             dot_acc_f(accf[0], accf[1], lo2(rk), av0);       // <rhat, v>
@@ -1034,8 +1102,9 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
           const float ae = has_e ? *reinterpret_cast<const float*>(bC + Ly::OA + ea + 4) : 1.0f;
           const float bb = bRow, tt = tRow;
           const float2 rk = *reinterpret_cast<const float2*>(bC + Ly::ORH + 8 * tid);
-          const float2 av = stencil_pts_f<ADJ>(g, sf, row_in && col_in0, i, j, ac, ae, aw, as, an, bb, tt, zc, ze, zw,
-                                               zs, zn);
+          const float2 av = inside ? stencil_plain<ADJ>(kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw, zs, zn)
+                                   : stencil_pml<ADJ>(pml, k, tid, kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw,
+                                                      zs, zn);
           out[(long long)i * nx + j] = av;
           if (half == 0) {
             dot_acc_f(accf[0], accf[1], rk, av);       // <rhat, v>
@@ -1339,7 +1408,7 @@ struct TileChoice {
 };
 
 static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileChoice* c) {
-  c->sw = 256; c->sd = 4; c->sr = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
+  c->sw = 256; c->sd = 0; c->sr = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
   c->tc = nsr_cols_tc(g);
   c->rows = nsr_rows_per_cta(g);
   c->groups = n_slots >= 8 ? 2 : 1;
@@ -1355,6 +1424,11 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     c->cols_staged = t->cols_staged != 0;
     c->rows_staged = t->rows_staged != 0;
   }
+  // Default ring depth 5 (256 columns, two per thread): three CTAs per SM, which
+  // leaves shared memory for a row-pass CTA of the other slot group.  22 learned
+  // 768 x 1024 systems: 47.6 us per system and iteration, 51.0 at depth 4 (four
+  // CTAs fill the shared memory), 52.1 at depth 6.
+  if (c->sd == 0) c->sd = c->sw == 256 && c->scpt == 2 ? 5 : 4;
   if (!stn_kernel(c->sw, c->sd, c->scpt, false, 1)) return NSR_ERR_ARGUMENT;
   if (c->sr != 0 && (c->sr < NSR_STN_MIN_ROWS || c->sr > 64)) return NSR_ERR_ARGUMENT;
   if (c->sctas < 0 || c->sctas > 8) return NSR_ERR_ARGUMENT;
