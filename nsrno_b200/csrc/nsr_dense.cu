@@ -12,7 +12,7 @@
 // with a = (1225/1024, -245/3072, 49/5120, -5/7168).
 // One kernel forms the staggered fluxes of a tile in shared memory and takes
 // their divergence.
-#include "nsr_internal.cuh"
+#include "nsr_dense.cuh"
 
 #include <string.h>
 
@@ -24,12 +24,6 @@ struct DenseCoef {
   // profiles along x [W] and z [H]
   const double2 *svx, *gvx, *lx, *rx;
   const double2 *svz, *gvz, *lz, *rz;
-};
-
-struct DenseGeo {
-  int H, W, pz, px, h, w;
-  double dx;
-  double2 scal;   // (D - 1) / (D k0^2)
 };
 
 __host__ __device__ inline size_t dense_coef_doubles(int H, int W) { return (size_t)H * W * 4 + 8 * (size_t)W + 8 * (size_t)H; }
@@ -265,14 +259,21 @@ static cudaError_t dense_apply_t(const DenseGeo& g, const double* coef, int nf, 
                           : launch_dense_apply<T, ADJ, 8>(g, coef, nf, x, y, st);
 }
 
-extern "C" size_t nsr_dense_coef_bytes(const NsrDenseGrid* g) {
-  if (!g || g->H <= 0 || g->W <= 0) return 0;
-  return sizeof(double) * dense_coef_doubles(g->H, g->W);
+DenseGeo nsr_dense_geo(const NsrDenseGrid* grid, double scal_re, double scal_im) {
+  DenseGeo g;
+  g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
+  g.scal = make_double2(scal_re, scal_im);
+  return g;
 }
 
-extern "C" size_t nsr_dense_workspace_size(const NsrDenseGrid* g, int32_t n_fields, int32_t precision) {
-  if (!g || g->H <= 0 || g->W <= 0 || n_fields < 0 || (precision != 0 && precision != 1)) return 0;
-  return n_fields > 0 ? 256 : 0;   // the fluxes live in shared memory
+int nsr_dense_apply_geo(const DenseGeo& g, const double* coef, int n_fields, int adjoint, int precision,
+                        const void* x, void* y, cudaStream_t st) {
+  const cudaError_t e =
+      precision == 0 ? (adjoint ? dense_apply_t<float, true>(g, coef, n_fields, x, y, st)
+                                : dense_apply_t<float, false>(g, coef, n_fields, x, y, st))
+                     : (adjoint ? dense_apply_t<double, true>(g, coef, n_fields, x, y, st)
+                                : dense_apply_t<double, false>(g, coef, n_fields, x, y, st));
+  return e == cudaSuccess ? 0 : (int)e;
 }
 
 extern "C" int nsr_dense_apply(const NsrDenseGrid* grid, const double* coef, double scal_re, double scal_im,
@@ -285,16 +286,8 @@ extern "C" int nsr_dense_apply(const NsrDenseGrid* grid, const double* coef, dou
   if (precision != 0 && precision != 1) return NSR_ERR_ARGUMENT;
   if (n_fields == 0) return 0;
   if (!workspace || workspace_bytes < nsr_dense_workspace_size(grid, n_fields, precision)) return NSR_ERR_WORKSPACE;
-  DenseGeo g;
-  g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
-  g.scal = make_double2(scal_re, scal_im);
-  cudaStream_t st = (cudaStream_t)stream;
-  const cudaError_t e =
-      precision == 0 ? (adjoint ? dense_apply_t<float, true>(g, coef, n_fields, x, y, st)
-                                : dense_apply_t<float, false>(g, coef, n_fields, x, y, st))
-                     : (adjoint ? dense_apply_t<double, true>(g, coef, n_fields, x, y, st)
-                                : dense_apply_t<double, false>(g, coef, n_fields, x, y, st));
-  return e == cudaSuccess ? 0 : (int)e;
+  return nsr_dense_apply_geo(nsr_dense_geo(grid, scal_re, scal_im), coef, n_fields, adjoint, precision, x, y,
+                             (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -375,9 +368,7 @@ extern "C" int nsr_dense_grad(const NsrDenseGrid* grid, const double* coef, doub
   if (grid->H < 3 || grid->W < 3 || grid->h < 1 || grid->w < 1 || grid->pz < 0 || grid->px < 0 ||
       grid->pz + grid->h > grid->H || grid->px + grid->w > grid->W || !(grid->dx > 0))
     return NSR_ERR_ARGUMENT;
-  DenseGeo g;
-  g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
-  g.scal = make_double2(scal_re, scal_im);
+  const DenseGeo g = nsr_dense_geo(grid, scal_re, scal_im);
   const long long n = (long long)g.H * g.W;
   int bx = (int)((n + 255) / 256);
   if (bx > 4096) bx = 4096;
@@ -483,33 +474,46 @@ extern "C" int nsr_dense_precondition(const NsrDenseGrid* grid, double k0dx2, do
   if (need == 0) return NSR_ERR_UNSUPPORTED_SIZE;
   if (workspace_bytes < need) return NSR_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
+  DensePrec M;
+  const int err = nsr_dense_prec_setup(grid, k0dx2, shift, n_fields, adjoint, workspace, st, &M);
+  if (err) return err;
+  const auto fwd = M.gx ? k_dense_rows_fwd<true> : k_dense_rows_fwd<false>;
+  fwd<<<M.g_rows, 256, M.row_smem, st>>>(grid->H, grid->W, M.t, (const float2*)x, M.w, M.rows);
+  nsr_dense_prec_finish(M, (float2*)y, st);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : (int)e;
+}
+
+int nsr_dense_prec_setup(const NsrDenseGrid* grid, double k0dx2, double shift, int n_fields, int adjoint,
+                         void* workspace, cudaStream_t st, DensePrec* M) {
   NsrGrid q = dense_fft_grid(grid);
   char* ws = (char*)workspace;
-  PrecTables t;
-  float* d2x = (float*)(ws + nsr_align(nsr_prec_table_bytes(&q)));
-  float* d2z = d2x + grid->W;
-  int err = nsr_prec_setup(&q, &t, ws, st, d2x, d2z);
+  M->geo = nsr_dense_geo(grid, 0.0, 0.0);
+  M->d2x = (float*)(ws + nsr_align(nsr_prec_table_bytes(&q)));
+  M->d2z = M->d2x + grid->W;
+  M->w = (float2*)(ws + nsr_align(nsr_prec_table_bytes(&q)) + nsr_align(sizeof(float) * (grid->H + grid->W)));
+  const int err = nsr_prec_setup(&q, &M->t, ws, st, M->d2x, M->d2z);
   if (err) return err;
-  float2* w = (float2*)(ws + nsr_align(nsr_prec_table_bytes(&q)) + nsr_align(sizeof(float) * (grid->H + grid->W)));
-  const int rows = nsr_rows_per_cta(&q);
-  const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->W);
-  const dim3 gr((grid->H + rows - 1) / rows, n_fields);
-  const bool gx = !nsr_specialised(grid->W), gz = !nsr_specialised(grid->H);
-  DenseGeo g;
-  g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
-  g.scal = make_double2(0.0, 0.0);
-  const auto fwd = gx ? k_dense_rows_fwd<true> : k_dense_rows_fwd<false>;
-  const auto inv = gx ? k_dense_rows_inv<true> : k_dense_rows_inv<false>;
-  fwd<<<gr, 256, row_smem, st>>>(grid->H, grid->W, t, (const float2*)x, w, rows);
-  const int tc = nsr_cols_tc(&q);
-  const dim3 gc((grid->W + tc - 1) / tc, n_fields);
-  const size_t csm = nsr_cols_smem(&q);
-  const auto cols = tc == 16 ? (gz ? k_dense_cols<16, true> : k_dense_cols<16, false>)
-                             : (gz ? k_dense_cols<8, true> : k_dense_cols<8, false>);
-  cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
-  cols<<<gc, nsr_cols_threads(gz), csm, st>>>(grid->H, grid->W, t, d2z, d2x, w, (float)(1.0 / k0dx2), (float)shift,
-                                              adjoint);
-  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
+  M->inv_k0dx2 = (float)(1.0 / k0dx2);
+  M->shift = (float)shift;
+  M->adjoint = adjoint;
+  M->rows = nsr_rows_per_cta(&q);
+  M->tc = nsr_cols_tc(&q);
+  M->gx = !nsr_specialised(grid->W);
+  M->gz = !nsr_specialised(grid->H);
+  M->g_rows = dim3((grid->H + M->rows - 1) / M->rows, n_fields);
+  M->g_cols = dim3((grid->W + M->tc - 1) / M->tc, n_fields);
+  M->row_smem = sizeof(float2) * (size_t)M->rows * nsr_row_stride(grid->W);
+  M->col_smem = nsr_cols_smem(&q);
+  return 0;
+}
+
+void nsr_dense_prec_finish(const DensePrec& M, float2* y, cudaStream_t st) {
+  const auto cols = M.tc == 16 ? (M.gz ? k_dense_cols<16, true> : k_dense_cols<16, false>)
+                               : (M.gz ? k_dense_cols<8, true> : k_dense_cols<8, false>);
+  cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M.col_smem);
+  cols<<<M.g_cols, nsr_cols_threads(M.gz), M.col_smem, st>>>(M.geo.H, M.geo.W, M.t, M.d2z, M.d2x, M.w, M.inv_k0dx2,
+                                                             M.shift, M.adjoint);
+  const auto inv = M.gx ? k_dense_rows_inv<true> : k_dense_rows_inv<false>;
+  inv<<<M.g_rows, 256, M.row_smem, st>>>(M.geo, M.t, M.w, y, M.rows);
 }

@@ -12,23 +12,30 @@
 // into the restart.
 //
 // Per Arnoldi step j the host enqueues (no synchronisation):
-//   z_j = M v_j                 nsr_dense_precondition (fixed shifted Laplacian)
-//   w   = A z_j                 nsr_dense_apply (complex64)
-//   h   = V_{0..j}^H w          k_dg_dots     (FP64 partials, last CTA sums)
-//   w  -= V h                   k_dg_update
-//   h' = V^H w ; w -= V h'      k_dg_dots, k_dg_update (+ ||w||^2, Givens)
-//   v_{j+1} = w / ||w||         k_dg_next
+//   rows  v_j = (w - sum_i h'_i v_i) / ||w|| (the correction of the second
+//         Gram-Schmidt pass; r / beta for j = 0), stored, and its row FFT
+//   cols, rows   z_j = M v_j, the rest of the fixed shifted Laplacian
+//   w   = A z_j                 the dense operator (complex64)
+//   h   = V_{0..j}^H w          k_dg_dots     (FP64, last CTA sums)
+//   w  -= V h, h' = V^H w, ||w||^2   k_dg_gs; the last CTA takes
+//         ||w - V h'||^2 = ||w||^2 - sum |h'_i|^2 (V is orthonormal and h' of
+//         rounding size) and forms the Givens rotation
 // and per cycle the FP64 residual, the back substitution and x += Z y.  The
-// host reads one small state record per cycle to decide whether to go on.
+// host reads one small state record per cycle to decide whether to go on.  The
+// transform tables are built once per solve.  Five fields on 160 x 192, 72
+// steps: 13.9 ms with 17 launches a step and dots whose blocks summed one value
+// at a time (37 us a launch), 5.9 ms in this form (11.0 with the new transforms
+// alone).
 #include "nsr_internal.cuh"
 #include "nsr_device.cuh"
+#include "nsr_gs.cuh"
+#include "nsr_dense.cuh"
 
 #include <stdlib.h>
 #include <string.h>
 
 #define NSR_DG_MAX_M 64
 #define NSR_DG_THREADS 256
-#define NSR_DG_GROUP 8   // basis vectors per accumulation pass of k_dg_dots
 
 struct DgState {
   int done;        // 1: converged / budget / non-finite, status is final
@@ -39,7 +46,7 @@ struct DgState {
   int cycles;      // cycles started
   int pad0, pad1;
   double bnorm;    // ||b||
-  double beta;     // ||r|| at the start of the cycle
+  double beta;     // ||r|| at the start of the cycle, then the norm that normalises the next vector
   double rel;      // true relative residual at the start of the last cycle
 };
 
@@ -49,12 +56,13 @@ struct DgArgs {
   int nb;              // CTAs of the vector kernels
   DgState* st;
   int* arrive;
-  double* part;        // [nb][2 (m + 1)]
+  double* part;        // [2 (m + 1) + 1][CTAs of the launch]
   double2* H;          // [(m + 1) m], column j at H[j (m + 1) + i]
   double* cs;          // [m]
   double2* sn;         // [m]
   double2* gv;         // [m + 1]
-  double2* hc;         // [m + 1] coefficients of the current Gram-Schmidt pass
+  double2* hc;         // [m + 1] coefficients of the first Gram-Schmidt pass
+  double2* hc2;        // [m + 1] and of the second
   double2* y;          // [m]
   float2* V;           // [m + 1][n]
   float2* Z;           // [m][n]
@@ -85,7 +93,7 @@ __device__ bool dg_arrive(const DgArgs& A, const double* mine, int nv, double* t
   __shared__ int last;
   __shared__ double red[NSR_DG_THREADS / 32];
   if (threadIdx.x == 0) {
-    for (int q = 0; q < nv; ++q) A.part[(long long)blockIdx.x * 2 * (A.m + 1) + q] = mine[q];
+    for (int q = 0; q < nv; ++q) A.part[(long long)blockIdx.x * nv + q] = mine[q];
     __threadfence();
     last = atomicAdd(A.arrive, 1) == (int)gridDim.x - 1;
   }
@@ -95,7 +103,7 @@ __device__ bool dg_arrive(const DgArgs& A, const double* mine, int nv, double* t
   for (int q = 0; q < nv; ++q) {
     double s = 0.0;
     for (int b = threadIdx.x; b < (int)gridDim.x; b += NSR_DG_THREADS)
-      s += __ldcg(&A.part[(long long)b * 2 * (A.m + 1) + q]);
+      s += __ldcg(&A.part[(long long)b * nv + q]);
     s = dg_block_sum(s, red);
     if (threadIdx.x == 0) tot[q] = s;
   }
@@ -167,158 +175,191 @@ __global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_residual(DgArgs A) {
   }
 }
 
-// v_0 /= beta (the division of the reference's basis[0] = r / beta).
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_scale0(DgArgs A) {
-  const DgState& S = *A.st;
-  if (S.done) return;
-  const float inv = (float)(1.0 / S.beta);
-  for (long long e = blockIdx.x * (long long)NSR_DG_THREADS + threadIdx.x; e < A.n;
-       e += (long long)gridDim.x * NSR_DG_THREADS) {
-    const float2 v = A.V[e];
-    A.V[e] = make_float2(v.x * inv, v.y * inv);
-  }
-}
-
 __device__ __forceinline__ bool dg_skip(const DgState& S) { return S.done || S.stop; }
 
-// hc[i] = <v_i, w> for i <= j, also added to column j of the Hessenberg matrix
-// (the two Gram-Schmidt passes sum into it).
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_dots(DgArgs A, int j) {
-  __shared__ double red[NSR_DG_THREADS / 32];
-  __shared__ double mine[2 * (NSR_DG_MAX_M + 1)], tot[2 * (NSR_DG_MAX_M + 1)];
+// hc[i] = <v_i, w> for i <= j of one tile of w.
+template <int TILE>
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_dots(DgArgs A, int j) {
+  __shared__ double2 wt[TILE];
+  __shared__ double tot[2 * (NSR_DG_MAX_M + 1)];
   if (dg_skip(*A.st)) return;
-  const int nv = j + 1;
-  for (int i0 = 0; i0 < nv; i0 += NSR_DG_GROUP) {
-    const int cnt = min(NSR_DG_GROUP, nv - i0);
-    double re[NSR_DG_GROUP], im[NSR_DG_GROUP];
+  const int nv = j + 1, nb = gridDim.x;
+  const long long base = (long long)blockIdx.x * TILE;
 #pragma unroll
-    for (int k = 0; k < NSR_DG_GROUP; ++k) re[k] = im[k] = 0.0;
-    for (long long e = blockIdx.x * (long long)NSR_DG_THREADS + threadIdx.x; e < A.n;
-         e += (long long)gridDim.x * NSR_DG_THREADS) {
-      const float2 wv = A.w[e];
-#pragma unroll
-      for (int k = 0; k < NSR_DG_GROUP; ++k)
-        if (k < cnt) dot_acc(re[k], im[k], A.V[(long long)(i0 + k) * A.n + e], wv);
-    }
-#pragma unroll
-    for (int k = 0; k < NSR_DG_GROUP; ++k) {
-      if (k < cnt) {
-        const double sr = dg_block_sum(re[k], red);
-        const double si = dg_block_sum(im[k], red);
-        if (threadIdx.x == 0) { mine[2 * (i0 + k)] = sr; mine[2 * (i0 + k) + 1] = si; }
-      }
-    }
-  }
+  for (int e = threadIdx.x; e < TILE; e += NSR_GS_THREADS)
+    wt[e] = base + e < A.n ? to_d(A.w[base + e]) : make_double2(0.0, 0.0);
   __syncthreads();
-  if (dg_arrive(A, mine, 2 * nv, tot)) {
-    for (int i = threadIdx.x; i < nv; i += NSR_DG_THREADS) {
-      const double2 h = make_double2(tot[2 * i], tot[2 * i + 1]);
-      A.hc[i] = h;
-      A.H[(long long)j * (A.m + 1) + i] = A.H[(long long)j * (A.m + 1) + i] + h;
-    }
-  }
+  gs_dots<TILE>(wt, A.V, A.n, nv, [&](int e) -> long long { return min(base + e, A.n - 1); }, A.part, nb,
+                blockIdx.x);
+  if (gs_arrive(A.part, nb, 2 * nv, A.arrive, tot))
+    for (int i = threadIdx.x; i < nv; i += NSR_GS_THREADS) A.hc[i] = make_double2(tot[2 * i], tot[2 * i + 1]);
 }
 
-// w -= sum_i hc[i] v_i.  With `last`, also ||w||^2; the last CTA then
-// completes column j of the Hessenberg matrix, applies the earlier Givens
-// rotations, forms the new one and detects a happy breakdown.
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_update(DgArgs A, int j, int last) {
-  __shared__ double red[NSR_DG_THREADS / 32];
-  __shared__ double mine[1], tot[1];
+// Column j of the Hessenberg matrix, the earlier Givens rotations on it, the new
+// one, and the happy breakdown (one thread).
+__device__ void dg_finish_step(const DgArgs& A, int j, const double* tot) {
+  DgState& S = *A.st;
+  const int m1 = A.m + 1;
+  double2* col = A.H + (long long)j * m1;
+  double nrm = tot[2 * (j + 1)];
+  for (int i = 0; i <= j; ++i) {
+    const double2 h2 = make_double2(tot[2 * i], tot[2 * i + 1]);
+    A.hc2[i] = h2;
+    col[i] = A.hc[i] + h2;
+    nrm -= h2.x * h2.x + h2.y * h2.y;
+  }
+  const double hn = nrm > 0.0 ? sqrt(nrm) : (nrm <= 0.0 ? 0.0 : nrm);   // a NaN stays one
+  col[j + 1] = make_double2(hn, 0.0);
+  S.steps += 1;
+  S.used = j + 1;
+  // Givens rotations G_i = [[c, s], [-conj(s), c]] (c real) applied to rows i, i+1.
+  for (int i = 0; i < j; ++i) {
+    const double2 a = col[i], b = col[i + 1];
+    col[i] = A.cs[i] * a + A.sn[i] * b;
+    col[i + 1] = A.cs[i] * b - conjc(A.sn[i]) * a;
+  }
+  const double2 a = col[j];
+  const double an = sqrt(a.x * a.x + a.y * a.y);
+  const double den = sqrt(an * an + hn * hn);
+  double c;
+  double2 sgn;
+  if (den == 0.0) {
+    c = 1.0; sgn = make_double2(0.0, 0.0);
+  } else if (an == 0.0) {
+    c = 0.0; sgn = make_double2(1.0, 0.0);
+  } else {
+    c = an / den;
+    const double2 ph = make_double2(a.x / an, a.y / an);
+    sgn = (hn / den) * ph;   // s = (a / |a|) hn / den
+  }
+  A.cs[j] = c;
+  A.sn[j] = sgn;
+  col[j] = c * a + hn * sgn;   // = (a / |a|) den
+  col[j + 1] = make_double2(0.0, 0.0);
+  const double2 g = A.gv[j];
+  A.gv[j] = c * g;
+  A.gv[j + 1] = make_double2(0.0, 0.0) - conjc(sgn) * g;
+  if (!isfinite(hn)) {
+    S.done = 1;
+    S.status = NSR_NONFINITE;
+  } else if (hn < 1e-12) {
+    S.stop = 1;   // happy breakdown (nsrno/wave_solver.py:29-31)
+  }
+  S.beta = hn;   // normaliser of v_{j+1}
+}
+
+// w -= sum_i hc[i] v_i (FP64), then of the new w the second pass's inner products
+// and ||w||^2; the last CTA finishes the step.
+template <int TILE>
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_gs(DgArgs A, int j) {
+  __shared__ double2 wt[TILE];
+  __shared__ double tot[2 * (NSR_DG_MAX_M + 1) + 1];
   __shared__ double2 h[NSR_DG_MAX_M + 1];
   if (dg_skip(*A.st)) return;
-  const int nv = j + 1;
-  for (int i = threadIdx.x; i < nv; i += NSR_DG_THREADS) h[i] = A.hc[i];
+  const int nv = j + 1, nb = gridDim.x;
+  for (int i = threadIdx.x; i < nv; i += NSR_GS_THREADS) h[i] = A.hc[i];
   __syncthreads();
-  double s = 0.0;
-  for (long long e = blockIdx.x * (long long)NSR_DG_THREADS + threadIdx.x; e < A.n;
-       e += (long long)gridDim.x * NSR_DG_THREADS) {
-    float2 wv = A.w[e];
-    double2 acc = make_double2(wv.x, wv.y);
-    for (int i = 0; i < nv; ++i) {
-      const float2 v = A.V[(long long)i * A.n + e];
-      const double2 hi = h[i];
-      acc.x -= hi.x * v.x - hi.y * v.y;
-      acc.y -= hi.x * v.y + hi.y * v.x;
-    }
-    wv = to_f(acc);
-    A.w[e] = wv;
-    if (last) s += (double)wv.x * wv.x + (double)wv.y * wv.y;
+  const long long base = (long long)blockIdx.x * TILE;
+  constexpr int C = TILE / NSR_GS_THREADS;
+  const float2 zero = make_float2(0.f, 0.f);
+  double2 acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
+    acc[c] = to_d(k < A.n ? A.w[k] : zero);
   }
-  if (!last) return;
-  s = dg_block_sum(s, red);
-  if (threadIdx.x == 0) mine[0] = s;
-  if (dg_arrive(A, mine, 1, tot) && threadIdx.x == 0) {
-    DgState& S = *A.st;
-    const int m1 = A.m + 1;
-    double2* col = A.H + (long long)j * m1;
-    const double hn = sqrt(tot[0]);
-    col[j + 1] = make_double2(hn, 0.0);
-    S.steps += 1;
-    S.used = j + 1;
-    // Givens rotations G_i = [[c, s], [-conj(s), c]] (c real) applied to rows i, i+1.
-    for (int i = 0; i < j; ++i) {
-      const double2 a = col[i], b = col[i + 1];
-      col[i] = A.cs[i] * a + A.sn[i] * b;
-      col[i + 1] = A.cs[i] * b - conjc(A.sn[i]) * a;
+#pragma unroll 4
+  for (int i = 0; i < nv; ++i) {
+    const float2* __restrict__ v = A.V + i * A.n;
+    const double2 hi = h[i];
+    float2 x[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
+      x[c] = k < A.n ? v[k] : zero;
     }
-    const double2 a = col[j];
-    const double an = sqrt(a.x * a.x + a.y * a.y);
-    const double den = sqrt(an * an + hn * hn);
-    double c;
-    double2 sgn;
-    if (den == 0.0) {
-      c = 1.0; sgn = make_double2(0.0, 0.0);
-    } else if (an == 0.0) {
-      c = 0.0; sgn = make_double2(1.0, 0.0);
-    } else {
-      c = an / den;
-      const double2 ph = make_double2(a.x / an, a.y / an);
-      sgn = (hn / den) * ph;   // s = (a / |a|) hn / den
-    }
-    A.cs[j] = c;
-    A.sn[j] = sgn;
-    col[j] = c * a + hn * sgn;   // = (a / |a|) den
-    col[j + 1] = make_double2(0.0, 0.0);
-    const double2 g = A.gv[j];
-    A.gv[j] = c * g;
-    A.gv[j + 1] = make_double2(0.0, 0.0) - conjc(sgn) * g;
-    if (!isfinite(hn)) {
-      S.done = 1;
-      S.status = NSR_NONFINITE;
-    } else if (hn < 1e-12) {
-      S.stop = 1;   // happy breakdown (nsrno/wave_solver.py:29-31)
-    }
-    S.beta = hn;   // normaliser of v_{j+1}
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = acc[c] - hi * to_d(x[c]);
   }
+  double nrm = 0.0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int e = c * NSR_GS_THREADS + threadIdx.x;
+    const float2 f = to_f(acc[c]);
+    const double2 d = to_d(f);
+    if (base + e < A.n) A.w[base + e] = f;
+    wt[e] = d;
+    nrm += d.x * d.x + d.y * d.y;
+  }
+  nrm = gs_block_sum(nrm);   // its barriers also publish wt
+  if (threadIdx.x == 0) A.part[(long long)(2 * nv) * nb + blockIdx.x] = nrm;
+  gs_dots<TILE>(wt, A.V, A.n, nv, [&](int e) -> long long { return min(base + e, A.n - 1); }, A.part, nb,
+                blockIdx.x);
+  if (gs_arrive(A.part, nb, 2 * nv + 1, A.arrive, tot) && threadIdx.x == 0) dg_finish_step(A, j, tot);
 }
 
-// v_{j+1} = w / ||w|| (skipped after a happy breakdown).
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_next(DgArgs A, int j) {
+// v_j and its row transform: the elementwise work runs inside the transform's
+// first stage.
+template <bool GEN>
+__global__ void __launch_bounds__(256, GEN ? 2 : 3) k_dg_rows(DgArgs A, int nz, int nx, PrecTables t,
+                                                              float2* __restrict__ W, int rows, int j) {
+  extern __shared__ float2 sm[];
+  __shared__ double2 c2[NSR_DG_MAX_M];
   const DgState& S = *A.st;
   if (dg_skip(S)) return;
+  for (int i = threadIdx.x; i < j; i += blockDim.x) c2[i] = A.hc2[i];
+  __syncthreads();
   const float inv = (float)(1.0 / S.beta);
-  float2* v = A.V + (long long)(j + 1) * A.n;
-  for (long long e = blockIdx.x * (long long)NSR_DG_THREADS + threadIdx.x; e < A.n;
-       e += (long long)gridDim.x * NSR_DG_THREADS) {
-    const float2 wv = A.w[e];
-    v[e] = make_float2(wv.x * inv, wv.y * inv);
-  }
+  const int z0 = blockIdx.x * rows;
+  const long long off = blockIdx.y * (long long)nz * nx + (long long)z0 * nx;
+  const float2* src = (j == 0 ? A.V : A.w) + off;   // k_dg_residual leaves r in V
+  float2* vj = A.V + (long long)j * A.n + off;
+  const float2* V = A.V + off;
+  rows_forward<GEN>(sm, min(rows, nz - z0), t.px, W + off, [&](auto tag, int k0, int step, float2* v) {
+    constexpr int R = decltype(tag)::value;
+    if (j == 0) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = inv * src[k0 + q * step];
+    } else {
+      constexpr int CH = R <= 4 ? R : 1;
+#pragma unroll
+      for (int c = 0; c < R; c += CH) {
+        double2 acc[CH];
+#pragma unroll
+        for (int q = 0; q < CH; ++q) acc[q] = to_d(src[k0 + (c + q) * step]);
+        for (int i = 0; i < j; ++i) {
+          const double2 h = c2[i];
+#pragma unroll
+          for (int q = 0; q < CH; ++q) acc[q] = acc[q] - h * to_d(V[(long long)i * A.n + k0 + (c + q) * step]);
+        }
+#pragma unroll
+        for (int q = 0; q < CH; ++q) v[c + q] = inv * to_f(acc[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) vj[k0 + q * step] = v[q];
+  });
 }
 
-// y = R^-1 g over the steps of the cycle (FP64, one thread).
+// y = R^-1 g over the steps of the cycle (FP64).
 __global__ void k_dg_solve(DgArgs A) {
+  // One warp, column by column: once y_i is known every lane takes its share of
+  // the rows above it.
+  __shared__ double2 g[NSR_DG_MAX_M];
   const DgState& S = *A.st;
-  if (S.done || threadIdx.x != 0) return;
+  if (S.done) return;
   const int k = S.used;
   const int m1 = A.m + 1;
+  for (int i = threadIdx.x; i < k; i += 32) g[i] = A.gv[i];
+  __syncwarp();
   for (int i = k - 1; i >= 0; --i) {
-    double2 s = A.gv[i];
-    for (int l = i + 1; l < k; ++l) s = s - A.H[(long long)l * m1 + i] * A.y[l];
-    A.y[i] = divc(s, A.H[(long long)i * m1 + i]);
+    const double2* col = A.H + (long long)i * m1;
+    const double2 y = divc(g[i], col[i]);
+    __syncwarp();
+    if (threadIdx.x == 0) A.y[i] = y;
+    for (int l = threadIdx.x; l < i; l += 32) g[l] = g[l] - col[l] * y;
+    __syncwarp();
   }
-  // a fresh Hessenberg matrix for the next cycle
-  for (int e = 0; e < m1 * A.m; ++e) A.H[e] = make_double2(0.0, 0.0);
 }
 
 // x += sum_j y_j z_j (FP64).
@@ -383,8 +424,8 @@ __global__ void k_dg_zero_ints(int* p, int n) {
 // Host side.
 // ---------------------------------------------------------------------------
 struct DgLayout {
-  size_t state, arrive, part, small, V, Z, w, ax, apply_ws, prec_ws, total;
-  int nb;
+  size_t state, arrive, part, small, V, Z, w, ax, prec_ws, total;
+  int nb, tile, nb_gs;
 };
 
 static int dg_blocks() {
@@ -400,13 +441,19 @@ static DgLayout dg_layout(const NsrDenseGrid* g, int n_fields, int m, int nb) {
   L.nb = nb;
   L.state = off; off += nsr_align(sizeof(DgState));
   L.arrive = off; off += nsr_align(sizeof(int) * (1 + (size_t)n_fields));
-  L.part = off; off += nsr_align(sizeof(double) * 2 * (size_t)(m + 1) * (nb > n_fields * 64 ? nb : n_fields * 64));
-  L.small = off; off += nsr_align(sizeof(double2) * ((size_t)(m + 1) * m + 4 * (m + 1)) + sizeof(double) * m);
+  // Gram-Schmidt tiles: 2,048 nodes, or 512 where those would be fewer than three per SM.
+  L.tile = (n + 2047) / 2048 >= 3 * 148 ? 2048 : 512;
+  L.nb_gs = (int)((n + L.tile - 1) / L.tile);
+  size_t parts = (size_t)(2 * (m + 1) + 1) * L.nb_gs;
+  if (parts < (size_t)2 * nb) parts = (size_t)2 * nb;
+  if (parts < (size_t)2 * n_fields * (nb / n_fields > 8 ? nb / n_fields : 8))
+    parts = (size_t)2 * n_fields * (nb / n_fields > 8 ? nb / n_fields : 8);
+  L.part = off; off += nsr_align(sizeof(double) * parts);
+  L.small = off; off += nsr_align(sizeof(double2) * ((size_t)(m + 1) * m + 5 * (m + 1)) + sizeof(double) * m);
   L.V = off; off += nsr_align(sizeof(float2) * n * (m + 1));
   L.Z = off; off += nsr_align(sizeof(float2) * n * m);
   L.w = off; off += nsr_align(sizeof(float2) * n);
   L.ax = off; off += nsr_align(sizeof(double2) * n);
-  L.apply_ws = off; off += nsr_align(nsr_dense_workspace_size(g, n_fields, 1));
   L.prec_ws = off; off += nsr_align(nsr_dense_precondition_workspace_size(g, n_fields));
   L.total = off;
   return L;
@@ -426,6 +473,9 @@ extern "C" int nsr_dense_solve(const NsrDenseGrid* grid, const double* coef, con
   if (m < 1 || m > NSR_DG_MAX_M || p->max_cycles < 1 || !(p->tolerance > 0) || !(p->k0dx2 > 0) || !(p->shift >= 0))
     return NSR_ERR_ARGUMENT;
   if (nsr_dense_precondition_workspace_size(grid, n_fields) == 0) return NSR_ERR_UNSUPPORTED_SIZE;
+  if (grid->h < 1 || grid->w < 1 || grid->pz < 0 || grid->px < 0 || grid->pz + grid->h > grid->H ||
+      grid->px + grid->w > grid->W || !(grid->dx > 0))
+    return NSR_ERR_ARGUMENT;
   const int nb = dg_blocks();
   const DgLayout L = dg_layout(grid, n_fields, m, nb);
   if (workspace_bytes < L.total) return NSR_ERR_WORKSPACE;
@@ -445,7 +495,8 @@ extern "C" int nsr_dense_solve(const NsrDenseGrid* grid, const double* coef, con
   A.sn = A.H + (size_t)(m + 1) * m;
   A.gv = A.sn + (m + 1);
   A.hc = A.gv + (m + 1);
-  A.y = A.hc + (m + 1);
+  A.hc2 = A.hc + (m + 1);
+  A.y = A.hc2 + (m + 1);
   A.cs = (double*)(A.y + (m + 1));
   A.V = (float2*)(ws + L.V);
   A.Z = (float2*)(ws + L.Z);
@@ -455,10 +506,6 @@ extern "C" int nsr_dense_solve(const NsrDenseGrid* grid, const double* coef, con
   A.ax = (const double2*)(ws + L.ax);
   A.tol = p->tolerance;
   A.max_cycles = p->max_cycles;
-  void* apply_ws = ws + L.apply_ws;
-  const size_t apply_bytes = nsr_dense_workspace_size(grid, n_fields, 1);
-  void* prec_ws = ws + L.prec_ws;
-  const size_t prec_bytes = nsr_dense_precondition_workspace_size(grid, n_fields);
   const int adj = p->adjoint ? 1 : 0;
   int err = 0;
   // Pinned host record of the solve state, one per host thread, kept for the
@@ -468,30 +515,30 @@ extern "C" int nsr_dense_solve(const NsrDenseGrid* grid, const double* coef, con
     host = nullptr;
     return cudaErrorMemoryAllocation;
   }
+  DensePrec M;
+  err = nsr_dense_prec_setup(grid, p->k0dx2, p->shift, n_fields, adj, ws + L.prec_ws, st, &M);
+  if (err) return err;
+  const DenseGeo geo = nsr_dense_geo(grid, p->scal_re, p->scal_im);
+  const auto rows_fn = M.gx ? k_dg_rows<true> : k_dg_rows<false>;
+  const auto dots_fn = L.tile == 2048 ? k_dg_dots<2048> : k_dg_dots<512>;
+  const auto gs_fn = L.tile == 2048 ? k_dg_gs<2048> : k_dg_gs<512>;
 #define DG_TRY(expr) do { int e_ = (int)(expr); if (e_) { err = e_; goto done; } } while (0)
   k_dg_zero_ints<<<1, 256, 0, st>>>(A.arrive, 1 + n_fields);
-  DG_TRY(cudaMemsetAsync(A.H, 0, sizeof(double2) * (size_t)(m + 1) * m, st));
   k_dg_bnorm<<<nb, NSR_DG_THREADS, 0, st>>>(A);
   DG_TRY(cudaGetLastError());
   for (;;) {
-    DG_TRY(nsr_dense_apply(grid, coef, p->scal_re, p->scal_im, n_fields, adj, 1, x, (void*)A.ax, apply_ws,
-                           apply_bytes, stream));
+    DG_TRY(nsr_dense_apply_geo(geo, coef, n_fields, adj, 1, x, (void*)A.ax, st));
     k_dg_residual<<<nb, NSR_DG_THREADS, 0, st>>>(A);
     DG_TRY(cudaGetLastError());
     DG_TRY(cudaMemcpyAsync(host, A.st, sizeof(DgState), cudaMemcpyDeviceToHost, st));
     DG_TRY(cudaStreamSynchronize(st));
     if (host->done) break;
-    k_dg_scale0<<<nb, NSR_DG_THREADS, 0, st>>>(A);
     for (int j = 0; j < m; ++j) {
-      DG_TRY(nsr_dense_precondition(grid, p->k0dx2, p->shift, n_fields, adj, (const float*)(A.V + j * A.n),
-                                    (float*)(A.Z + j * A.n), prec_ws, prec_bytes, stream));
-      DG_TRY(nsr_dense_apply(grid, coef, p->scal_re, p->scal_im, n_fields, adj, 0, A.Z + j * A.n, A.w, apply_ws,
-                             apply_bytes, stream));
-      k_dg_dots<<<nb, NSR_DG_THREADS, 0, st>>>(A, j);
-      k_dg_update<<<nb, NSR_DG_THREADS, 0, st>>>(A, j, 0);
-      k_dg_dots<<<nb, NSR_DG_THREADS, 0, st>>>(A, j);
-      k_dg_update<<<nb, NSR_DG_THREADS, 0, st>>>(A, j, 1);
-      k_dg_next<<<nb, NSR_DG_THREADS, 0, st>>>(A, j);
+      rows_fn<<<M.g_rows, 256, M.row_smem, st>>>(A, grid->H, grid->W, M.t, M.w, M.rows, j);
+      nsr_dense_prec_finish(M, A.Z + j * A.n, st);
+      DG_TRY(nsr_dense_apply_geo(geo, coef, n_fields, adj, 0, A.Z + j * A.n, A.w, st));
+      dots_fn<<<L.nb_gs, NSR_GS_THREADS, 0, st>>>(A, j);
+      gs_fn<<<L.nb_gs, NSR_GS_THREADS, 0, st>>>(A, j);
       DG_TRY(cudaGetLastError());
     }
     k_dg_solve<<<1, 32, 0, st>>>(A);
