@@ -259,6 +259,16 @@ static cudaError_t dense_apply_t(const DenseGeo& g, const double* coef, int nf, 
                           : launch_dense_apply<T, ADJ, 8>(g, coef, nf, x, y, st);
 }
 
+extern "C" size_t nsr_dense_coef_bytes(const NsrDenseGrid* g) {
+  if (!g || g->H <= 0 || g->W <= 0) return 0;
+  return sizeof(double) * dense_coef_doubles(g->H, g->W);
+}
+
+extern "C" size_t nsr_dense_workspace_size(const NsrDenseGrid* g, int32_t n_fields, int32_t precision) {
+  if (!g || g->H <= 0 || g->W <= 0 || n_fields < 0 || (precision != 0 && precision != 1)) return 0;
+  return n_fields > 0 ? 256 : 0;   // the fluxes live in shared memory
+}
+
 DenseGeo nsr_dense_geo(const NsrDenseGrid* grid, double scal_re, double scal_im) {
   DenseGeo g;
   g.H = grid->H; g.W = grid->W; g.pz = grid->pz; g.px = grid->px; g.h = grid->h; g.w = grid->w; g.dx = grid->dx;
