@@ -114,88 +114,238 @@ __device__ __forceinline__ void node_maps(const T* __restrict__ maps, int hw, in
 // ---------------------------------------------------------------------------
 // Set-up: context and pooling, convolutions, gains.
 // ---------------------------------------------------------------------------
+// A thread takes one column of a low-resolution row (8 nodes) and eight lanes
+// combine to a pixel, so the grid fills the chip at every size (one thread per
+// pixel left 96 blocks with 192 serial logarithms each: 63 us at 768 x 1024).
+// Four nodes share a logarithm: the logs of c and rho add up in a product (four
+// floats stay in double range), log1p(alpha) in 1 + q = prod (1 + alpha) with q
+// kept apart from the 1.  Bound by the logarithms' FP64; 6 us.
 template <typename T>
-__global__ void k_lp_pool(int nz, int nx, int h8, int w8, const float* __restrict__ c, const float* __restrict__ rho,
-                          const float* __restrict__ alpha, const double* __restrict__ freq, int n_freq,
-                          T* __restrict__ state) {
+__global__ void __launch_bounds__(256) k_lp_pool(int nz, int nx, int h8, int w8, const float* __restrict__ c,
+                                                 const float* __restrict__ rho, const float* __restrict__ alpha,
+                                                 const double* __restrict__ freq, int n_freq, T* __restrict__ state) {
   const int hw = h8 * w8;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= hw) return;
-  const int py = p / w8, px = p - py * w8;
+  const int nbx = (8 * w8 + 255) / 256;
+  const int py = blockIdx.x / nbx, x = (blockIdx.x % nbx) * 256 + threadIdx.x;
+  const bool own = x < 8 * w8;
+  const int xc = own ? x : 8 * w8 - 1;
+  const double c4 = 1540.0 * 1540.0 * 1540.0 * 1540.0, r4 = 1e12;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (int dy = 0; dy < 8; ++dy)
-    for (int dx = 0; dx < 8; ++dx) {
-      const long long k = (long long)(8 * py + dy) * nx + 8 * px + dx;
-      s0 += log((double)c[k] / 1540.0) / 0.06;
-      s1 += log((double)rho[k] / 1000.0) / 0.08;
-      s2 += log1p((double)alpha[k]);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    double pc = 1.0, pr = 1.0, q = 0.0;
+    bool bad = false;
+#pragma unroll
+    for (int dy = 0; dy < 4; ++dy) {
+      const long long k = (long long)(8 * py + 4 * h + dy) * nx + xc;
+      const double a = alpha[k];
+      pc *= (double)c[k];
+      pr *= (double)rho[k];
+      q = q + a + q * a;
+      bad = bad || !(a >= -1.0);
     }
-  for (int f = 0; f < n_freq; ++f) {
+    s0 += log(pc / c4);
+    s1 += log(pr / r4);
+    s2 += bad ? NAN : log1p(q);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    s0 += __shfl_down_sync(0xffffffffu, s0, o, 8);
+    s1 += __shfl_down_sync(0xffffffffu, s1, o, 8);
+    s2 += __shfl_down_sync(0xffffffffu, s2, o, 8);
+  }
+  // every lane of the pixel writes some of the frequencies
+  s0 = __shfl_sync(0xffffffffu, s0, 0, 8);
+  s1 = __shfl_sync(0xffffffffu, s1, 0, 8);
+  s2 = __shfl_sync(0xffffffffu, s2, 0, 8);
+  if (!own) return;
+  const int p = py * w8 + (x >> 3);
+  for (int f = x & 7; f < n_freq; f += 8) {
     T* sp = state + (long long)f * LP_PLANES * hw + LP_POOL * hw;
-    stv(sp + p, (float)(s0 / 64.0));
-    stv(sp + hw + p, (float)(s1 / 64.0));
+    stv(sp + p, (float)(s0 / 0.06 / 64.0));
+    stv(sp + hw + p, (float)(s1 / 0.08 / 64.0));
     stv(sp + 2 * hw + p, (float)(s2 / 64.0));
     stv(sp + 3 * hw + p, (float)(freq[f] / 6e6 - 1.0));
     stv(sp + 4 * hw + p, 1.0f);
   }
 }
 
-// 3x3 cross-correlation, zero padding 1, one thread per pixel and all COUT outputs.
-template <typename T, int CIN, int COUT, bool TANH>
-__global__ void __launch_bounds__(128) k_lp_conv(int h8, int w8, const float* __restrict__ wt,
-                                                 const float* __restrict__ bias, T* __restrict__ state,
-                                                 int in_plane, int out_plane) {
-  __shared__ float sw[COUT * CIN * 9];
-  __shared__ float sb[COUT];
-  for (int k = threadIdx.x; k < COUT * CIN * 9; k += blockDim.x) sw[k] = wround<T>(wt[k]);
-  for (int k = threadIdx.x; k < COUT; k += blockDim.x) sb[k] = wround<T>(bias[k]);
-  __syncthreads();
-  const int hw = h8 * w8;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= hw) return;
-  const T* in = state + (long long)blockIdx.y * LP_PLANES * hw + in_plane * hw;
-  T* out = state + (long long)blockIdx.y * LP_PLANES * hw + out_plane * hw;
-  const int y = p / w8, x = p - y * w8;
-  float acc[COUT];
+// The three 3x3 convolutions of a tile of LPN_Y x LPN_X pixels in one launch,
+// with a halo of three pixels: layer 1 on the tile and two rings, layer 2 on the
+// tile and one, all in shared memory; every layer's own tile also goes to the
+// state planes (training reads them).  Each thread forms all outputs of a pixel;
+// the weights lie output-fastest in shared memory, so a tap costs one activation
+// load and four 16-byte weight loads for 16 multiply-adds (16 scalar loads in the
+// layer-by-layer form).  Zero padding is a zero activation, as in the reference.
+// Four 96 x 128 maps: 53 us in three launches, 34 us here, bound by shared-memory
+// loads (five per 16 multiply-adds) at 2.6 CTAs per SM.
+#define LPN_Y 8
+#define LPN_X 16
+#define LPN_THREADS 256
+struct LpNetSmem {
+  float in[5][LPN_Y + 6][LPN_X + 6];
+  float a1[16][LPN_Y + 4][LPN_X + 4];
+  float a2[16][LPN_Y + 2][LPN_X + 2];
+  float4 w1[5 * 9][4], w2[16 * 9][4], w3[16 * 9];
+  float b1[16], b2[16], b3[4];
+};
+
+// Activation rounding of storage type T.
+template <typename T> __device__ __forceinline__ float around(float v) { return wround<T>(v); }
+
+template <typename T, int CIN, int H, int W>
+__device__ __forceinline__ void lpn_conv16(const float (&in)[CIN][H][W], const float4 (*w)[4], const float* b, int y,
+                                           int x, float* acc) {
 #pragma unroll
-  for (int co = 0; co < COUT; ++co) acc[co] = sb[co];
+  for (int co = 0; co < 16; ++co) acc[co] = b[co];
   for (int ci = 0; ci < CIN; ++ci)
 #pragma unroll
-    for (int ky = 0; ky < 3; ++ky) {
-      const int yy = y + ky - 1;
-      if (yy < 0 || yy >= h8) continue;
+    for (int k = 0; k < 9; ++k) {
+      const float v = in[ci][y + k / 3][x + k % 3];
+      const float4* wk = w[ci * 9 + k];
 #pragma unroll
-      for (int kx = 0; kx < 3; ++kx) {
-        const int xx = x + kx - 1;
-        if (xx < 0 || xx >= w8) continue;
-        const float v = ld(in + ci * hw + yy * w8 + xx);
-#pragma unroll
-        for (int co = 0; co < COUT; ++co) acc[co] += sw[((co * CIN + ci) * 3 + ky) * 3 + kx] * v;
+      for (int q = 0; q < 4; ++q) {
+        const float4 t = wk[q];
+        acc[4 * q] += t.x * v;
+        acc[4 * q + 1] += t.y * v;
+        acc[4 * q + 2] += t.z * v;
+        acc[4 * q + 3] += t.w * v;
       }
     }
-#pragma unroll
-  for (int co = 0; co < COUT; ++co) stv(out + co * hw + p, TANH ? tanhf(acc[co]) : acc[co]);
 }
 
-// inner = (1 + tanh(m0)/2) exp(-i tanh(m1)/2), outer likewise from m2, m3.
 template <typename T>
-__global__ void k_lp_gains(int nz, int nx, int h8, int w8, const T* __restrict__ state,
-                           float2* __restrict__ gains) {
+__global__ void __launch_bounds__(LPN_THREADS) k_lp_net(int h8, int w8, const float* __restrict__ params,
+                                                        T* __restrict__ state) {
+  extern __shared__ __align__(16) unsigned char lpn_smem[];
+  LpNetSmem& s = *reinterpret_cast<LpNetSmem*>(lpn_smem);
+  const int hw = h8 * w8, tid = threadIdx.x;
+  T* st = state + (long long)blockIdx.y * LP_PLANES * hw;
+  const int nbx = (w8 + LPN_X - 1) / LPN_X;
+  const int y0 = (blockIdx.x / nbx) * LPN_Y, x0 = (blockIdx.x % nbx) * LPN_X;
+  float* w1 = reinterpret_cast<float*>(s.w1);
+  float* w2 = reinterpret_cast<float*>(s.w2);
+  float* w3 = reinterpret_cast<float*>(s.w3);
+  for (int k = tid; k < 16 * 45; k += LPN_THREADS) w1[(k % 45) * 16 + k / 45] = wround<T>(params[LP_W1 + k]);
+  for (int k = tid; k < 16 * 144; k += LPN_THREADS) w2[(k % 144) * 16 + k / 144] = wround<T>(params[LP_W2 + k]);
+  for (int k = tid; k < 4 * 144; k += LPN_THREADS) w3[(k % 144) * 4 + k / 144] = wround<T>(params[LP_W3 + k]);
+  if (tid < 16) { s.b1[tid] = wround<T>(params[LP_B1 + tid]); s.b2[tid] = wround<T>(params[LP_B2 + tid]); }
+  if (tid < 4) s.b3[tid] = wround<T>(params[LP_B3 + tid]);
+  constexpr int IH = LPN_Y + 6, IW = LPN_X + 6;
+  for (int k = tid; k < 5 * IH * IW; k += LPN_THREADS) {
+    const int ci = k / (IH * IW), r = (k / IW) % IH, c = k % IW;
+    const int y = y0 - 3 + r, x = x0 - 3 + c;
+    s.in[ci][r][c] = y >= 0 && y < h8 && x >= 0 && x < w8 ? ld(st + (LP_POOL + ci) * hw + y * w8 + x) : 0.0f;
+  }
+  __syncthreads();
+  constexpr int H1 = LPN_Y + 4, W1 = LPN_X + 4, H2 = LPN_Y + 2, W2 = LPN_X + 2;
+  for (int k = tid; k < H1 * W1; k += LPN_THREADS) {
+    const int r = k / W1, c = k - r * W1, y = y0 - 2 + r, x = x0 - 2 + c;
+    const bool in = y >= 0 && y < h8 && x >= 0 && x < w8;
+    const bool own = in && r >= 2 && r < 2 + LPN_Y && c >= 2 && c < 2 + LPN_X;
+    float acc[16];
+    lpn_conv16<T>(s.in, s.w1, s.b1, r, c, acc);
+#pragma unroll
+    for (int co = 0; co < 16; ++co) {
+      const float v = in ? around<T>(tanhf(acc[co])) : 0.0f;
+      s.a1[co][r][c] = v;
+      if (own) stv(st + (LP_A1 + co) * hw + y * w8 + x, v);
+    }
+  }
+  __syncthreads();
+  for (int k = tid; k < H2 * W2; k += LPN_THREADS) {
+    const int r = k / W2, c = k - r * W2, y = y0 - 1 + r, x = x0 - 1 + c;
+    const bool in = y >= 0 && y < h8 && x >= 0 && x < w8;
+    const bool own = in && r >= 1 && r < 1 + LPN_Y && c >= 1 && c < 1 + LPN_X;
+    float acc[16];
+    lpn_conv16<T>(s.a1, s.w2, s.b2, r, c, acc);
+#pragma unroll
+    for (int co = 0; co < 16; ++co) {
+      const float v = in ? around<T>(tanhf(acc[co])) : 0.0f;
+      s.a2[co][r][c] = v;
+      if (own) stv(st + (LP_A2 + co) * hw + y * w8 + x, v);
+    }
+  }
+  __syncthreads();
+  if (tid < LPN_Y * LPN_X) {
+    const int r = tid / LPN_X, c = tid - r * LPN_X, y = y0 + r, x = x0 + c;
+    if (y < h8 && x < w8) {
+      float4 acc = make_float4(s.b3[0], s.b3[1], s.b3[2], s.b3[3]);
+      for (int ci = 0; ci < 16; ++ci)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          const float v = s.a2[ci][r + k / 3][c + k % 3];
+          const float4 t = s.w3[ci * 9 + k];
+          acc.x += t.x * v;
+          acc.y += t.y * v;
+          acc.z += t.z * v;
+          acc.w += t.w * v;
+        }
+      T* m = st + LP_MAPS * hw + y * w8 + x;
+      stv(m, acc.x);
+      stv(m + hw, acc.y);
+      stv(m + 2 * hw, acc.z);
+      stv(m + 3 * hw, acc.w);
+    }
+  }
+}
+
+// sin and cos of |x| <= 1/2 by their Taylor series to x^9 and x^8 (truncation
+// below 3e-10): the angles are halves of a tanh.
+__device__ __forceinline__ void sincos_half(float x, float* sn, float* cs) {
+  const float q = x * x;
+  *sn = x * fmaf(q, fmaf(q, fmaf(q, fmaf(q, 2.75573192e-6f, -1.98412698e-4f), 8.33333333e-3f), -1.66666667e-1f), 1.0f);
+  *cs = fmaf(q, fmaf(q, fmaf(q, fmaf(q, 2.48015873e-5f, -1.38888889e-3f), 4.16666667e-2f), -0.5f), 1.0f);
+}
+
+// inner = (1 + tanh(m0)/2) exp(-i tanh(m1)/2), outer likewise from m2, m3.  A
+// thread walks down LPG_ROWS rows of a column: the horizontal interpolation is
+// formed once per low-resolution row it meets, not per node.  Four 768 x 1024
+// pairs of planes: 37 us with the interpolation and a range-reduced sincos per
+// node, 22 us here (8 us to write them), bound by the four tanh per node.
+#define LPG_ROWS 16
+template <typename T>
+__global__ void __launch_bounds__(256) k_lp_gains(int nz, int nx, int h8, int w8, const T* __restrict__ state,
+                                                  float2* __restrict__ gains) {
   const long long n = (long long)nz * nx;
   const int hw = h8 * w8;
   const int f = blockIdx.y;
   const T* maps = state + (long long)f * LP_PLANES * hw + LP_MAPS * hw;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k / nx), j = (int)(k - (long long)i * nx);
+  const int nbx = (nx + 255) / 256;
+  const int j = (blockIdx.x % nbx) * 256 + threadIdx.x;
+  const int i0 = (blockIdx.x / nbx) * LPG_ROWS;
+  if (j >= nx) return;
+  const Lerp lx = lerp_of(j, w8, nx);
+  // maps of low-resolution row r at this column
+  auto line = [&](int r, float* m) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const T* M = maps + c * hw + r * w8;
+      m[c] = (1.0f - lx.l1) * ld(M + lx.i0) + lx.l1 * ld(M + lx.i1);
+    }
+  };
+  float2* gi = gains + (2LL * f) * n + j;
+  float2* go = gi + n;
+  float top[4], bot[4];
+  int r0 = -1, r1 = -1;
+  for (int i = i0; i < min(i0 + LPG_ROWS, nz); ++i) {
+    const Lerp lz = lerp_of(i, h8, nz);
+    if (lz.i0 != r0 || lz.i1 != r1) {
+      line(lz.i0, top);
+      line(lz.i1, bot);
+      r0 = lz.i0;
+      r1 = lz.i1;
+    }
     float m[4];
-    node_maps(maps, hw, w8, lerp_of(i, h8, nz), lerp_of(j, w8, nx), m);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) m[c] = (1.0f - lz.l1) * top[c] + lz.l1 * bot[c];
     float s1, c1, s3, c3;
-    sincosf(0.5f * tanhf(m[1]), &s1, &c1);
-    sincosf(0.5f * tanhf(m[3]), &s3, &c3);
+    sincos_half(0.5f * tanhf(m[1]), &s1, &c1);
+    sincos_half(0.5f * tanhf(m[3]), &s3, &c3);
     const float g0 = 1.0f + 0.5f * tanhf(m[0]);
     const float g2 = 1.0f + 0.5f * tanhf(m[2]);
-    gains[(2LL * f) * n + k] = make_float2(g0 * c1, -g0 * s1);
-    gains[(2LL * f + 1) * n + k] = make_float2(g2 * c3, -g2 * s3);
+    gi[(long long)i * nx] = make_float2(g0 * c1, -g0 * s1);
+    go[(long long)i * nx] = make_float2(g2 * c3, -g2 * s3);
   }
 }
 
@@ -208,17 +358,14 @@ template <typename T>
 static void learned_setup_t(const NsrGrid* grid, const float* c, const float* rho, const float* alpha,
                             const double* freq_hz, int n_freq, const float* params, T* state, void* gains,
                             cudaStream_t st) {
-  const int h8 = lp_h(grid), w8 = lp_w(grid), hw = h8 * w8;
-  const int pb = (hw + 127) / 128;
-  k_lp_pool<T><<<pb, 128, 0, st>>>(grid->nz, grid->nx, h8, w8, c, rho, alpha, freq_hz, n_freq, state);
-  const dim3 gconv(pb, n_freq);
-  k_lp_conv<T, 5, 16, true><<<gconv, 128, 0, st>>>(h8, w8, params + LP_W1, params + LP_B1, state, LP_POOL, LP_A1);
-  k_lp_conv<T, 16, 16, true><<<gconv, 128, 0, st>>>(h8, w8, params + LP_W2, params + LP_B2, state, LP_A1, LP_A2);
-  k_lp_conv<T, 16, 4, false><<<gconv, 128, 0, st>>>(h8, w8, params + LP_W3, params + LP_B3, state, LP_A2, LP_MAPS);
+  const int h8 = lp_h(grid), w8 = lp_w(grid);
+  k_lp_pool<T><<<h8 * ((8 * w8 + 255) / 256), 256, 0, st>>>(grid->nz, grid->nx, h8, w8, c, rho, alpha, freq_hz, n_freq,
+                                                            state);
+  cudaFuncSetAttribute(k_lp_net<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LpNetSmem));
+  const dim3 gn(((h8 + LPN_Y - 1) / LPN_Y) * ((w8 + LPN_X - 1) / LPN_X), n_freq);
+  k_lp_net<T><<<gn, LPN_THREADS, sizeof(LpNetSmem), st>>>(h8, w8, params, state);
   if (gains) {
-    const long long n = (long long)grid->nz * grid->nx;
-    int bx = (int)((n + 255) / 256);
-    if (bx > 1184) bx = 1184;
+    const int bx = ((grid->nx + 255) / 256) * ((grid->nz + LPG_ROWS - 1) / LPG_ROWS);
     k_lp_gains<T><<<dim3(bx, n_freq), 256, 0, st>>>(grid->nz, grid->nx, h8, w8, state, (float2*)gains);
   }
 }
@@ -231,6 +378,7 @@ extern "C" int nsr_learned_setup_ex(const NsrGrid* grid, const float* c, const f
   if (!c || !rho || !alpha || !freq_hz || !params || !state || n_freq < 0 || n_freq > 65535) return NSR_ERR_ARGUMENT;
   if (precision != NSR_LEARNED_FP32 && precision != NSR_LEARNED_BF16) return NSR_ERR_ARGUMENT;
   if (n_freq == 0) return 0;
+  if (lp_h(grid) < 1 || lp_w(grid) < 1) return NSR_ERR_ARGUMENT;   // no low-resolution pixel
   cudaStream_t st = (cudaStream_t)stream;
   if (precision == NSR_LEARNED_BF16)
     learned_setup_t(grid, c, rho, alpha, freq_hz, n_freq, params, (__nv_bfloat16*)state, gains, st);
