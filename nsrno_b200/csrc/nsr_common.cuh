@@ -563,14 +563,14 @@ __device__ __forceinline__ void gen_rows_inverse(float2* s, int nl, const FftPla
                 gen_twiddle<R, true>(v, P.tws, j, m);
                 small_dft<R, true>(v);
 #pragma unroll
-                for (int q = 0; q < R; ++q) out(l * N + j + q * m, v[q]);
+                for (int q = 0; q < R; ++q) out(l * N + j + q * m, v[q], l, j + q * m);
               }
             },
             [&] {
               gen_stage_prime<true, 0>(s, nl, P, P.radix[0], N, P.tws);
               __syncthreads();
               for (int l = 0; l < nl; ++l)
-                for (int c = threadIdx.x; c < N; c += blockDim.x) out(l * N + c, s[l * rs + row_pos(c)]);
+                for (int c = threadIdx.x; c < N; c += blockDim.x) out(l * N + c, s[l * rs + row_pos(c)], l, c);
             });
 }
 
@@ -1023,8 +1023,8 @@ __device__ __forceinline__ bool fft_cols_direct(float2* s, const FftPlan& P, flo
 //    whatever elementwise work produces it; stage 0 runs on those registers,
 //    the middle stages in shared memory, the last stage writes `g`;
 //  * inverse: the first stage reads `g`, the middle stages run in shared
-//    memory, and `out(k, v)` receives each output of stage 0 (flat index k)
-//    and stores it.
+//    memory, and `out(k, v, l, c)` receives each output of stage 0 (flat index
+//    k, row l, column c) and stores it.
 // Two shared-memory round trips fewer than load, transform, store.
 template <int N, typename IN>
 __device__ __forceinline__ void ct_rows_forward_direct(float2* s, int nl, const float2* __restrict__ tws,
@@ -1105,7 +1105,7 @@ __device__ __forceinline__ void ct_rows_inverse_direct(float2* s, int nl, const 
     for (int k = 1; k < R0; ++k) v[k] = v[k] * conjc(__ldg(tw0 + (k - 1) * M0 + j));
     small_dft<R0, true>(v);
 #pragma unroll
-    for (int q = 0; q < R0; ++q) out(l * N + j + q * M0, v[q]);
+    for (int q = 0; q < R0; ++q) out(l * N + j + q * M0, v[q], l, j + q * M0);
   }
 }
 

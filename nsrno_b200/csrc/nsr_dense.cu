@@ -447,9 +447,8 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) k_dense_rows_inv(DenseGeo g,
     for (int k = threadIdx.x; k < nr * nx; k += blockDim.x) ys[k] = make_float2(0.f, 0.f);
     return;
   }
-  rows_inverse<GEN>(sm, nr, t.px, w + off, [&](int k, float2 v) {
-    const int l = k / nx;
-    ys[k] = dense_inside(g, z0 + l, k - l * nx) ? v : make_float2(0.f, 0.f);
+  rows_inverse<GEN>(sm, nr, t.px, w + off, [&](int k, float2 v, int l, int c) {
+    ys[k] = dense_inside(g, z0 + l, c) ? v : make_float2(0.f, 0.f);
   });
 }
 
@@ -507,14 +506,14 @@ int nsr_dense_prec_setup(const NsrDenseGrid* grid, double k0dx2, double shift, i
   M->inv_k0dx2 = (float)(1.0 / k0dx2);
   M->shift = (float)shift;
   M->adjoint = adjoint;
-  M->rows = nsr_rows_per_cta(&q);
-  M->tc = nsr_cols_tc(&q);
+  M->rows = nsr_rows_per_cta(&q, n_fields);
+  M->tc = nsr_cols_tc(&q, n_fields);
   M->gx = !nsr_specialised(grid->W);
   M->gz = !nsr_specialised(grid->H);
   M->g_rows = dim3((grid->H + M->rows - 1) / M->rows, n_fields);
   M->g_cols = dim3((grid->W + M->tc - 1) / M->tc, n_fields);
   M->row_smem = sizeof(float2) * (size_t)M->rows * nsr_row_stride(grid->W);
-  M->col_smem = nsr_cols_smem(&q);
+  M->col_smem = sizeof(float2) * (size_t)grid->H * M->tc;
   return 0;
 }
 

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(GArgs A, int j) {
   const long long off = (long long)z0 * g.nx;
   float2* Wp = A.W + slot * n + off;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
-  rows_inverse<GEN>(sm, nr, A.tab.px, Wp, [&](int k, float2 v) {
+  rows_inverse<GEN>(sm, nr, A.tab.px, Wp, [&](int k, float2 v, int, int) {
     Wp[k] = G.post ? gain_mul(G.post, off + k, G.conj, v) : v;
   });
 }
@@ -695,8 +695,8 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     A.m = m;
     A.n_slots = n_slots;
     A.nb_max = L.nb_max;
-    A.rows = nsr_rows_per_cta(grid);
-    A.tc = nsr_cols_tc(grid);
+    A.rows = nsr_rows_per_cta(grid, n_slots);
+    A.tc = nsr_cols_tc(grid, n_slots);
     A.tol = params->tolerance;
     A.shift = params->shift;
     A.max_it = params->max_iterations;
@@ -729,7 +729,7 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     }
 
     const size_t fwd_smem = sizeof(float2) * A.rows * nsr_row_stride(grid->nx);
-    const size_t col_smem = nsr_cols_smem(grid);
+    const size_t col_smem = sizeof(float2) * (size_t)grid->nz * A.tc;
     const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
     const auto fwd_fn = gx ? gk_fwd<true> : gk_fwd<false>;
     const auto rinv_fn = gx ? gk_rinv<true> : gk_rinv<false>;

@@ -17,9 +17,9 @@ int nsr_check_grid(const NsrGrid* g, bool need_fft);
 int nsr_prec_setup(const NsrGrid* g, PrecTables* t, void* table_mem, cudaStream_t st, float* d2x = nullptr,
                    float* d2z = nullptr);
 size_t nsr_prec_table_bytes(const NsrGrid* g);
-int nsr_cols_tc(const NsrGrid* g);
-size_t nsr_cols_smem(const NsrGrid* g);
-int nsr_rows_per_cta(const NsrGrid* g);
+// Columns and rows per CTA of the transform passes over ns fields.
+int nsr_cols_tc(const NsrGrid* g, int ns);
+int nsr_rows_per_cta(const NsrGrid* g, int ns);
 
 // Threads of a column-pass CTA: the run-time transforms take half as many
 // (their butterflies hold up to 19 points in registers).

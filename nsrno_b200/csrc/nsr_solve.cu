@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_rinv(Solv
   float2* w = A.B.w + slot * n + goff;
   const GainPair G = gain_pair(A.gains, S.gidx, n, A.adjoint);
   if constexpr (PASS != PASS_STAGED) {
-    rows_inverse<PASS == PASS_GENERIC>(sm, nr, A.tab.px, w, [&](int k, float2 v) {
+    rows_inverse<PASS == PASS_GENERIC>(sm, nr, A.tab.px, w, [&](int k, float2 v, int, int) {
       w[k] = G.post ? gain_mul(G.post, goff + k, G.conj, v) : v;
     });
     return;
@@ -1409,9 +1409,9 @@ struct TileChoice {
 
 static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileChoice* c) {
   c->sw = 256; c->sd = 0; c->sr = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
-  c->tc = nsr_cols_tc(g);
-  c->rows = nsr_rows_per_cta(g);
   c->groups = n_slots >= 8 ? 2 : 1;
+  c->tc = nsr_cols_tc(g, n_slots);
+  c->rows = nsr_rows_per_cta(g, n_slots);
   if (t) {
     if (t->stencil_width) c->sw = t->stencil_width;
     if (t->stencil_depth) c->sd = t->stencil_depth;
@@ -1598,7 +1598,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     }
 
     const size_t fwd_smem = sizeof(float2) * A.rows * nsr_row_stride(grid->nx);
-    const size_t col_smem = nsr_cols_smem(grid);
+    const size_t col_smem = sizeof(float2) * (size_t)grid->nz * A.tc;
     const int nb_st = stencil_ctas(grid);
     const bool pairs = grid->nx % 2 == 0;
     const bool use_stn = stn_ok(grid);
