@@ -1308,17 +1308,13 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
 }
 
 
-__global__ void k_solve_outputs(SolveArgs A) {
+__global__ void k_solve_init(SolveArgs A, int n_slots) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < A.n_systems; s += gridDim.x * blockDim.x) {
     A.status[s] = NSR_NOT_RUN;
     A.iterations[s] = 0;
     A.residual[s] = NAN;
   }
-}
-
-__global__ void k_solve_init(SolveArgs A, int n_slots) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < n_slots; s += gridDim.x * blockDim.x) {
     SlotState st;
     memset(&st, 0, sizeof(st));
@@ -1351,14 +1347,27 @@ __global__ void k_solve_init(SolveArgs A, int n_slots) {
 // graph node): ends the loop once every system has finished, a kernel has
 // reported an error, or the round budget (an upper bound on the rounds a full
 // queue can need) is spent.
+__device__ __forceinline__ bool loop_ends(const SolveArgs& A, unsigned long long rounds, long long max_rounds) {
+  const int done = *(volatile int*)A.B.done;
+  const int error = *(volatile int*)A.B.error;
+  return done >= A.n_systems || error || rounds >= (unsigned long long)max_rounds;
+}
 __global__ void k_loop_control(SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   unsigned long long* rounds = reinterpret_cast<unsigned long long*>(A.B.queue + 6);
   const unsigned long long r = *rounds + 1;
   *rounds = r;
-  const int done = *(volatile int*)A.B.done;
-  const int error = *(volatile int*)A.B.error;
-  if (done >= A.n_systems || error || r >= (unsigned long long)max_rounds) cudaGraphSetConditional(loop, 0);
+  if (loop_ends(A, r, max_rounds)) cudaGraphSetConditional(loop, 0);
+}
+// Last launch of the first round, which runs outside the loop.
+__global__ void k_round_count(SolveArgs A) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) *reinterpret_cast<unsigned long long*>(A.B.queue + 6) += 1;
+}
+// First node of the loop's graph: whether the loop runs at all.
+__global__ void k_loop_begin(SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const unsigned long long r = *reinterpret_cast<unsigned long long*>(A.B.queue + 6);
+  cudaGraphSetConditional(loop, loop_ends(A, r, max_rounds) ? 0 : 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1535,7 +1544,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
 #define NSR_TRY(x) do { ce = (x); if (ce != cudaSuccess) { err = (int)ce; goto cleanup; } } while (0)
   {
     NSR_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    for (int g = 1; g < NSR_MAX_GROUPS; ++g) {
+    for (int g = 1; g < T.groups; ++g) {   // a stream costs about 0.1 ms to make and release
       NSR_TRY(cudaStreamCreateWithFlags(&sg[g], cudaStreamNonBlocking));
       NSR_TRY(cudaEventCreateWithFlags(&ev_join[g], cudaEventDisableTiming));
     }
@@ -1647,10 +1656,9 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     NSR_TRY(cudaFuncSetAttribute((const void*)cols_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
     NSR_TRY(cudaFuncSetAttribute((const void*)rinv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem));
 
-    k_solve_outputs<<<64, 256, 0, st>>>(A);
     k_solve_init<<<64, 256, 0, st>>>(A, n_slots);
     NSR_TRY(cudaGetLastError());
-    launches = 3;  // the tables, the outputs and the slots
+    launches = 3;  // the tables, the slots, the check before the device loop
 
     // The slots run as independent groups on branches of the captured graph,
     // so that one group's kernels fill the tail waves of the others'.
@@ -1751,8 +1759,8 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     const long long per_sys = (long long)params->max_iterations * 2 + 16;
     const long long waves = (n_systems + n_slots - 1) / n_slots + 1;
     const long long max_launch = waves * ((per_sys + K - 1) / K) + 4;
-    // The K iterations of one round, captured from both slot-group streams.
-    auto capture_round = [&]() -> cudaError_t {
+    // The K iterations of one round on the slot groups' streams, launched or captured.
+    auto issue_round = [&]() -> cudaError_t {
       cudaError_t e = cudaSuccess;
       if (n_groups > 1 && (e = cudaEventRecord(ev_fork, st)) != cudaSuccess) return e;
       for (int g = 1; g < n_groups; ++g)
@@ -1768,21 +1776,39 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     };
 
     if (!blocking) {
-      // Device-side loop: a conditional WHILE node whose body is one round
-      // followed by k_loop_control, so the whole solve is one graph launch
-      // on the stream and the host returns at once.
+      // The first round is launched kernel by kernel, so that the device works
+      // while the host builds the graph of the others (0.5 to 1 ms of a 256 x 256
+      // solve's 5).  They are a device-side loop: a conditional WHILE node whose
+      // body is one round followed by k_loop_control, behind k_loop_begin, which
+      // skips it when the first round was enough.  The host returns without
+      // waiting for either.
+      NSR_TRY(issue_round());
+      k_round_count<<<1, 32, 0, st>>>(A);
+      NSR_TRY(cudaGetLastError());
       cudaGraphConditionalHandle handle;
       NSR_TRY(cudaGraphCreate(&loop_graph, 0));
-      NSR_TRY(cudaGraphConditionalHandleCreate(&handle, loop_graph, 1, cudaGraphCondAssignDefault));
+      NSR_TRY(cudaGraphConditionalHandleCreate(&handle, loop_graph, 0, cudaGraphCondAssignDefault));
+      NSR_TRY(cudaStreamBeginCaptureToGraph(st, loop_graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+      k_loop_begin<<<1, 32, 0, st>>>(A, handle, max_launch);
+      ce = cudaGetLastError();
+      {
+        cudaGraph_t begun = nullptr;
+        const cudaError_t ce2 = cudaStreamEndCapture(st, &begun);
+        if (ce == cudaSuccess) ce = ce2;
+      }
+      if (ce != cudaSuccess) { err = (int)ce; goto cleanup; }
+      cudaGraphNode_t begin_node;
+      size_t n_begin = 1;
+      NSR_TRY(cudaGraphGetRootNodes(loop_graph, &begin_node, &n_begin));
       cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
       cp.conditional.handle = handle;
       cp.conditional.type = cudaGraphCondTypeWhile;
       cp.conditional.size = 1;
       cudaGraphNode_t while_node;
-      NSR_TRY(cudaGraphAddNode(&while_node, loop_graph, nullptr, 0, &cp));
+      NSR_TRY(cudaGraphAddNode(&while_node, loop_graph, &begin_node, 1, &cp));
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       NSR_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      ce = capture_round();
+      ce = issue_round();
       if (ce == cudaSuccess) {
         k_loop_control<<<1, 32, 0, st>>>(A, handle, max_launch);
         ce = cudaGetLastError();
@@ -1804,7 +1830,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     }
 
     NSR_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    ce = capture_round();
+    ce = issue_round();
     {
       const cudaError_t ce2 = cudaStreamEndCapture(st, &graph);
       if (ce == cudaSuccess) ce = ce2;
