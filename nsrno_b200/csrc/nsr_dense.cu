@@ -15,6 +15,7 @@
 #include "nsr_dense.cuh"
 
 #include <string.h>
+#include <type_traits>
 
 struct DenseCoef {
   // planes [H][W]
@@ -249,11 +250,377 @@ static cudaError_t launch_dense_apply(const DenseGeo& g, const double* coef, int
   return cudaGetLastError();
 }
 
-// Tile height: tall tiles form the fewest fluxes twice (23 rows for 16); grids
-// whose 16-row tiles are fewer than three per SM take 8-row ones.
+// The same operator as a walk down the rows, for grids that fill the chip with
+// bands of rows.  A thread owns CPT adjacent columns of a strip and keeps the
+// last eight rows of mask p and of Z in registers, so the z part reads no shared
+// memory at all; the x part writes a row of p (and then of X) once and reads ten
+// neighbours of two columns as five 16-byte loads.  A step takes in row q, forms
+// Z of row q - 4 and finishes row q - 7; the strip's halo columns and the next
+// rows are in flight meanwhile.  A strip yields all but its four outermost columns
+// on each side, whose X lacks neighbours.
+// Eleven complex64 fields on 1056 x 1216: 260 us (tiles 316, two passes 695);
+// bound by instruction issue at three CTAs per SM.
+#define DS_THREADS 128
+#define DS_ROWS 64     // most rows of a band
+#define DS_UNROLL 2
+
+template <typename T, int CPT>
+struct __align__(16) DenseRowsSmem {
+  typedef typename DC<T>::C C;
+  static constexpr int N = DS_THREADS * CPT + 8;   // columns b0 - 4 .. b0 + strip + 3
+  C a[2][N], b[2][N];                              // p, or conj(l) p and conj(r) p (adjoint in the PML)
+  C x[N], gx[N];                                   // X, gvx X (forward in the PML)
+  C halo[8][8];                                    // p at columns b0 - 3 .. b0 - 1 and the four after the strip
+  C prz[4][DS_ROWS + 16];                          // sv, gv, l, r of rows z0 - 8 ..
+};
+
+__device__ __forceinline__ void ds_cp_async(float2* dst, const float2* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void ds_cp_async(double2* dst, const double2* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+// CPT adjacent values, as one 16-byte access where CPT is 2.
+template <int CPT>
+__device__ __forceinline__ void ds_vec(const float2* p, float2* v) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = make_float2(t.x, t.y);
+  v[1] = make_float2(t.z, t.w);
+}
+template <int CPT>
+__device__ __forceinline__ void ds_vec(const double2* p, double2* v) { v[0] = *p; }
+template <int CPT>
+__device__ __forceinline__ void ds_vec(const double* p, double* v) {
+  if constexpr (CPT == 2) {
+    const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    v[0] = __ldg(p);
+  }
+}
+template <int CPT>
+__device__ __forceinline__ void ds_store(float2* p, const float2* v) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+}
+template <int CPT>
+__device__ __forceinline__ void ds_store(double2* p, const double2* v) { *p = v[0]; }
+
+// CPT + 8 consecutive row entries, from an entry that is a multiple of CPT.
+template <int CPT>
+__device__ __forceinline__ void ds_load(const float2* row, float2 (&v)[CPT + 8]) {
+  static_assert(CPT == 2, "pairs");
+#pragma unroll
+  for (int q = 0; q < (CPT + 8) / 2; ++q) {
+    const float4 t = reinterpret_cast<const float4*>(row)[q];
+    v[2 * q] = make_float2(t.x, t.y);
+    v[2 * q + 1] = make_float2(t.z, t.w);
+  }
+}
+template <int CPT>
+__device__ __forceinline__ void ds_load(const double2* row, double2 (&v)[CPT + 8]) {
+#pragma unroll
+  for (int q = 0; q < CPT + 8; ++q) v[q] = row[q];
+}
+
+template <typename T, bool ADJ, int CPT>
+__global__ void __launch_bounds__(DS_THREADS, sizeof(T) == 4 ? 3 : 2)
+    k_dense_stream(DenseGeo g, const double* __restrict__ coef, const typename DC<T>::C* __restrict__ p,
+                   typename DC<T>::C* __restrict__ y, int nf, int rows) {
+  typedef typename DC<T>::C C;
+  typedef DenseRowsSmem<T, CPT> Smem;
+  extern __shared__ __align__(16) unsigned char da_smem[];
+  Smem& sm = *reinterpret_cast<Smem*>(da_smem);
+  constexpr int STRIP = DS_THREADS * CPT, OUT = STRIP - 8;
+  const DenseCoef dc = dense_unpack(coef, g.H, g.W);
+  const long long n = (long long)g.H * g.W;
+  const int f = blockIdx.x % nf, tile = blockIdx.x / nf;
+  const int nbx = (g.W + OUT - 1) / OUT;
+  const int z0 = (tile / nbx) * rows, z1 = min(z0 + rows, g.H);
+  const int c0 = (tile % nbx) * OUT, b0 = c0 - 4;   // outputs c0 .. c0 + OUT - 1
+  const C* __restrict__ pf = p + (long long)f * n;
+  C* __restrict__ yf = y + (long long)f * n;
+  const C zero = cx<C>(T(0), T(0));
+  const int tid = threadIdx.x, jt = b0 + CPT * tid;
+  const int j0 = min(max(jt, 0), g.W - CPT);   // W is a multiple of CPT and jt too: a thread's columns are in or out together
+  if (!(z0 < g.pz + g.h && z1 > g.pz && c0 < g.px + g.w && c0 + OUT > g.px)) {   // no native node: copy
+    for (int i = z0; i < z1; ++i)
+      for (int j = c0 + tid; j < min(c0 + OUT, g.W); j += DS_THREADS) yf[(long long)i * g.W + j] = pf[(long long)i * g.W + j];
+    return;
+  }
+  C rxc[CPT], lxc[CPT], svc[CPT], gvc[CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    svc[c] = DC<T>::from(dc.svx[j0 + c]);
+    gvc[c] = DC<T>::from(dc.gvx[j0 + c]);
+    lxc[c] = DC<T>::from(dc.lx[j0 + c]);
+    rxc[c] = DC<T>::from(dc.rx[j0 + c]);
+  }
+  // Whether every column (row) the block touches is off the PML, with one right factor.
+  const C r0x = DC<T>::from(dc.rx[min(c0, g.W - 1)]), r0z = DC<T>::from(dc.rz[z0]);
+  bool px = true, pz = true;
+  for (int e = tid; e < STRIP + 8; e += DS_THREADS) {
+    const int j = min(max(b0 - 4 + e, 0), g.W - 1);
+    const C r = DC<T>::from(dc.rx[j]);
+    px = px && is_real(DC<T>::from(dc.svx[j]), 1.0) && is_real(DC<T>::from(dc.gvx[j]), 1.0) &&
+         is_real(DC<T>::from(dc.lx[j]), 0.0) && r.x == r0x.x && r.y == r0x.y;
+  }
+  for (int e = tid; e < rows + 16; e += DS_THREADS) {
+    const int i = z0 - 8 + e;
+    const bool in = i >= 0 && i < g.H;
+    const C sv = in ? DC<T>::from(dc.svz[i]) : zero, gv = in ? DC<T>::from(dc.gvz[i]) : zero;
+    const C l = in ? DC<T>::from(dc.lz[i]) : zero, r = in ? DC<T>::from(dc.rz[i]) : zero;
+    sm.prz[0][e] = sv; sm.prz[1][e] = gv; sm.prz[2][e] = l; sm.prz[3][e] = r;
+    pz = pz && is_real(sv, 1.0) && is_real(gv, 1.0) && is_real(l, 0.0) && r.x == r0z.x && r.y == r0z.y;
+  }
+  const bool plain_x = __syncthreads_and(px) != 0, plain_z = __syncthreads_and(pz) != 0;
+  const T a4[4] = {(T)nsr_dense_stencil(0), (T)nsr_dense_stencil(1), (T)nsr_dense_stencil(2), (T)nsr_dense_stencil(3)};
+  const T inv_dx = (T)(1.0 / g.dx), sgn = ADJ ? T(-1) * inv_dx : inv_dx;
+  const C scal = DC<T>::from(g.scal);
+  const C adj_x = conjc(scal * r0x), adj_z = conjc(scal * r0z);
+  bool col_in[CPT], col_out[CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    col_in[c] = jt + c >= g.px && jt + c < g.px + g.w;
+    col_out[c] = jt + c >= c0 && jt + c < min(c0 + OUT, g.W);
+  }
+  const bool live_cols = jt >= 0 && jt < g.W;
+  const C* __restrict__ pcol = pf + j0;
+  const double* __restrict__ axt = dc.ax + j0;
+  const double* __restrict__ azt = dc.az + j0;
+  const double2* __restrict__ mt = dc.mass + j0;
+  auto load_p = [&](int i, C* v) {   // mask p of row i at the thread's columns
+    C t[CPT];
+    ds_vec<CPT>(pcol + (long long)min(max(i, 0), g.H - 1) * g.W, t);
+    const bool row_in = i >= g.pz && i < g.pz + g.h;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) v[c] = row_in && col_in[c] ? t[c] : zero;
+  };
+  // halo entry of this thread (the first seven)
+  const int hj = tid < 3 ? b0 - 3 + tid : b0 + STRIP + tid - 3;
+  const int he = tid < 3 ? 1 + tid : STRIP + 4 + tid - 3;   // its entry in a row
+  const bool h_in = hj >= g.px && hj < g.px + g.w;
+  const int hjc = min(max(hj, 0), g.W - 1);
+  const C hl = ADJ ? conjc(DC<T>::from(dc.lx[hjc])) : zero, hr = ADJ ? conjc(DC<T>::from(dc.rx[hjc])) : zero;
+
+  // Windows of mask p and of Z: entry 8 + k takes the row of step k of a group of
+  // DS_UNROLL, entries 0 .. 7 hold the eight before.  (A ring of eight without the
+  // shift needs eight copies of the step, which missed the instruction cache: 327
+  // us where this form takes 260.)
+  C pw[8 + DS_UNROLL][CPT], zw[8 + DS_UNROLL][CPT];
+#pragma unroll
+  for (int k = 0; k < 8 + DS_UNROLL; ++k)
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) pw[k][c] = zw[k][c] = zero;
+  C pn[2][CPT];   // rows q + 1, q + 2 in flight
+  load_p(z0 - 7, pn[0]);
+  load_p(z0 - 6, pn[1]);
+  double raw_az[CPT], raw_ax[CPT];
+  double2 raw_m[CPT];
+  auto load_coef = [&](int q) {   // az of row q - 4, ax and mass of row q - 7
+    const long long rz = (long long)min(max(q - 4, 0), g.H - 1) * g.W, ri = (long long)min(max(q - 7, 0), g.H - 1) * g.W;
+    ds_vec<CPT>(azt + rz, raw_az);
+    ds_vec<CPT>(axt + ri, raw_ax);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) raw_m[c] = __ldg(mt + ri + c);
+  };
+  load_coef(z0 - 7);
+  const int steps = z1 - z0 + 14;
+  // One copy of the loop per kind of block: with every case in one body it did
+  // not fit the instruction cache.
+  auto walk = [&](auto tag_x, auto tag_z) {
+  constexpr bool plain_x = decltype(tag_x)::value, plain_z = decltype(tag_z)::value;
+#pragma unroll 1
+  for (int s0 = 0; s0 < steps; s0 += DS_UNROLL) {
+#pragma unroll
+    for (int k = 0; k < DS_UNROLL; ++k) {
+      const int s = s0 + k;
+      if (s >= steps) break;
+      const int q = z0 - 7 + s;
+      if (tid < 7) {
+        const bool live = h_in && q >= g.pz && q < g.pz + g.h;
+        ds_cp_async(&sm.halo[s & 7][tid], pf + (live ? (long long)q * g.W + hjc : 0), live);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const int zr = q - 4, i = q - 7;
+      // this step's coefficients (loaded during the step before), then the next's
+      T caz[CPT], cax[CPT];
+      C cm[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        caz[c] = (T)raw_az[c];
+        cax[c] = (T)raw_ax[c];
+        cm[c] = DC<T>::from(raw_m[c]);
+      }
+      load_coef(q + 1);
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) pw[8 + k][c] = pn[k & 1][c];
+      load_p(q + 2, pn[k & 1]);
+      // Z of row q - 4 from rows q - 7 .. q
+      if (s >= 7) {
+        const bool live = zr >= 0 && zr < g.H;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          C v;
+          const T az = live ? sgn * caz[c] : T(0);
+          if (!ADJ || plain_z) {
+            C d = zero;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) d = d + a4[t] * (pw[k + 5 + t][c] - pw[k + 4 - t][c]);
+            v = plain_z ? (ADJ ? az * (adj_z * d) : az * d) : az * (sm.prz[0][zr - z0 + 8] * d);
+          } else {
+            C fl = zero, fr = zero;
+            const int e = zr - z0 + 8;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const C ps = pw[k + 5 + t][c], pm = pw[k + 4 - t][c];
+              fl = fl + a4[t] * (conjc(sm.prz[2][e + 1 + t]) * ps - conjc(sm.prz[2][e - t]) * pm);
+              fr = fr + a4[t] * (conjc(sm.prz[3][e + 1 + t]) * ps - conjc(sm.prz[3][e - t]) * pm);
+            }
+            v = az * (conjc(sm.prz[0][e] * scal) * (fl + conjc(sm.prz[1][e]) * fr));
+          }
+          zw[8 + k][c] = v;
+        }
+      }
+      if (s < 14) continue;
+      // finish row i = q - 7, whose p is the oldest row of the window
+      const C* pi = pw[k + 1];
+      C* ra = sm.a[s & 1];
+      C* rb = sm.b[s & 1];
+      asm volatile("cp.async.wait_group 7;" ::: "memory");
+      if (tid < 7) {
+        const C h = sm.halo[(s + 1) & 7][tid];
+        ra[he] = !ADJ || plain_x ? h : hl * h;
+        if (ADJ && !plain_x) rb[he] = hr * h;
+      }
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        ra[4 + CPT * tid + c] = !ADJ || plain_x ? pi[c] : conjc(lxc[c]) * pi[c];
+        if (ADJ && !plain_x) rb[4 + CPT * tid + c] = conjc(rxc[c]) * pi[c];
+      }
+      __syncthreads();
+      {
+        C v[CPT + 8], d[CPT];
+        auto grad = [&](int c) -> C {   // D at the thread's column c
+          C u = zero;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) u = u + a4[t] * (v[c + 5 + t] - v[c + 4 - t]);
+          return u;
+        };
+        ds_load<CPT>(ra + CPT * tid, v);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) d[c] = grad(c);
+        if (ADJ && !plain_x) {
+          ds_load<CPT>(rb + CPT * tid, v);
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) d[c] = d[c] + conjc(gvc[c]) * grad(c);
+        }
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          const T ax = live_cols ? sgn * cax[c] : T(0);
+          const C x = ax * (plain_x ? (ADJ ? adj_x * d[c] : d[c]) : (ADJ ? conjc(svc[c] * scal) : svc[c]) * d[c]);
+          sm.x[4 + CPT * tid + c] = x;
+          if (!ADJ && !plain_x) sm.gx[4 + CPT * tid + c] = gvc[c] * x;
+        }
+      }
+      __syncthreads();
+      {
+        C v[CPT + 8], part[CPT];
+        auto div = [&](int c) -> C {   // sum a (X[c + t] - X[c - 1 - t])
+          C u = zero;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) u = u + a4[t] * (v[c + 4 + t] - v[c + 3 - t]);
+          return u;
+        };
+        ds_load<CPT>(sm.x + CPT * tid, v);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) part[c] = ADJ ? div(c) : (plain_x ? rxc[c] : lxc[c]) * div(c);
+        if (!ADJ && !plain_x) {
+          ds_load<CPT>(sm.gx + CPT * tid, v);
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) part[c] = part[c] + rxc[c] * div(c);
+        }
+        const bool row_in = i >= g.pz && i < g.pz + g.h;
+        C res[CPT];
+        bool all = row_in;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          C dz = zero, dg = zero;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const C zs = zw[k + 5 + t][c], zm = zw[k + 4 - t][c];
+            dz = dz + a4[t] * (zs - zm);
+            if (!ADJ && !plain_z) dg = dg + a4[t] * (sm.prz[1][i - z0 + 8 + t] * zs - sm.prz[1][i - z0 + 7 - t] * zm);
+          }
+          if (ADJ) {
+            res[c] = sgn * (part[c] + dz) + conjc(cm[c]) * pi[c];
+          } else {
+            const C sum = part[c] + (plain_z ? r0z * dz : sm.prz[2][i - z0 + 8] * dz + sm.prz[3][i - z0 + 8] * dg);
+            res[c] = scal * (inv_dx * sum) + cm[c] * pi[c];
+          }
+          all = all && col_out[c] && col_in[c];
+        }
+        const long long id = (long long)i * g.W + jt;
+        if (all) {
+          ds_store<CPT>(yf + id, res);
+        } else {
+#pragma unroll
+          for (int c = 0; c < CPT; ++c)
+            if (col_out[c]) yf[id + c] = row_in && col_in[c] ? res[c] : pf[id + c];
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        pw[e][c] = pw[e + DS_UNROLL][c];
+        zw[e][c] = zw[e + DS_UNROLL][c];
+      }
+  }
+  };
+  if (plain_x) {
+    if (plain_z) walk(std::true_type{}, std::true_type{});
+    else walk(std::true_type{}, std::false_type{});
+  } else {
+    if (plain_z) walk(std::false_type{}, std::true_type{});
+    else walk(std::false_type{}, std::false_type{});
+  }
+}
+
+// Launch: the walk where its bands give every SM three blocks or more (and, for
+// complex64, even widths and 16-byte aligned buffers let it read pairs); else
+// the tiles, 16 rows high (23 rows of fluxes for 16) or, where those are
+// fewer than three per SM, 8.
 template <typename T, bool ADJ>
 static cudaError_t dense_apply_t(const DenseGeo& g, const double* coef, int nf, const void* x, void* y,
                                  cudaStream_t st) {
+  typedef typename DC<T>::C C;
+  constexpr int CPT = sizeof(T) == 4 ? 2 : 1, OUT = DS_THREADS * CPT - 8;
+  constexpr int RESIDENT = 148 * (sizeof(T) == 4 ? 3 : 2);
+  const long long strips = (long long)((g.W + OUT - 1) / OUT) * nf;
+  const bool pairs = CPT == 1 || (g.W % 2 == 0 && (((uintptr_t)coef | (uintptr_t)x | (uintptr_t)y) & 15) == 0);
+  if (strips * ((g.H + 31) / 32) >= 3 * 148 && pairs) {
+    // Band height: a band walks 14 rows more than it yields, and the last wave of
+    // blocks should be full, so take the height with the fewest row steps over
+    // all waves (1056 rows of eleven fields: 44 rows, 262 us at 32).
+    int rows = 32;
+    long long best = -1;
+    for (int r = 16; r <= DS_ROWS; ++r) {
+      const long long waves = (strips * ((g.H + r - 1) / r) + RESIDENT - 1) / RESIDENT, cost = waves * (r + 14);
+      if (best < 0 || cost < best) { best = cost; rows = r; }
+    }
+    const long long bands = strips * ((g.H + rows - 1) / rows);
+    const int smem = (int)sizeof(DenseRowsSmem<T, CPT>);
+    const cudaError_t ce = cudaFuncSetAttribute(k_dense_stream<T, ADJ, CPT>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (ce != cudaSuccess) return ce;
+    k_dense_stream<T, ADJ, CPT><<<(unsigned)bands, DS_THREADS, smem, st>>>(g, coef, (const C*)x, (C*)y, nf, rows);
+    return cudaGetLastError();
+  }
   const long long tiles = (long long)((g.W + DA_TX - 1) / DA_TX) * ((g.H + 15) / 16) * nf;
   return tiles >= 3 * 148 ? launch_dense_apply<T, ADJ, 16>(g, coef, nf, x, y, st)
                           : launch_dense_apply<T, ADJ, 8>(g, coef, nf, x, y, st);
