@@ -546,9 +546,20 @@ __device__ __forceinline__ void gen_rows_forward(float2* s, int nl, const FftPla
 
 template <typename OUT>
 __device__ __forceinline__ void gen_rows_inverse(float2* s, int nl, const FftPlan& P, const float2* g, OUT out) {
-  const int N = P.n, rs = nsr_row_stride(N);
-  for (int l = 0; l < nl; ++l)
-    for (int c = threadIdx.x; c < N; c += blockDim.x) s[l * rs + row_pos(c)] = g[(long long)l * N + c];
+  const int N = P.n, rs = nsr_row_stride(N), total = nl * N;
+  for (int k0 = threadIdx.x; k0 < total; k0 += 4 * blockDim.x) {   // four loads in flight per thread
+    float2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = g[min(k0 + u * (int)blockDim.x, total - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = k0 + u * blockDim.x;
+      if (k < total) {
+        const int l = k / N;
+        s[l * rs + row_pos(k - l * N)] = v[u];
+      }
+    }
+  }
   __syncthreads();
   gen_stages<true, 0>(s, nl, P, 1, P.nst);
   gen_radix(P.radix[0],

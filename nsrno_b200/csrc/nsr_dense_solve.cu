@@ -113,7 +113,7 @@ __device__ bool dg_arrive(const DgArgs& A, const double* mine, int nv, double* t
 }
 
 // ||b||^2 (once per solve).
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_bnorm(DgArgs A) {
+__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_bnorm(const __grid_constant__ DgArgs A) {
   __shared__ double red[NSR_DG_THREADS / 32];
   __shared__ double mine[1], tot[1];
   double s = 0.0;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_bnorm(DgArgs A) {
 
 // r = b - A x (FP64), v_0 = r in complex64, ||r||^2; the last CTA decides
 // whether the solve has converged and sets up the cycle.
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_residual(DgArgs A) {
+__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_residual(const __grid_constant__ DgArgs A) {
   __shared__ double red[NSR_DG_THREADS / 32];
   __shared__ double mine[1], tot[1];
   if (A.st->done) return;
@@ -179,7 +179,7 @@ __device__ __forceinline__ bool dg_skip(const DgState& S) { return S.done || S.s
 
 // hc[i] = <v_i, w> for i <= j of one tile of w.
 template <int TILE>
-__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_dots(DgArgs A, int j) {
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_dots(const __grid_constant__ DgArgs A, int j) {
   __shared__ double2 wt[TILE];
   __shared__ double tot[2 * (NSR_DG_MAX_M + 1)];
   if (dg_skip(*A.st)) return;
@@ -195,63 +195,42 @@ __global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_dots(DgArgs A, int j) 
     for (int i = threadIdx.x; i < nv; i += NSR_GS_THREADS) A.hc[i] = make_double2(tot[2 * i], tot[2 * i + 1]);
 }
 
-// Column j of the Hessenberg matrix, the earlier Givens rotations on it, the new
-// one, and the happy breakdown (one thread).
-__device__ void dg_finish_step(const DgArgs& A, int j, const double* tot) {
+// Column j of the Hessenberg matrix, the Givens rotations and the happy breakdown
+// (the last CTA).  Rotations G_i = [[c, s], [-conj(s), c]], c real, act on rows i, i+1.
+__device__ __noinline__ void dg_finish_step(const DgArgs& A, int j, const double* tot) {
+  __shared__ GsColumn k;
+  gs_finish_column(k, j, tot, A.hc, A.hc2, A.H + (long long)j * (A.m + 1), A.cs, A.sn, A.gv,
+                   [](double2 a, double hn, double* c, double2* s, double2* d) {
+                     const double an = sqrt(a.x * a.x + a.y * a.y);
+                     const double den = sqrt(an * an + hn * hn);
+                     if (den == 0.0) {
+                       *c = 1.0; *s = make_double2(0.0, 0.0);
+                     } else if (an == 0.0) {
+                       *c = 0.0; *s = make_double2(1.0, 0.0);
+                     } else {
+                       *c = an / den;
+                       const double2 ph = make_double2(a.x / an, a.y / an);
+                       *s = (hn / den) * ph;   // s = (a / |a|) hn / den
+                     }
+                     *d = *c * a + hn * *s;   // = (a / |a|) den
+                   });
+  if (threadIdx.x != 0) return;
   DgState& S = *A.st;
-  const int m1 = A.m + 1;
-  double2* col = A.H + (long long)j * m1;
-  double nrm = tot[2 * (j + 1)];
-  for (int i = 0; i <= j; ++i) {
-    const double2 h2 = make_double2(tot[2 * i], tot[2 * i + 1]);
-    A.hc2[i] = h2;
-    col[i] = A.hc[i] + h2;
-    nrm -= h2.x * h2.x + h2.y * h2.y;
-  }
-  const double hn = nrm > 0.0 ? sqrt(nrm) : (nrm <= 0.0 ? 0.0 : nrm);   // a NaN stays one
-  col[j + 1] = make_double2(hn, 0.0);
   S.steps += 1;
   S.used = j + 1;
-  // Givens rotations G_i = [[c, s], [-conj(s), c]] (c real) applied to rows i, i+1.
-  for (int i = 0; i < j; ++i) {
-    const double2 a = col[i], b = col[i + 1];
-    col[i] = A.cs[i] * a + A.sn[i] * b;
-    col[i + 1] = A.cs[i] * b - conjc(A.sn[i]) * a;
-  }
-  const double2 a = col[j];
-  const double an = sqrt(a.x * a.x + a.y * a.y);
-  const double den = sqrt(an * an + hn * hn);
-  double c;
-  double2 sgn;
-  if (den == 0.0) {
-    c = 1.0; sgn = make_double2(0.0, 0.0);
-  } else if (an == 0.0) {
-    c = 0.0; sgn = make_double2(1.0, 0.0);
-  } else {
-    c = an / den;
-    const double2 ph = make_double2(a.x / an, a.y / an);
-    sgn = (hn / den) * ph;   // s = (a / |a|) hn / den
-  }
-  A.cs[j] = c;
-  A.sn[j] = sgn;
-  col[j] = c * a + hn * sgn;   // = (a / |a|) den
-  col[j + 1] = make_double2(0.0, 0.0);
-  const double2 g = A.gv[j];
-  A.gv[j] = c * g;
-  A.gv[j + 1] = make_double2(0.0, 0.0) - conjc(sgn) * g;
-  if (!isfinite(hn)) {
+  if (!isfinite(k.norm)) {
     S.done = 1;
     S.status = NSR_NONFINITE;
-  } else if (hn < 1e-12) {
+  } else if (k.norm < 1e-12) {
     S.stop = 1;   // happy breakdown (nsrno/wave_solver.py:29-31)
   }
-  S.beta = hn;   // normaliser of v_{j+1}
+  S.beta = k.norm;   // normaliser of v_{j+1}
 }
 
 // w -= sum_i hc[i] v_i (FP64), then of the new w the second pass's inner products
 // and ||w||^2; the last CTA finishes the step.
 template <int TILE>
-__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_gs(DgArgs A, int j) {
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_gs(const __grid_constant__ DgArgs A, int j) {
   __shared__ double2 wt[TILE];
   __shared__ double tot[2 * (NSR_DG_MAX_M + 1) + 1];
   __shared__ double2 h[NSR_DG_MAX_M + 1];
@@ -268,19 +247,25 @@ __global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_gs(DgArgs A, int j) {
     const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
     acc[c] = to_d(k < A.n ? A.w[k] : zero);
   }
-#pragma unroll 4
-  for (int i = 0; i < nv; ++i) {
-    const float2* __restrict__ v = A.V + i * A.n;
-    const double2 hi = h[i];
-    float2 x[C];
+  constexpr int B = C >= 8 ? 1 : 8 / C;   // vectors whose loads are in flight together
+  for (int i0 = 0; i0 < nv; i0 += B) {
+    float2 x[B][C];
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const long long k = base + c * NSR_GS_THREADS + threadIdx.x;
-      x[c] = k < A.n ? v[k] : zero;
-    }
+    for (int b = 0; b < B; ++b)
 #pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = acc[c] - hi * to_d(x[c]);
+      for (int c = 0; c < C; ++c)
+        x[b][c] = A.V[min(i0 + b, nv - 1) * A.n + min(base + c * NSR_GS_THREADS + threadIdx.x, A.n - 1)];
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+      if (i0 + b < nv) {
+        const double2 hi = h[i0 + b];
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[c] = acc[c] - hi * to_d(x[b][c]);
+      }
   }
+#pragma unroll
+  for (int c = 0; c < C; ++c)   // nodes past the end hold what their clamped loads gave
+    if (base + c * NSR_GS_THREADS + threadIdx.x >= A.n) acc[c] = make_double2(0.0, 0.0);
   double nrm = 0.0;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
@@ -295,13 +280,13 @@ __global__ void __launch_bounds__(NSR_GS_THREADS, 4) k_dg_gs(DgArgs A, int j) {
   if (threadIdx.x == 0) A.part[(long long)(2 * nv) * nb + blockIdx.x] = nrm;
   gs_dots<TILE>(wt, A.V, A.n, nv, [&](int e) -> long long { return min(base + e, A.n - 1); }, A.part, nb,
                 blockIdx.x);
-  if (gs_arrive(A.part, nb, 2 * nv + 1, A.arrive, tot) && threadIdx.x == 0) dg_finish_step(A, j, tot);
+  if (gs_arrive(A.part, nb, 2 * nv + 1, A.arrive, tot)) dg_finish_step(A, j, tot);
 }
 
 // v_j and its row transform: the elementwise work runs inside the transform's
 // first stage.
 template <bool GEN>
-__global__ void __launch_bounds__(256, GEN ? 2 : 3) k_dg_rows(DgArgs A, int nz, int nx, PrecTables t,
+__global__ void __launch_bounds__(256, GEN ? 2 : 3) k_dg_rows(const __grid_constant__ DgArgs A, int nz, int nx, PrecTables t,
                                                               float2* __restrict__ W, int rows, int j) {
   extern __shared__ float2 sm[];
   __shared__ double2 c2[NSR_DG_MAX_M];
@@ -312,9 +297,10 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 3) k_dg_rows(DgArgs A, int nz, 
   const float inv = (float)(1.0 / S.beta);
   const int z0 = blockIdx.x * rows;
   const long long off = blockIdx.y * (long long)nz * nx + (long long)z0 * nx;
-  const float2* src = (j == 0 ? A.V : A.w) + off;   // k_dg_residual leaves r in V
+  // k_dg_residual leaves r in v_0, so for j = 0 src and vj are one buffer
+  const float2* src = (j == 0 ? A.V : A.w) + off;
   float2* vj = A.V + (long long)j * A.n + off;
-  const float2* V = A.V + off;
+  const float2* __restrict__ V = A.V + off;
   rows_forward<GEN>(sm, min(rows, nz - z0), t.px, W + off, [&](auto tag, int k0, int step, float2* v) {
     constexpr int R = decltype(tag)::value;
     if (j == 0) {
@@ -342,7 +328,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 3) k_dg_rows(DgArgs A, int nz, 
 }
 
 // y = R^-1 g over the steps of the cycle (FP64).
-__global__ void k_dg_solve(DgArgs A) {
+__global__ void k_dg_solve(const __grid_constant__ DgArgs A) {
   // One warp, column by column: once y_i is known every lane takes its share of
   // the rows above it.
   __shared__ double2 g[NSR_DG_MAX_M];
@@ -363,7 +349,7 @@ __global__ void k_dg_solve(DgArgs A) {
 }
 
 // x += sum_j y_j z_j (FP64).
-__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_xupdate(DgArgs A) {
+__global__ void __launch_bounds__(NSR_DG_THREADS) k_dg_xupdate(const __grid_constant__ DgArgs A) {
   __shared__ double2 y[NSR_DG_MAX_M];
   const DgState& S = *A.st;
   if (S.done) return;

@@ -90,7 +90,6 @@ __device__ __forceinline__ bool g_active(const GSlot& S, int j) {
   return S.sys >= 0 && !S.done && !S.stop && j >= S.used;
 }
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) { return a * b; }
 __device__ __forceinline__ double cabs(double2 a) { return sqrt(a.x * a.x + a.y * a.y); }
 
 __device__ __forceinline__ double* g_part(const GArgs& A, int slot) {
@@ -102,7 +101,7 @@ __device__ __forceinline__ double* g_part(const GArgs& A, int slot) {
 // stored in V and transformed by rows.
 // ---------------------------------------------------------------------------
 template <bool GEN>
-__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(const __grid_constant__ GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -142,7 +141,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_fwd(GArgs A, int j) {
 
 // cols for slots active at step j (j < 0: slots that run a cycle-end update)
 template <int TC, bool GEN, bool LEARNED>
-__global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(GArgs A, int j) {
+__global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(const __grid_constant__ GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(GArgs A, int j) {
 // once per system, in the digit-reversed (z, x) order of the transformed field,
 // and read by every column pass (94 us for eleven 768 x 1024 systems with the
 // two tanh, the exponential and the sincos evaluated in the pass).
-__global__ void __launch_bounds__(256) gk_sym(GArgs A) {
+__global__ void __launch_bounds__(256) gk_sym(const __grid_constant__ GArgs A) {
   const GSlot& S = A.slots[blockIdx.y];
   if (S.sys < 0) return;
   const Geo& g = A.g;
@@ -183,7 +182,7 @@ __global__ void __launch_bounds__(256) gk_sym(GArgs A) {
 // rinv: inverse row FFT of W in place, times the outer gain (W becomes M^-1 v_j,
 // or M^-1 u at the end of a cycle when j < 0).
 template <bool GEN>
-__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(GArgs A, int j) {
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(const __grid_constant__ GArgs A, int j) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -206,7 +205,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_rinv(GArgs A, int j) {
 // with the north/centre/south values of z and a in registers.
 #define NSR_GST_TX NSR_GS_THREADS
 template <bool ADJ, int TZ>
-__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_inv(GArgs A, int j) {
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_inv(const __grid_constant__ GArgs A, int j) {
   extern __shared__ __align__(16) double2 wt[];   // TZ x NSR_GST_TX nodes of w
   __shared__ double tot[2 * (NSR_GMRES_MAX_M + 1)];
   __shared__ RowFactors<float> rowf[TZ];
@@ -304,68 +303,43 @@ __global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_inv(GArgs A, int j) {
       A.hc[(long long)slot * (A.m + 1) + i] = make_double2(tot[2 * i], tot[2 * i + 1]);
 }
 
-// Column j of the Hessenberg matrix, its Givens rotations, and whether the
-// cycle stops (one thread).
-__device__ void g_finish_step(const GArgs& A, GSlot& S, int slot, int j, const double* tot) {
+// Column j of the Hessenberg matrix, its Givens rotations, and whether the cycle
+// stops (the last CTA).
+__device__ __noinline__ void g_finish_step(const GArgs& A, GSlot& S, int slot, int j, const double* tot) {
+  __shared__ GsColumn k;
   const int m = A.m;
-  double2* Hc = A.H + (long long)slot * (m + 1) * m + j * (m + 1);   // column j
-  const double2* hc = A.hc + (long long)slot * (m + 1);
-  double2* hc2 = A.hc2 + (long long)slot * (m + 1);
-  double nrm = tot[2 * (j + 1)];
-  for (int i = 0; i <= j; ++i) {
-    const double2 h2 = make_double2(tot[2 * i], tot[2 * i + 1]);
-    hc2[i] = h2;
-    Hc[i] = hc[i] + h2;
-    nrm -= h2.x * h2.x + h2.y * h2.y;
-  }
-  const double hnext = nrm > 0.0 ? sqrt(nrm) : (nrm <= 0.0 ? 0.0 : nrm);   // a NaN stays one
-  Hc[j + 1] = make_double2(hnext, 0.0);
-  S.hlast = hnext;
-  double* cs = A.cs + (long long)slot * m;
-  double2* sn = A.sn + (long long)slot * m;
-  double2* gv = A.gv + (long long)slot * (m + 1);
-  // previous rotations on column j
-  for (int i = 0; i < j; ++i) {
-    const double2 a = Hc[i], b = Hc[i + 1];
-    Hc[i] = cs[i] * a + cmul(sn[i], b);
-    Hc[i + 1] = cs[i] * b - cmul(conjc(sn[i]), a);
-  }
-  // new rotation zeroing Hc[j+1]
-  const double2 a = Hc[j];
-  const double b = hnext;
-  const double aa = cabs(a);
-  const double nu = sqrt(aa * aa + b * b);
-  double c;
-  double2 s;
-  if (aa == 0.0) {
-    c = 0.0;
-    s = make_double2(1.0, 0.0);
-    Hc[j] = make_double2(b, 0.0);
-  } else {
-    const double2 ph = make_double2(a.x / aa, a.y / aa);
-    c = aa / nu;
-    s = make_double2(ph.x * b / nu, ph.y * b / nu);
-    Hc[j] = make_double2(ph.x * nu, ph.y * nu);
-  }
-  Hc[j + 1] = make_double2(0.0, 0.0);
-  cs[j] = c;
-  sn[j] = s;
-  const double2 gj = gv[j];
-  gv[j] = c * gj;
-  gv[j + 1] = make_double2(0.0, 0.0) - cmul(conjc(s), gj);
+  gs_finish_column(k, j, tot, A.hc + (long long)slot * (m + 1), A.hc2 + (long long)slot * (m + 1),
+                   A.H + (long long)slot * (m + 1) * m + j * (m + 1), A.cs + (long long)slot * m,
+                   A.sn + (long long)slot * m, A.gv + (long long)slot * (m + 1),
+                   [](double2 a, double b, double* c, double2* s, double2* d) {
+                     const double aa = cabs(a);
+                     const double nu = sqrt(aa * aa + b * b);
+                     if (aa == 0.0) {
+                       *c = 0.0;
+                       *s = make_double2(1.0, 0.0);
+                       *d = make_double2(b, 0.0);
+                     } else {
+                       const double2 ph = make_double2(a.x / aa, a.y / aa);
+                       *c = aa / nu;
+                       *s = make_double2(ph.x * b / nu, ph.y * b / nu);
+                       *d = make_double2(ph.x * nu, ph.y * nu);
+                     }
+                   });
+  if (threadIdx.x != 0) return;
+  S.hlast = k.norm;
   S.used = j + 1;
   S.iters += 1;
-  const double est = cabs(gv[j + 1]) / S.bnorm;
+  const double est = cabs(k.g1) / S.bnorm;
   // Stop the cycle on convergence of the estimate, on a happy breakdown
   // (nsrno/wave_solver.py:31-32), at the restart length or at the budget.
-  if (est < 0.5 * A.tol || !(hnext > 1e-12 * S.beta) || j + 1 == m || S.iters >= A.max_it || !isfinite(est))
+  if (est < 0.5 * A.tol || !(k.norm > 1e-12 * S.beta) || j + 1 == m || S.iters >= A.max_it || !isfinite(est))
     S.stop = 1;
 }
 
 // gs: w -= sum_i h_i v_i, then of the new w the second pass's inner products and
 // ||w||^2; the last CTA finishes the step.
 template <int TILE>
-__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_gs(GArgs A, int j) {
+__global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_gs(const __grid_constant__ GArgs A, int j) {
   extern __shared__ __align__(16) double2 wt[];   // TILE nodes of w
   __shared__ double tot[2 * (NSR_GMRES_MAX_M + 1) + 1];
   __shared__ float2 coef[NSR_GMRES_MAX_M + 1];
@@ -412,11 +386,11 @@ __global__ void __launch_bounds__(NSR_GS_THREADS, 4) gk_gs(GArgs A, int j) {
   nrm = gs_block_sum(nrm);   // its barriers also publish wt
   if (threadIdx.x == 0) part[(long long)(2 * nv) * nb + blockIdx.x] = nrm;
   gs_dots<TILE>(wt, V, n, nv, [&](int e) -> long long { return min(base + e, n - 1); }, part, nb, blockIdx.x);
-  if (gs_arrive(part, nb, 2 * nv + 1, &A.arrive[slot], tot) && threadIdx.x == 0) g_finish_step(A, S, slot, j, tot);
+  if (gs_arrive(part, nb, 2 * nv + 1, &A.arrive[slot], tot)) g_finish_step(A, S, slot, j, tot);
 }
 
 // Back substitution R y = g for the slots that ran a cycle.
-__global__ void gk_solve(GArgs A) {
+__global__ void gk_solve(const __grid_constant__ GArgs A) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.n_slots) return;
   GSlot& S = A.slots[slot];
@@ -427,14 +401,14 @@ __global__ void gk_solve(GArgs A) {
   double2* y = A.y + (long long)slot * m;
   for (int i = u - 1; i >= 0; --i) {
     double2 acc = gv[i];
-    for (int k = i + 1; k < u; ++k) acc = acc - cmul(H[k * (m + 1) + i], y[k]);
+    for (int k = i + 1; k < u; ++k) acc = acc - H[k * (m + 1) + i] * y[k];
     y[i] = divc(acc, H[i * (m + 1) + i]);
   }
 }
 
 // u = V y, forward row FFT into W.
 template <bool GEN>
-__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_comb(GArgs A) {
+__global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_comb(const __grid_constant__ GArgs A) {
   extern __shared__ float2 sm[];
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -469,7 +443,7 @@ __global__ void __launch_bounds__(256, GEN ? 2 : 4) gk_comb(GArgs A) {
 
 // FP64 true residual.  init = 1: x = x0 (or 0); init = 0: x += M^-1 V y.
 template <bool ADJ>
-__global__ void __launch_bounds__(NSR_RES_TX) gk_res(GArgs A, int init) {
+__global__ void __launch_bounds__(NSR_RES_TX) gk_res(const __grid_constant__ GArgs A, int init) {
   __shared__ double tot[2];
   const int slot = blockIdx.y;
   GSlot& S = A.slots[slot];
@@ -540,7 +514,7 @@ __global__ void __launch_bounds__(NSR_RES_TX) gk_res(GArgs A, int init) {
 }
 
 // Outputs of one batch: IQ, residual, iterations, status, fields.
-__global__ void gk_emit(GArgs A, double2* iq, const int* rx, int n_rx, double* residual, int* iterations,
+__global__ void gk_emit(const __grid_constant__ GArgs A, double2* iq, const int* rx, int n_rx, double* residual, int* iterations,
                         int* status, void* fields, int fields_fp64) {
   const int slot = blockIdx.y;
   const GSlot& S = A.slots[slot];
@@ -569,7 +543,7 @@ __global__ void gk_emit(GArgs A, double2* iq, const int* rx, int n_rx, double* r
   }
 }
 
-__global__ void gk_load(GArgs A, int first, int count, const double* freq, const double* angle) {
+__global__ void gk_load(const __grid_constant__ GArgs A, int first, int count, const double* freq, const double* angle) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= A.n_slots) return;
   GSlot S;
@@ -588,7 +562,7 @@ __global__ void gk_load(GArgs A, int first, int count, const double* freq, const
   A.arrive[slot] = 0;
 }
 
-__global__ void gk_count(GArgs A, int* remaining) {
+__global__ void gk_count(const __grid_constant__ GArgs A, int* remaining) {
   __shared__ int cnt;
   if (threadIdx.x == 0) cnt = 0;
   __syncthreads();

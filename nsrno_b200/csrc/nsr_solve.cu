@@ -182,7 +182,7 @@ enum { PASS_STAGED = 0, PASS_DIRECT = 1, PASS_GENERIC = 2 };
 // runs inside the transform's first stage (rows_forward).
 // ---------------------------------------------------------------------------
 template <int PASS>
-__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(SolveArgs A, int half) {
+__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(const __grid_constant__ SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const SlotState& S = A.B.slots[slot];
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(Solve
 // cols: column FFT, preconditioner multiply, inverse column FFT (in place).
 // ---------------------------------------------------------------------------
 template <int TC, bool LEARNED, int PASS>
-__global__ void __launch_bounds__(PASS == PASS_GENERIC ? 256 : 512, 2) k_cols(SolveArgs A, int half) {
+__global__ void __launch_bounds__(PASS == PASS_GENERIC ? 256 : 512, 2) k_cols(const __grid_constant__ SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const int mode = A.B.slots[slot].mode;
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(PASS == PASS_GENERIC ? 256 : 512, 2) k_cols(So
 // registers (rows_inverse).
 // ---------------------------------------------------------------------------
 template <int PASS>
-__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_rinv(SolveArgs A, int half) {
+__global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_rinv(const __grid_constant__ SolveArgs A, int half) {
   extern __shared__ float2 sm[];
   const int slot = A.slot0 + blockIdx.x;
   const SlotState& S = A.B.slots[slot];
@@ -658,7 +658,7 @@ __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); 
 __device__ __forceinline__ float4 pack2(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
 
 template <bool ADJ>
-__global__ void __launch_bounds__(256, 4) k_inv(SolveArgs A, int half) {
+__global__ void __launch_bounds__(256, 4) k_inv(const __grid_constant__ SolveArgs A, int half) {
   const int slot = A.slot0 + blockIdx.y;
   SlotState& S = A.B.slots[slot];
   const int mode = S.mode;
@@ -874,7 +874,7 @@ __device__ __forceinline__ float2 stencil_plain(float kh2, float fpow, float a_c
 
 template <int W, int D, int CPT, bool ADJ, int H>
 __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>()))
-    k_stn(SolveArgs A, int /*half: H*/, StnItems it, int ns) {
+    k_stn(const __grid_constant__ SolveArgs A, int /*half: H*/, StnItems it, int ns) {
   typedef StnLayout<W, H> Ly;
   constexpr int half = H;
   constexpr int NP = stn_parts(H);
@@ -1188,7 +1188,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
 // neighbours are the adjacent threads' loads (L1 hits).
 // ---------------------------------------------------------------------------
 template <bool ADJ>
-__global__ void __launch_bounds__(256, 4) k_inv1(SolveArgs A, int half) {
+__global__ void __launch_bounds__(256, 4) k_inv1(const __grid_constant__ SolveArgs A, int half) {
   const int slot = A.slot0 + blockIdx.y;
   SlotState& S = A.B.slots[slot];
   const int mode = S.mode;
@@ -1262,7 +1262,7 @@ __global__ void __launch_bounds__(256, 4) k_inv1(SolveArgs A, int half) {
 // each, and receivers gathered by one thread, 9 ms on residual_tiles.
 // ---------------------------------------------------------------------------
 template <bool ADJ>
-__global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
+__global__ void __launch_bounds__(NSR_RES_TX) k_res(const __grid_constant__ SolveArgs A) {
   const int slot = A.slot0 + blockIdx.y;
   SlotState& S = A.B.slots[slot];
   const int mode = S.mode;
@@ -1308,7 +1308,7 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(SolveArgs A) {
 }
 
 
-__global__ void k_solve_init(SolveArgs A, int n_slots) {
+__global__ void k_solve_init(const __grid_constant__ SolveArgs A, int n_slots) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < A.n_systems; s += gridDim.x * blockDim.x) {
     A.status[s] = NSR_NOT_RUN;
@@ -1352,7 +1352,7 @@ __device__ __forceinline__ bool loop_ends(const SolveArgs& A, unsigned long long
   const int error = *(volatile int*)A.B.error;
   return done >= A.n_systems || error || rounds >= (unsigned long long)max_rounds;
 }
-__global__ void k_loop_control(SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
+__global__ void k_loop_control(const __grid_constant__ SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   unsigned long long* rounds = reinterpret_cast<unsigned long long*>(A.B.queue + 6);
   const unsigned long long r = *rounds + 1;
@@ -1360,11 +1360,11 @@ __global__ void k_loop_control(SolveArgs A, cudaGraphConditionalHandle loop, lon
   if (loop_ends(A, r, max_rounds)) cudaGraphSetConditional(loop, 0);
 }
 // Last launch of the first round, which runs outside the loop.
-__global__ void k_round_count(SolveArgs A) {
+__global__ void k_round_count(const __grid_constant__ SolveArgs A) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *reinterpret_cast<unsigned long long*>(A.B.queue + 6) += 1;
 }
 // First node of the loop's graph: whether the loop runs at all.
-__global__ void k_loop_begin(SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
+__global__ void k_loop_begin(const __grid_constant__ SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const unsigned long long r = *reinterpret_cast<unsigned long long*>(A.B.queue + 6);
   cudaGraphSetConditional(loop, loop_ends(A, r, max_rounds) ? 0 : 1);
