@@ -368,14 +368,16 @@ extern "C" int nsr_precondition(const NsrGrid* grid, const double* freq_hz, int3
   return last_error();
 }
 
-// Row tiles near 32 KB of shared memory, at most 8 rows; half or a quarter of
-// that for batches of fewer than two such tiles per SM (solves of three
-// 256 x 256 and six 256 x 384 systems take 4% less with the tile rules).
+// Row tiles near 32 KB of shared memory (40 KB where the transform's first radix
+// may be a large prime: four rows of 1216 give all 256 threads a butterfly, 107 ->
+// 96 us for eleven 1056 x 1216 fields), at most 8 rows; half or a quarter of that
+// for batches of fewer than four such tiles for three SMs (solves of three 256 x
+// 256 and six 256 x 384 systems take 4% less with the tile rules).
 int nsr_rows_per_cta(const NsrGrid* g, int ns) {
-  int rows = (int)(4096 / g->nx);
+  int rows = (int)((nsr_specialised(g->nx) ? 4096 : 5120) / g->nx);
   if (rows < 1) rows = 1;
   if (rows > 8) rows = 8;
-  while (rows > 2 && (long long)ns * ((g->nz + rows - 1) / rows) < 2 * 148) rows = (rows + 1) / 2;
+  while (rows > 2 && 3LL * ns * ((g->nz + rows - 1) / rows) < 4 * 148) rows = (rows + 1) / 2;
   return rows;
 }
 
@@ -426,13 +428,14 @@ extern "C" int nsr_plane_wave_rhs(const NsrGrid* grid, const double* freq_hz, co
 // registers while the systems go by; the tile of u and lam of the next system is
 // copied into shared memory (cp.async) while the present one is summed.  The edge term is the same product at both
 // ends of an edge, so each south edge is formed once and carried to the next
-// row.  With c = (k0 h)^2 sx sz and onepie = 1 + i e the sums are kept without
+// row, each east edge once and handed to the next lane.  With c = (k0 h)^2 sx sz and onepie = 1 + i e the sums are kept without
 // b and a:  acc_c = 2 sum Re(conj(lam) u c onepie),  acc_r = sum Re(conj(lam) u
 // c onepie^2),  acc_e = sum Re(edges); everything is FP64 as before.  Bound by
-// FP64 issue and conversions (about 30 FP64 operations and 8 conversions per
+// FP64 issue and conversions (about 40 FP64 operations and 8 conversions per
 // node and system).  22 systems of 1024 x 1536: 1,152 us with one thread per
-// node, a pow and six PML profiles per node and system; 270 us in this form.
+// node, a pow and six PML profiles per node and system; 270 us with the x edges formed at both ends, 251 us in this form.
 #define NSR_GRAD_TX 128      // threads of a block, one column each
+#define NSR_GRAD_OWN 124     // columns a block yields: a warp's first lane only forms the east edge its neighbour needs
 #define NSR_GRAD_CHUNK 64    // systems whose scalars are staged in shared memory at a time
 
 __device__ __forceinline__ void cp_async_zfill(float2* dst, const float2* src, bool live) {
@@ -447,11 +450,11 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int PENDING>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-// Columns c0 - 1 .. c0 + NSR_GRAD_TX of the rows z0 - 1 .. z0 + TZ of a field
-// (zero outside the grid).
+// Columns c0 .. c0 + NSR_GRAD_OWN + 1 of the rows z0 - 1 .. z0 + TZ of a field (zero
+// outside the grid).
 template <typename CT, int TZ>
 struct GradTile {
-  CT u[TZ + 2][NSR_GRAD_TX + 2], l[TZ + 2][NSR_GRAD_TX + 2];
+  CT u[TZ + 2][NSR_GRAD_TX], l[TZ + 2][NSR_GRAD_TX];
 };
 template <typename CT, int TZ>
 __device__ __forceinline__ void grad_fetch(GradTile<CT, TZ>& t, const Geo& g, const CT* us, const CT* ls, int z0,
@@ -461,19 +464,10 @@ __device__ __forceinline__ void grad_fetch(GradTile<CT, TZ>& t, const Geo& g, co
     const int i = z0 - 1 + r;
     const bool row = i >= 0 && i < g.nz;
     const int j = c0 + threadIdx.x;
-    const bool live = row && j < g.nx;
+    const bool live = row && j >= 0 && j < g.nx;
     const long long id = live ? (long long)i * g.nx + j : 0;
-    cp_async_zfill(&t.u[r][threadIdx.x + 1], us + id, live);
-    cp_async_zfill(&t.l[r][threadIdx.x + 1], ls + id, live);
-  }
-  // the two halo columns
-  for (int q = threadIdx.x; q < 2 * (TZ + 2); q += NSR_GRAD_TX) {
-    const int r = q >> 1, i = z0 - 1 + r, j = (q & 1) ? c0 + NSR_GRAD_TX : c0 - 1;
-    const bool live = i >= 0 && i < g.nz && j >= 0 && j < g.nx;
-    const long long id = live ? (long long)i * g.nx + j : 0;
-    const int c = (q & 1) ? NSR_GRAD_TX + 1 : 0;
-    cp_async_zfill(&t.u[r][c], us + id, live);
-    cp_async_zfill(&t.l[r][c], ls + id, live);
+    cp_async_zfill(&t.u[r][threadIdx.x], us + id, live);
+    cp_async_zfill(&t.l[r][threadIdx.x], ls + id, live);
   }
   cp_async_commit();
 }
@@ -488,20 +482,22 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
   GradTile<CT, TZ>* tiles = reinterpret_cast<GradTile<CT, TZ>*>(grad_smem);   // two: one in use, one in flight
   const long long n = (long long)g.nz * g.nx;
   const int nx = g.nx, nz = g.nz;
-  const int nbx = (nx + NSR_GRAD_TX - 1) / NSR_GRAD_TX;
-  const int c0 = (blockIdx.x % nbx) * NSR_GRAD_TX;
-  const int j = c0 + threadIdx.x, tx = threadIdx.x + 1;
+  // Tile column tx is grid column c0 + tx; warp w takes 32 of them from 31 w on, and
+  // its lanes 1 .. 31 own theirs.
+  const int nbx = (nx + NSR_GRAD_OWN - 1) / NSR_GRAD_OWN;
+  const int c0 = (blockIdx.x % nbx) * NSR_GRAD_OWN - 1;
+  const int lane = threadIdx.x & 31, tx = 31 * (threadIdx.x >> 5) + lane;
+  const int j = c0 + tx;
   const int z0 = (blockIdx.x / nbx) * TZ;
-  const bool own = j < nx;
-  const int jc = own ? j : nx - 1;
+  const bool own = lane > 0 && j < nx;
+  const int jc = min(max(j, 0), nx - 1);
   const MatPlanes mp = nsr_planes(mat, n);
   grad_fetch(tiles[0], g, u, lam, z0, c0);
   const bool col_plain = j > g.n_pml && j < nx - 1 - g.n_pml;
-  // PML profiles of the column at j, j + 1/2, j - 1/2 (zero off the PML)
-  const double px = col_plain ? 0.0 : pml_profile<double>((double)jc, nx, g.n_pml);
-  const double pxe = col_plain ? 0.0 : pml_profile<double>(jc + 0.5, nx, g.n_pml);
-  const double pxw = col_plain ? 0.0 : pml_profile<double>(jc - 0.5, nx, g.n_pml);
-  const bool warp_plain = __all_sync(0xffffffffu, col_plain || !own);
+  // PML profiles of the column at j and j + 1/2 (zero off the PML)
+  const double px = col_plain ? 0.0 : pml_profile<double>((double)j, nx, g.n_pml);
+  const double pxe = col_plain ? 0.0 : pml_profile<double>(j + 0.5, nx, g.n_pml);
+  const bool warp_plain = __all_sync(0xffffffffu, col_plain || j >= nx);
   double acc_c[TZ], acc_r[TZ], acc_e[TZ];
   double t64[TZ];
 #pragma unroll
@@ -530,9 +526,9 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
       __syncthreads();
       const GradTile<CT, TZ>& t = tiles[sys & 1];
       const SysScalars s = scs[q];
-      // 1 / (1 + i sig p) of the column's east and west half nodes
-      double2 ie = make_double2(1.0, 0.0), iw = ie;
-      if (!warp_plain) { ie = inv_stretch(s.sig * pxe); iw = inv_stretch(s.sig * pxw); }
+      // 1 / (1 + i sig p) of the column's east half node
+      double2 ie = make_double2(1.0, 0.0);
+      if (!warp_plain) ie = inv_stretch(s.sig * pxe);
       const double2 sx = make_double2(1.0, s.sig * px);
       double2 uc = D(t.u[1][tx]), lc = D(t.l[1][tx]);
       double north;   // Re(w conj(dl) du) of the edge to the row above
@@ -549,26 +545,28 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
         const int i = z0 + r;
         const double2 un = D(t.u[r + 2][tx]), ln = D(t.l[r + 2][tx]);
         const double2 due = D(t.u[r + 1][tx + 1]) - uc, dle = D(t.l[r + 1][tx + 1]) - lc;
-        const double2 duw = D(t.u[r + 1][tx - 1]) - uc, dlw = D(t.l[r + 1][tx - 1]) - lc;
         const double2 dus = un - uc, dls = ln - lc;
         const double2 lu = prod(lc, uc);
         const double e = t64[r] * s.fpow;
         const bool row_plain = i > g.n_pml && i < nz - 1 - g.n_pml;
         if (row_plain && warp_plain) {
           const double south = dls.x * dus.x + dls.y * dus.y;
-          const double ew = dle.x * due.x + dle.y * due.y + (dlw.x * duw.x + dlw.y * duw.y);
-          acc_e[r] += 0.5 * (ew + south + north);
+          const double east = dle.x * due.x + dle.y * due.y;
+          const double west = __shfl_up_sync(0xffffffffu, east, 1);
+          acc_e[r] += 0.5 * (east + west + south + north);
           north = south;
           const double ei = e * lu.y;
           acc_c[r] += s.kh2 * (lu.x - ei);
           acc_r[r] += s.kh2 * (lu.x * (1.0 - e * e) - 2.0 * ei);
         } else {
-          const double2 pe = prod(dle, due), pw = prod(dlw, duw), ps = prod(dls, dus);
+          const double2 pe = prod(dle, due), ps = prod(dls, dus);
           const double2 sz = make_double2(1.0, s.sig * pml_profile<double>((double)i, nz, g.n_pml));
-          const double2 we = sz * ie, ww = sz * iw;
+          const double2 we = sz * ie;
           const double2 ws = sx * inv_stretch(s.sig * pml_profile<double>(i + 0.5, nz, g.n_pml));
           const double south = ws.x * ps.x - ws.y * ps.y;
-          acc_e[r] += 0.5 * ((we.x * pe.x - we.y * pe.y) + (ww.x * pw.x - ww.y * pw.y) + south + north);
+          const double east = we.x * pe.x - we.y * pe.y;
+          const double west = __shfl_up_sync(0xffffffffu, east, 1);
+          acc_e[r] += 0.5 * (east + west + south + north);
           north = south;
           const double2 cell = sx * sz;
           const double2 c1 = cell * make_double2(1.0, e), c2 = cell * make_double2(1.0 - e * e, 2.0 * e);
@@ -597,7 +595,7 @@ static cudaError_t launch_grad(const Geo& g, const void* coef, const double* fre
                                const void* lam, double* gc, double* gr, cudaStream_t st) {
   // 4-row tiles read 6 rows for 4, from L2; a grid whose 4-row tiles would
   // leave SMs without four blocks takes 2-row tiles.
-  const int bx = (g.nx + NSR_GRAD_TX - 1) / NSR_GRAD_TX;
+  const int bx = (g.nx + NSR_GRAD_OWN - 1) / NSR_GRAD_OWN;
   const CT *pu = (const CT*)u, *pl = (const CT*)lam;
   cudaError_t ce;
   if ((long long)bx * ((g.nz + 3) / 4) >= 4 * 148) {
