@@ -300,8 +300,42 @@ __host__ __device__ constexpr PrimeTable<R> make_prime_table() {
   return t;
 }
 
-template <int R, bool INV>
+// Complex sums, packed or not.
+template <bool PACKED>
+struct Sum2 {
+  static __device__ __forceinline__ float2 add(float2 a, float2 b) { return a + b; }
+  static __device__ __forceinline__ float2 sub(float2 a, float2 b) { return a - b; }
+};
+template <>
+struct Sum2<true> {
+  static __device__ __forceinline__ unsigned long long bits(float2 a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+  }
+  static __device__ __forceinline__ float2 of(unsigned long long r) {
+    float2 a;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+  }
+  static __device__ __forceinline__ float2 add(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
+    return of(r);
+  }
+  static __device__ __forceinline__ float2 sub(float2 a, float2 b) {   // a + (-1) b, exact in the product
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits(b)), "l"(bits(make_float2(-1.f, -1.f))), "l"(bits(a)));
+    return of(r);
+  }
+};
+
+// PACKED: complex sums as one add.rn.f32x2 instead of two adds (the same
+// rounding).  It shortens the row passes, which are short of issue slots next to
+// their loads; in the column passes the register pairs cost more than they save.
+template <int R, bool INV, bool PACKED = false>
 __device__ __forceinline__ void small_dft(float2* x) {
+  typedef Sum2<PACKED> S2;
   if constexpr (R == 5 || R == 7 || R == 11 || R == 13 || R == 17 || R == 19) {
     // Direct DFT of an odd prime length on the sums and differences of x[q] and
     // x[R - q]: (R - 1)^2 real multiply-adds instead of 4 (R - 1)^2.
@@ -329,19 +363,19 @@ __device__ __forceinline__ void small_dft(float2* x) {
     }
   } else if (R == 2) {
     float2 a = x[0], b = x[1];
-    x[0] = a + b; x[1] = a - b;
+    x[0] = S2::add(a, b); x[1] = S2::sub(a, b);
   } else if (R == 3) {
     const float h3 = 0.86602540378443864676f;
-    float2 t1 = x[1] + x[2];
+    float2 t1 = S2::add(x[1], x[2]);
     float2 t2 = x[0] - 0.5f * t1;
-    float2 d = x[1] - x[2];
+    float2 d = S2::sub(x[1], x[2]);
     // forward: t3 = -i (sqrt3/2) d ; inverse: +i (sqrt3/2) d
     float2 t3 = INV ? make_float2(-h3 * d.y, h3 * d.x) : make_float2(h3 * d.y, -h3 * d.x);
-    x[0] = x[0] + t1; x[1] = t2 + t3; x[2] = t2 - t3;
+    x[0] = S2::add(x[0], t1); x[1] = S2::add(t2, t3); x[2] = S2::sub(t2, t3);
   } else if (R == 4) {
-    float2 a = x[0] + x[2], b = x[0] - x[2], c = x[1] + x[3], e = x[1] - x[3];
+    float2 a = S2::add(x[0], x[2]), b = S2::sub(x[0], x[2]), c = S2::add(x[1], x[3]), e = S2::sub(x[1], x[3]);
     float2 d = INV ? make_float2(-e.y, e.x) : make_float2(e.y, -e.x);
-    x[0] = a + c; x[2] = a - c; x[1] = b + d; x[3] = b - d;
+    x[0] = S2::add(a, c); x[2] = S2::sub(a, c); x[1] = S2::add(b, d); x[3] = S2::sub(b, d);
   } else if (R == 16) {
     // 16 = 4 x 4: DFT4 over n1 for each n2, twiddle W16^(n2 k1), DFT4 over n2.
     const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, r2 = 0.70710678118654752440f;
@@ -349,7 +383,7 @@ __device__ __forceinline__ void small_dft(float2* x) {
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
       float2 t[4] = {x[n2], x[4 + n2], x[8 + n2], x[12 + n2]};
-      small_dft<4, INV>(t);
+      small_dft<4, INV, PACKED>(t);
 #pragma unroll
       for (int k1 = 0; k1 < 4; ++k1) y[n2][k1] = t[k1];
     }
@@ -366,25 +400,25 @@ __device__ __forceinline__ void small_dft(float2* x) {
 #pragma unroll
     for (int k1 = 0; k1 < 4; ++k1) {
       float2 t[4] = {y[0][k1], y[1][k1], y[2][k1], y[3][k1]};
-      small_dft<4, INV>(t);
+      small_dft<4, INV, PACKED>(t);
 #pragma unroll
       for (int k2 = 0; k2 < 4; ++k2) x[k1 + 4 * k2] = t[k2];
     }
   } else if (R == 8) {
     float2 ev[4] = {x[0], x[2], x[4], x[6]};
     float2 od[4] = {x[1], x[3], x[5], x[7]};
-    small_dft<4, INV>(ev);
-    small_dft<4, INV>(od);
+    small_dft<4, INV, PACKED>(ev);
+    small_dft<4, INV, PACKED>(od);
     const float r2 = 0.70710678118654752440f;
     // W8^k = exp(-+ i pi k / 4)
     float2 w1 = INV ? make_float2(r2, r2) : make_float2(r2, -r2);
     float2 w2 = INV ? make_float2(0.f, 1.f) : make_float2(0.f, -1.f);
     float2 w3 = INV ? make_float2(-r2, r2) : make_float2(-r2, -r2);
     float2 o1 = w1 * od[1], o2 = w2 * od[2], o3 = w3 * od[3];
-    x[0] = ev[0] + od[0]; x[4] = ev[0] - od[0];
-    x[1] = ev[1] + o1;    x[5] = ev[1] - o1;
-    x[2] = ev[2] + o2;    x[6] = ev[2] - o2;
-    x[3] = ev[3] + o3;    x[7] = ev[3] - o3;
+    x[0] = S2::add(ev[0], od[0]); x[4] = S2::sub(ev[0], od[0]);
+    x[1] = S2::add(ev[1], o1);    x[5] = S2::sub(ev[1], o1);
+    x[2] = S2::add(ev[2], o2);    x[6] = S2::sub(ev[2], o2);
+    x[3] = S2::add(ev[3], o3);    x[7] = S2::sub(ev[3], o3);
   }
 }
 
@@ -782,11 +816,11 @@ __device__ __forceinline__ void ct_stage(float2* s, int nl, const float2* __rest
         }
       };
       if (!INV) {
-        small_dft<R, false>(v[u]);
+        small_dft<R, false, PAD>(v[u]);
         twiddle(v[u]);
       } else {
         twiddle(v[u]);
-        small_dft<R, true>(v[u]);
+        small_dft<R, true, PAD>(v[u]);
       }
     }
 #pragma unroll
@@ -1050,7 +1084,7 @@ __device__ __forceinline__ void ct_rows_forward_direct(float2* s, int nl, const 
     const int l = b / M0, j = b - l * M0;
     float2 v[R0];
     in(RadixTag<R0>{}, l * N + j, M0, v);
-    small_dft<R0, false>(v);
+    small_dft<R0, false, true>(v);
 #pragma unroll
     for (int k = 1; k < R0; ++k) v[k] = v[k] * __ldg(tw0 + (k - 1) * M0 + j);
     float2* d = s + l * LS;
@@ -1069,7 +1103,7 @@ __device__ __forceinline__ void ct_rows_forward_direct(float2* s, int nl, const 
     float2 v[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) v[q] = src[q];
-    small_dft<16, false>(v);
+    small_dft<16, false, true>(v);
     float4* dst = reinterpret_cast<float4*>(g + (long long)l * N + o * 16);
 #pragma unroll
     for (int q = 0; q < 8; ++q) dst[q] = make_float4(v[2 * q].x, v[2 * q].y, v[2 * q + 1].x, v[2 * q + 1].y);
@@ -1094,7 +1128,7 @@ __device__ __forceinline__ void ct_rows_inverse_direct(float2* s, int nl, const 
       v[2 * q] = make_float2(t.x, t.y);
       v[2 * q + 1] = make_float2(t.z, t.w);
     }
-    small_dft<16, true>(v);
+    small_dft<16, true, true>(v);
     float2* d = s + l * LS + o * 17;
 #pragma unroll
     for (int q = 0; q < 16; ++q) d[q] = v[q];
@@ -1114,7 +1148,7 @@ __device__ __forceinline__ void ct_rows_inverse_direct(float2* s, int nl, const 
     }
 #pragma unroll
     for (int k = 1; k < R0; ++k) v[k] = v[k] * conjc(__ldg(tw0 + (k - 1) * M0 + j));
-    small_dft<R0, true>(v);
+    small_dft<R0, true, true>(v);
 #pragma unroll
     for (int q = 0; q < R0; ++q) out(l * N + j + q * M0, v[q], l, j + q * M0);
   }
