@@ -56,17 +56,17 @@ FALLBACK_HBM_GBS = 6650.0
 # per resident system (complex64 vectors; coefficient planes counted once per
 # launch and listed separately): fwd h0 reads r,v,t,p,y and writes r,p,y,w;
 # cols and rinv read and write w; inv h0 reads z (= w after rinv), rhat and
-# writes v; fwd h1 reads r,v and writes w; inv h1 reads z, rhat, r, v and
-# writes t.  res h1 (the FP64 true residual) has no work in the timed
+# writes v; fwd h1 reads r,v and writes s (over r) and w; inv h1 reads z,
+# rhat, s and writes t.  res h1 (the FP64 true residual) has no work in the timed
 # iterations of a fresh batch.
-KERNEL_BYTES = {"fwd_h0": 72, "cols_h0": 16, "rinv_h0": 16, "inv_h0": 24, "fwd_h1": 24, "cols_h1": 16,
-                "rinv_h1": 16, "res_h1": 0, "inv_h1": 40}
+KERNEL_BYTES = {"fwd_h0": 72, "cols_h0": 16, "rinv_h0": 16, "inv_h0": 24, "fwd_h1": 32, "cols_h1": 16,
+                "rinv_h1": 16, "res_h1": 0, "inv_h1": 32}
 # The learned preconditioner adds one complex64 read per node to every fwd
 # launch (inner gain), every cols launch (the multiplier plane of the slot's
 # system) and every rinv launch (outer gain).
 LEARNED_BYTES = {k: v + (8 if k.startswith(("fwd", "cols", "rinv")) else 0) for k, v in KERNEL_BYTES.items()}
 COEF_BYTES = {"inv_h0": 12, "inv_h1": 12}
-LEARNED_SETUP_LAUNCHES = 5     # pool, three convolutions, gains
+LEARNED_SETUP_LAUNCHES = 3     # pool, network, gains
 
 
 def parse():

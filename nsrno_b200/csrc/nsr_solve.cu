@@ -53,7 +53,8 @@ struct __align__(16) SlotState {
   SysScalars sc;                    // scalars of freq (set when the slot starts)
   float kh2f, sigf, fpowf, pad_f;   // per-system stencil scalars in float (set when the slot starts)
   double2 rho, alpha, omega, beta;
-  // s = r + c_sv v ; r_new = s + c_rt t ; y += c_yp p + c_ys s ; p_new = r_new + c_pp p + c_pv v
+  // Second half: s = r + c_sv v, written over r by its fwd pass.  First half: r_new = s + c_rt t ;
+  // y += c_yp p + c_ys s ; p_new = r_new + c_pp p + c_pv v.
   double2 c_sv, c_rt, c_yp, c_ys, c_pp, c_pv;
 };
 
@@ -142,7 +143,7 @@ __device__ __forceinline__ void fwd_staged(const SolveArgs& A, const SlotState& 
 #pragma unroll 4
     for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
       const float2 rk = rr_[k], vk = vv_[k], tk = tt_[k], pk = pp_[k], yk = yy_[k];
-      const float2 s1 = rk + sv * vk;
+      const float2 s1 = rk;   // r holds s after a second half
       const float2 rn = s1 + rt * tk;
       const float2 yn = yk + yp * pk + ys * s1;
       const float2 pn = rn + pp * pk + pv * vk;
@@ -154,12 +155,12 @@ __device__ __forceinline__ void fwd_staged(const SolveArgs& A, const SlotState& 
 #pragma unroll 8
     for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
       const float2 s1 = rr_[k] + sv * vv_[k];
+      rr_[k] = s1;
       sm[row_pos(k)] = G.pre ? gain_mul(G.pre, goff + k, G.conj, s1) : s1;
     }
   } else {  // MODE_RES: apply the pending update to y, transform y, clear it
     for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-      const float2 s1 = rr_[k] + sv * vv_[k];
-      const float2 yn = yy_[k] + yp * pp_[k] + ys * s1;
+      const float2 yn = yy_[k] + yp * pp_[k] + ys * rr_[k];
       sm[row_pos(k)] = G.pre ? gain_mul(G.pre, goff + k, G.conj, yn) : yn;
       yy_[k] = make_float2(0.f, 0.f);
     }
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(const
 #pragma unroll
           for (int q = 0; q < CH; ++q) {
             const int k = k0 + (c + q) * step;
-            const float2 s1 = rk[q] + sv * vk[q];
+            const float2 s1 = rk[q];   // r holds s after a second half
             const float2 rn = s1 + rt * tk[q];
             const float2 yn = yk[q] + yp * pk[q] + ys * s1;
             const float2 pn = rn + pp * pk[q] + pv * vk[q];
@@ -271,13 +272,15 @@ __global__ void __launch_bounds__(256, PASS == PASS_GENERIC ? 2 : 4) k_fwd(const
           rk[q] = rr_[k]; vk[q] = vv_[k];
         }
 #pragma unroll
-        for (int q = 0; q < R; ++q) out[q] = rk[q] + sv * vk[q];
+        for (int q = 0; q < R; ++q) {
+          out[q] = rk[q] + sv * vk[q];
+          rr_[k0 + q * step] = out[q];
+        }
       } else {  // MODE_RES: apply the pending update to y, transform y, clear it
 #pragma unroll
         for (int q = 0; q < R; ++q) {
           const int k = k0 + q * step;
-          const float2 s1 = rr_[k] + sv * vv_[k];
-          out[q] = yy_[k] + yp * pp_[k] + ys * s1;
+          out[q] = yy_[k] + yp * pp_[k] + ys * rr_[k];
           yy_[k] = make_float2(0.f, 0.f);
         }
       }
@@ -687,9 +690,7 @@ __global__ void __launch_bounds__(256, 4) k_inv(const __grid_constant__ SolveArg
     const float2* __restrict__ z = A.B.w + soff;
     const float2* __restrict__ rh = A.B.rh + soff;
     const float2* __restrict__ r = A.B.r + soff;
-    const float2* __restrict__ v = A.B.v + soff;
     float2* __restrict__ out = (half == 0 ? A.B.v : A.B.t) + soff;
-    const float2 sv = f2(S.c_sv);
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     const float2 zero = make_float2(0.f, 0.f);
     const int jc = own ? j : 0;
@@ -731,8 +732,7 @@ __global__ void __launch_bounds__(256, 4) k_inv(const __grid_constant__ SolveArg
           dot_acc(acc[0], acc[1], hi2(rk), av1);
         } else {
           const float4 rr = *reinterpret_cast<const float4*>(r + idx);
-          const float4 vv = *reinterpret_cast<const float4*>(v + idx);
-          const float2 s0 = lo2(rr) + sv * lo2(vv), s1 = hi2(rr) + sv * hi2(vv);
+          const float2 s0 = lo2(rr), s1 = hi2(rr);     // s, left by the fwd pass
           dot_acc(acc[0], acc[1], av0, s0);            // <t, s>
           dot_acc(acc[0], acc[1], av1, s1);
           acc[2] += (double)av0.x * av0.x + (double)av0.y * av0.y + (double)av1.x * av1.x + (double)av1.y * av1.y;
@@ -762,21 +762,24 @@ __global__ void __launch_bounds__(256, 4) k_inv(const __grid_constant__ SolveArg
 // entry; W/2 consumer threads (two columns each) compute row i from the
 // buffers of rows i-1, i, i+1 and release the buffer of row i-1 on an `empty`
 // mbarrier.  Every row buffer holds z (with two halo columns each side) and
-// a (four each side), and for the band's own rows b, t, rhat and, in the
-// second half, r and v: a row step moves about 22 B per column, and D-3 row
-// steps are in flight per CTA while the consumers compute.  Nothing but the
-// copies themselves touches HBM on the read side, so the loads overlap the
-// stencil and FP64 dot products completely.
+// a (four each side), and for the band's own rows rhat and, in the second
+// half, s: a row step moves 20 to 28 B per column, and D-3 row steps are in
+// flight per CTA while the consumers compute.  Nothing but the copies
+// themselves touches HBM on the read side, so the loads overlap the stencil
+// and FP64 dot products completely.
 // ---------------------------------------------------------------------------
-// One row of the ring.  The first half (H = 0) needs no r and v, so its rows
-// are two fifths smaller and the same ring bytes hold more of them.
+// One row of the ring.  The second half reads s from r, where its forward pass
+// left it: r and v and their sum cost 8 B per node more here and a wider row
+// than the 8 B that the forward pass now writes (one launch over the 22 systems
+// of the 1024 x 768 record, second half: 182 -> 145 us here, 125 -> 135 us
+// there).  The first half (H = 0) needs no s, so its rows are a quarter smaller
+// and the same ring bytes hold more of them.
 template <int W, int H>
 struct StnLayout {
   static constexpr int OZ = 0;                    // float2 z[W + 4], column c0 - 2 + e
   static constexpr int ORH = OZ + (W + 4) * 8;    // float2 rhat[W]
-  static constexpr int OR = ORH + W * 8;          // float2 r[W] (second half)
-  static constexpr int OV = OR + (H ? W * 8 : 0);   // float2 v[W] (second half)
-  static constexpr int OA = OV + (H ? W * 8 : 0);   // float a[W + 8], column c0 - 4 + e
+  static constexpr int OR = ORH + W * 8;          // float2 s[W] (second half; kept in r)
+  static constexpr int OA = OR + (H ? W * 8 : 0);   // float a[W + 8], column c0 - 4 + e
   static constexpr int SLOT = OA + (W + 8) * 4;
   static_assert(ORH % 16 == 0 && OA % 16 == 0 && SLOT % 16 == 0, "alignment");
 };
@@ -922,7 +925,6 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
       const float2* zsrc = A.B.w + soff;
       const float2* rhsrc = A.B.rh + soff;
       const float2* rsrc = A.B.r + soff;
-      const float2* vsrc = A.B.v + soff;
       const int zlo = max(c0 - 2, 0), zhi = min(c0 + W + 2, nx);
       const int alo = max(c0 - 4, 0), ahi = min(c0 + W + 4, nx);
       const int phi = min(c0 + W, nx);
@@ -937,7 +939,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
         const bool own = row >= z0 && row < z1;
         uint32_t bytes = 0;
         if (in) bytes += (zhi - zlo) * 8 + (ahi - alo) * 4;
-        if (own) bytes += (phi - c0) * 8 + (half ? 2 * (phi - c0) * 8 : 0);
+        if (own) bytes += (phi - c0) * 8 + (half ? (phi - c0) * 8 : 0);
         mbar_arrive_expect_tx(&full[e], bytes);
         if (in) {
           const long long ro = (long long)row * nx;
@@ -946,10 +948,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
           if (own) {
             const uint32_t cb = (phi - c0) * 8;
             bulk_load(buf + Ly::ORH, rhsrc + ro + c0, cb, &full[e]);
-            if (half) {
-              bulk_load(buf + Ly::OR, rsrc + ro + c0, cb, &full[e]);
-              bulk_load(buf + Ly::OV, vsrc + ro + c0, cb, &full[e]);
-            }
+            if (half) bulk_load(buf + Ly::OR, rsrc + ro + c0, cb, &full[e]);
           }
         }
       }
@@ -999,7 +998,6 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
       }
       named_sync(1, NC);
     }
-    const float2 sv = f2(S.c_sv);
     // Inner products: float partial sums over NSR_STN_FLUSH rows (2 NSR_STN_FLUSH
     // products per thread), accumulated in FP64.
     float accf[NSR_NPART];
@@ -1082,8 +1080,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
             dot_acc_f(accf[0], accf[1], hi2(rk), av1);
           } else {
             const float4 rr = *reinterpret_cast<const float4*>(bC + Ly::OR + 16 * tid);
-            const float4 vv = *reinterpret_cast<const float4*>(bC + Ly::OV + 16 * tid);
-            const float2 s0 = lo2(rr) + sv * lo2(vv), s1 = hi2(rr) + sv * hi2(vv);
+            const float2 s0 = lo2(rr), s1 = hi2(rr);
             dot_acc_f(accf[0], accf[1], av0, s0);            // <t, s>
             dot_acc_f(accf[0], accf[1], av1, s1);
             accf[2] = fmaf(av0.x, av0.x, fmaf(av0.y, av0.y, fmaf(av1.x, av1.x, fmaf(av1.y, av1.y, accf[2]))));
@@ -1110,8 +1107,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
             dot_acc_f(accf[0], accf[1], rk, av);       // <rhat, v>
           } else {
             const float2 rr = *reinterpret_cast<const float2*>(bC + Ly::OR + 8 * tid);
-            const float2 vv = *reinterpret_cast<const float2*>(bC + Ly::OV + 8 * tid);
-            const float2 s0 = rr + sv * vv;
+            const float2 s0 = rr;
             dot_acc_f(accf[0], accf[1], av, s0);       // <t, s>
             accf[2] = fmaf(av.x, av.x, fmaf(av.y, av.y, accf[2]));
             accf[3] = fmaf(s0.x, s0.x, fmaf(s0.y, s0.y, accf[3]));
@@ -1213,9 +1209,7 @@ __global__ void __launch_bounds__(256, 4) k_inv1(const __grid_constant__ SolveAr
     const float2* __restrict__ z = A.B.w + soff;
     const float2* __restrict__ rh = A.B.rh + soff;
     const float2* __restrict__ r = A.B.r + soff;
-    const float2* __restrict__ v = A.B.v + soff;
     float2* __restrict__ out = (half == 0 ? A.B.v : A.B.t) + soff;
-    const float2 sv = f2(S.c_sv);
     const float2 zero = make_float2(0.f, 0.f);
     const bool has_e = j + 1 < nx, has_w = j > 0;
     long long idx = (long long)z0 * nx + j;
@@ -1238,7 +1232,7 @@ __global__ void __launch_bounds__(256, 4) k_inv1(const __grid_constant__ SolveAr
       if (half == 0) {
         dot_acc(acc[0], acc[1], rk, av);       // <rhat, v>
       } else {
-        const float2 s1 = r[idx] + sv * v[idx];
+        const float2 s1 = r[idx];              // s, left by the fwd pass
         dot_acc(acc[0], acc[1], av, s1);       // <t, s>
         acc[2] += (double)av.x * av.x + (double)av.y * av.y;
         acc[3] += (double)s1.x * s1.x + (double)s1.y * s1.y;
