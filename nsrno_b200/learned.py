@@ -33,7 +33,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .solver import Geometry, Medium, _ptr, _require_cuda, _stream, apply, plane_wave_rhs, solve_batched
+from .solver import Geometry, Medium, _float64_vector, _ptr, _require_cuda, _stream, apply, plane_wave_rhs, solve_batched
 
 N_PARAMS = _lib.LEARNED_PARAMS
 SHAPES = (("spectral", (2, 4)), ("log_shift", ()), ("context.0.weight", (16, 5, 3, 3)), ("context.0.bias", (16,)),
@@ -157,7 +157,7 @@ def learned_precondition(medium: Medium, setup: LearnedSetup | None, x: torch.Te
         raise ValueError("x must be complex64 [S, nz, nx]")
     x = x.contiguous()
     S = x.shape[0]
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=x.device).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, x.device)
     lib = _lib.load()
     nbytes = lib.nsr_precondition_workspace_size(ctypes.byref(medium._grid), S)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)

@@ -27,7 +27,21 @@ def _require_cuda(t: torch.Tensor, name: str):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle of torch.cuda.current_stream(), without building its Python object
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+def _float64_vector(v, device):
+    """``v`` as a contiguous float64 vector on ``device`` (itself when it is one).
+
+    A 256 x 256 apply is bound by this host path: its kernel takes 4.8 us, the
+    call 14.5 us with the conversions below and a stream object on every call
+    and 8.5 us without.
+    """
+    if (type(v) is torch.Tensor and v.dtype is torch.float64 and v.dim() == 1 and v.device == device
+            and v.is_contiguous()):
+        return v
+    return torch.as_tensor(v, dtype=torch.float64, device=device).reshape(-1).contiguous()
 
 
 def _ptr(t):
@@ -170,7 +184,7 @@ def solve_batched(medium: Medium, freqs, angles=None, *, rhs=None, x0=None, tole
     lib = _lib.load()
     g = medium.geometry
     dev = medium.device
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, dev)
     S = int(freqs.numel())
     if angles is None and rhs is None:
         raise ValueError("either angles (plane-wave sources) or rhs must be given")
@@ -303,7 +317,7 @@ def gmres_batched(medium: Medium, freqs, angles=None, *, rhs=None, x0=None, tole
     lib = _lib.load()
     g = medium.geometry
     dev = medium.device
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, dev)
     S = int(freqs.numel())
     if angles is None and rhs is None:
         raise ValueError("either angles (plane-wave sources) or rhs must be given")
@@ -350,15 +364,16 @@ def apply(medium: Medium, x: torch.Tensor, freqs, adjoint=False):
     """``A x`` (or ``A^H x``) of the h^2-scaled operator for fields x [S, nz, nx]."""
     g = medium.geometry
     _require_cuda(x, "x")
-    if x.dtype not in (torch.complex64, torch.complex128) or x.dim() != 3 or tuple(x.shape[1:]) != (g.nz, g.nx):
+    dtype, shape = x.dtype, x.shape
+    if dtype not in (torch.complex64, torch.complex128) or len(shape) != 3 or shape[1:] != (g.nz, g.nx):
         raise ValueError("x must be complex64/complex128 [S, nz, nx]")
     x = x.contiguous()
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=x.device).reshape(-1).contiguous()
-    if freqs.numel() != x.shape[0]:
+    freqs = _float64_vector(freqs, x.device)
+    if freqs.numel() != shape[0]:
         raise ValueError("one frequency per field")
     y = torch.empty_like(x)
-    _lib.check(_lib.load().nsr_apply(ctypes.byref(medium._grid), _ptr(medium.material), _ptr(freqs), x.shape[0],
-                                     int(bool(adjoint)), 0 if x.dtype == torch.complex64 else 1,
+    _lib.check(_lib.load().nsr_apply(ctypes.byref(medium._grid), _ptr(medium.material), _ptr(freqs), shape[0],
+                                     int(bool(adjoint)), 0 if dtype == torch.complex64 else 1,
                                      _ptr(x), _ptr(y), _stream()))
     return y
 
@@ -371,7 +386,7 @@ def precondition(medium: Medium, x: torch.Tensor, freqs, shift=DEFAULT_SHIFT, ad
         raise ValueError("x must be complex64 [S, nz, nx]")
     x = x.contiguous()
     S = x.shape[0]
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=x.device).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, x.device)
     lib = _lib.load()
     nbytes = lib.nsr_precondition_workspace_size(ctypes.byref(medium._grid), S)
     if nbytes == 0:
@@ -387,7 +402,7 @@ def plane_wave_rhs(medium: Medium, freqs, angles):
     """SI right-hand sides ``-line/h^2`` on the array row, complex128 [S, nz, nx]."""
     g = medium.geometry
     dev = medium.device
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, dev)
     angles = torch.as_tensor(angles, dtype=torch.float64, device=dev).reshape(-1).contiguous()
     b = torch.empty((freqs.numel(), g.nz, g.nx), dtype=torch.complex128, device=dev)
     _lib.check(_lib.load().nsr_plane_wave_rhs(ctypes.byref(medium._grid), _ptr(freqs), _ptr(angles),
@@ -406,7 +421,7 @@ def grad_accum(medium: Medium, freqs, u: torch.Tensor, lam: torch.Tensor, g_logc
     dtype = torch.complex128 if torch.complex128 in (u.dtype, lam.dtype) else torch.complex64
     u = u.to(dtype).contiguous()
     lam = lam.to(dtype).contiguous()
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, dev)
     if g_logc is None:
         g_logc = torch.zeros((g.nz, g.nx), dtype=torch.float64, device=dev)
     if g_logrho is None:
@@ -481,7 +496,7 @@ def true_residual(medium: Medium, x: torch.Tensor, freqs, angles=None, rhs=None,
     dev = x.device
     x = x.to(torch.complex128).contiguous()
     S = x.shape[0]
-    freqs = torch.as_tensor(freqs, dtype=torch.float64, device=dev).reshape(-1).contiguous()
+    freqs = _float64_vector(freqs, dev)
     if rhs is None and angles is None:
         raise ValueError("either angles or rhs must be given")
     ang = None if angles is None else torch.as_tensor(angles, dtype=torch.float64, device=dev).reshape(-1).contiguous()
