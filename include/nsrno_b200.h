@@ -75,7 +75,7 @@ typedef struct NsrTiles {
   int32_t stencil_depth;     /* row buffers of the second half's stencil ring:
                                 4 (default), 5, 6 (width 512: 4; one column per
                                 thread: 4); the first half's smaller rows fill
-                                the same bytes (7, 8 or 10 of them)            */
+                                the same bytes (5, 6 or 8 of them)             */
   int32_t stencil_rows;      /* rows per stencil work item (band): 4..64       */
   int32_t stencil_ctas;      /* resident stencil CTAs per SM (0: occupancy)    */
   int32_t cols_width;        /* columns per column-FFT CTA: 8 or 16            */
@@ -342,6 +342,8 @@ typedef struct NsrDenseGrid {
  * svx, gvx, lx = mx/(D-arx), rx = 1 + (1-mx)/(D-arx), then along z
  * (c128 [H] each) svz, gvz, lz, rz.  Built by nsrno_b200.dense. */
 size_t nsr_dense_coef_bytes(const NsrDenseGrid* grid);
+/* The fluxes stay on the chip, so nsr_dense_apply needs no more than a token
+ * workspace (256 bytes); 0 for a grid it does not take. */
 size_t nsr_dense_workspace_size(const NsrDenseGrid* grid, int32_t n_fields, int32_t precision);
 
 /* y = A x (adjoint 0) or A^H x (adjoint 1) for n_fields fields [n][H][W]

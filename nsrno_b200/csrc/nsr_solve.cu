@@ -16,8 +16,10 @@
 //   * The update of x is deferred: y accumulates alpha p + omega s and
 //     x += M^-1 y is applied at every true-residual replacement, where
 //     r = b - A x is recomputed in FP64 from an FP64 x.
-//   * The host captures `graph_iterations` iterations in a CUDA graph and
-//     relaunches it, polling a completion counter.
+//   * The first round of `graph_iterations` iterations is launched directly;
+//     the others are the body of a WHILE node of a CUDA graph that the host
+//     builds meanwhile (the _sync variant relaunches a captured round and polls
+//     a completion counter).
 // Algorithmic reference: bicgstab, nsrno/dense_wave.py:118-148 (right
 // preconditioned, shared-angle inner products, true residual every 40
 // iterations, breakdown/divergence reasons) and the fixed preconditioner of
@@ -1427,11 +1429,11 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     c->cols_staged = t->cols_staged != 0;
     c->rows_staged = t->rows_staged != 0;
   }
-  // Default ring depth 5 (256 columns, two per thread): three CTAs per SM, which
-  // leaves shared memory for a row-pass CTA of the other slot group.  22 learned
-  // 768 x 1024 systems: 47.6 us per system and iteration, 51.0 at depth 4 (four
-  // CTAs fill the shared memory), 52.1 at depth 6.
-  if (c->sd == 0) c->sd = c->sw == 256 && c->scpt == 2 ? 5 : 4;
+  // Default ring depth 4, the one that every width takes.  22 learned 768 x 1024
+  // systems: 46.8 us per system and iteration, 46.6 at depth 5, 50.4 at depth 6
+  // (fewer CTAs per SM and no shared memory left for a row-pass CTA of the other
+  // slot group).
+  if (c->sd == 0) c->sd = 4;
   if (!stn_kernel(c->sw, c->sd, c->scpt, false, 1)) return NSR_ERR_ARGUMENT;
   if (c->sr != 0 && (c->sr < NSR_STN_MIN_ROWS || c->sr > 64)) return NSR_ERR_ARGUMENT;
   if (c->sctas < 0 || c->sctas > 8) return NSR_ERR_ARGUMENT;
