@@ -249,10 +249,12 @@ inline int res_ctas(const NsrGrid* g, int ns) {
 
 // Tiles blockIdx.x, blockIdx.x + gridDim.x, ... : `P(id)` is x at node id,
 // `b_at(idx, i, j)` the h^2-scaled right-hand side, `out(idx, x, b, r)` takes
-// each node's x, b and r = b - A x.
-template <bool ADJ, typename XF, typename BF, typename OUT>
+// each node's x, b and r = b - A x, and `end(tile)` closes a tile.  Sums are
+// published by tile: how many CTAs a launch spreads the tiles over follows from
+// the slots beside this one, and must not regroup them.
+template <bool ADJ, typename XF, typename BF, typename OUT, typename END>
 __device__ __forceinline__ void residual_tiles(const Geo& g, const MatPlanes& mat, const SysScalars& sc, XF P,
-                                               BF b_at, OUT out) {
+                                               BF b_at, OUT out, END end) {
   __shared__ RowFactors<double> rowf[NSR_RES_TZ];
   const int nx = g.nx;
   const int nbx = (nx + NSR_RES_TX - 1) / NSR_RES_TX;
@@ -308,6 +310,7 @@ __device__ __forceinline__ void residual_tiles(const Geo& g, const MatPlanes& ma
       an = ac;
       ac = as;
     }
+    end(tile);
   }
 }
 

@@ -460,6 +460,8 @@ __global__ void __launch_bounds__(NSR_RES_TX) gk_res(const __grid_constant__ GAr
   const double st = sin(S.angle);
   float2* r = A.r + slot * n;
   double rr = 0.0, bb = 0.0;
+  double* part = g_part(A, slot);
+  const int nb = res_tiles(g.nz, g.nx);
   residual_tiles<ADJ>(
       g, A.mat, sc,
       [&](long long id) -> double2 {
@@ -472,15 +474,16 @@ __global__ void __launch_bounds__(NSR_RES_TX) gk_res(const __grid_constant__ GAr
         r[idx] = to_f(res);
         rr += res.x * res.x + res.y * res.y;
         bb += b.x * b.x + b.y * b.y;
+      },
+      [&](int tile) {
+        rr = gs_block_sum(rr);
+        bb = gs_block_sum(bb);
+        if (threadIdx.x == 0) {
+          part[tile] = rr;
+          part[nb + tile] = bb;
+        }
+        rr = bb = 0.0;
       });
-  double* part = g_part(A, slot);
-  const int nb = gridDim.x;
-  rr = gs_block_sum(rr);
-  bb = gs_block_sum(bb);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = rr;
-    part[nb + blockIdx.x] = bb;
-  }
   if (gs_arrive(part, nb, 2, &A.arrive[slot], tot) && threadIdx.x == 0) {
     rr = tot[0];
     bb = tot[1];
@@ -592,7 +595,7 @@ static GLayout g_layout(const NsrGrid* g, int n_slots, int m) {
   L.nb_st = bx * ((g->nz + L.tz - 1) / L.tz);
   L.nb_gs = (int)((n + L.tile - 1) / L.tile);
   L.nb_max = L.nb_st > L.nb_gs ? L.nb_st : L.nb_gs;
-  if (res_ctas(g, 1) > L.nb_max) L.nb_max = res_ctas(g, 1);
+  if (res_tiles(g->nz, g->nx) > L.nb_max) L.nb_max = res_tiles(g->nz, g->nx);
   size_t off = 0;
   L.tables = off; off += nsr_align(nsr_prec_table_bytes(g));
   L.slots = off; off += nsr_align(sizeof(GSlot) * n_slots);

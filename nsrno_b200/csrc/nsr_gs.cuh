@@ -87,15 +87,15 @@ __device__ __forceinline__ double gs_block_sum(double v) {
   return t;
 }
 
-// Counts this block in; in the last of `nb` blocks returns true with the sums
-// of the `nv` partial columns (in block order within each lane, then over the
-// lanes: the same on every run) in tot.
+// Counts this block in; in the last block of the launch's row returns true with
+// the sums of the `nv` columns of `nb` partials (in order within each lane, then
+// over the lanes: the same on every run) in tot.
 __device__ __forceinline__ bool gs_arrive(double* part, int nb, int nv, int* arrive, double* tot) {
   __shared__ int last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(arrive, 1) == nb - 1;
+    last = atomicAdd(arrive, 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return false;

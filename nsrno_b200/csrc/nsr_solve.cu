@@ -622,16 +622,18 @@ __device__ __forceinline__ void sum_partials(const double* part, int count, int 
   sync();
 }
 
-__device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotState& S, int slot, int mode,
-                                                    double* acc) {
-  __shared__ double red[NSR_NPART];
+// Partials of a slot; thread 0 of a block writes its rows.
+__device__ __forceinline__ double* slot_partials(const SolveArgs& A, int slot) {
+  return A.B.partials + (long long)slot * A.nb_inv * NSR_NPART;
+}
+
+// Counts the block in; the slot's last one sums the `count` rows of partials and
+// runs the recurrence.
+__device__ __forceinline__ void arrive_and_finalize(const SolveArgs& A, SlotState& S, int slot, int mode, int count) {
   __shared__ double tot[NSR_NPART];
   __shared__ double run[256];   // the blocks have 256 threads
   __shared__ int am_last, finished;
-  block_sum<NSR_NPART>(acc, red);
-  double* part = A.B.partials + (long long)slot * A.nb_inv * NSR_NPART;
   if (threadIdx.x == 0) {
-    for (int q = 0; q < NSR_NPART; ++q) part[blockIdx.x * NSR_NPART + q] = red[q];
     __threadfence();
     const int prev = atomicAdd(&A.B.arrive[slot], 1);
     am_last = (prev == (int)gridDim.x - 1);
@@ -639,7 +641,7 @@ __device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotStat
   __syncthreads();
   if (!am_last) return;
   __threadfence();
-  sum_partials(part, (int)gridDim.x, threadIdx.x, blockDim.x, run, tot, [] { __syncthreads(); });
+  sum_partials(slot_partials(A, slot), count, threadIdx.x, blockDim.x, run, tot, [] { __syncthreads(); });
   if (threadIdx.x == 0) {
     A.B.arrive[slot] = 0;
     finalize(A, S, mode, tot);
@@ -648,6 +650,18 @@ __device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotStat
   }
   __syncthreads();
   if (finished) finish_block(A, S, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+}
+
+// One row of partials per CTA of the launch.
+__device__ __forceinline__ void reduce_and_finalize(const SolveArgs& A, SlotState& S, int slot, int mode,
+                                                    double* acc) {
+  __shared__ double red[NSR_NPART];
+  block_sum<NSR_NPART>(acc, red);
+  if (threadIdx.x == 0) {
+    double* part = slot_partials(A, slot) + blockIdx.x * NSR_NPART;
+    for (int q = 0; q < NSR_NPART; ++q) part[q] = red[q];
+  }
+  arrive_and_finalize(A, S, slot, mode, (int)gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1265,10 +1279,10 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(const __grid_constant__ Solv
   if (!(mode == MODE_RES || mode == MODE_INIT || mode == MODE_EMIT)) return;
   const Geo& g = A.g;
   const long long n = (long long)g.nz * g.nx;
-  double acc[NSR_NPART];
-#pragma unroll
-  for (int q = 0; q < NSR_NPART; ++q) acc[q] = 0.0;
   if (mode != MODE_EMIT) {
+    __shared__ double red[3];
+    double* part = slot_partials(A, slot);
+    double acc[3] = {0.0, 0.0, 0.0};
     const bool init = mode == MODE_INIT;
     const SysScalars sc = S.sc;
     const float2* zw = A.B.w + slot * n;   // z = M^-1 y after the rinv pass
@@ -1298,9 +1312,15 @@ __global__ void __launch_bounds__(NSR_RES_TX) k_res(const __grid_constant__ Solv
             acc[0] += (double)rf.x * rf.x + (double)rf.y * rf.y;
             dot_acc(acc[1], acc[2], rh[idx], rf);
           }
+        },
+        [&](int tile) {
+          block_sum<3>(acc, red);
+          if (threadIdx.x == 0)
+            for (int q = 0; q < NSR_NPART; ++q) part[(long long)tile * NSR_NPART + q] = q < 3 ? red[q] : 0.0;
+          acc[0] = acc[1] = acc[2] = 0.0;
         });
   }
-  reduce_and_finalize(A, S, slot, mode, acc);
+  arrive_and_finalize(A, S, slot, mode, mode == MODE_EMIT ? 0 : res_tiles(g.nz, g.nx));
 }
 
 
@@ -1462,7 +1482,7 @@ struct Layout {
 static Layout layout(const NsrGrid* g, int n_slots) {
   Layout L;
   const size_t n = (size_t)g->nz * g->nx;
-  const int nb_res = res_ctas(g, 1);
+  const int nb_res = res_tiles(g->nz, g->nx);
   int nb_st = stencil_ctas(g);
   if (stn_ok(g) && stn_items_max(g) > nb_st) nb_st = stn_items_max(g);
   L.nb_inv = nb_res > nb_st ? nb_res : nb_st;
