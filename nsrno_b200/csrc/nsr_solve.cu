@@ -807,20 +807,11 @@ struct StnLayout {
 // slot i % ns: the slots run fastest, so the CTAs in flight at any time work
 // on the same few bands of every slot, and the medium's coefficient rows
 // (read by every slot) come from L2 after the first slot's copy.
+#define NSR_STN_UNITS 4   // most units of a band
 struct StnItems {
   int tz, nbands, nstrips, per_slot, n_items;
+  int unit, n_units;   // rows of one partial sum (tz is at most NSR_STN_UNITS of them), partials per slot
 };
-
-template <int W>
-__host__ __device__ inline StnItems stn_items(int nz, int nx, int tz, int ns) {
-  StnItems it;
-  it.tz = tz;
-  it.nbands = (nz + tz - 1) / tz;
-  it.nstrips = (nx + W - 1) / W;
-  it.per_slot = it.nbands * it.nstrips;
-  it.n_items = ns * it.per_slot;
-  return it;
-}
 
 // Resident CTAs per SM that the shared-memory ring of a k_stn shape allows
 // (at most 4): its register budget follows from it.
@@ -903,7 +894,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
   __shared__ __align__(8) uint64_t full[D], empty[D];
   __shared__ int abort_word;
   volatile int& abort_flag = abort_word;
-  __shared__ double wsum[NC / 32][NSR_NPART];
+  __shared__ double wsum[NSR_STN_UNITS][NC / 32][NSR_NPART];
   __shared__ double tot[NSR_NPART];
   // Each consumer's FP64 accumulators live in shared memory (column tid; reused
   // as scratch of the slot's last sum): in
@@ -1053,6 +1044,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     AT bNext = bt(bpl, z0), tNext = bt(tpl, z0);
     // Interior test (no PML stretch) per column, once per item; per row below.
     const bool cols_in = j > lo && j + CPT - 1 < hi_x;
+    int unit = 0, unit_end = min(it.unit, nrows);
     for (int k = 0; k < nrows; ++k) {
       const int i = z0 + k;
       const bool inside = i > lo && i < hi_z && cols_in;
@@ -1133,12 +1125,22 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
         }
       }
       zN = zC; zC = zS; aN = aC; aC = aS;
-      if ((k + 1) % FLUSH == 0 || k + 1 == nrows) {
+      if ((k + 1) % FLUSH == 0 || k + 1 == unit_end) {
 #pragma unroll
         for (int qq = 0; qq < NSR_NPART; ++qq) {
           if (qq < NP) accs[qq][tid] += (double)accf[qq];
           accf[qq] = 0.0f;
         }
+      }
+      if (k + 1 == unit_end) {
+#pragma unroll
+        for (int qq = 0; qq < NP; ++qq) {
+          const double s = warp_sum(accs[qq][tid]);
+          if (lane == 0) wsum[unit][wid][qq] = s;
+          accs[qq][tid] = 0.0;
+        }
+        ++unit;
+        unit_end = min(unit_end + it.unit, nrows);
       }
       // The buffer of row i - 1 goes back to the producer one row after its
       // last use as centre.  Its values were loaded into registers during row
@@ -1159,28 +1161,26 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     }
     q = q0 + nrows + 2;
 
-    // Block sum of the partials (consumer threads only), then the arrival.
-#pragma unroll
-    for (int k = 0; k < NSR_NPART; ++k) {
-      const double s = k < NP ? warp_sum(accs[k][tid]) : 0.0;
-      if (lane == 0) wsum[wid][k] = s;
-    }
+    // Block sums of the band's units (one warp of the consumers), then the arrival.
     named_sync(1, NC);
-    double* part = A.B.partials + (long long)slot * A.nb_inv * NSR_NPART;
-    if (tid == 0) {
-      for (int k = 0; k < NSR_NPART; ++k) {
+    double* part = slot_partials(A, slot);
+    if (tid < 32) {
+      const int u = tid / NSR_NPART, k = tid % NSR_NPART;
+      static_assert(NSR_STN_UNITS * NSR_NPART == 32, "one lane per sum");
+      if (u < unit) {
         double s = 0.0;
-        for (int w2 = 0; w2 < NC / 32; ++w2) s += wsum[w2][k];
-        part[rem * NSR_NPART + k] = s;
+        if (k < NP)
+          for (int w2 = 0; w2 < NC / 32; ++w2) s += wsum[u][w2][k];
+        part[((long long)(z0 / it.unit + u) * it.nstrips + strip) * NSR_NPART + k] = s;
       }
       __threadfence();
-      const int prev = atomicAdd(&A.B.arrive[slot], 1);
-      am_last = (prev == it.per_slot - 1);
+      __syncwarp();
+      if (tid == 0) am_last = atomicAdd(&A.B.arrive[slot], 1) == it.per_slot - 1;
     }
     named_sync(1, NC);
     if (am_last) {
       __threadfence();
-      sum_partials(part, it.per_slot, tid, NC, &accs[0][0], tot, [] { named_sync(1, NC); });
+      sum_partials(part, it.n_units, tid, NC, &accs[0][0], tot, [] { named_sync(1, NC); });
       if (tid == 0) {
         A.B.arrive[slot] = 0;
         finalize(A, S, want, tot);   // ITER modes never finish a system: no finish_block here
@@ -1429,11 +1429,11 @@ static size_t stn_smem(int w, int d, int half) {
 
 // Launch shapes of one call: NsrTiles with zero fields replaced by defaults.
 struct TileChoice {
-  int sw, sd, sr, sctas, tc, rows, groups, scpt, cols_staged, rows_staged;
+  int sw, sd, sr, su, sctas, tc, rows, groups, scpt, cols_staged, rows_staged;
 };
 
 static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileChoice* c) {
-  c->sw = 256; c->sd = 0; c->sr = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
+  c->sw = 256; c->sd = 0; c->sr = 0; c->su = 0; c->sctas = 0; c->scpt = 2; c->cols_staged = 0; c->rows_staged = 0;
   c->groups = n_slots >= 8 ? 2 : 1;
   c->tc = nsr_cols_tc(g, n_slots);
   c->rows = nsr_rows_per_cta(g, n_slots);
@@ -1462,14 +1462,24 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     return NSR_ERR_ARGUMENT;
   if (c->groups < 1 || c->groups > NSR_MAX_GROUPS) return NSR_ERR_ARGUMENT;
   if (c->groups > n_slots) c->groups = n_slots;
+  c->su = c->sr;
   if (c->sr == 0) {
-    // Band height of the stencil: the tallest whose items give every SM about
-    // three CTAs.  Tall bands re-read the fewest halo rows, but a band is walked
-    // row by row, about 0.8 us each: three 256 x 256 systems in 64-row bands
-    // were 12 CTAs and 52 us a launch, in 4-row bands 192 CTAs.
+    // Band height of the stencil.  Its inner products are summed by units of rows
+    // whose height follows from the grid alone (the tallest power of two that
+    // gives one system 64 units), so that the slots and groups of a call never
+    // regroup them; a band is one, two or four units, the tallest whose items give
+    // every SM about three CTAs.  Tall bands re-read the fewest halo rows, but a
+    // band is walked row by row, about 0.8 us each.  Microseconds per iteration of
+    // 1 / 11 / 22 systems with bands of 4, 8, 16, 32 and 64 rows: 256 x 256
+    // 78 / 123 / 167, 82 / 123 / 161, 90 / 128 / 163, 105 / 140 / 176,
+    // 138 / 176 / 201 (units of 4); 768 x 1024 133 / 654 / 1245, 121 / 611 / 1143,
+    // 127 / 579 / 1093, 140 / 561 / 1056, 175 / 581 / 1042 (units of 32).
     const int strips = (g->nx + c->sw - 1) / c->sw, ns = (n_slots + c->groups - 1) / c->groups;
-    c->sr = 64;
-    while (c->sr > NSR_STN_MIN_ROWS && (long long)ns * ((g->nz + c->sr - 1) / c->sr) * strips < 3 * 148) c->sr /= 2;
+    auto items = [&](int rows) { return (long long)((g->nz + rows - 1) / rows) * strips; };
+    c->su = 64;
+    while (c->su > NSR_STN_MIN_ROWS && items(c->su) < 64) c->su /= 2;
+    c->sr = c->su;
+    while (c->sr < 64 && c->sr < NSR_STN_UNITS * c->su && ns * items(2 * c->sr) >= 3 * 148) c->sr *= 2;
   }
   return 0;
 }
@@ -1720,6 +1730,8 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
         si.nstrips = (grid->nx + T.sw - 1) / T.sw;
         si.per_slot = si.nbands * si.nstrips;
         si.n_items = ns * si.per_slot;
+        si.unit = T.su;
+        si.n_units = (grid->nz + T.su - 1) / T.su * si.nstrips;
         int hv = half, nsv = ns;
         const int gx = si.n_items < stn_per_sm[half] * n_sms ? si.n_items : stn_per_sm[half] * n_sms;
         void* args[] = {&Ag, &hv, &si, &nsv};

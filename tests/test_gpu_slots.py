@@ -43,3 +43,7 @@ def check_solve(record, **shape):
 def test_residual_sums_do_not_depend_on_the_slots(record):
     check_solve(record, stencil_rows=64)
 
+
+def test_solves_do_not_depend_on_the_slots(record):
+    check_solve(record)
+
