@@ -586,10 +586,15 @@ struct GLayout {
 static GLayout g_layout(const NsrGrid* g, int n_slots, int m) {
   GLayout L;
   const size_t n = (size_t)g->nz * g->nx;
-  // Tall tiles (8 rows, 2,048 nodes) amortise the reductions; a batch whose tall
-  // tiles are fewer than three CTAs per SM takes 2-row tiles of 512 nodes.
+  // Tall tiles (8 rows, 2,048 nodes) amortise the reductions; a grid of fewer than
+  // 64 of them takes 2-row tiles of 512 nodes.  Tiles group the partial sums, so
+  // the rule looks at the grid alone and not at the slots of a call.  Cycles of 8
+  // steps with 1 / 4 / 11 systems, us, tall against short: 768 x 1024
+  // 1003 / 2139 / 4564 and 1161 / 2495 / 5503, 243 x 729 849 / 1192 / 2294 and
+  // 856 / 1271 / 2487, 256 x 256 (32 tall tiles) 758 / 784 / 940 and
+  // 741 / 779 / 1016, 128 x 192 (16) 711 / 729 / 846 and 690 / 713 / 849.
   const int bx = (g->nx + NSR_GST_TX - 1) / NSR_GST_TX;
-  const bool tall = (long long)bx * ((g->nz + 7) / 8) * n_slots >= 3 * 148;
+  const bool tall = (long long)bx * ((g->nz + 7) / 8) >= 64;
   L.tz = tall ? 8 : 2;
   L.tile = L.tz * NSR_GST_TX;
   L.nb_st = bx * ((g->nz + L.tz - 1) / L.tz);

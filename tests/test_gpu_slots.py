@@ -47,3 +47,12 @@ def test_residual_sums_do_not_depend_on_the_slots(record):
 def test_solves_do_not_depend_on_the_slots(record):
     check_solve(record)
 
+
+def test_gmres_does_not_depend_on_the_slots(record):
+    from nsrno_b200 import gmres_batched
+    med, f, a = record
+    runs = {s: gmres_batched(med, f[:11], a[:11], tolerance=1e-30, restart=6, max_iterations=6, n_slots=s,
+                             return_fields=True) for s in (11, 3, 1)}
+    for s in (3, 1):
+        assert torch.equal(runs[s].residual, runs[11].residual)
+        assert torch.equal(runs[s].fields, runs[11].fields)
