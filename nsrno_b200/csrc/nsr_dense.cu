@@ -875,7 +875,7 @@ int nsr_dense_prec_setup(const NsrDenseGrid* grid, double k0dx2, double shift, i
   M->adjoint = adjoint;
   M->rows = nsr_rows_per_cta(&q, n_fields);
   M->tc = nsr_cols_tc(&q, n_fields);
-  M->gx = !nsr_specialised(grid->W);
+  M->gx = nsr_rows_generic(grid->W, M->w);
   M->gz = !nsr_specialised(grid->H);
   M->g_rows = dim3((grid->H + M->rows - 1) / M->rows, n_fields);
   M->g_cols = dim3((grid->W + M->tc - 1) / M->tc, n_fields);

@@ -25,4 +25,9 @@ int nsr_rows_per_cta(const NsrGrid* g, int ns);
 // (their butterflies hold up to 19 points in registers).
 inline int nsr_cols_threads(bool gen) { return gen ? 256 : 512; }
 
+// Whether a row pass between caller's fields and the work field `w` runs the
+// run-time stages: the specialised transforms read and write w in 16-byte pairs,
+// which a workspace that is only 8-byte aligned does not allow.
+inline bool nsr_rows_generic(int nx, const void* w) { return !nsr_specialised(nx) || ((uintptr_t)w & 15) != 0; }
+
 int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st);

@@ -534,7 +534,7 @@ extern "C" int nsr_learned_precondition(const NsrGrid* grid, const NsrLearned* l
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
   const float2* gains = (const float2*)learned->gains;
-  const bool gx = !nsr_specialised(grid->nx), gz = !nsr_specialised(grid->nz);
+  const bool gx = nsr_rows_generic(grid->nx, w), gz = !nsr_specialised(grid->nz);
   const auto fwd = gx ? k_lp_rows_fwd<true> : k_lp_rows_fwd<false>;
   const auto inv = gx ? k_lp_rows_inv<true> : k_lp_rows_inv<false>;
   fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows, gains, learned->gain_index, learned->n_gain, adjoint);
@@ -928,7 +928,7 @@ extern "C" int nsr_learned_spectral_backward(const NsrGrid* grid, const float* p
   const int rows = nsr_rows_per_cta(grid, n_systems);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   const dim3 gr((grid->nz + rows - 1) / rows, n_systems);
-  const auto fwd = nsr_specialised(grid->nx) ? k_lp_rows_fwd<false> : k_lp_rows_fwd<true>;
+  const auto fwd = nsr_rows_generic(grid->nx, xr) ? k_lp_rows_fwd<true> : k_lp_rows_fwd<false>;
   fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, xr, rows, nullptr, nullptr, 0, 0);
   fwd<<<gr, 256, row_smem, st>>>(g, t, (const float2*)y, yr, rows, nullptr, nullptr, 0, 0);
   const int tc = spec_tc(grid);

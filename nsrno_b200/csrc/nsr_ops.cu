@@ -353,7 +353,8 @@ extern "C" int nsr_precondition(const NsrGrid* grid, const double* freq_hz, int3
   const int rows = nsr_rows_per_cta(grid, n_systems);
   const size_t row_smem = sizeof(float2) * (size_t)rows * nsr_row_stride(grid->nx);
   dim3 gr((grid->nz + rows - 1) / rows, n_systems);
-  if (nsr_specialised(grid->nx)) k_prec_rows_fwd<false><<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
+  const bool gx = nsr_rows_generic(grid->nx, w);
+  if (!gx) k_prec_rows_fwd<false><<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
   else k_prec_rows_fwd<true><<<gr, 256, row_smem, st>>>(g, t, (const float2*)x, w, rows);
   const int tc = nsr_cols_tc(grid, n_systems);
   const bool gen = !nsr_specialised(grid->nz);
@@ -363,7 +364,7 @@ extern "C" int nsr_precondition(const NsrGrid* grid, const double* freq_hz, int3
                              : (gen ? k_prec_cols<8, true> : k_prec_cols<8, false>);
   cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
   cols<<<gc, nsr_cols_threads(gen), csm, st>>>(g, t, freq_hz, w, shift, adjoint);
-  if (nsr_specialised(grid->nx)) k_prec_rows_inv<false><<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
+  if (!gx) k_prec_rows_inv<false><<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
   else k_prec_rows_inv<true><<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows);
   return last_error();
 }
