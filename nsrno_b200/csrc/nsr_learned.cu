@@ -32,6 +32,7 @@
 //                                 nsrno/train_dense_wave.py:37,76)
 #include "nsr_internal.cuh"
 #include "nsr_device.cuh"
+#include "nsr_gain_check.cuh"
 
 #include <cuda_bf16.h>
 #include <stdlib.h>
@@ -392,62 +393,6 @@ extern "C" int nsr_learned_setup(const NsrGrid* grid, const float* c, const floa
                                  void* gains, void* stream) {
   return nsr_learned_setup_ex(grid, c, rho, alpha, freq_hz, n_freq, params, NSR_LEARNED_FP32, state, gains, stream);
 }
-
-// ---------------------------------------------------------------------------
-// Gain-index validation shared by every entry point that reads gains.
-// ---------------------------------------------------------------------------
-namespace {
-// The check in two parts: start() refuses what the host can see and copies the
-// indices to pinned memory behind the stream's earlier work, finish() waits for
-// that copy alone and looks at them.  What a caller launches in between runs
-// while the host waits (four 256 x 384 fields through nsr_learned_precondition:
-// 71 us a call with the stream drained first, 59 us this way).
-struct GainCheck {
-  const int32_t* host = nullptr;
-  int count = 0, n_gain = 0;
-  cudaEvent_t copied = nullptr;
-  ~GainCheck() { if (copied) cudaEventDestroy(copied); }
-
-  int start(const NsrLearned* L, int n_systems, cudaStream_t st) {
-    if (!L) return 0;
-    if (!L->params) return NSR_ERR_ARGUMENT;
-    if (!L->gains) return 0;
-    if (L->n_gain <= 0) return NSR_ERR_ARGUMENT;
-    if (!L->gain_index) return n_systems <= L->n_gain ? 0 : NSR_ERR_ARGUMENT;
-    if (n_systems <= 0) return 0;
-    // Pinned index buffer of this host thread, kept for its life; calls of one
-    // thread use it one after the other (finish() has read it before the next).
-    static thread_local int32_t* pinned = nullptr;
-    static thread_local int capacity = 0;
-    if (capacity < n_systems) {
-      if (pinned) cudaFreeHost(pinned);
-      pinned = nullptr;
-      const int want = n_systems < 1024 ? 1024 : n_systems;
-      const cudaError_t ce = cudaHostAlloc((void**)&pinned, sizeof(int32_t) * (size_t)want, cudaHostAllocDefault);
-      if (ce != cudaSuccess) { pinned = nullptr; capacity = 0; return (int)ce; }
-      capacity = want;
-    }
-    cudaError_t ce = cudaEventCreateWithFlags(&copied, cudaEventDisableTiming);
-    if (ce == cudaSuccess)
-      ce = cudaMemcpyAsync(pinned, L->gain_index, sizeof(int32_t) * (size_t)n_systems, cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaEventRecord(copied, st);
-    if (ce != cudaSuccess) return (int)ce;
-    host = pinned;
-    count = n_systems;
-    n_gain = L->n_gain;
-    return 0;
-  }
-
-  int finish() {
-    if (!host) return 0;
-    const cudaError_t ce = cudaEventSynchronize(copied);
-    if (ce != cudaSuccess) return (int)ce;
-    for (int s = 0; s < count; ++s)
-      if (host[s] < 0 || host[s] >= n_gain) return NSR_ERR_ARGUMENT;
-    return 0;
-  }
-};
-}  // namespace
 
 int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st) {
   GainCheck check;
