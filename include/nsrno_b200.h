@@ -110,7 +110,8 @@ typedef struct NsrLearned {
                                 multiplier only (no diagonal gains)            */
   const int32_t* gain_index; /* device int32 [n_systems]: gain pair of each
                                 system; NULL: system s uses pair s. Checked on
-                                the host (one small copy) before any launch     */
+                                the host (one small copy); a call that refuses
+                                one writes no result                           */
   int32_t n_gain;            /* gain pairs in `gains`                          */
   int32_t reserved;
 } NsrLearned;

@@ -403,7 +403,7 @@ int nsr_check_learned(const NsrLearned* L, int n_systems, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Learned apply: rows (pre gain) -> columns (learned multiplier) -> rows (post gain).
 // ---------------------------------------------------------------------------
-// Pair of system s.  The host checks the indices while these kernels run, so an
+// Pair of system s.  The host checks the indices while the first passes run, so an
 // index it is about to refuse is held inside the pairs here.
 __device__ __forceinline__ int lp_gidx(const int* gain_index, int s, int n_gain) {
   return gain_index ? min(max(gain_index[s], 0), n_gain - 1) : s;
@@ -490,10 +490,13 @@ extern "C" int nsr_learned_precondition(const NsrGrid* grid, const NsrLearned* l
                              : (gz ? k_lp_cols<8, true> : k_lp_cols<8, false>);
   cudaFuncSetAttribute((const void*)cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm);
   cols<<<gc, nsr_cols_threads(gz), csm, st>>>(g, t, freq_hz, w, learned->params, adjoint);
-  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, learned->n_gain, adjoint);
   err = last_error();
+  // The passes above write the workspace only.  The one that writes y follows the
+  // check (they are still running then), so a refused call leaves y alone.
   const int bad = check.finish();
-  return err ? err : bad;
+  if (err || bad) return err ? err : bad;
+  inv<<<gr, 256, row_smem, st>>>(g, t, w, (float2*)y, rows, gains, learned->gain_index, learned->n_gain, adjoint);
+  return last_error();
 }
 
 // ---------------------------------------------------------------------------

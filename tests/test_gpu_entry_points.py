@@ -63,3 +63,26 @@ def test_workspaces_aligned_to_eight_bytes(cuda, nx):
     for want, got in zip(results(0), results(8)):
         assert np.abs(want).max() > 0
         assert rel(got, want) < 6e-6
+
+
+@pytest.mark.parametrize("bad", [-1, 2, 1 << 30])
+def test_refused_gain_index_leaves_the_output_alone(cuda, bad):
+    from nsrno_b200 import _lib
+    from nsrno_b200.learned import LearnedPreconditioner
+    rec = small_record(nz=64, nx=96)
+    med = medium_of(rec, cuda)
+    setup = LearnedPreconditioner.load(device=cuda).setup(med, rec.frequencies)
+    lib = _lib.load()
+    S = 3
+    index = torch.tensor([0, 1, bad], dtype=torch.int32, device=cuda)
+    f = torch.as_tensor(rec.frequencies[[0, 1, 1]], device=cuda)
+    x = torch.randn((S, rec.nz, rec.nx), dtype=torch.complex64, device=cuda)
+    y = torch.full_like(x, 7.0)
+    size = lib.nsr_precondition_workspace_size(ctypes.byref(med._grid), S)
+    ws = torch.empty(size, dtype=torch.uint8, device=cuda)
+    struct = setup.struct(index)
+    code = lib.nsr_learned_precondition(ctypes.byref(med._grid), ctypes.byref(struct), ptr(f), S, 0, ptr(x), ptr(y),
+                                        ptr(ws), size, stream())
+    torch.cuda.synchronize()
+    assert code != 0
+    assert (y == 7.0).all()
