@@ -119,8 +119,19 @@ __device__ __forceinline__ void node_maps(const T* __restrict__ maps, int hw, in
 // combine to a pixel, so the grid fills the chip at every size (one thread per
 // pixel left 96 blocks with 192 serial logarithms each: 63 us at 768 x 1024).
 // Four nodes share a logarithm: the logs of c and rho add up in a product (four
-// floats stay in double range), log1p(alpha) in 1 + q = prod (1 + alpha) with q
-// kept apart from the 1.  Bound by the logarithms' FP64; 6 us.
+// positive floats stay in double range), log1p(alpha) in 1 + q = prod (1 + alpha)
+// with q kept apart from the 1.  A group with a value for which that differs from
+// the sum of its logarithms (two negative factors cancel, an infinite one meets
+// a zero q, 1 + q loses its digits near alpha = -1) takes them node by node.
+// Bound by the logarithms' FP64; 6 us.
+__device__ __noinline__ void lp_pool_nodes(const float* __restrict__ c, const float* __restrict__ rho,
+                                           const float* __restrict__ alpha, int nx, double* s) {
+  for (int dy = 0; dy < 4; ++dy) {
+    s[0] += log((double)c[(long long)dy * nx] / 1540.0);
+    s[1] += log((double)rho[(long long)dy * nx] / 1000.0);
+    s[2] += log1p((double)alpha[(long long)dy * nx]);
+  }
+}
 template <typename T>
 __global__ void __launch_bounds__(256) k_lp_pool(int nz, int nx, int h8, int w8, const float* __restrict__ c,
                                                  const float* __restrict__ rho, const float* __restrict__ alpha,
@@ -135,19 +146,30 @@ __global__ void __launch_bounds__(256) k_lp_pool(int nz, int nx, int h8, int w8,
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     double pc = 1.0, pr = 1.0, q = 0.0;
-    bool bad = false;
+    float least = INFINITY, least_a = INFINITY;   // a NaN passes by and comes back in the products
+    const long long k0 = (long long)(8 * py + 4 * h) * nx + xc;
 #pragma unroll
     for (int dy = 0; dy < 4; ++dy) {
-      const long long k = (long long)(8 * py + 4 * h + dy) * nx + xc;
-      const double a = alpha[k];
-      pc *= (double)c[k];
-      pr *= (double)rho[k];
+      const long long k = k0 + (long long)dy * nx;
+      const float cv = c[k], rv = rho[k], av = alpha[k];
+      const double a = av;
+      pc *= (double)cv;
+      pr *= (double)rv;
       q = q + a + q * a;
-      bad = bad || !(a >= -1.0);
+      least = fminf(least, fminf(cv, rv));
+      least_a = fminf(least_a, av);
     }
-    s0 += log(pc / c4);
-    s1 += log(pr / r4);
-    s2 += bad ? NAN : log1p(q);
+    if (least > 0.f && least_a >= -0.5f && pc < INFINITY && pr < INFINITY && q < INFINITY) {
+      s0 += log(pc / c4);
+      s1 += log(pr / r4);
+      s2 += log1p(q);
+    } else {
+      double s[3] = {s0, s1, s2};
+      lp_pool_nodes(c + k0, rho + k0, alpha + k0, nx, s);
+      s0 = s[0];
+      s1 = s[1];
+      s2 = s[2];
+    }
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) {

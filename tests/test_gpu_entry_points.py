@@ -86,3 +86,38 @@ def test_refused_gain_index_leaves_the_output_alone(cuda, bad):
     torch.cuda.synchronize()
     assert code != 0
     assert (y == 7.0).all()
+
+
+@pytest.mark.parametrize("c_bad,rho_bad,alpha_bad", [
+    (-1500.0, None, None), (None, -1000.0, None), (0.0, None, None), (None, np.inf, None), (None, None, np.inf),
+    (None, None, -1.0), (None, None, -1.0 + 2.0 ** -24), (None, None, -2.0)])
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+def test_context_of_values_outside_the_physical_range(cuda, c_bad, rho_bad, alpha_bad, count):
+    """The pooled context is the mean of the nodes' logarithms also where a
+    medium has values that no tissue has, one to four of them in a column:
+    negative ones give NaN, zeros and infinities what their logarithms give."""
+    from nsrno_b200 import _lib
+    from nsrno_b200.learned import LearnedPreconditioner
+    rec = small_record(nz=24, nx=40, n_pml=3)
+    med = medium_of(rec, cuda)
+    net = LearnedPreconditioner.load(device=cuda)
+    planes = [np.array(v, np.float32) for v in (rec.c, rec.rho, rec.alpha)]
+    for v, value in zip(planes, (c_bad, rho_bad, alpha_bad)):
+        if value is not None:
+            v[8:8 + count, 19] = value
+    lib = _lib.load()
+    f = torch.tensor([2.3e6], dtype=torch.float64, device=cuda)
+    state = torch.zeros(lib.nsr_learned_state_bytes(ctypes.byref(med._grid), 1), dtype=torch.uint8, device=cuda)
+    dev = [torch.as_tensor(v, device=cuda) for v in planes]
+    assert lib.nsr_learned_setup(ctypes.byref(med._grid), *[ptr(v) for v in dev], ptr(f), 1, ptr(net.params),
+                                 ptr(state), None, stream()) == 0
+    got = state[:4 * 3 * 15].view(torch.float32).reshape(3, 3, 5).cpu().numpy()
+    with np.errstate(all="ignore"):
+        c, rho, alpha = (v.astype(np.float64) for v in planes)
+        logs = np.stack((np.log(c / 1540) / 0.06, np.log(rho / 1000) / 0.08, np.log1p(alpha)))
+        want = logs.reshape(3, 3, 8, 5, 8).mean(axis=(2, 4))
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    ok = np.isfinite(want)
+    # rounding of the mean to float: 6e-8 of the largest term
+    assert np.abs(got[ok] - want[ok]).max() < 1e-6 * np.abs(want[ok]).max()
