@@ -70,10 +70,9 @@ struct GArgs {
   double2* hc;         // [n_slots][m+1]  coefficients of the first CGS pass
   double2* hc2;        // [n_slots][m+1]  and of the second
   double2* y;          // [n_slots][m]
-  float2* V;           // [n_slots][m+1][n]
+  float2* V;           // [n_slots][m+1][n]; plane m: learned multiplier of the slot's system (a cycle's basis ends at m - 1)
   float2* w;           // [n_slots][n]
   float2* W;           // [n_slots][n]   FFT work field
-  float2* sym;         // [n_slots][n]   learned multiplier of the slot's system (learned solves only)
   float2* r;           // [n_slots][n]
   double2* x;          // [n_slots][2][n]
   const double* freq;
@@ -91,6 +90,10 @@ __device__ __forceinline__ bool g_active(const GSlot& S, int j) {
 }
 
 __device__ __forceinline__ double cabs(double2 a) { return sqrt(a.x * a.x + a.y * a.y); }
+
+__device__ __forceinline__ float2* g_sym(const GArgs& A, int slot, long long n) {
+  return A.V + ((long long)slot * (A.m + 1) + A.m) * n;
+}
 
 __device__ __forceinline__ double* g_part(const GArgs& A, int slot) {
   return A.partials + (long long)slot * (2 * (A.m + 1) + 1) * A.nb_max;
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(GEN ? 256 : 512, 2) gk_cols(const __grid_const
   float2* w = A.W + slot * n;
   const int c0 = blockIdx.x * TC;
   if (LEARNED) {
-    const float2* __restrict__ symp = A.sym + slot * n;
+    const float2* __restrict__ symp = g_sym(A, slot, n);
     const int nx = A.g.nx, adjoint = A.adjoint;
     cols_pass_with<TC, GEN, false>(sm, A.g, A.tab, w, c0, [&](int c, int z) -> float2 {
       const float2 mul = symp[(long long)z * nx + c0 + c];
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(256) gk_sym(const __grid_constant__ GArgs A) {
   const long long n = (long long)g.nz * g.nx;
   const LearnedSpec L = load_learned_spec(A.lp);
   const float kh2 = (float)S.sc.kh2;
-  float2* __restrict__ sym = A.sym + blockIdx.y * n;
+  float2* __restrict__ sym = g_sym(A, blockIdx.y, n);
   for (int z = blockIdx.x; z < g.nz; z += gridDim.x)
     for (int x = threadIdx.x; x < g.nx; x += blockDim.x)
       sym[(long long)z * g.nx + x] = learned_plane_value(L, g, A.tab, kh2, z, x);
@@ -579,7 +582,7 @@ __global__ void gk_count(const __grid_constant__ GArgs A, int* remaining) {
 // Host side.
 // ---------------------------------------------------------------------------
 struct GLayout {
-  size_t tables, slots, arrive, count, partials, H, cs, sn, gv, hc, hc2, y, V, w, W, sym, r, x, total;
+  size_t tables, slots, arrive, count, partials, H, cs, sn, gv, hc, hc2, y, V, w, W, r, x, total;
   int tz, tile, nb_st, nb_gs, nb_max;   // stencil rows and Gram-Schmidt nodes of a CTA, CTAs per slot
 };
 
@@ -617,7 +620,6 @@ static GLayout g_layout(const NsrGrid* g, int n_slots, int m) {
   L.V = off; off += nsr_align(sizeof(float2) * n * (m + 1) * n_slots);
   L.w = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.W = off; off += nsr_align(sizeof(float2) * n * n_slots);
-  L.sym = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.r = off; off += nsr_align(sizeof(float2) * n * n_slots);
   L.x = off; off += nsr_align(sizeof(double2) * n * 2 * n_slots);
   L.total = off;
@@ -697,7 +699,6 @@ extern "C" int nsr_gmres_batched(const NsrGrid* grid, const void* material, cons
     A.V = (float2*)(ws + L.V);
     A.w = (float2*)(ws + L.w);
     A.W = (float2*)(ws + L.W);
-    A.sym = (float2*)(ws + L.sym);
     A.r = (float2*)(ws + L.r);
     A.x = (double2*)(ws + L.x);
     A.freq = freq_hz;
