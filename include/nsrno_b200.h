@@ -343,8 +343,9 @@ typedef struct NsrDenseGrid {
  * svx, gvx, lx = mx/(D-arx), rx = 1 + (1-mx)/(D-arx), then along z
  * (c128 [H] each) svz, gvz, lz, rz.  Built by nsrno_b200.dense. */
 size_t nsr_dense_coef_bytes(const NsrDenseGrid* grid);
-/* The fluxes stay on the chip, so nsr_dense_apply needs no more than a token
- * workspace (256 bytes); 0 for a grid it does not take. */
+/* Workspace of nsr_dense_apply in place (y = x): 256 bytes and one copy of the
+ * fields.  A call with separate buffers needs the 256 bytes only.  0 for a grid
+ * it does not take. */
 size_t nsr_dense_workspace_size(const NsrDenseGrid* grid, int32_t n_fields, int32_t precision);
 
 /* y = A x (adjoint 0) or A^H x (adjoint 1) for n_fields fields [n][H][W]

@@ -631,9 +631,14 @@ extern "C" size_t nsr_dense_coef_bytes(const NsrDenseGrid* g) {
   return sizeof(double) * dense_coef_doubles(g->H, g->W);
 }
 
+// The fluxes live in shared memory: separate buffers need no workspace to speak
+// of.  A call in place copies its fields there first, because tiles read the
+// halos of their neighbours' nodes.
+#define NSR_DENSE_WORKSPACE_MIN 256
 extern "C" size_t nsr_dense_workspace_size(const NsrDenseGrid* g, int32_t n_fields, int32_t precision) {
   if (!g || g->H <= 0 || g->W <= 0 || n_fields < 0 || (precision != 0 && precision != 1)) return 0;
-  return n_fields > 0 ? 256 : 0;   // the fluxes live in shared memory
+  if (n_fields == 0) return 0;
+  return NSR_DENSE_WORKSPACE_MIN + (size_t)g->H * g->W * n_fields * (precision ? 16 : 8);
 }
 
 DenseGeo nsr_dense_geo(const NsrDenseGrid* grid, double scal_re, double scal_im) {
@@ -662,7 +667,14 @@ extern "C" int nsr_dense_apply(const NsrDenseGrid* grid, const double* coef, dou
     return NSR_ERR_ARGUMENT;
   if (precision != 0 && precision != 1) return NSR_ERR_ARGUMENT;
   if (n_fields == 0) return 0;
-  if (!workspace || workspace_bytes < nsr_dense_workspace_size(grid, n_fields, precision)) return NSR_ERR_WORKSPACE;
+  const size_t full = nsr_dense_workspace_size(grid, n_fields, precision);
+  if (!workspace || workspace_bytes < (x == y ? full : NSR_DENSE_WORKSPACE_MIN)) return NSR_ERR_WORKSPACE;
+  if (x == y) {
+    const cudaError_t ce = cudaMemcpyAsync(workspace, x, full - NSR_DENSE_WORKSPACE_MIN, cudaMemcpyDeviceToDevice,
+                                           (cudaStream_t)stream);
+    if (ce != cudaSuccess) return (int)ce;
+    x = workspace;
+  }
   return nsr_dense_apply_geo(nsr_dense_geo(grid, scal_re, scal_im), coef, n_fields, adjoint, precision, x, y,
                              (cudaStream_t)stream);
 }

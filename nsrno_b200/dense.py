@@ -186,7 +186,7 @@ class DenseSystem:
         p = p.contiguous()
         prec = 1 if p.dtype == torch.complex128 else 0
         lib = _lib.load()
-        nbytes = lib.nsr_dense_workspace_size(ctypes.byref(g.struct), p.shape[0], prec)
+        nbytes = 256   # separate buffers: no copy of the fields
         ws = torch.empty(nbytes, dtype=torch.uint8, device=p.device)
         y = torch.empty_like(p)
         _lib.check(lib.nsr_dense_apply(ctypes.byref(g.struct), ctypes.c_void_p(self.coef.data_ptr()),

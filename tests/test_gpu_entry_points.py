@@ -121,3 +121,27 @@ def test_context_of_values_outside_the_physical_range(cuda, c_bad, rho_bad, alph
     ok = np.isfinite(want)
     # rounding of the mean to float: 6e-8 of the largest term
     assert np.abs(got[ok] - want[ok]).max() < 1e-6 * np.abs(want[ok]).max()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("h,w,pml,n", [(70, 300, 12, 2), (260, 300, 24, 40), (130, 150, 12, 19)])
+def test_dense_apply_in_place(cuda, h, w, pml, n, dtype):
+    """y = x is the same buffer: the result of separate buffers, bit for bit (row
+    walk and tiles)."""
+    from nsrno_b200 import _lib
+    from nsrno_b200.dense import DenseSystem
+    from test_gpu_tiles import dense_case
+    _, g, medium, alpha, rng = dense_case(h, w, pml)
+    s = DenseSystem(g, medium, alpha, 5.1e6, device=cuda)
+    p = torch.as_tensor(rng.standard_normal((n, g.H, g.W)) + 1j * rng.standard_normal((n, g.H, g.W)),
+                        device=cuda).to(dtype)
+    lib = _lib.load()
+    prec = int(dtype == torch.complex128)
+    size = lib.nsr_dense_workspace_size(ctypes.byref(g.struct), n, prec)
+    ws = torch.empty(size, dtype=torch.uint8, device=cuda)
+    for adj in (0, 1):
+        want = (s.adjoint if adj else s.apply)(p)
+        y = p.clone()
+        assert lib.nsr_dense_apply(ctypes.byref(g.struct), ptr(s.coef), s.scal.real, s.scal.imag, n, adj, prec,
+                                   ptr(y), ptr(y), ptr(ws), size, stream()) == 0
+        assert torch.equal(y, want)
