@@ -16,9 +16,9 @@
 //   * The update of x is deferred: y accumulates alpha p + omega s and
 //     x += M^-1 y is applied at every true-residual replacement, where
 //     r = b - A x is recomputed in FP64 from an FP64 x.
-//   * The first round of `graph_iterations` iterations is launched directly;
-//     the others are the body of a WHILE node of a CUDA graph that the host
-//     builds meanwhile (the _sync variant relaunches a captured round and polls
+//   * The first iterations are launched directly; rounds of `graph_iterations`
+//     others are the body of a WHILE node of a CUDA graph that the host builds
+//     meanwhile (the _sync variant relaunches a captured round and polls
 //     a completion counter).
 // Algorithmic reference: bicgstab, nsrno/dense_wave.py:118-148 (right
 // preconditioned, shared-angle inner products, true residual every 40
@@ -1375,15 +1375,10 @@ __global__ void k_loop_control(const __grid_constant__ SolveArgs A, cudaGraphCon
   *rounds = r;
   if (loop_ends(A, r, max_rounds)) cudaGraphSetConditional(loop, 0);
 }
-// Last launch of the first round, which runs outside the loop.
-__global__ void k_round_count(const __grid_constant__ SolveArgs A) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *reinterpret_cast<unsigned long long*>(A.B.queue + 6) += 1;
-}
 // First node of the loop's graph: whether the loop runs at all.
 __global__ void k_loop_begin(const __grid_constant__ SolveArgs A, cudaGraphConditionalHandle loop, long long max_rounds) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const unsigned long long r = *reinterpret_cast<unsigned long long*>(A.B.queue + 6);
-  cudaGraphSetConditional(loop, loop_ends(A, r, max_rounds) ? 0 : 1);
+  cudaGraphSetConditional(loop, loop_ends(A, 0, max_rounds) ? 0 : 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1787,13 +1782,13 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     const long long per_sys = (long long)params->max_iterations * 2 + 16;
     const long long waves = (n_systems + n_slots - 1) / n_slots + 1;
     const long long max_launch = waves * ((per_sys + K - 1) / K) + 4;
-    // The K iterations of one round on the slot groups' streams, launched or captured.
-    auto issue_round = [&]() -> cudaError_t {
+    // Iterations on the slot groups' streams, launched or captured.
+    auto issue = [&](int iterations) -> cudaError_t {
       cudaError_t e = cudaSuccess;
       if (n_groups > 1 && (e = cudaEventRecord(ev_fork, st)) != cudaSuccess) return e;
       for (int g = 1; g < n_groups; ++g)
         if ((e = cudaStreamWaitEvent(sg[g], ev_fork, 0)) != cudaSuccess) return e;
-      for (int it = 0; it < K; ++it)
+      for (int it = 0; it < iterations; ++it)
         for (int q = 0; q < NSR_LAUNCHES_PER_IT; ++q)
           for (int g = 0; g < n_groups; ++g) launch(q, g, g ? sg[g] : st);
       for (int g = 1; g < n_groups; ++g) {
@@ -1804,15 +1799,22 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     };
 
     if (!blocking) {
-      // The first round is launched kernel by kernel, so that the device works
-      // while the host builds the graph of the others (0.5 to 1 ms of a 256 x 256
-      // solve's 5).  They are a device-side loop: a conditional WHILE node whose
-      // body is one round followed by k_loop_control, behind k_loop_begin, which
-      // skips it when the first round was enough.  The host returns without
-      // waiting for either.
-      NSR_TRY(issue_round());
-      k_round_count<<<1, 32, 0, st>>>(A);
-      NSR_TRY(cudaGetLastError());
+      // The first iterations are launched kernel by kernel, so that the device
+      // works while the host builds the graph of the others (0.5 to 1 ms of a 256 x
+      // 256 solve's 5): as many as keep it busy until then and no more, because
+      // each costs the host 20 us a slot group, which a call whose systems all start
+      // converged only waits for (22 such systems of 768 x 1024: 2.4 ms a call with
+      // a whole round ahead, 1.7 ms with two iterations, the first of which only
+      // starts the systems).  The others are a device-side loop: a conditional WHILE node whose body is one round of K
+      // iterations followed by k_loop_control, behind k_loop_begin, which skips it
+      // when the first iterations were enough.  The host returns without waiting
+      // for either.
+      const double resident = n_systems < n_slots ? n_systems : n_slots;
+      const double it_us = 70.0 + resident * (double)grid->nz * grid->nx * 272.0 / 4.2e6;   // latency, bytes
+      const double spare_us = it_us - 20.0 * T.groups;   // of one iteration, next to its launches
+      int ahead = K;
+      if (spare_us > 0.0 && 900.0 / spare_us + 2.0 < K) ahead = (int)(900.0 / spare_us) + 2;
+      NSR_TRY(issue(ahead));
       cudaGraphConditionalHandle handle;
       NSR_TRY(cudaGraphCreate(&loop_graph, 0));
       NSR_TRY(cudaGraphConditionalHandleCreate(&handle, loop_graph, 0, cudaGraphCondAssignDefault));
@@ -1836,7 +1838,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
       NSR_TRY(cudaGraphAddNode(&while_node, loop_graph, &begin_node, 1, &cp));
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       NSR_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-      ce = issue_round();
+      ce = issue(K);
       if (ce == cudaSuccess) {
         k_loop_control<<<1, 32, 0, st>>>(A, handle, max_launch);
         ce = cudaGetLastError();
@@ -1858,7 +1860,7 @@ static int solve_impl(const NsrGrid* grid, const void* coef, const double* freq_
     }
 
     NSR_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    ce = issue_round();
+    ce = issue(K);
     {
       const cudaError_t ce2 = cudaStreamEndCapture(st, &graph);
       if (ce == cudaSuccess) ce = ce2;

@@ -264,7 +264,8 @@ def solve_batched(medium: Medium, freqs, angles=None, *, rhs=None, x0=None, tole
 def solve_progress(result: BatchResult):
     """(systems finished, device loop rounds, error flag, kernels launched) of a
     non-blocking solve, from the progress record copied behind it (call after
-    the stream has passed the solve, e.g. after torch.cuda.synchronize()).
+    the stream has passed the solve, e.g. after torch.cuda.synchronize()).  The
+    iterations that the host launches ahead of the loop are in neither count.
     For a blocking solve the host already counted everything: (systems,
     graph launches, 0, kernels launched)."""
     if result.extra.get("blocking"):
