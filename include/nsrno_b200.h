@@ -68,15 +68,19 @@ typedef struct NsrGrid {
 } NsrGrid;
 
 /* Launch shapes of nsr_solve_batched (all zero: the built-in defaults).
- * Chosen per grid and device by the autotuner of nsrno_b200.tune; every
- * choice gives bitwise the same results for a fixed slot count. */
+ * Chosen per grid and device by the autotuner of nsrno_b200.tune.  Shapes of
+ * the transforms, slot groups and the slot count leave a system's results as
+ * they are, bit for bit; stencil_width, stencil_rows and stencil_cols regroup
+ * the partial sums of its inner products. */
 typedef struct NsrTiles {
   int32_t stencil_width;     /* columns per stencil work item: 256 or 512      */
   int32_t stencil_depth;     /* row buffers of the second half's stencil ring:
                                 4 (default), 5, 6 (width 512: 4; one column per
                                 thread: 4); the first half's smaller rows fill
                                 the same bytes (5, 6 or 8 of them)             */
-  int32_t stencil_rows;      /* rows per stencil work item (band): 4..64       */
+  int32_t stencil_rows;      /* rows per stencil work item (band): 4..64 (0: from
+                                the grid and the slots, summed by units of rows
+                                that the grid alone decides)                   */
   int32_t stencil_ctas;      /* resident stencil CTAs per SM (0: occupancy)    */
   int32_t cols_width;        /* columns per column-FFT CTA: 8 or 16            */
   int32_t row_tile;          /* rows per row-FFT CTA: 1..8                     */
@@ -244,9 +248,10 @@ int nsr_plane_wave_rhs(const NsrGrid* grid, const double* freq_hz, const double*
  * stats NULL or a host NsrSolveStats.
  *
  * nsr_solve_batched does not block: it enqueues the whole solve on the
- * caller's stream and returns.  The iteration loop runs on the device, as a
- * CUDA graph whose conditional WHILE node repeats graph_iterations
- * iterations until every system has finished (or a round budget derived
+ * caller's stream and returns.  The first iterations (at most
+ * graph_iterations) are launched as they are, then the loop runs on the
+ * device, as a CUDA graph whose conditional WHILE node repeats
+ * graph_iterations iterations until every system has finished (or a round budget derived
  * from max_iterations is spent; systems never finished keep NSR_NOT_RUN).
  * Inputs, outputs and the workspace must stay valid until the stream passes
  * the solve.  stats (if given) gets only what is known at enqueue time;
@@ -277,8 +282,8 @@ int nsr_solve_batched_sync(const NsrGrid* grid, const void* material,
                            void* fields, NsrSolveStats* stats, void* stream);
 
 /* Progress of the last solve in `workspace` (n_slots as given to it): systems
- * finished, device loop rounds run, and 1 if a kernel gave up on its copy
- * ring.  Synchronises `stream` (reads a few words). */
+ * finished, device loop rounds run (without the iterations launched ahead of
+ * the loop), and 1 if a kernel gave up on its copy ring.  Synchronises `stream` (reads a few words). */
 int nsr_solve_progress(const NsrGrid* grid, int32_t n_slots, const void* workspace, int32_t* done,
                        int64_t* rounds, int32_t* error, void* stream);
 /* Byte offset in the workspace of the progress record read by

@@ -1205,20 +1205,18 @@ __device__ __forceinline__ void cols_multiply(float2* s, const FftPlan& P, float
   else fft_cols_direct<TC>(s, P, g, nx, ncol, mul);
 }
 
-// Column pass with the fused middle stage for the specialised sizes; other
-// sizes run the separate transforms and multiply.  Returns false for those
-// other sizes, which the caller then handles itself.
+// Column pass of a tile that lies in shared memory, with the fused middle stage;
+// launched for the specialised sizes only.
 template <int TC, typename MUL>
-__device__ __forceinline__ bool fft_cols_fused(float2* s, const FftPlan& P, MUL mul) {
+__device__ __forceinline__ void fft_cols_fused(float2* s, const FftPlan& P, MUL mul) {
   switch (P.n) {
-    case 256: ct_cols_fused<256, TC>(s, P.tws, mul); return true;
-    case 384: ct_cols_fused<384, TC>(s, P.tws, mul); return true;
-    case 512: ct_cols_fused<512, TC>(s, P.tws, mul); return true;
-    case 768: ct_cols_fused<768, TC>(s, P.tws, mul); return true;
-    case 1024: ct_cols_fused<1024, TC>(s, P.tws, mul); return true;
-    case 1536: ct_cols_fused<1536, TC>(s, P.tws, mul); return true;
-    case 2048: ct_cols_fused<2048, TC>(s, P.tws, mul); return true;
-    default: return false;
+    case 256: ct_cols_fused<256, TC>(s, P.tws, mul); break;
+    case 384: ct_cols_fused<384, TC>(s, P.tws, mul); break;
+    case 512: ct_cols_fused<512, TC>(s, P.tws, mul); break;
+    case 768: ct_cols_fused<768, TC>(s, P.tws, mul); break;
+    case 1024: ct_cols_fused<1024, TC>(s, P.tws, mul); break;
+    case 1536: ct_cols_fused<1536, TC>(s, P.tws, mul); break;
+    case 2048: ct_cols_fused<2048, TC>(s, P.tws, mul); break;
   }
 }
 

@@ -777,7 +777,7 @@ extern "C" int nsr_dense_grad(const NsrDenseGrid* grid, const double* coef, doub
 // prime factors are at most 61, e.g. the 1056 x 1216 padding of the reference).
 // ---------------------------------------------------------------------------
 // Eleven 1056 x 1216 fields (radices 11 3 2 16 and 19 4 16): 1,365 us with the
-// prime radices as loops over local arrays and unpadded rows, 490 us with
+// prime radices as loops over local arrays and unpadded rows, 420 us with
 // register butterflies and the ends of the transforms fused.
 template <bool GEN>
 __global__ void __launch_bounds__(256, GEN ? 2 : 4) k_dense_rows_fwd(int nz, int nx, PrecTables t,

@@ -16,8 +16,9 @@
 //         ||w - V h'||^2 = ||w||^2 - sum |h'_i|^2 (V is orthonormal and h' is
 //         of rounding size), applies the previous Givens rotations to column j
 //         and forms the new one, all in FP64 on the device.
-// So the basis is read three times a step (four, with w twice more, when every
-// dot and axpy was its own launch).  Eleven 768 x 1024 systems, 8 steps: 9.1 ms
+// So a step sweeps the basis four times: in fwd, in inv and twice in gs, whose
+// second sweep finds the tile in cache while a CTA's tiles of the vectors fit
+// (8 steps do, the longest restart does not).  Eleven 768 x 1024 systems, 8 steps: 9.1 ms
 // with eight launches a step and one-thread-per-node dots, 4.9 ms in this form.
 // At the end of a cycle: back substitution for y (FP64), u = V y fused with
 // the forward row FFT, the column and inverse row passes, and an FP64 pass

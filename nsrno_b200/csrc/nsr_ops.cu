@@ -286,9 +286,12 @@ size_t nsr_prec_table_bytes(const NsrGrid* g) {
          nsr_align(sizeof(float2) * nsr_twiddle_offset(g->nz, 0));
 }
 
-// 16 columns (128-byte row segments) up to 1024 points; 8 for longer columns,
-// whose tile would not leave room for two CTAs, and for batches of fewer 16-column
-// tiles than SMs.
+// 16 columns (128-byte row segments) up to 1024 points; 8 for longer columns, and
+// for batches of fewer 16-column tiles than SMs.  Two 16-column tiles fit an SM's
+// shared memory up to 908 points; between there and 1024, which the solver has
+// taken 16 wide from its first version, 8 are faster (22 learned systems of
+// 1024 x 1536: 0.233 ms a launch against 0.309) and the autotuner's cols_width
+// finds them.
 int nsr_cols_tc(const NsrGrid* g, int ns) {
   return g->nz <= 1024 && (long long)ns * ((g->nx + 15) / 16) >= 148 ? 16 : 8;
 }
@@ -371,7 +374,8 @@ extern "C" int nsr_precondition(const NsrGrid* grid, const double* freq_hz, int3
 
 // Row tiles near 32 KB of shared memory (40 KB where the transform's first radix
 // may be a large prime: four rows of 1216 give all 256 threads a butterfly, 107 ->
-// 96 us for eleven 1056 x 1216 fields), at most 8 rows; half or a quarter of that
+// 96 us for eleven 1056 x 1216 fields, the one width it was measured at), at most
+// 8 rows; half or a quarter of that
 // for batches of fewer than four such tiles for three SMs (solves of three 256 x
 // 256 and six 256 x 384 systems take 4% less with the tile rules).
 int nsr_rows_per_cta(const NsrGrid* g, int ns) {
