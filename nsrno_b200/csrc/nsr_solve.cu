@@ -807,7 +807,10 @@ struct StnLayout {
 // slot i % ns: the slots run fastest, so the CTAs in flight at any time work
 // on the same few bands of every slot, and the medium's coefficient rows
 // (read by every slot) come from L2 after the first slot's copy.
-#define NSR_STN_UNITS 4   // most units of a band
+// Most units of a band.  Four would take another 512 bytes of shared memory: four
+// CTAs at ring depth 5 then pass 196 KB and the SM's next partition of it, and an
+// iteration of 22 learned 768 x 1024 systems took 1.147 ms where it takes 1.045.
+#define NSR_STN_UNITS 2
 struct StnItems {
   int tz, nbands, nstrips, per_slot, n_items;
   int unit, n_units;   // rows of one partial sum (tz is at most NSR_STN_UNITS of them), partials per slot
@@ -1044,114 +1047,113 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     AT bNext = bt(bpl, z0), tNext = bt(tpl, z0);
     // Interior test (no PML stretch) per column, once per item; per row below.
     const bool cols_in = j > lo && j + CPT - 1 < hi_x;
-    int unit = 0, unit_end = min(it.unit, nrows);
-    for (int k = 0; k < nrows; ++k) {
-      const int i = z0 + k;
-      const bool inside = i > lo && i < hi_z && cols_in;
-      const AT bRow = bNext, tRow = tNext;
-      if (k + 1 < nrows) { bNext = bt(bpl, i + 1); tNext = bt(tpl, i + 1); }
-      const uint32_t sS = q0 + k + 2;
-      const int eS = (eC + 1 == D) ? 0 : eC + 1;
-      if (ok) ok = mbar_wait(&full[eS], (sS / D) & 1, &abort_word, NSR_STN_WAIT_NS);
-      if (!ok) abort_flag = 1;
-      ZT zS = ZT{};
-      AT aS;
-      if constexpr (CPT == 2) aS = make_float2(1.f, 1.f); else aS = 1.0f;
-      if (ok && i + 1 < nz) { zS = zload(eS); aS = aload(eS); }
-      if (ok && own) {
-        const unsigned char* bC = ring + (size_t)eC * Ly::SLOT;
-        const float2 zero = make_float2(0.f, 0.f);
-        if constexpr (CPT == 2) {
-          const float4 zc = zC, zn = zN, zs = zS;
-          const float2 zw = has_w ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez - 8) : zero;
-          const float2 ze = has_e ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez + 16) : zero;
-          const float2 ac = aC, an = aN, as = aS;
-          const float aw = has_w ? *reinterpret_cast<const float*>(bC + Ly::OA + ea - 4) : 1.0f;
-          const float ae = has_e ? *reinterpret_cast<const float*>(bC + Ly::OA + ea + 8) : 1.0f;
-          const float2 bb = bRow, tt = tRow;
-          const float4 rk = *reinterpret_cast<const float4*>(bC + Ly::ORH + 16 * tid);
-          const float2 c0v = lo2(zc), c1v = hi2(zc);
-          float2 av0, av1;
-          if (inside) {
-            av0 = stencil_plain<ADJ>(kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs), lo2(zn));
-            av1 = stencil_plain<ADJ>(kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v, hi2(zs), hi2(zn));
+    int unit = 0;
+    for (int k = 0; k < nrows; ++unit) {
+      const int unit_end = min(k + it.unit, nrows);
+      for (; k < unit_end; ++k) {
+        const int i = z0 + k;
+        const bool inside = i > lo && i < hi_z && cols_in;
+        const AT bRow = bNext, tRow = tNext;
+        if (k + 1 < nrows) { bNext = bt(bpl, i + 1); tNext = bt(tpl, i + 1); }
+        const uint32_t sS = q0 + k + 2;
+        const int eS = (eC + 1 == D) ? 0 : eC + 1;
+        if (ok) ok = mbar_wait(&full[eS], (sS / D) & 1, &abort_word, NSR_STN_WAIT_NS);
+        if (!ok) abort_flag = 1;
+        ZT zS = ZT{};
+        AT aS;
+        if constexpr (CPT == 2) aS = make_float2(1.f, 1.f); else aS = 1.0f;
+        if (ok && i + 1 < nz) { zS = zload(eS); aS = aload(eS); }
+        if (ok && own) {
+          const unsigned char* bC = ring + (size_t)eC * Ly::SLOT;
+          const float2 zero = make_float2(0.f, 0.f);
+          if constexpr (CPT == 2) {
+            const float4 zc = zC, zn = zN, zs = zS;
+            const float2 zw = has_w ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez - 8) : zero;
+            const float2 ze = has_e ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez + 16) : zero;
+            const float2 ac = aC, an = aN, as = aS;
+            const float aw = has_w ? *reinterpret_cast<const float*>(bC + Ly::OA + ea - 4) : 1.0f;
+            const float ae = has_e ? *reinterpret_cast<const float*>(bC + Ly::OA + ea + 8) : 1.0f;
+            const float2 bb = bRow, tt = tRow;
+            const float4 rk = *reinterpret_cast<const float4*>(bC + Ly::ORH + 16 * tid);
+            const float2 c0v = lo2(zc), c1v = hi2(zc);
+            float2 av0, av1;
+            if (inside) {
+              av0 = stencil_plain<ADJ>(kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs), lo2(zn));
+              av1 = stencil_plain<ADJ>(kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v, hi2(zs), hi2(zn));
+            } else {
+              const int c = CPT * tid;
+              av0 = stencil_pml<ADJ>(pml, k, c, kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs),
+                                     lo2(zn));
+              av1 = stencil_pml<ADJ>(pml, k, c + 1, kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v,
+                                     hi2(zs), hi2(zn));
+            }
+            *reinterpret_cast<float4*>(out + (long long)i * nx + j) = pack2(av0, av1);
+            if (half == 0) {
+              dot_acc_f(accf[0], accf[1], lo2(rk), av0);       // <rhat, v>
+              dot_acc_f(accf[0], accf[1], hi2(rk), av1);
+            } else {
+              const float4 rr = *reinterpret_cast<const float4*>(bC + Ly::OR + 16 * tid);
+              const float2 s0 = lo2(rr), s1 = hi2(rr);
+              dot_acc_f(accf[0], accf[1], av0, s0);            // <t, s>
+              dot_acc_f(accf[0], accf[1], av1, s1);
+              accf[2] = fmaf(av0.x, av0.x, fmaf(av0.y, av0.y, fmaf(av1.x, av1.x, fmaf(av1.y, av1.y, accf[2]))));
+              accf[3] = fmaf(s0.x, s0.x, fmaf(s0.y, s0.y, fmaf(s1.x, s1.x, fmaf(s1.y, s1.y, accf[3]))));
+              dot_acc_f(accf[4], accf[5], lo2(rk), av0);       // <rhat, t>
+              dot_acc_f(accf[4], accf[5], hi2(rk), av1);
+              dot_acc_f(accf[6], accf[7], lo2(rk), s0);        // <rhat, s>
+              dot_acc_f(accf[6], accf[7], hi2(rk), s1);
+            }
           } else {
-            const int c = CPT * tid;
-            av0 = stencil_pml<ADJ>(pml, k, c, kh2, fpow, ac.x, ac.y, aw, as.x, an.x, bb.x, tt.x, c0v, c1v, zw, lo2(zs),
-                                   lo2(zn));
-            av1 = stencil_pml<ADJ>(pml, k, c + 1, kh2, fpow, ac.y, ae, ac.x, as.y, an.y, bb.y, tt.y, c1v, ze, c0v,
-                                   hi2(zs), hi2(zn));
-          }
-          *reinterpret_cast<float4*>(out + (long long)i * nx + j) = pack2(av0, av1);
-          if (half == 0) {
-            dot_acc_f(accf[0], accf[1], lo2(rk), av0);       // <rhat, v>
-            dot_acc_f(accf[0], accf[1], hi2(rk), av1);
-          } else {
-            const float4 rr = *reinterpret_cast<const float4*>(bC + Ly::OR + 16 * tid);
-            const float2 s0 = lo2(rr), s1 = hi2(rr);
-            dot_acc_f(accf[0], accf[1], av0, s0);            // <t, s>
-            dot_acc_f(accf[0], accf[1], av1, s1);
-            accf[2] = fmaf(av0.x, av0.x, fmaf(av0.y, av0.y, fmaf(av1.x, av1.x, fmaf(av1.y, av1.y, accf[2]))));
-            accf[3] = fmaf(s0.x, s0.x, fmaf(s0.y, s0.y, fmaf(s1.x, s1.x, fmaf(s1.y, s1.y, accf[3]))));
-            dot_acc_f(accf[4], accf[5], lo2(rk), av0);       // <rhat, t>
-            dot_acc_f(accf[4], accf[5], hi2(rk), av1);
-            dot_acc_f(accf[6], accf[7], lo2(rk), s0);        // <rhat, s>
-            dot_acc_f(accf[6], accf[7], hi2(rk), s1);
-          }
-        } else {
-          const float2 zc = zC, zn = zN, zs = zS;
-          const float2 zw = has_w ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez - 8) : zero;
-          const float2 ze = has_e ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez + 8) : zero;
-          const float ac = aC, an = aN, as = aS;
-          const float aw = has_w ? *reinterpret_cast<const float*>(bC + Ly::OA + ea - 4) : 1.0f;
-          const float ae = has_e ? *reinterpret_cast<const float*>(bC + Ly::OA + ea + 4) : 1.0f;
-          const float bb = bRow, tt = tRow;
-          const float2 rk = *reinterpret_cast<const float2*>(bC + Ly::ORH + 8 * tid);
-          const float2 av = inside ? stencil_plain<ADJ>(kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw, zs, zn)
-                                   : stencil_pml<ADJ>(pml, k, tid, kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw,
-                                                      zs, zn);
-          out[(long long)i * nx + j] = av;
-          if (half == 0) {
-            dot_acc_f(accf[0], accf[1], rk, av);       // <rhat, v>
-          } else {
-            const float2 rr = *reinterpret_cast<const float2*>(bC + Ly::OR + 8 * tid);
-            const float2 s0 = rr;
-            dot_acc_f(accf[0], accf[1], av, s0);       // <t, s>
-            accf[2] = fmaf(av.x, av.x, fmaf(av.y, av.y, accf[2]));
-            accf[3] = fmaf(s0.x, s0.x, fmaf(s0.y, s0.y, accf[3]));
-            dot_acc_f(accf[4], accf[5], rk, av);       // <rhat, t>
-            dot_acc_f(accf[6], accf[7], rk, s0);       // <rhat, s>
+            const float2 zc = zC, zn = zN, zs = zS;
+            const float2 zw = has_w ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez - 8) : zero;
+            const float2 ze = has_e ? *reinterpret_cast<const float2*>(bC + Ly::OZ + ez + 8) : zero;
+            const float ac = aC, an = aN, as = aS;
+            const float aw = has_w ? *reinterpret_cast<const float*>(bC + Ly::OA + ea - 4) : 1.0f;
+            const float ae = has_e ? *reinterpret_cast<const float*>(bC + Ly::OA + ea + 4) : 1.0f;
+            const float bb = bRow, tt = tRow;
+            const float2 rk = *reinterpret_cast<const float2*>(bC + Ly::ORH + 8 * tid);
+            const float2 av = inside ? stencil_plain<ADJ>(kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw, zs, zn)
+                                     : stencil_pml<ADJ>(pml, k, tid, kh2, fpow, ac, ae, aw, as, an, bb, tt, zc, ze, zw,
+                                                        zs, zn);
+            out[(long long)i * nx + j] = av;
+            if (half == 0) {
+              dot_acc_f(accf[0], accf[1], rk, av);       // <rhat, v>
+            } else {
+              const float2 rr = *reinterpret_cast<const float2*>(bC + Ly::OR + 8 * tid);
+              const float2 s0 = rr;
+              dot_acc_f(accf[0], accf[1], av, s0);       // <t, s>
+              accf[2] = fmaf(av.x, av.x, fmaf(av.y, av.y, accf[2]));
+              accf[3] = fmaf(s0.x, s0.x, fmaf(s0.y, s0.y, accf[3]));
+              dot_acc_f(accf[4], accf[5], rk, av);       // <rhat, t>
+              dot_acc_f(accf[6], accf[7], rk, s0);       // <rhat, s>
+            }
           }
         }
-      }
-      zN = zC; zC = zS; aN = aC; aC = aS;
-      if ((k + 1) % FLUSH == 0 || k + 1 == unit_end) {
+        zN = zC; zC = zS; aN = aC; aC = aS;
+        if ((k + 1) % FLUSH == 0 || k + 1 == unit_end) {
 #pragma unroll
-        for (int qq = 0; qq < NSR_NPART; ++qq) {
-          if (qq < NP) accs[qq][tid] += (double)accf[qq];
-          accf[qq] = 0.0f;
+          for (int qq = 0; qq < NSR_NPART; ++qq) {
+            if (qq < NP) accs[qq][tid] += (double)accf[qq];
+            accf[qq] = 0.0f;
+          }
         }
+        // The buffer of row i - 1 goes back to the producer one row after its
+        // last use as centre.  Its values were loaded into registers during row
+        // i - 1, but a release right after those loads can overtake them: the
+        // arrival does not wait for shared-memory loads still in flight, and
+        // the producer's next bulk copy into the buffer then races them (seen
+        // as nondeterministic inner products with two slot groups).
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[eN]);
+        eN = eC;
+        eC = eS;
       }
-      if (k + 1 == unit_end) {
 #pragma unroll
-        for (int qq = 0; qq < NP; ++qq) {
-          const double s = warp_sum(accs[qq][tid]);
-          if (lane == 0) wsum[unit][wid][qq] = s;
-          accs[qq][tid] = 0.0;
-        }
-        ++unit;
-        unit_end = min(unit_end + it.unit, nrows);
+      for (int qq = 0; qq < NP; ++qq) {
+        const double s = warp_sum(accs[qq][tid]);
+        if (lane == 0) wsum[unit][wid][qq] = s;
+        accs[qq][tid] = 0.0;
       }
-      // The buffer of row i - 1 goes back to the producer one row after its
-      // last use as centre.  Its values were loaded into registers during row
-      // i - 1, but a release right after those loads can overtake them: the
-      // arrival does not wait for shared-memory loads still in flight, and
-      // the producer's next bulk copy into the buffer then races them (seen
-      // as nondeterministic inner products with two slot groups).
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[eN]);
-      eN = eC;
-      eC = eS;
     }
     // rows z1 - 1 and z1
     __syncwarp();
@@ -1166,7 +1168,7 @@ __global__ void __launch_bounds__(W / CPT + 32, (stn_min_blocks<W, D, CPT, H>())
     double* part = slot_partials(A, slot);
     if (tid < 32) {
       const int u = tid / NSR_NPART, k = tid % NSR_NPART;
-      static_assert(NSR_STN_UNITS * NSR_NPART == 32, "one lane per sum");
+      static_assert(NSR_STN_UNITS * NSR_NPART <= 32, "one lane per sum");
       if (u < unit) {
         double s = 0.0;
         if (k < NP)
@@ -1463,7 +1465,7 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     // Band height of the stencil.  Its inner products are summed by units of rows
     // whose height follows from the grid alone (the tallest power of two that
     // gives one system 64 units), so that the slots and groups of a call never
-    // regroup them; a band is one, two or four units, the tallest whose items give
+    // regroup them; a band is one or two units, the tallest whose items give
     // every SM about three CTAs.  Tall bands re-read the fewest halo rows, but a
     // band is walked row by row, about 0.8 us each.  Microseconds per iteration of
     // 1 / 11 / 22 systems with bands of 4, 8, 16, 32 and 64 rows: 256 x 256
