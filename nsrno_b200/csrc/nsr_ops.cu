@@ -102,20 +102,18 @@ template <> struct PlaneOf<double> {
 // and by launch latency for one small field.  Six complex128 243 x 729 fields,
 // adjoint: 42 us with one thread per node and four complex divisions each,
 // 19 us in this form.
-#define NSR_APPLY_TX 128
-template <typename T, bool ADJ, int TZ>
-__global__ void __launch_bounds__(NSR_APPLY_TX) k_apply(Geo g, const void* __restrict__ mat,
-                                                        const double* __restrict__ freq,
-                                                        const typename CxT<T>::type* __restrict__ x,
-                                                        typename CxT<T>::type* __restrict__ y) {
+template <typename T, bool ADJ, int TZ, int TX>
+__global__ void __launch_bounds__(TX) k_apply(Geo g, const void* __restrict__ mat, const double* __restrict__ freq,
+                                              const typename CxT<T>::type* __restrict__ x,
+                                              typename CxT<T>::type* __restrict__ y) {
   typedef typename CxT<T>::type C;
   __shared__ SysScalars sc;
   __shared__ RowFactors<T> rowf[TZ];
   const long long n = (long long)g.nz * g.nx;
   const int nx = g.nx, nz = g.nz;
-  const int nbx = (nx + NSR_APPLY_TX - 1) / NSR_APPLY_TX;
+  const int nbx = (nx + TX - 1) / TX;
   const int z0 = (blockIdx.x / nbx) * TZ;
-  const int j = (blockIdx.x % nbx) * NSR_APPLY_TX + threadIdx.x;
+  const int j = (blockIdx.x % nbx) * TX + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool own = j < nx;
   const C* __restrict__ xs = x + blockIdx.y * n;
@@ -162,17 +160,52 @@ __global__ void __launch_bounds__(NSR_APPLY_TX) k_apply(Geo g, const void* __res
   }
 }
 
+// One thread per node, for grids so narrow that a warp of columns would be half
+// empty or more.
+template <typename T, bool ADJ>
+__global__ void __launch_bounds__(256) k_apply_nodes(Geo g, const void* __restrict__ mat,
+                                                     const double* __restrict__ freq,
+                                                     const typename CxT<T>::type* __restrict__ x,
+                                                     typename CxT<T>::type* __restrict__ y) {
+  typedef typename CxT<T>::type C;
+  const long long n = (long long)g.nz * g.nx, k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const SysScalars s = sys_scalars(g, freq[blockIdx.y]);
+  const MatPlanes mp = nsr_planes(mat, n);
+  const T* __restrict__ ca = PlaneOf<T>::a(mp);
+  const C* __restrict__ xs = x + blockIdx.y * n;
+  auto inside = [&](int i, int j) { return i >= 0 && i < g.nz && j >= 0 && j < g.nx; };
+  auto P = [&](int i, int j) -> C { return inside(i, j) ? xs[(long long)i * g.nx + j] : cx<C>(T(0), T(0)); };
+  auto A = [&](int i, int j) -> T { return inside(i, j) ? ca[(long long)i * g.nx + j] : T(1); };
+  const int i = (int)(k / g.nx), j = (int)(k - (long long)i * g.nx);
+  y[blockIdx.y * n + k] = stencil<T, ADJ>(g, s, i, j, PlaneOf<T>::b(mp)[k], PlaneOf<T>::t(mp)[k], P, A);
+}
+
+template <typename T, bool ADJ, int TX>
+static void launch_apply_tx(const Geo& g, const void* coef, const double* freq, int ns, const void* x, void* y,
+                            cudaStream_t st) {
+  typedef typename CxT<T>::type C;
+  // 8-row tiles read 10 rows for 8; small grids take 2-row tiles so that every
+  // SM gets a few blocks.
+  const int bx = (g.nx + TX - 1) / TX;
+  if ((long long)bx * ((g.nz + 7) / 8) * ns * TX >= 8 * 148 * 128)
+    k_apply<T, ADJ, 8, TX><<<dim3(bx * ((g.nz + 7) / 8), ns), TX, 0, st>>>(g, coef, freq, (const C*)x, (C*)y);
+  else
+    k_apply<T, ADJ, 2, TX><<<dim3(bx * ((g.nz + 1) / 2), ns), TX, 0, st>>>(g, coef, freq, (const C*)x, (C*)y);
+}
+// Columns of a block: 128, one warp's where 128 would be largely empty, a thread
+// per node where a warp would.  Us a call, 22 complex64 fields of 2048 x 8: 45 with
+// 128 columns, 19 with 32, 15 by nodes; of 2048 x 16: 45 and 23 by nodes; six of
+// 2048 x 60: 17.6 with 128, 18.7 with 32.
 template <typename T, bool ADJ>
 static void launch_apply(const Geo& g, const void* coef, const double* freq, int ns, const void* x, void* y,
                          cudaStream_t st) {
   typedef typename CxT<T>::type C;
-  // 8-row tiles read 10 rows for 8; small grids take 2-row tiles so that every
-  // SM gets a few blocks.
-  const int bx = (g.nx + NSR_APPLY_TX - 1) / NSR_APPLY_TX;
-  if ((long long)bx * ((g.nz + 7) / 8) * ns >= 8 * 148)
-    k_apply<T, ADJ, 8><<<dim3(bx * ((g.nz + 7) / 8), ns), NSR_APPLY_TX, 0, st>>>(g, coef, freq, (const C*)x, (C*)y);
-  else
-    k_apply<T, ADJ, 2><<<dim3(bx * ((g.nz + 1) / 2), ns), NSR_APPLY_TX, 0, st>>>(g, coef, freq, (const C*)x, (C*)y);
+  if (g.nx <= 16)
+    k_apply_nodes<T, ADJ><<<dim3((unsigned)(((long long)g.nz * g.nx + 255) / 256), ns), 256, 0, st>>>(g, coef, freq,
+                                                                                                      (const C*)x, (C*)y);
+  else if (g.nx <= 48) launch_apply_tx<T, ADJ, 32>(g, coef, freq, ns, x, y, st);
+  else launch_apply_tx<T, ADJ, 128>(g, coef, freq, ns, x, y, st);
 }
 
 extern "C" int nsr_apply(const NsrGrid* grid, const void* coef, const double* freq_hz,
@@ -439,8 +472,10 @@ extern "C" int nsr_plane_wave_rhs(const NsrGrid* grid, const double* freq_hz, co
 // FP64 issue and conversions (about 40 FP64 operations and 8 conversions per
 // node and system).  22 systems of 1024 x 1536: 1,152 us with one thread per
 // node, a pow and six PML profiles per node and system; 270 us with the x edges formed at both ends, 251 us in this form.
-#define NSR_GRAD_TX 128      // threads of a block, one column each
-#define NSR_GRAD_OWN 124     // columns a block yields: a warp's first lane only forms the east edge its neighbour needs
+// TX threads of a block take one column each.  Columns a block yields: a warp's
+// first lane only forms the east edge its neighbour needs, and the last lane of a
+// one-warp block has no east neighbour in the tile.
+__host__ __device__ constexpr int grad_own(int TX) { return TX == 32 ? 30 : 31 * (TX / 32); }
 #define NSR_GRAD_CHUNK 64    // systems whose scalars are staged in shared memory at a time
 
 __device__ __forceinline__ void cp_async_zfill(float2* dst, const float2* src, bool live) {
@@ -455,14 +490,14 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int PENDING>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-// Columns c0 .. c0 + NSR_GRAD_OWN + 1 of the rows z0 - 1 .. z0 + TZ of a field (zero
-// outside the grid).
-template <typename CT, int TZ>
+// Columns c0 .. c0 + TX - 1 of the rows z0 - 1 .. z0 + TZ of a field (zero outside
+// the grid).
+template <typename CT, int TZ, int TX>
 struct GradTile {
-  CT u[TZ + 2][NSR_GRAD_TX], l[TZ + 2][NSR_GRAD_TX];
+  CT u[TZ + 2][TX], l[TZ + 2][TX];
 };
-template <typename CT, int TZ>
-__device__ __forceinline__ void grad_fetch(GradTile<CT, TZ>& t, const Geo& g, const CT* us, const CT* ls, int z0,
+template <typename CT, int TZ, int TX>
+__device__ __forceinline__ void grad_fetch(GradTile<CT, TZ, TX>& t, const Geo& g, const CT* us, const CT* ls, int z0,
                                            int c0) {
 #pragma unroll
   for (int r = 0; r < TZ + 2; ++r) {
@@ -477,24 +512,27 @@ __device__ __forceinline__ void grad_fetch(GradTile<CT, TZ>& t, const Geo& g, co
   cp_async_commit();
 }
 
-template <typename CT, int TZ>
-__global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, const void* __restrict__ mat,
+template <typename CT, int TZ, int TX>
+__global__ void __launch_bounds__(TX, TX == 32 ? 16 : 5) k_grad(Geo g, const void* __restrict__ mat,
                                                          const double* __restrict__ freq, int ns,
                                                          const CT* __restrict__ u, const CT* __restrict__ lam,
                                                          double* __restrict__ gc, double* __restrict__ gr) {
   __shared__ SysScalars scs[NSR_GRAD_CHUNK];
   extern __shared__ __align__(16) unsigned char grad_smem[];
-  GradTile<CT, TZ>* tiles = reinterpret_cast<GradTile<CT, TZ>*>(grad_smem);   // two: one in use, one in flight
+  GradTile<CT, TZ, TX>* tiles = reinterpret_cast<GradTile<CT, TZ, TX>*>(grad_smem);   // two: one in use, one in flight
   const long long n = (long long)g.nz * g.nx;
   const int nx = g.nx, nz = g.nz;
   // Tile column tx is grid column c0 + tx; warp w takes 32 of them from 31 w on, and
   // its lanes 1 .. 31 own theirs.
-  const int nbx = (nx + NSR_GRAD_OWN - 1) / NSR_GRAD_OWN;
-  const int c0 = (blockIdx.x % nbx) * NSR_GRAD_OWN - 1;
+  constexpr int OWN = grad_own(TX);
+  const int nbx = (nx + OWN - 1) / OWN;
+  const int c0 = (blockIdx.x % nbx) * OWN - 1;
   const int lane = threadIdx.x & 31, tx = 31 * (threadIdx.x >> 5) + lane;
   const int j = c0 + tx;
   const int z0 = (blockIdx.x / nbx) * TZ;
-  const bool own = lane > 0 && j < nx;
+  // The east neighbour; a one-warp block's last lane has none.
+  const int te = TX == 32 ? min(tx + 1, TX - 1) : tx + 1;
+  const bool own = lane > 0 && (TX > 32 || lane < 31) && j < nx;
   const int jc = min(max(j, 0), nx - 1);
   const MatPlanes mp = nsr_planes(mat, n);
   grad_fetch(tiles[0], g, u, lam, z0, c0);
@@ -518,7 +556,7 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
   for (int s0 = 0; s0 < ns; s0 += NSR_GRAD_CHUNK) {
     const int cnt = min(NSR_GRAD_CHUNK, ns - s0);
     __syncthreads();
-    for (int q = threadIdx.x; q < cnt; q += NSR_GRAD_TX) scs[q] = sys_scalars(g, freq[s0 + q]);
+    for (int q = threadIdx.x; q < cnt; q += TX) scs[q] = sys_scalars(g, freq[s0 + q]);
     for (int q = 0; q < cnt; ++q) {
       const int sys = s0 + q;
       __syncthreads();   // the tile about to be refilled has been read
@@ -529,7 +567,7 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
         cp_async_wait<0>();
       }
       __syncthreads();
-      const GradTile<CT, TZ>& t = tiles[sys & 1];
+      const GradTile<CT, TZ, TX>& t = tiles[sys & 1];
       const SysScalars s = scs[q];
       // 1 / (1 + i sig p) of the column's east half node
       double2 ie = make_double2(1.0, 0.0);
@@ -549,7 +587,7 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
       for (int r = 0; r < TZ; ++r) {
         const int i = z0 + r;
         const double2 un = D(t.u[r + 2][tx]), ln = D(t.l[r + 2][tx]);
-        const double2 due = D(t.u[r + 1][tx + 1]) - uc, dle = D(t.l[r + 1][tx + 1]) - lc;
+        const double2 due = D(t.u[r + 1][te]) - uc, dle = D(t.l[r + 1][te]) - lc;
         const double2 dus = un - uc, dls = ln - lc;
         const double2 lu = prod(lc, uc);
         const double e = t64[r] * s.fpow;
@@ -595,24 +633,32 @@ __global__ void __launch_bounds__(NSR_GRAD_TX, TZ <= 4 ? 5 : 4) k_grad(Geo g, co
   }
 }
 
+template <typename CT, int TX>
+static cudaError_t launch_grad_tx(const Geo& g, const void* coef, const double* freq, int ns, const void* u,
+                                  const void* lam, double* gc, double* gr, cudaStream_t st) {
+  // 4-row tiles read 6 rows for 4, from L2; a grid whose 4-row tiles would
+  // leave SMs without sixteen warps takes 2-row tiles.
+  const int bx = (g.nx + grad_own(TX) - 1) / grad_own(TX);
+  const CT *pu = (const CT*)u, *pl = (const CT*)lam;
+  cudaError_t ce;
+  if ((long long)bx * ((g.nz + 3) / 4) * TX >= 4 * 148 * 128) {
+    const int smem = 2 * (int)sizeof(GradTile<CT, 4, TX>);
+    ce = cudaFuncSetAttribute(k_grad<CT, 4, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (ce != cudaSuccess) return ce;
+    k_grad<CT, 4, TX><<<bx * ((g.nz + 3) / 4), TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
+  } else {
+    const int smem = 2 * (int)sizeof(GradTile<CT, 2, TX>);
+    k_grad<CT, 2, TX><<<bx * ((g.nz + 1) / 2), TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
+  }
+  return cudaGetLastError();
+}
+// One-warp blocks where a block of 128 columns would be half empty or more (22
+// fields of 2048 x 8: 58 us a call with 128 columns, 30 us with 32).
 template <typename CT>
 static cudaError_t launch_grad(const Geo& g, const void* coef, const double* freq, int ns, const void* u,
                                const void* lam, double* gc, double* gr, cudaStream_t st) {
-  // 4-row tiles read 6 rows for 4, from L2; a grid whose 4-row tiles would
-  // leave SMs without four blocks takes 2-row tiles.
-  const int bx = (g.nx + NSR_GRAD_OWN - 1) / NSR_GRAD_OWN;
-  const CT *pu = (const CT*)u, *pl = (const CT*)lam;
-  cudaError_t ce;
-  if ((long long)bx * ((g.nz + 3) / 4) >= 4 * 148) {
-    const int smem = 2 * (int)sizeof(GradTile<CT, 4>);
-    ce = cudaFuncSetAttribute(k_grad<CT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (ce != cudaSuccess) return ce;
-    k_grad<CT, 4><<<bx * ((g.nz + 3) / 4), NSR_GRAD_TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
-  } else {
-    const int smem = 2 * (int)sizeof(GradTile<CT, 2>);
-    k_grad<CT, 2><<<bx * ((g.nz + 1) / 2), NSR_GRAD_TX, smem, st>>>(g, coef, freq, ns, pu, pl, gc, gr);
-  }
-  return cudaGetLastError();
+  return g.nx <= 60 ? launch_grad_tx<CT, 32>(g, coef, freq, ns, u, lam, gc, gr, st)
+                    : launch_grad_tx<CT, 128>(g, coef, freq, ns, u, lam, gc, gr, st);
 }
 
 extern "C" int nsr_grad_accum(const NsrGrid* grid, const void* coef, const double* freq_hz,
