@@ -591,19 +591,27 @@ __global__ void __launch_bounds__(DS_THREADS, sizeof(T) == 4 ? 3 : 2)
   }
 }
 
-// Launch: the walk where its bands give every SM three blocks or more (and, for
-// complex64, even widths and 16-byte aligned buffers let it read pairs); else
-// the tiles, 16 rows high (23 rows of fluxes for 16) or, where those are
-// fewer than three per SM, 8.
+// Launch: the walk where it is the faster one and, for complex64, even widths and
+// 16-byte aligned buffers let it read pairs; else the tiles, 16 rows high (23 rows
+// of fluxes for 16) or, where those are fewer than three per SM, 8.
+// The walk's time goes by the columns of its strips, filled or not, the tiles' by
+// the nodes, more of it once the fields pass the L2.  us, walk against tiles
+// (forward, complex64, then complex128): 11 of 480 x 480 (2.5 M nodes, strips
+// filled to 0.97 and 1.0) 52 / 54, 105 / 98; 11 of 672 x 576 (4.3 M, 0.77 and 0.96)
+// 113 / 102, 187 / 182; 2 of 1056 x 1216 (2.6 M, 0.98 and 0.92) 52 / 70, 118 / 126;
+// 3 of 768 x 992 (2.3 M, 1.0 and 0.92) 61 / 54, 106 / 107; 11 of them (8.4 M)
+// 166 / 239, 305 / 352; 60 of 128 x 128 (1.0 M, 0.52 and 0.53) 44 / 23, 78 / 27.
 template <typename T, bool ADJ>
 static cudaError_t dense_apply_t(const DenseGeo& g, const double* coef, int nf, const void* x, void* y,
                                  cudaStream_t st) {
   typedef typename DC<T>::C C;
   constexpr int CPT = sizeof(T) == 4 ? 2 : 1, OUT = DS_THREADS * CPT - 8;
   constexpr int RESIDENT = 148 * (sizeof(T) == 4 ? 3 : 2);
-  const long long strips = (long long)((g.W + OUT - 1) / OUT) * nf;
+  const long long across = (g.W + OUT - 1) / OUT, strips = across * nf, nodes = (long long)nf * g.H * g.W;
+  const bool walk = (nodes >= 2500000 && 8LL * g.W >= 7 * across * OUT) ||
+                    (nodes >= 6000000 && 4LL * g.W >= 3 * across * OUT);
   const bool pairs = CPT == 1 || (g.W % 2 == 0 && (((uintptr_t)coef | (uintptr_t)x | (uintptr_t)y) & 15) == 0);
-  if (strips * ((g.H + 31) / 32) >= 3 * 148 && pairs) {
+  if (walk && pairs) {
     // Band height: a band walks 14 rows more than it yields, and the last wave of
     // blocks should be full, so take the height with the fewest row steps over
     // all waves (1056 rows of eleven fields: 44 rows, 262 us at 32).
