@@ -1463,8 +1463,8 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
   c->su = c->sr;
   if (c->sr == 0) {
     // Band height of the stencil.  Its inner products are summed by units of rows
-    // whose height follows from the grid alone (the tallest power of two that
-    // gives one system 64 units), so that the slots and groups of a call never
+    // whose height follows from the grid alone (32, or the tallest power of two
+    // that gives one system 64 units), so that the slots and groups of a call never
     // regroup them; a band is one or two units, the tallest whose items give
     // every SM about three CTAs.  Tall bands re-read the fewest halo rows, but a
     // band is walked row by row, about 0.8 us each.  Microseconds per iteration of
@@ -1474,7 +1474,7 @@ static int resolve_tiles(const NsrGrid* g, const NsrTiles* t, int n_slots, TileC
     // 127 / 579 / 1093, 140 / 561 / 1056, 175 / 581 / 1042 (units of 32).
     const int strips = (g->nx + c->sw - 1) / c->sw, ns = (n_slots + c->groups - 1) / c->groups;
     auto items = [&](int rows) { return (long long)((g->nz + rows - 1) / rows) * strips; };
-    c->su = 64;
+    c->su = 32;
     while (c->su > NSR_STN_MIN_ROWS && items(c->su) < 64) c->su /= 2;
     c->sr = c->su;
     while (c->sr < 64 && c->sr < NSR_STN_UNITS * c->su && ns * items(2 * c->sr) >= 3 * 148) c->sr *= 2;
